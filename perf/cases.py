@@ -473,7 +473,9 @@ def _diff_arms(case, seed):
 def _diff_inputs(case, seed):
     n = case["n"]
     # below 1: at exactly 1 the transfer function's border is one rounding away
-    vol = hy.synth_blobs_f32(seed, (n, n, n), 12) * np.float32(0.95)
+    vol = np.zeros((n, n, n), np.float32)
+    # and an empty rim: a ray's first sample falls on either side of its face
+    vol[2:-2, 2:-2, 2:-2] = hy.synth_blobs_f32(seed, (n - 4,) * 3, 12) * np.float32(0.95)
     tf = _knots(f"seeded{case['ntf']}", seed)
     rng = np.random.default_rng([seed, 5])
     # dL/dimage of a mean squared error: small, of both signs
