@@ -761,7 +761,7 @@ def main_ours(args):
         c = batch.config
         tuned = {"tile_w": c.tile_w, "grab": c.grab, "block_warps": c.block_warps,
                  "blocks_per_sm": c.blocks_per_sm, "block_queue": c.block_queue,
-                 "steps_per_iter": max(1, c.steps_per_iter),
+                 "steps_per_iter": c.steps_per_iter,
                  "source": "fixed" if args.launch_shape else "default"}
     else:
         tuned = autotune.tuned_config(batch, key, out.data_ptr(), reps=1)

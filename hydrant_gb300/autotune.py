@@ -60,7 +60,7 @@ def tuned_config(batch, key: str, rgba_ptr: int, reps: int = 2, path: Path = DEF
     best = batch.autotune(rgba_ptr, reps)
     c = {"tile_w": best.tile_w, "grab": best.grab, "block_warps": best.block_warps,
          "blocks_per_sm": best.blocks_per_sm, "block_queue": best.block_queue,
-         "steps_per_iter": max(1, best.steps_per_iter)}
+         "steps_per_iter": best.steps_per_iter}
     cache[key] = c
     try:
         Path(path).write_text(json.dumps(cache, indent=1, sort_keys=True))

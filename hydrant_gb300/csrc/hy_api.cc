@@ -43,6 +43,8 @@ extern "C" int hy_ctx_create(int device, hy_ctx **out) {
     ctx->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->counter_dev, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
@@ -106,6 +108,7 @@ extern "C" int hy_tf_set(hy_ctx *ctx, const float *rgba, int32_t n) {
                                  cudaMemcpyHostToDevice, ctx->stream));
     HY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->ntf = n;
+    hy_skip_tf_ranges(rgba, n, &ctx->tf_ranges, &ctx->tf_alpha_max);
     return HY_OK;
 }
 

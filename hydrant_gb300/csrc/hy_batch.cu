@@ -224,29 +224,46 @@ __global__ void __launch_bounds__(kMaxBlockThreads,
 #ifndef HY_BATCH_GATHER_REGS
 #define HY_BATCH_GATHER_REGS 48
 #endif
-template <int DT, bool PADDED, int GATHER>
+template <int DT, bool PADDED, int GATHER, int LOOP>
 constexpr int lean_regs() {
-    return GATHER ? HY_BATCH_GATHER_REGS : (DT == HY_DTYPE_U8 && PADDED) ? HY_BATCH_LEAN_REGS : 64;
+    return LOOP == kLoopBatch4 ? 128
+           : LOOP == kLoopBatch2 ? 64
+           : GATHER ? HY_BATCH_GATHER_REGS : (DT == HY_DTYPE_U8 && PADDED) ? HY_BATCH_LEAN_REGS : 64;
 }
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER, int LOOP>
-__global__ void __maxnreg__((lean_regs<DT, PADDED, GATHER>()))
+__global__ void __maxnreg__((lean_regs<DT, PADDED, GATHER, LOOP>()))
     batch_lean_kernel(const __grid_constant__ BatchArgs B) {
     batch_body<SHADER, PC, DT, PADDED, 0, true, GATHER, LOOP>(B);
 }
 
+// The lean march's samples in flight (volume_batches), where steps_per_iter
+// leaves it open: four (128 registers) for a batch of fewer than 8 warps of
+// rays a scheduler, which is bound by latency; else two at 64 registers, for
+// bricks of 32 voxels and more: 16 views of the 1024^3 volume 25.6 ms against
+// 25.7 with one at 48 registers (26.5 for two at 72 or 80, 29.9 for four at
+// 96), 11 views of a 99x213x412 volume 887 against 946 us, 9 views of 128^3
+// bricks 157 against 175; with 16^3 bricks a batch ends at a brick face
+// after a few steps and one sample at a time is faster (526 against 558 us).
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
-const void *pick_lean(const ShadeArgs &a, int steps_per_iter) {
+const void *pick_lean(const ShadeArgs &a, int steps_per_iter, long long rays) {
     if (a.ert > 0.f)
         return reinterpret_cast<const void *>(
             &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopErt>);
-    if (steps_per_iter == 2)
-        return reinterpret_cast<const void *>(
-            &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopTwo>);
+    if constexpr (PADDED) {
+        if (steps_per_iter != 1 && a.vol.P <= kMaxBatchesP) {
+            if (steps_per_iter == 0 && rays < 8 * 32ll * a.schedulers)
+                return reinterpret_cast<const void *>(
+                    &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopBatch4>);
+            if (steps_per_iter == 2 || a.vol.P >= 34)
+                return reinterpret_cast<const void *>(
+                    &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopBatch2>);
+        }
+    }
     return reinterpret_cast<const void *>(&batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopOne>);
 }
 
 template <int SHADER, int PC, int DT, bool PADDED>
-const void *pick_c(const ShadeArgs &a, int steps_per_iter) {
+const void *pick_c(const ShadeArgs &a, int steps_per_iter, long long rays) {
     if (a.composite) {
         // the Volume shader's per-brick segments sample by gathers too
         if constexpr (SHADER == HY_SHADER_VOLUME && DT == HY_DTYPE_U8 && PADDED) {
@@ -259,43 +276,43 @@ const void *pick_c(const ShadeArgs &a, int steps_per_iter) {
         if (a.mode == HY_VOLUME_DEFAULT) {
             if constexpr (DT == HY_DTYPE_U8 && PADDED) {
                 if (a.vol.tex)  // bricks in gather textures
-                    return pick_lean<SHADER, PC, DT, PADDED, true>(a, steps_per_iter);
+                    return pick_lean<SHADER, PC, DT, PADDED, true>(a, steps_per_iter, rays);
             }
-            return pick_lean<SHADER, PC, DT, PADDED, false>(a, steps_per_iter);
+            return pick_lean<SHADER, PC, DT, PADDED, false>(a, steps_per_iter, rays);
         }
     }
     return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, PADDED, 0>);
 }
 
 template <int SHADER>
-const void *pick_shader(const ShadeArgs &a, int spi) {
+const void *pick_shader(const ShadeArgs &a, int spi, long long rays) {
     if constexpr (SHADER == HY_SHADER_BLOCKS || SHADER == HY_SHADER_PAGING) {
-        return pick_c<SHADER, 0, HY_DTYPE_U8, false>(a, spi);
+        return pick_c<SHADER, 0, HY_DTYPE_U8, false>(a, spi, rays);
     } else {
         const bool padded = a.vol.pad > 0;
         if (a.vol.dtype == HY_DTYPE_F32) {
-            return padded ? pick_c<SHADER, 0, HY_DTYPE_F32, true>(a, spi)
-                          : pick_c<SHADER, 0, HY_DTYPE_F32, false>(a, spi);
+            return padded ? pick_c<SHADER, 0, HY_DTYPE_F32, true>(a, spi, rays)
+                          : pick_c<SHADER, 0, HY_DTYPE_F32, false>(a, spi, rays);
         }
-        if (padded && a.vol.P == 66) return pick_c<SHADER, 66, HY_DTYPE_U8, true>(a, spi);
-        if (padded && a.vol.P == 130) return pick_c<SHADER, 130, HY_DTYPE_U8, true>(a, spi);
-        return padded ? pick_c<SHADER, 0, HY_DTYPE_U8, true>(a, spi)
-                      : pick_c<SHADER, 0, HY_DTYPE_U8, false>(a, spi);
+        if (padded && a.vol.P == 66) return pick_c<SHADER, 66, HY_DTYPE_U8, true>(a, spi, rays);
+        if (padded && a.vol.P == 130) return pick_c<SHADER, 130, HY_DTYPE_U8, true>(a, spi, rays);
+        return padded ? pick_c<SHADER, 0, HY_DTYPE_U8, true>(a, spi, rays)
+                      : pick_c<SHADER, 0, HY_DTYPE_U8, false>(a, spi, rays);
     }
 }
 
-// steps_per_iter: march steps per loop iteration of the lean Volume march
-// (1 or 2; early termination keeps 1)
-const void *pick_kernel(const ShadeArgs &a, int steps_per_iter = 1) {
+// steps_per_iter: samples in flight of the lean Volume march (1 or 2, 0: by
+// the rule of pick_lean for this many rays; early termination keeps 1)
+const void *pick_kernel(const ShadeArgs &a, int steps_per_iter, long long rays) {
     switch (a.shader) {
         case HY_SHADER_VOLUME:
-            return pick_shader<HY_SHADER_VOLUME>(a, steps_per_iter);
+            return pick_shader<HY_SHADER_VOLUME>(a, steps_per_iter, rays);
         case HY_SHADER_BLOCKS:
-            return pick_shader<HY_SHADER_BLOCKS>(a, steps_per_iter);
+            return pick_shader<HY_SHADER_BLOCKS>(a, steps_per_iter, rays);
         case HY_SHADER_PAGING:
-            return pick_shader<HY_SHADER_PAGING>(a, steps_per_iter);
+            return pick_shader<HY_SHADER_PAGING>(a, steps_per_iter, rays);
         default:
-            return pick_shader<HY_SHADER_ISOSURFACE>(a, steps_per_iter);
+            return pick_shader<HY_SHADER_ISOSURFACE>(a, steps_per_iter, rays);
     }
 }
 
@@ -384,7 +401,9 @@ void fill_view(BatchView &d, const hy_batch_view &v, int tiles_x, int tile0) {
 // (Re)build the tile layout for the current config and the persistent grid.
 int layout(hy_batch *b) {
     hy_ctx *ctx = b->ctx;
-    b->kernel = pick_kernel(b->base, b->cfg.steps_per_iter == 2 ? 2 : 1);
+    long long rays = 0;
+    for (auto &v : b->in) rays += (long long)v.width * v.height;
+    b->kernel = pick_kernel(b->base, b->cfg.steps_per_iter, rays);
     int bx, by;
     unit_shape(b->cfg, bx, by);
     const int tw = b->cfg.tile_w * bx, th = (32 / b->cfg.tile_w) * by;
@@ -434,6 +453,15 @@ int launch(hy_batch *b, uint8_t *out) {
         b->base.ntf = ctx->ntf;
         int rc = layout(b);
         if (rc) return rc;
+    }
+    // the skip grid follows the knots; a launch that gains or loses it is a
+    // new graph
+    SkipGrid skip;
+    int rc = hy_skip_view(ctx, b->vol, &b->params, &skip);
+    if (rc) return rc;
+    if (skip.d != b->base.skip.d) {
+        b->base.skip = skip;
+        drop_graph(b);
     }
     const int count = b->params.count_samples ? 1 : 0;
     if (!b->exec || b->graph_out != out || b->graph_count != count) {
@@ -510,7 +538,6 @@ extern "C" int hy_batch_create(hy_ctx *ctx, const hy_volume *vol, const hy_shade
     b->params = *params;
     b->in.assign(views, views + nviews);
     b->base = base;
-    b->kernel = pick_kernel(base);
     for (auto &v : b->in)
         b->out_bytes = std::max<int64_t>(b->out_bytes, v.rgba_offset + (int64_t)v.width * v.height * 4);
     cudaError_t e = cudaMalloc(&b->views_dev, sizeof(BatchView) * nviews);
@@ -663,7 +690,7 @@ extern "C" int hy_batch_autotune(hy_batch *b, uint8_t *rgba_dev, int32_t reps,
     for (int tw : tws)
         for (int g : grabs)
             for (int w : warps) {
-                hy_batch_config c{tw, g, w, 0, bq, 1};
+                hy_batch_config c{tw, g, w, 0, bq, 0};
                 b->cfg = c;
                 if ((rc = layout(b))) goto done;
                 if ((rc = launch(b, rgba_dev))) goto done;  // warm-up and graph build
@@ -679,24 +706,26 @@ extern "C" int hy_batch_autotune(hy_batch *b, uint8_t *rgba_dev, int32_t reps,
                     best = c;
                 }
             }
-    // samples per loop iteration on the fastest shape
+    // one or two samples in flight on the fastest shape
     if (b->base.shader == HY_SHADER_VOLUME && b->base.mode == HY_VOLUME_DEFAULT &&
         !b->base.composite && !(b->base.ert > 0.f)) {
         hy_batch_config c = best;
-        c.steps_per_iter = 2;
-        b->cfg = c;
-        if ((rc = layout(b))) goto done;
-        if ((rc = launch(b, rgba_dev))) goto done;
-        HY_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
-        for (int r = 0; r < reps; ++r)
+        for (int steps = 1; steps <= 2; ++steps) {
+            c.steps_per_iter = steps;
+            b->cfg = c;
+            if ((rc = layout(b))) goto done;
             if ((rc = launch(b, rgba_dev))) goto done;
-        HY_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
-        HY_CUDA(ctx, cudaEventSynchronize(e1));
-        float ms = 0.f;
-        HY_CUDA(ctx, cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best_ms) {
-            best_ms = ms;
-            best = c;
+            HY_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
+            for (int r = 0; r < reps; ++r)
+                if ((rc = launch(b, rgba_dev))) goto done;
+            HY_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
+            HY_CUDA(ctx, cudaEventSynchronize(e1));
+            float ms = 0.f;
+            HY_CUDA(ctx, cudaEventElapsedTime(&ms, e0, e1));
+            if (ms < best_ms) {
+                best_ms = ms;
+                best = c;
+            }
         }
     }
 done:
@@ -783,6 +812,8 @@ extern "C" int hy_render_views_noalloc(hy_ctx *ctx, const hy_volume *vol,
     if (rc) return rc;
     base.count = 0;  // sample counting is not available on this entry point
     HY_CUDA(ctx, cudaSetDevice(ctx->device));
+    rc = hy_skip_view(ctx, vol, params, &base.skip);
+    if (rc) return rc;
     // The descriptors are copied from this call's stack: a captured copy
     // would replay from a dead address, so capture is refused.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -803,7 +834,7 @@ extern "C" int hy_render_views_noalloc(hy_ctx *ctx, const hy_volume *vol,
     const int uw = cfg.tile_w * bx, uh = (32 / cfg.tile_w) * by;
     BatchView hv[kNoAllocMaxViews];
     int hs[kNoAllocMaxViews];
-    long long tile = 0;
+    long long tile = 0, rays = 0;
     for (int i = 0; i < nviews; ++i) {
         const hy_batch_view &v = views[i];
         if (v.width <= 0 || v.height <= 0 || v.rgba_offset < 0 || (v.rgba_offset & 3))
@@ -824,6 +855,7 @@ extern "C" int hy_render_views_noalloc(hy_ctx *ctx, const hy_volume *vol,
         d.tile0 = int(tile);
         hs[i] = int(tile);
         tile += (long long)d.tiles_x * ((v.height + uh - 1) / uh);
+        rays += (long long)v.width * v.height;
         if (tile >= (1ll << 31) - 64) return hy_fail(ctx, HY_ERR_INVALID, "noalloc: too many tiles");
     }
     unsigned int *queue = reinterpret_cast<unsigned int *>(scratch);
@@ -849,7 +881,7 @@ extern "C" int hy_render_views_noalloc(hy_ctx *ctx, const hy_volume *vol,
     args.by = by;
     args.queue = queue;
     args.out = rgba_dev;
-    const void *kernel = pick_kernel(base);
+    const void *kernel = pick_kernel(base, 0, rays);
     const int threads = cfg.block_warps * 32;
     const size_t smem = size_t(base.ntf + kTfPad) * sizeof(float4) + 256 * sizeof(float) +
                         size_t(nviews) * sizeof(int);

@@ -97,6 +97,19 @@ struct ViewArgs {
     int W, H;
 };
 
+// The skip grid as a launch reads it (hy_skip.cu): a byte per cell of the
+// whole volume, cx cells a row and cy rows a slice; null: none.
+struct SkipGrid {
+    const unsigned char *d;
+    int plane;            // cells: plane (x < 0) + 2 (y < 0) + 4 (z < 0) of the directions
+    int cx, cy;
+    float fcx, fcy, fcz;  // cells per axis
+    float nc, cell;       // cells per brick edge (a power of two) and 1 / nc
+    float shrink;         // margin of a box in bricks
+    int stride;           // steps between two looks at the grid
+    float fstride;
+};
+
 // Everything one shading launch reads; passed as a __grid_constant__ kernel
 // parameter (the reference copies its shader struct into a 16 KiB
 // __constant__ buffer per launch, cuda_shading.cu:5-10).
@@ -114,6 +127,7 @@ struct ShadeArgs {
     int lowest_blkcnt;
     float to_world[16];
     int composite, srgb, count;
+    SkipGrid skip;
     float ert;  // early ray termination opacity (lean Volume march; 0 = off)
     unsigned char clear_u8[4];
     ViewArgs view;
@@ -126,17 +140,28 @@ struct ShadeArgs {
     void *film;
     void *dst;
     unsigned long long *counter;
+    int schedulers;  // warp schedulers of the device (host: launch shapes)
 };
 
 }  // namespace hy
 
+// Sample values without effect: up to HY_SKIP_RANGES closed intervals.
+constexpr int HY_SKIP_RANGES = 8;
+struct hy_skip_ranges {
+    int n = 0;
+    float lo[HY_SKIP_RANGES], hi[HY_SKIP_RANGES];
+};
+
 struct hy_ctx {
     int device = 0;
+    int sms = 0;
     cudaStream_t stream = nullptr;
     std::string err;
     float4 *tf_dev = nullptr;
     int ntf = 0;
     int tf_cap = 0;
+    hy_skip_ranges tf_ranges;  // of the knots (hy_skip_tf_ranges)
+    float tf_alpha_max = 0.f;
     unsigned long long *counter_dev = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     hy_render_stats stats{};
@@ -151,6 +176,21 @@ struct hy_ctx {
 };
 // Frees ctx->diff_gather (hy_diff.cu).
 void hy_diff_release(hy_ctx *ctx);
+
+// A resident volume's skip grid (hy_skip.cu): the cells' smallest and largest
+// voxels, and the distances for the ranges last asked for, one grid for the
+// transfer function and one for the isovalue.
+struct hy_skip {
+    int nc = 0;  // cells per brick edge; 0: none
+    int c[3] = {0, 0, 0};
+    long long cells = 0;
+    float shrink = 0.f;
+    void *minmax = nullptr;
+    unsigned char *tmp = nullptr, *tmp2 = nullptr;  // one allocation with the grids
+    unsigned char *grid[2] = {nullptr, nullptr};
+    bool valid[2] = {false, false};
+    hy_skip_ranges key[2];
+};
 
 struct hy_volume {
     hy_ctx *ctx = nullptr;
@@ -182,6 +222,7 @@ struct hy_volume {
     int4 *info4_dev = nullptr;
     bool tex_sampling = true;  // hy_volume_set_gather_sampling
     bool paged_gather = false;  // a pager's cache held in atlas (gather textures)
+    hy_skip skip;
 };
 
 // Brick store: every non-empty padded brick in pinned host memory, laid out
@@ -235,6 +276,15 @@ int hy_store_alloc(hy_store *s, int nonempty);
 // Chebyshev distance over the brick grid (hy_page.cu)
 void hy_chebyshev_transform(const std::vector<unsigned char> &nonempty, const int grid[3],
                             std::vector<int> &out);
+
+// Skip grid (hy_skip.cu): built from the brick pool by the upload, freed with
+// it; hy_skip_view brings it in line with the context's knots (or the
+// isovalue) on the context's stream and fills a launch's view of it, with a
+// null grid where the launch has to sample every cell.
+int hy_skip_build(hy_volume *v);
+void hy_skip_free(hy_volume *v);
+int hy_skip_view(hy_ctx *ctx, const hy_volume *v, const hy_shader_params *p, hy::SkipGrid *out);
+void hy_skip_tf_ranges(const float *rgba, int n, hy_skip_ranges *r, float *alpha_max);
 
 // error helpers (hy_api.cc)
 int hy_fail(hy_ctx *ctx, int code, const std::string &msg);

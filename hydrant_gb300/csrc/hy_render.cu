@@ -118,9 +118,10 @@ __global__ void HY_RENDER_LEAN_BOUNDS render_lean_kernel(const __grid_constant__
     render_body<SHADER, PC, DT, PADDED, 0, true, false, LOOP>(A);
 }
 // The same march sampling by texture gathers (u8 bricks with an apron in
-// the volume's gather textures): 64-view step, one launch per view, 169.6
-// ms at 48 registers against 172.4 at 56, 173.1 at 64 and 198.8 for the
-// loads (HY_RENDER_GATHER=0 builds the per-view path without it).
+// the volume's gather textures), one sample at a time, for early termination
+// and for paged caches: 64-view step, one launch per view, 169.6 ms at 48
+// registers against 172.4 at 56, 173.1 at 64 and 198.8 for the loads
+// (HY_RENDER_GATHER=0 builds the per-view path without gathers).
 #ifndef HY_RENDER_GATHER
 #define HY_RENDER_GATHER 1
 #endif
@@ -140,6 +141,44 @@ __global__ void __maxnreg__(GATHER == kGatherPaged ? HY_RENDER_PAGED_GATHER_REGS
     render_body<SHADER, PC, DT, PADDED, 0, true, GATHER, LOOP>(A);
 }
 
+
+// Lean march with 2 or 4 samples of a ray in flight (volume_batches), 64 or
+// 128 registers: with fewer the compiler fetches the samples one after the
+// other again.
+template <int SHADER, int PC, int DT, int GATHER, int LOOP>
+__global__ void __launch_bounds__(kThreads, LOOP == kLoopBatch4 ? 4 : 8)
+    render_batches_kernel(const __grid_constant__ ShadeArgs A) {
+    render_body<SHADER, PC, DT, true, 0, true, GATHER, LOOP>(A);
+}
+
+// Small launches of the lean march: 8 lanes a ray (volume_group).  A warp
+// holds 2x2 rays, a block 4 warps.
+constexpr int kGroup = 8, kGroupW = 2, kGroupH = 32 / kGroup / kGroupW;
+template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
+__global__ void __launch_bounds__(kThreads) render_group_kernel(const __grid_constant__ ShadeArgs A) {
+    extern __shared__ float4 smem[];
+    float4 *tf = smem;
+    float *lut = reinterpret_cast<float *>(smem + A.ntf + kTfPad);
+    load_shared(A, tf, lut);
+    const Shared S = make_shared(tf, A.ntf, lut);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane / kGroup;
+    const int x = (blockIdx.x * 2 + (warp & 1)) * kGroupW + r % kGroupW;
+    const int y = (blockIdx.y * 2 + (warp >> 1)) * kGroupH + r / kGroupW;
+    const bool on = x < A.view.W && y < A.view.H;
+    float ox, oy, oz, dx, dy, dz;
+    gen_ray(A.view, x, y, ox, oy, oz, dx, dy, dz);
+    Px p;
+    const bool hit = emit_setup<SHADER>(p, A, ox, oy, oz, dx, dy, dz, 0.f, 0.f, 0.f, A.bbox_max[0],
+                                        A.bbox_max[1], A.bbox_max[2]);
+    const unsigned int samples = volume_group<kGroup, PC, DT, PADDED, GATHER>(p, on && hit, A, S);
+    if (on && (lane & (kGroup - 1)) == 0) {
+        const float4 v = make_float4(p.vx, p.vy, p.vz, p.vw);
+        const size_t idx = size_t(y) * A.view.W + x;
+        A.rgba[idx] = quantise(A, v);
+        if (A.vout) A.vout[idx] = v;
+    }
+    count_samples(A, samples);
+}
 
 // The per-brick compositing variants of the Volume and Isosurface shaders,
 // held to 64 registers (8 resident blocks): on the 512^3 tubes at 1024^2,
@@ -313,6 +352,50 @@ dim3 grid_of(const ShadeArgs &a) {
     return dim3((a.view.W + kTileW - 1) / kTileW, (a.view.H + kTileH - 1) / kTileH);
 }
 
+template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
+void launch_group(const ShadeArgs &a, cudaStream_t s) {
+    const dim3 g((a.view.W + 2 * kGroupW - 1) / (2 * kGroupW),
+                 (a.view.H + 2 * kGroupH - 1) / (2 * kGroupH));
+    render_group_kernel<SHADER, PC, DT, PADDED, GATHER><<<g, kThreads, smem_bytes(a), s>>>(a);
+}
+
+// The lean march of one view in the form its size wants, by the warps (of 32
+// rays) a scheduler would get.  u8 by gathers, 1-voxel steps, us at 0.8, 3.4,
+// 13.5 and 54 warps (256^3, 512^3, 512^3, 512^3 blobs at 128^2, 256^2, 512^2,
+// 1024^2): 8 lanes a ray 65, 244, 783, 2871; 4 samples in flight 97, 196, 363,
+// 1100; 2 in flight 112, 247, 323, 904; one sample at a time 163, 361, 364, 941
+// (the last column row with boxes on all sides).  f32 (200^3, quarter-voxel
+// steps): 97, 155, 449, 1643; 163, 169, 230, 587; 191, 198, 248, 526; 288, 286,
+// 311, 581.  Without an apron only the group and the plain march are built:
+// 83, 228, 738 against 233, 235, 400.
+template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
+void launch_lean(const ShadeArgs &a, cudaStream_t s) {
+    const dim3 g = grid_of(a);
+    const size_t sm = smem_bytes(a);
+    if (a.ert > 0.f) {
+        if constexpr (GATHER != 0)
+            render_lean_gather_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopErt><<<g, kThreads, sm, s>>>(a);
+        else
+            render_lean_kernel<SHADER, PC, DT, PADDED, kLoopErt><<<g, kThreads, sm, s>>>(a);
+        return;
+    }
+    const long long rays = (long long)a.view.W * a.view.H, per_warp = 32ll * a.schedulers;
+    if (rays < 2 * per_warp) {
+        launch_group<SHADER, PC, DT, PADDED, GATHER>(a, s);
+        return;
+    }
+    if constexpr (PC == 0 && GATHER == 0) {
+        if (!PADDED || a.vol.P > kMaxBatchesP) {
+            render_lean_kernel<SHADER, PC, DT, PADDED, kLoopOne><<<g, kThreads, sm, s>>>(a);
+            return;
+        }
+    }
+    if (rays < 8 * per_warp)
+        render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
+    else
+        render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch2><<<g, kThreads, sm, s>>>(a);
+}
+
 template <int SHADER, int PC, int DT, bool PADDED>
 void launch_fused(const ShadeArgs &a, cudaStream_t s) {
     if (a.composite) {
@@ -332,10 +415,9 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
     }
     if constexpr (SHADER == HY_SHADER_VOLUME) {
         if (a.mode == HY_VOLUME_DEFAULT && !a.aux) {
-            const bool ert = a.ert > 0.f;
             if constexpr (DT == HY_DTYPE_U8 && PADDED) {
                 if (a.vol.paged_gather) {  // a pager's cache in gather textures
-                    if (ert)
+                    if (a.ert > 0.f)
                         render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherPaged, kLoopErt>
                             <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
                     else
@@ -346,21 +428,11 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
             }
             if constexpr (HY_RENDER_GATHER && DT == HY_DTYPE_U8 && PADDED) {
                 if (a.vol.tex) {  // bricks in gather textures
-                    if (ert)
-                        render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherResident, kLoopErt>
-                            <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
-                    else
-                        render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherResident, kLoopOne>
-                            <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+                    launch_lean<SHADER, PC, DT, PADDED, kGatherResident>(a, s);
                     return;
                 }
             }
-            if (ert)
-                render_lean_kernel<SHADER, PC, DT, PADDED, kLoopErt>
-                    <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
-            else
-                render_lean_kernel<SHADER, PC, DT, PADDED, kLoopOne>
-                    <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+            launch_lean<SHADER, PC, DT, PADDED, 0>(a, s);
             return;
         }
     }
@@ -445,6 +517,7 @@ int hy_fill_args(hy_ctx *ctx, const hy_volume *vol, const hy_shader_params *p, c
     if (p->shader == HY_SHADER_VOLUME && ctx->ntf <= 0)
         return hy_fail(ctx, HY_ERR_STATE, "render: Volume shader needs a transfer function");
     std::memset(a, 0, sizeof(*a));
+    a->skip.stride = 1 << 30;  // no skip grid unless hy_skip_view gives one
     a->vol = DevVolume{vol->pool, vol->info_dev, vol->reg_dev, vol->mean_dev, vol->grid[0],
                        vol->grid[1], vol->grid[2], vol->P, vol->desc.dtype, vol->desc.padding,
                        nullptr, {0ull, 0ull}, vol->k, vol->b, nullptr};
@@ -490,6 +563,7 @@ int hy_fill_args(hy_ctx *ctx, const hy_volume *vol, const hy_shader_params *p, c
     a->view.H = H;
     a->tf = ctx->tf_dev;
     a->ntf = ctx->ntf;
+    a->schedulers = 4 * ctx->sms;
     a->counter = ctx->counter_dev;
     return HY_OK;
 }
@@ -589,6 +663,8 @@ extern "C" int hy_render_device(hy_ctx *ctx, const hy_volume *vol, const hy_shad
     ShadeArgs a;
     int rc = hy_fill_args(ctx, vol, p, view, W, H, &a);
     if (rc) return rc;
+    rc = hy_skip_view(ctx, vol, p, &a.skip);
+    if (rc) return rc;
     a.rgba = reinterpret_cast<uchar4 *>(rgba_dev);
     a.vout = reinterpret_cast<float4 *>(v_dev);
     a.aux = reinterpret_cast<float4 *>(aux_dev);
@@ -615,6 +691,8 @@ extern "C" int hy_render(hy_ctx *ctx, const hy_volume *vol, const hy_shader_para
     int rc = hy_fill_args(ctx, vol, p, view, W, H, &a);
     if (rc) return rc;
     HY_CUDA(ctx, cudaSetDevice(ctx->device));
+    rc = hy_skip_view(ctx, vol, p, &a.skip);
+    if (rc) return rc;
     // outputs in pinned, mapped host memory are written by the kernel itself
     // (as in hy_batch_render); the others are staged in device memory and
     // copied once

@@ -457,6 +457,41 @@ __device__ __forceinline__ float sample_brick_gather(const DevVolume &V, const B
 #endif
 }
 
+// A trilinear sample in three parts, for marches that keep several in flight:
+// the footprint, its eight taps, the lerps -- the arithmetic of
+// sample_brick_gather and of sample_brick's interior case.
+constexpr int kMaxBatchesP = 1290;  // tap indices of a brick are ints: P^3 < 2^31
+struct Footprint {
+    float X, Y;  // gather coordinates
+    int off;     // or the lower tap's index in the brick (P <= kMaxBatchesP)
+    float2 axy;
+    float az;
+};
+template <int PC, bool GATHER>
+__device__ __forceinline__ Footprint footprint(const DevVolume &V, const BrickRef &b, float lx,
+                                               float ly, float lz) {
+    const int P = PC ? PC : V.P;
+    const float fd = float(P);
+    const float k = GATHER ? V.map_k : b.k;
+    const float mbx = GATHER ? V.map_b : b.bx, mby = GATHER ? V.map_b : b.by,
+                mbz = GATHER ? V.map_b : b.bz;
+    const float2 kl = mul2(f2(k, k), f2(lx, ly));
+    const float2 fxy = mul2(f2(fd, fd), f2(__fadd_rn(kl.x, mbx), __fadd_rn(kl.y, mby)));
+    const float fz = fd * (k * lz + mbz);
+    const float ux = fxy.x - .5f, uy = fxy.y - .5f, uz = fz - .5f;
+    const float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
+    Footprint f;
+    f.axy = sub2(f2(ux, uy), f2(flx, fly));
+    f.az = uz - flz;
+    if (GATHER) {
+        f.X = b.tx + flx;
+        f.Y = fabsf(b.ty) + (flz * fd + fly);
+    } else {
+        f.off = (int(flz) * P + int(fly)) * P + int(flx);
+    }
+    return f;
+}
+
 // The transfer function's knots in shared memory with the end knots
 // repeated and two zero knots after them: tfs[0] = knot 0, tfs[i + 1] =
 // knot i, tfs[n + 1] = knot n - 1, tfs[n + 2] = tfs[n + 3] = 0
@@ -615,6 +650,73 @@ struct BrickCursor {
     }
 };
 
+// Passes over the samples from p that change nothing (hy_skip.cu): while the
+// cell of p is free of effect, the ray takes every step whose sample lies in
+// the box of free cells ahead of it.  The axis that leaves the box first does
+// so after m steps (approximate division; the box is shrunk by more than its
+// error and the steps' roundings), so the samples at p, p + s, .., p + m s are
+// all in it: m + 1 steps (o + s), rounded one by one and counted as if they
+// had been sampled.  s >= 0 (a zero of either sign too) heads for the upper
+// face, so an axis the ray does not move along never limits it (x / 0 = inf,
+// and fminf drops 0 / 0).  A position outside the grid or NaN fails the range
+// test and is sampled.  step_size is 1..16.
+__device__ __forceinline__ float steps_to_face(float o, float s, float q, float up, float dn,
+                                               const SkipGrid &G) {
+    const float a = s >= 0.f ? ((q + up) * G.cell - G.shrink) - o
+                             : o - ((q + dn) * G.cell + G.shrink);
+    return __fdividef(a, fabsf(s));
+}
+// The plane of distances for rays of step (sx, sy, sz), as an offset.
+__device__ __forceinline__ int skip_plane(const SkipGrid &G, float sx, float sy, float sz) {
+    return (int(sx < 0.f) + 2 * int(sy < 0.f) + 4 * int(sz < 0.f)) * G.plane;
+}
+// The byte of the cell at (x, y, z); 0 outside the grid and for NaN.
+__device__ __forceinline__ int skip_cell(const SkipGrid &G, int plane, float x, float y, float z,
+                                         float &qx, float &qy, float &qz) {
+    qx = floorf(x * G.nc);
+    qy = floorf(y * G.nc);
+    qz = floorf(z * G.nc);
+    if (!(qx >= 0.f && qx < G.fcx && qy >= 0.f && qy < G.fcy && qz >= 0.f && qz < G.fcz)) return 0;
+    return __ldg(G.d + (plane + (int(qz) * G.cy + int(qy)) * G.cx + int(qx)));
+}
+__device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, float sy, float sz,
+                                          unsigned int &samples) {
+    const int plane = skip_plane(G, sx, sy, sz);
+    while (p.nsteps > 0) {
+        float qx, qy, qz;
+        const int d = skip_cell(G, plane, p.ox, p.oy, p.oz, qx, qy, qz);
+        if (d == 0) return;
+        const float up = float(d), dn = float(1 - d);
+        const float m = fminf(fminf(steps_to_face(p.ox, sx, qx, up, dn, G),
+                                    steps_to_face(p.oy, sy, qy, up, dn, G)),
+                              steps_to_face(p.oz, sz, qz, up, dn, G));
+        unsigned int n = 1u + unsigned(int(fminf(fmaxf(m, 0.f), 126.f)));
+        const unsigned int left = unsigned(p.nsteps), ss = unsigned(p.step_size);
+        n = min(n, ss == 1u ? left : (left + ss - 1u) / ss);
+        samples += n;
+        p.nsteps -= int(n * ss);
+        for (; n > 0; --n) {
+            p.ox = p.ox + sx;
+            p.oy = p.oy + sy;
+            p.oz = p.oz + sz;
+        }
+    }
+}
+// Between two looks at the grid a march takes 16 steps (G.stride), the warp
+// together.  The next look is a hint loaded before those steps, from about
+// where they end, so its latency is hidden behind them; only a free cell
+// there starts skip_free, which looks again where the ray is.  16-view batch of
+// the 1024^3 volume: 43.5 ms without the grid, 27.8 with a look every 4
+// steps, 26.0 every 8, 25.7 every 16, 24.7 with the distances kept per
+// direction.
+__device__ __forceinline__ int skip_hint(const Px &p, const SkipGrid &G, float sx, float sy,
+                                         float sz, float steps) {
+    if (!G.d) return 0;
+    float qx, qy, qz;
+    return skip_cell(G, skip_plane(G, sx, sy, sz), __fmaf_rn(steps, sx, p.ox), __fmaf_rn(steps, sy, p.oy),
+                     __fmaf_rn(steps, sz, p.oz), qx, qy, qz);
+}
+
 // VolumeShaderKernel::main (volume_shader.cu:32-81) as the per-ray state and
 // one loop iteration; volume_main is the loop.  PADDED: the volume has an
 // apron of >= 1 voxel, so the interior sampler applies.
@@ -745,20 +847,283 @@ struct VolumeMarch {
 //            alone stopping would not free its warp).  A lane stops only when
 //            its own ray is that opaque, whichever lanes vote with it, so what
 //            it leaves out adds at most 1 - A.ert per channel;
-//  kLoopTwo  two steps per iteration (the batch's steps_per_iter = 2): the
-//            same steps in the same order, one loop test per step still.
-constexpr int kLoopOne = 0, kLoopErt = 1, kLoopTwo = 2;
+//  kLoopBatch2, kLoopBatch4  volume_batches with 2 or 4 samples in flight.
+constexpr int kLoopOne = 0, kLoopErt = 1, kLoopBatch2 = 2, kLoopBatch4 = 4;
 template <int PC, int DT, bool PADDED, bool LEAN = false, int GATHER = 0, int LOOP = kLoopOne>
 __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, const Shared &S) {
     unsigned int samples = 0;
     VolumeMarch m;
     m.init(p, A.step);
-    while (p.nsteps > 0) {
-        if (!m.step<PC, DT, PADDED, LEAN, GATHER>(p, A, S, samples)) break;
-        if (LOOP == kLoopErt && __all_sync(__activemask(), p.vw >= A.ert)) break;
-        if (LOOP == kLoopTwo) {
-            if (p.nsteps <= 0) break;
+    if constexpr (LOOP == kLoopErt) {
+        while (p.nsteps > 0) {
             if (!m.step<PC, DT, PADDED, LEAN, GATHER>(p, A, S, samples)) break;
+            if (__all_sync(__activemask(), p.vw >= A.ert)) break;
+        }
+    } else {
+        bool go = true;
+        int hint = A.skip.d != nullptr;
+        while (go && p.nsteps > 0) {
+            if (hint) {
+                skip_free(p, A.skip, m.sx, m.sy, m.sz, samples);
+                if (p.nsteps <= 0) break;
+            }
+            hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, A.skip.fstride);
+            int r = A.skip.stride;  // at least one step whatever it is
+            do {
+                go = m.step<PC, DT, PADDED, LEAN, GATHER>(p, A, S, samples);
+            } while (go && p.nsteps > 0 && --r > 0);
+        }
+    }
+    return samples;
+}
+
+// The lean Volume march with U samples of the ray in flight: a step's taps
+// do not depend on the sample before it (only its position does, by one
+// addition), so the next U positions are stepped first, their taps fetched
+// together, and their colours composited in order -- the floats of
+// volume_main.  A batch takes the samples in the brick of its first one; the
+// sample after which the step size changes ends it (the samples fetched
+// beyond are dropped).
+template <int U, int PC, int DT, bool PADDED, int GATHER>
+__device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, const Shared &S) {
+    const DevVolume &V = A.vol;
+    unsigned int samples = 0;
+    VolumeMarch m;
+    m.init(p, A.step);
+    int hint = A.skip.d != nullptr;
+    while (p.nsteps > 0) {
+        if (hint) {
+            skip_free(p, A.skip, m.sx, m.sy, m.sz, samples);
+            if (p.nsteps <= 0) break;
+        }
+        hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, A.skip.fstride);
+        int r = A.skip.stride;
+        do {
+            float lx, ly, lz;
+            m.c.update<GATHER>(V, p.ox, p.oy, p.oz, lx, ly, lz);
+            if (!m.c.sample) {
+                if (m.c.cd == 0) return samples;
+                const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
+                p.nsteps -= skip_nblock_steps(p, 1.f / p.dx, 1.f / p.dy, 1.f / p.dz, m.c.ipx, m.c.ipy,
+                                              m.c.ipz, m.c.cd, cdu, A.step * float(p.step_size));
+                m.advance(p);
+                --r;
+                continue;
+            }
+            const int ss = p.step_size;
+            float qx[U], qy[U], qz[U], v[U];
+            Footprint fp[U];
+            bool ok = true;
+            int n = 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                qx[u] = u ? qx[u ? u - 1 : 0] + m.sx : p.ox;
+                qy[u] = u ? qy[u ? u - 1 : 0] + m.sy : p.oy;
+                qz[u] = u ? qz[u ? u - 1 : 0] + m.sz : p.oz;
+                float ux = lx, uy = ly, uz = lz;
+                if (u) {
+                    ux = qx[u] - m.c.ipx;
+                    uy = qy[u] - m.c.ipy;
+                    uz = qz[u] - m.c.ipz;
+                    ok = ok & unit_interval(ux) & unit_interval(uy) & unit_interval(uz) &
+                         (p.nsteps > u * ss);
+                    ux = ok ? ux : lx;
+                    uy = ok ? uy : ly;
+                    uz = ok ? uz : lz;
+                }
+                n += ok;
+                fp[u] = footprint<PC, GATHER != 0>(V, m.c.br, ux, uy, uz);
+            }
+            if constexpr (GATHER) {
+                const int P = PC ? PC : V.P;
+                const float fd = float(P);
+                float4 g0[U], g1[U];
+                const unsigned int am = __activemask();
+                if (__all_sync(am, m.c.br.which == 0)) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        g0[u] = gather_r(V.gtex[0], fp[u].X, fp[u].Y);
+                        g1[u] = gather_r(V.gtex[0], fp[u].X, fp[u].Y + fd);
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) gather2(V, m.c.br.which, fp[u].X, fp[u].Y, fd, g0[u], g1[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    v[u] = trilerp(f2(g0[u].w, g1[u].w), f2(g0[u].z, g1[u].z), f2(g0[u].x, g1[u].x),
+                                   f2(g0[u].y, g1[u].y), fp[u].axy, fp[u].az);
+            } else {
+                const int P = PC ? PC : V.P;
+                float t[U][8];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int at[8] = {0, P * P, 1, P * P + 1, P, P * P + P, P + 1, P * P + P + 1};
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        if (DT == HY_DTYPE_U8)
+                            t[u][k] = u8_norm(__ldg(m.c.br.base + fp[u].off + at[k]));
+                        else
+                            t[u][k] = __ldg(reinterpret_cast<const float *>(m.c.br.base) + fp[u].off + at[k]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    v[u] = trilerp(f2(t[u][0], t[u][1]), f2(t[u][2], t[u][3]), f2(t[u][4], t[u][5]),
+                                   f2(t[u][6], t[u][7]), fp[u].axy, fp[u].az);
+            }
+            int end = 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                float4 c = sample_tf<DT == HY_DTYPE_U8>(S.tf, S.ntf, S.fntf, v[u]);
+                c.w = c.w * A.density;
+                const float2 cxy = mul2(f2(c.x, c.y), f2(c.w, c.w));
+                c.z = c.z * c.w;
+                if (u < n) {
+                    const float t = 1.f - p.vw;
+                    const float2 txy = mul2(cxy, f2(t, t)), tzw = mul2(f2(c.z, c.w), f2(t, t));
+                    p.vx = __fadd_rn(p.vx, txy.x);
+                    p.vy = __fadd_rn(p.vy, txy.y);
+                    p.vz = __fadd_rn(p.vz, tzw.x);
+                    p.vw = __fadd_rn(p.vw, tzw.y);
+                    p.ox = qx[u];
+                    p.oy = qy[u];
+                    p.oz = qz[u];
+                    end = u;
+                    if (p.vw >= HY_T85) {
+                        const int s2 = p.vw >= HY_T93 ? 16 : 4;
+                        if (s2 != ss) {
+                            p.step_size = s2;
+                            m.set_step(p, A.step);
+                            n = 0;
+                        }
+                    }
+                }
+            }
+            samples += unsigned(end + 1);
+            p.nsteps -= end * ss;
+            m.advance(p);
+            r -= U;
+        } while (p.nsteps > 0 && r > 0);
+    }
+    return samples;
+}
+
+// The lean Volume march with a ray's consecutive samples on K neighbouring
+// lanes, for launches too small to fill the GPU: there a march is a chain of
+// samples, each waiting some 600 cycles for its taps, and K of them wait
+// together here.  Lane j of a ray's group takes sample j of the next K steps
+// (the position by j additions, as the march rounds it) up to its colour; then
+// every lane composites the group's K colours in order, so all hold the same
+// ray state and the floats are those of volume_main.  The group ends early at
+// the sample after which the step size changes, and before a sample whose
+// cell is an empty or absent brick.  The warp stays together: every lane of
+// the warp must call this (`on` false: no ray).  Costs about 13 instructions a
+// sample and ray more than volume_main.
+template <int K, int PC, int DT, bool PADDED, int GATHER>
+__device__ __forceinline__ unsigned int volume_group(Px &p, bool on, const ShadeArgs &A,
+                                                     const Shared &S) {
+    const DevVolume &V = A.vol;
+    const unsigned int full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, j = lane & (K - 1), base = lane - j;
+    const unsigned int group = (K == 32 ? full : ((1u << K) - 1u)) << base;
+    unsigned int samples = 0;
+    VolumeMarch m;
+    m.init(p, A.step);
+    if (!on) p.nsteps = 0;
+    int hint = A.skip.d != nullptr;
+    while (__any_sync(full, p.nsteps > 0)) {
+        if (hint && p.nsteps > 0) {
+            unsigned int n = 0;
+            skip_free(p, A.skip, m.sx, m.sy, m.sz, n);
+            if (j == 0) samples += n;
+        }
+        hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, float(K));
+        const int ss = p.step_size;
+        // this lane's sample
+        float px = p.ox, py = p.oy, pz = p.oz;
+#pragma unroll
+        for (int i = 0; i < K - 1; ++i)
+            if (i < j) {
+                px = px + m.sx;
+                py = py + m.sy;
+                pz = pz + m.sz;
+            }
+        const bool valid = p.nsteps > j * ss;
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool special = false;
+        if (valid) {
+            float lx, ly, lz;
+            m.c.update<GATHER>(V, px, py, pz, lx, ly, lz);
+            special = !m.c.sample;
+            if (m.c.sample) {
+                float s;
+                if constexpr (GATHER)
+                    s = sample_brick_gather<PC, GATHER>(V, m.c.br, V.P, lx, ly, lz);
+                else
+                    s = sample_brick<PC, DT, PADDED>(m.c.br, V.P, lx, ly, lz, S.lut);
+                c = sample_tf<DT == HY_DTYPE_U8>(S.tf, S.ntf, S.fntf, s);
+                c.w = c.w * A.density;
+                c.x = c.x * c.w;
+                c.y = c.y * c.w;
+                c.z = c.z * c.w;
+            }
+        }
+        const unsigned int vb = __ballot_sync(full, valid) & group;
+        const unsigned int sb = __ballot_sync(full, special) & group;
+        // samples to composite: the valid ones before the first special one
+        const int nv = __popc(vb);
+        const int take = sb ? __ffs(sb) - 1 - base : nv;
+        int end = -1;  // the sample after which the step size changed
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            const float4 q = make_float4(__shfl_sync(full, c.x, i, K), __shfl_sync(full, c.y, i, K),
+                                         __shfl_sync(full, c.z, i, K), __shfl_sync(full, c.w, i, K));
+            if (i < take && end < 0) {
+                const float t = 1.f - p.vw;
+                const float2 txy = mul2(f2(q.x, q.y), f2(t, t)), tzw = mul2(f2(q.z, q.w), f2(t, t));
+                p.vx = __fadd_rn(p.vx, txy.x);
+                p.vy = __fadd_rn(p.vy, txy.y);
+                p.vz = __fadd_rn(p.vz, tzw.x);
+                p.vw = __fadd_rn(p.vw, tzw.y);
+                if (p.vw >= HY_T85 && p.step_size != (p.vw >= HY_T93 ? 16 : 4)) end = i;
+            }
+        }
+        // the position to go on from: after the last sample, at the special
+        // sample, or at the one that changed the step size
+        const int at = end >= 0 ? end : sb ? take : K - 1;
+        const float qx = __shfl_sync(full, px, at, K), qy = __shfl_sync(full, py, at, K),
+                    qz = __shfl_sync(full, pz, at, K);
+        if (p.nsteps > 0) {
+            p.ox = qx;
+            p.oy = qy;
+            p.oz = qz;
+            if (end >= 0) {
+                if (j == 0) samples += unsigned(end + 1);
+                p.nsteps -= end * ss;
+                p.step_size = p.vw >= HY_T93 ? 16 : 4;
+                m.set_step(p, A.step);
+                m.advance(p);
+            } else if (sb) {
+                if (j == 0) samples += unsigned(take);
+                p.nsteps -= take * ss;
+                const float ipx = floorf(qx), ipy = floorf(qy), ipz = floorf(qz);
+                const int cd = __ldg(&V.info[thumb_index(V, ipx, ipy, ipz)].x);
+                if (cd == 0) {
+                    p.nsteps = 0;  // absent brick: the ray ends
+                } else {
+                    const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
+                    p.nsteps -= skip_nblock_steps(p, 1.f / p.dx, 1.f / p.dy, 1.f / p.dz, ipx, ipy,
+                                                  ipz, cd, cdu, A.step * float(ss));
+                    m.advance(p);
+                }
+            } else {
+                if (j == 0) samples += unsigned(nv);
+                p.nsteps -= nv * ss;
+                p.ox = p.ox + m.sx;
+                p.oy = p.oy + m.sy;
+                p.oz = p.oz + m.sz;
+            }
         }
     }
     return samples;
@@ -980,7 +1345,11 @@ template <int SHADER, int PC, int DT, bool PADDED, bool LEAN = false, int GATHER
           int LOOP = kLoopOne>
 __device__ __forceinline__ long long run_main(Px &p, const ShadeArgs &A, const ViewArgs &Vw,
                                              const Shared &S) {
-    if (SHADER == HY_SHADER_VOLUME)
+    if constexpr (SHADER == HY_SHADER_VOLUME && LOOP == kLoopBatch2)
+        return volume_batches<2, PC, DT, PADDED, GATHER>(p, A, S);
+    else if constexpr (SHADER == HY_SHADER_VOLUME && LOOP == kLoopBatch4)
+        return volume_batches<4, PC, DT, PADDED, GATHER>(p, A, S);
+    else if (SHADER == HY_SHADER_VOLUME)
         return volume_main<PC, DT, PADDED, LEAN, GATHER, LOOP>(p, A, S);
     if (SHADER == HY_SHADER_BLOCKS) return blocks_main(p, A);
     if (SHADER == HY_SHADER_PAGING) return paging_main(p, A);

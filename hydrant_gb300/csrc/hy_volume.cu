@@ -307,6 +307,7 @@ int build_gather(hy_volume *vol) {
 
 void free_volume_device(hy_volume *v) {
     free_gather(v);
+    hy_skip_free(v);
     if (v->pool) cudaFree(v->pool);
     if (v->info_dev) cudaFree(v->info_dev);
     if (v->reg_dev) cudaFree(v->reg_dev);
@@ -412,6 +413,8 @@ int upload_impl(hy_volume *vol, const void *host) {
 #undef HY_UP
     cleanup();
     vol->uploaded = true;
+    const int rc = hy_skip_build(vol);
+    if (rc) return rc;
     return build_gather(vol);
 }
 
