@@ -95,9 +95,16 @@ __device__ __forceinline__ void render_body(const ShadeArgs &A) {
     count_samples(A, samples);
 }
 
-template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE, bool LEAN, int LOOP = kLoopOne>
+template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE>
 __global__ void __launch_bounds__(kThreads) render_kernel(const __grid_constant__ ShadeArgs A) {
-    render_body<SHADER, PC, DT, PADDED, COMPOSITE, LEAN, false, LOOP>(A);
+    render_body<SHADER, PC, DT, PADDED, COMPOSITE, false>(A);
+}
+
+// The Isosurface march with 2 or 4 samples in flight (80 and 128 registers).
+template <int PC, int DT, int LOOP>
+__global__ void __launch_bounds__(kThreads, LOOP == kLoopBatch4 ? 4 : 6)
+    render_iso_kernel(const __grid_constant__ ShadeArgs A) {
+    render_body<HY_SHADER_ISOSURFACE, PC, DT, true, 0, false, false, LOOP>(A);
 }
 
 // The lean march of the per-view path by loads (f32 volumes, volumes without
@@ -400,7 +407,7 @@ template <int SHADER, int PC, int DT, bool PADDED>
 void launch_fused(const ShadeArgs &a, cudaStream_t s) {
     if (a.composite) {
         if constexpr (SHADER == HY_SHADER_BLOCKS)
-            render_kernel<SHADER, PC, DT, PADDED, 1, false><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+            render_kernel<SHADER, PC, DT, PADDED, 1><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
         else if constexpr (HY_RENDER_COMPOSITE_GATHER && SHADER == HY_SHADER_VOLUME &&
                            DT == HY_DTYPE_U8 && PADDED) {
             if (a.vol.tex)
@@ -436,7 +443,21 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
             return;
         }
     }
-    render_kernel<SHADER, PC, DT, PADDED, 0, false><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+    if constexpr (SHADER == HY_SHADER_ISOSURFACE && PADDED) {
+        // Samples in flight by the warps of rays a scheduler gets: 512^3 tubes
+        // at 256^2, 512^2 and 1024^2 (3.4, 13.5, 54 warps) 470, 596, 1160 us
+        // with four, 492, 590, 984 with two, 554, 602, 978 with one; 200^3 f32
+        // blobs at 600^2 (18.5 warps) 222, 216, 236.
+        const long long rays = (long long)a.view.W * a.view.H, per_warp = 32ll * a.schedulers;
+        if (rays < 24 * per_warp && a.vol.P <= kMaxBatchesP) {
+            if (rays < 8 * per_warp)
+                render_iso_kernel<PC, DT, kLoopBatch4><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+            else
+                render_iso_kernel<PC, DT, kLoopBatch2><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+            return;
+        }
+    }
+    render_kernel<SHADER, PC, DT, PADDED, 0><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
 }
 
 // Instantiations: Blocks reads no bricks; u8 volumes with a 1-voxel apron and

@@ -492,6 +492,27 @@ __device__ __forceinline__ Footprint footprint(const DevVolume &V, const BrickRe
     return f;
 }
 
+// U samples of one brick by loads: all taps first, then the lerps, so that
+// the loads are in flight together.
+template <int U, int PC, int DT>
+__device__ __forceinline__ void fetch_loads(const DevVolume &V, const BrickRef &b,
+                                            const Footprint (&fp)[U], float (&v)[U]) {
+    const int P = PC ? PC : V.P;
+    const int at[8] = {0, P * P, 1, P * P + 1, P, P * P + P, P + 1, P * P + P + 1};
+    float t[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            t[u][k] = DT == HY_DTYPE_U8
+                          ? u8_norm(__ldg(b.base + fp[u].off + at[k]))
+                          : __ldg(reinterpret_cast<const float *>(b.base) + fp[u].off + at[k]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        v[u] = trilerp(f2(t[u][0], t[u][1]), f2(t[u][2], t[u][3]), f2(t[u][4], t[u][5]),
+                       f2(t[u][6], t[u][7]), fp[u].axy, fp[u].az);
+}
+
 // The transfer function's knots in shared memory with the end knots
 // repeated and two zero knots after them: tfs[0] = knot 0, tfs[i + 1] =
 // knot i, tfs[n + 1] = knot n - 1, tfs[n + 2] = tfs[n + 3] = 0
@@ -679,7 +700,7 @@ __device__ __forceinline__ int skip_cell(const SkipGrid &G, int plane, float x, 
     if (!(qx >= 0.f && qx < G.fcx && qy >= 0.f && qy < G.fcy && qz >= 0.f && qz < G.fcz)) return 0;
     return __ldg(G.d + (plane + (int(qz) * G.cy + int(qy)) * G.cx + int(qx)));
 }
-__device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, float sy, float sz,
+__device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, float sy, float sz, int step_size,
                                           unsigned int &samples) {
     const int plane = skip_plane(G, sx, sy, sz);
     while (p.nsteps > 0) {
@@ -691,7 +712,7 @@ __device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, fl
                                     steps_to_face(p.oy, sy, qy, up, dn, G)),
                               steps_to_face(p.oz, sz, qz, up, dn, G));
         unsigned int n = 1u + unsigned(int(fminf(fmaxf(m, 0.f), 126.f)));
-        const unsigned int left = unsigned(p.nsteps), ss = unsigned(p.step_size);
+        const unsigned int left = unsigned(p.nsteps), ss = unsigned(step_size);
         n = min(n, ss == 1u ? left : (left + ss - 1u) / ss);
         samples += n;
         p.nsteps -= int(n * ss);
@@ -864,7 +885,7 @@ __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, cons
         int hint = A.skip.d != nullptr;
         while (go && p.nsteps > 0) {
             if (hint) {
-                skip_free(p, A.skip, m.sx, m.sy, m.sz, samples);
+                skip_free(p, A.skip, m.sx, m.sy, m.sz, p.step_size, samples);
                 if (p.nsteps <= 0) break;
             }
             hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, A.skip.fstride);
@@ -893,7 +914,7 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
     int hint = A.skip.d != nullptr;
     while (p.nsteps > 0) {
         if (hint) {
-            skip_free(p, A.skip, m.sx, m.sy, m.sz, samples);
+            skip_free(p, A.skip, m.sx, m.sy, m.sz, p.step_size, samples);
             if (p.nsteps <= 0) break;
         }
         hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, A.skip.fstride);
@@ -954,23 +975,7 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
                     v[u] = trilerp(f2(g0[u].w, g1[u].w), f2(g0[u].z, g1[u].z), f2(g0[u].x, g1[u].x),
                                    f2(g0[u].y, g1[u].y), fp[u].axy, fp[u].az);
             } else {
-                const int P = PC ? PC : V.P;
-                float t[U][8];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int at[8] = {0, P * P, 1, P * P + 1, P, P * P + P, P + 1, P * P + P + 1};
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        if (DT == HY_DTYPE_U8)
-                            t[u][k] = u8_norm(__ldg(m.c.br.base + fp[u].off + at[k]));
-                        else
-                            t[u][k] = __ldg(reinterpret_cast<const float *>(m.c.br.base) + fp[u].off + at[k]);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    v[u] = trilerp(f2(t[u][0], t[u][1]), f2(t[u][2], t[u][3]), f2(t[u][4], t[u][5]),
-                                   f2(t[u][6], t[u][7]), fp[u].axy, fp[u].az);
+                fetch_loads<U, PC, DT>(V, m.c.br, fp, v);
             }
             int end = 0;
 #pragma unroll
@@ -1035,7 +1040,7 @@ __device__ __forceinline__ unsigned int volume_group(Px &p, bool on, const Shade
     while (__any_sync(full, p.nsteps > 0)) {
         if (hint && p.nsteps > 0) {
             unsigned int n = 0;
-            skip_free(p, A.skip, m.sx, m.sy, m.sz, n);
+            skip_free(p, A.skip, m.sx, m.sy, m.sz, p.step_size, n);
             if (j == 0) samples += n;
         }
         hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, float(K));
@@ -1242,14 +1247,15 @@ __device__ __forceinline__ void normalize3(float &x, float &y, float &z) {
 }
 
 // IsosurfaceShaderKernel::main (isosurface_shader.cu:50-125).  prev_value
-// stays 0, as in the reference (it is never updated there).
-template <int PC, int DT, bool PADDED>
+// stays 0, as in the reference (it is never updated there).  U samples of the
+// ray in flight (U > 1: bricks with an apron, as in volume_batches; the
+// samples fetched beyond the hit are dropped); samples that cannot cross
+// the isovalue are passed over (skip_free).
+template <int U, int PC, int DT, bool PADDED>
 __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const ViewArgs &Vw,
                                              const Shared &S) {
     const DevVolume &V = A.vol;
-    long long samples = 0;
-    const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
-    const float rx = 1.f / p.dx, ry = 1.f / p.dy, rz = 1.f / p.dz;
+    unsigned int samples = 0;
     const float prev_value = 0.0f;
     const float iso = A.isovalue;
     // sign(value - iso) != sign(prev_value - iso), prev_value = 0 (never
@@ -1261,83 +1267,132 @@ __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const V
     const float sx = p.dx * A.step, sy = p.dy * A.step, sz = p.dz * A.step;
     BrickCursor c;
     c.reset();
-    while (p.nsteps > 0) {
-        float l0x, l0y, l0z;
-        c.update(V, p.ox, p.oy, p.oz, l0x, l0y, l0z);
-        const float ipx = c.ipx, ipy = c.ipy, ipz = c.ipz;
-        const BrickRef &br = c.br;
-        if (c.cd) {
-            p.nsteps -= skip_nblock_steps(p, rx, ry, rz, ipx, ipy, ipz, c.cd, cdu, A.step);
-        } else {
-            if (c.pg == -1) break;  // page fault: resume in the next march pass
-            float value = sample_brick<PC, DT, PADDED>(br, V.P, l0x, l0y, l0z, S.lut);
-            ++samples;
-            const bool crossed = prev_sign < 0.f   ? !(value < iso)
-                                 : prev_sign > 0.f ? !(value > iso)
-                                                   : (value < iso || value > iso);
-            if (crossed) {
-                const float dt = A.step;
-                p.vx = A.surface[0];
-                p.vy = A.surface[1];
-                p.vz = A.surface[2];
-                p.vw = 1.f;
-                const float a = (iso - prev_value) / (value - prev_value);
-                const float qx = p.ox - dt * p.dx, qy = p.oy - dt * p.dy, qz = p.oz - dt * p.dz;
-                const float ia = 1.f - a;
-                const float ipx2 = ia * qx + a * p.ox, ipy2 = ia * qy + a * p.oy,
-                            ipz2 = ia * qz + a * p.oz;
-                // central difference in brick-local coordinates, dt = du * 2
-                const float lx = ipx2 - ipx, ly = ipy2 - ipy, lz = ipz2 - ipz;
-                const float g = A.du * 2.f;
-                float nnx = sample_brick<0, DT>(br, V.P, lx - g, ly - 0.f, lz - 0.f, S.lut) -
-                            sample_brick<0, DT>(br, V.P, lx + g, ly + 0.f, lz + 0.f, S.lut);
-                float nny = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - g, lz - 0.f, S.lut) -
-                            sample_brick<0, DT>(br, V.P, lx + 0.f, ly + g, lz + 0.f, S.lut);
-                float nnz = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - 0.f, lz - g, S.lut) -
-                            sample_brick<0, DT>(br, V.P, lx + 0.f, ly + 0.f, lz + g, S.lut);
-                samples += 6;
-                float wx, wy, wz, nx, ny, nz;
-                mat_vec4(A.to_world, ipx2, ipy2, ipz2, 1.f, wx, wy, wz);
-                mat_vec4(A.to_world, nnx, nny, nnz, 0.f, nx, ny, nz);
-                normalize3(nx, ny, nz);
-                float lx2 = Vw.light[0] - wx, ly2 = Vw.light[1] - wy, lz2 = Vw.light[2] - wz;
-                normalize3(lx2, ly2, lz2);
-                float hx = lx2 - wx, hy = ly2 - wy, hz = lz2 - wz;
-                normalize3(hx, hy, hz);
-                const float ambient = 0.2f;
-                const float diffuse = .6f * fclamp(lx2 * nx + ly2 * ny + lz2 * nz, 0.f, 1.f);
-                const float specular =
-                    .2f * powf(fclamp(hx * nx + hy * ny + hz * nz, 0.f, 1.f), 100.f);
-                const float ex = wx - Vw.eye[0], ey = wy - Vw.eye[1], ez = wz - Vw.eye[2];
-                const float distance = sqrtf(ex * ex + ey * ey + ez * ez) / 2.f;
-                if (A.mode == HY_ISO_COLOR) {
-                    const float f = ambient + (diffuse + specular) / distance;
-                    p.vx = iso_linear_to_srgb(p.vx * f);
-                    p.vy = iso_linear_to_srgb(p.vy * f);
-                    p.vz = iso_linear_to_srgb(p.vz * f);
-                    p.vw = p.vw * f;
-                } else if (A.mode == HY_ISO_POSITION) {
-                    p.vx = ipx2 / A.bbox_max[0];
-                    p.vy = ipy2 / A.bbox_max[1];
-                    p.vz = ipz2 / A.bbox_max[2];
-                    p.vw = 1.f;
-                } else {
-                    p.vx = nx;
-                    p.vy = ny;
-                    p.vz = nz;
-                    p.vw = 1.f;
-                }
-                const float ddx = p.e0 - p.ox, ddy = p.e1 - p.oy, ddz = p.e2 - p.oz;
-                p.e3 = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
-                p.nsteps = 0;
-                break;
-            }
+    bool hit = false;
+    float value = 0.f;
+    int hint = A.skip.d != nullptr;
+    while (p.nsteps > 0 && !hit) {
+        if (hint) {
+            skip_free(p, A.skip, sx, sy, sz, 1, samples);
+            if (p.nsteps <= 0) break;
         }
-        p.ox = p.ox + sx;
-        p.oy = p.oy + sy;
-        p.oz = p.oz + sz;
-        p.nsteps -= 1;
+        hint = skip_hint(p, A.skip, sx, sy, sz, A.skip.fstride);
+        int r = A.skip.stride;
+        do {
+            float lx, ly, lz;
+            c.update(V, p.ox, p.oy, p.oz, lx, ly, lz);
+            if (c.cd) {
+                const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
+                p.nsteps -= skip_nblock_steps(p, 1.f / p.dx, 1.f / p.dy, 1.f / p.dz, c.ipx, c.ipy,
+                                              c.ipz, c.cd, cdu, A.step);
+                --r;
+            } else {
+                if (c.pg == -1) return samples;  // page fault: resume in the next march pass
+                float qx[U], qy[U], qz[U], v[U];
+                int n = 1;
+                qx[0] = p.ox;
+                qy[0] = p.oy;
+                qz[0] = p.oz;
+                if constexpr (U == 1) {
+                    v[0] = sample_brick<PC, DT, PADDED>(c.br, V.P, lx, ly, lz, S.lut);
+                } else {
+                    Footprint fp[U];
+                    fp[0] = footprint<PC, false>(V, c.br, lx, ly, lz);
+                    bool ok = true;
+#pragma unroll
+                    for (int u = 1; u < U; ++u) {
+                        qx[u] = qx[u - 1] + sx;
+                        qy[u] = qy[u - 1] + sy;
+                        qz[u] = qz[u - 1] + sz;
+                        float ux = qx[u] - c.ipx, uy = qy[u] - c.ipy, uz = qz[u] - c.ipz;
+                        ok = ok & unit_interval(ux) & unit_interval(uy) & unit_interval(uz) &
+                             (p.nsteps > u);
+                        ux = ok ? ux : lx;
+                        uy = ok ? uy : ly;
+                        uz = ok ? uz : lz;
+                        n += ok;
+                        fp[u] = footprint<PC, false>(V, c.br, ux, uy, uz);
+                    }
+                    fetch_loads<U, PC, DT>(V, c.br, fp, v);
+                }
+                // the first of them that crosses, or the last
+                int taken = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (u < n && !hit) {
+                        value = v[u];
+                        p.ox = qx[u];
+                        p.oy = qy[u];
+                        p.oz = qz[u];
+                        taken = u + 1;
+                        hit = prev_sign < 0.f   ? !(value < iso)
+                              : prev_sign > 0.f ? !(value > iso)
+                                                : (value < iso || value > iso);
+                    }
+                samples += unsigned(taken);
+                p.nsteps -= taken - 1;
+                if (hit) break;
+                r -= U;
+            }
+            p.ox = p.ox + sx;
+            p.oy = p.oy + sy;
+            p.oz = p.oz + sz;
+            p.nsteps -= 1;
+        } while (p.nsteps > 0 && r > 0);
     }
+    if (!hit) return samples;
+    const BrickRef &br = c.br;
+    const float dt = A.step;
+    p.vx = A.surface[0];
+    p.vy = A.surface[1];
+    p.vz = A.surface[2];
+    p.vw = 1.f;
+    const float a = (iso - prev_value) / (value - prev_value);
+    const float qx = p.ox - dt * p.dx, qy = p.oy - dt * p.dy, qz = p.oz - dt * p.dz;
+    const float ia = 1.f - a;
+    const float ipx2 = ia * qx + a * p.ox, ipy2 = ia * qy + a * p.oy, ipz2 = ia * qz + a * p.oz;
+    // central difference in brick-local coordinates, dt = du * 2
+    const float lx = ipx2 - c.ipx, ly = ipy2 - c.ipy, lz = ipz2 - c.ipz;
+    const float g = A.du * 2.f;
+    float nnx = sample_brick<0, DT>(br, V.P, lx - g, ly - 0.f, lz - 0.f, S.lut) -
+                sample_brick<0, DT>(br, V.P, lx + g, ly + 0.f, lz + 0.f, S.lut);
+    float nny = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - g, lz - 0.f, S.lut) -
+                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + g, lz + 0.f, S.lut);
+    float nnz = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - 0.f, lz - g, S.lut) -
+                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + 0.f, lz + g, S.lut);
+    samples += 6;
+    float wx, wy, wz, nx, ny, nz;
+    mat_vec4(A.to_world, ipx2, ipy2, ipz2, 1.f, wx, wy, wz);
+    mat_vec4(A.to_world, nnx, nny, nnz, 0.f, nx, ny, nz);
+    normalize3(nx, ny, nz);
+    float lx2 = Vw.light[0] - wx, ly2 = Vw.light[1] - wy, lz2 = Vw.light[2] - wz;
+    normalize3(lx2, ly2, lz2);
+    float hx = lx2 - wx, hy = ly2 - wy, hz = lz2 - wz;
+    normalize3(hx, hy, hz);
+    const float ambient = 0.2f;
+    const float diffuse = .6f * fclamp(lx2 * nx + ly2 * ny + lz2 * nz, 0.f, 1.f);
+    const float specular = .2f * powf(fclamp(hx * nx + hy * ny + hz * nz, 0.f, 1.f), 100.f);
+    const float ex = wx - Vw.eye[0], ey = wy - Vw.eye[1], ez = wz - Vw.eye[2];
+    const float distance = sqrtf(ex * ex + ey * ey + ez * ez) / 2.f;
+    if (A.mode == HY_ISO_COLOR) {
+        const float f = ambient + (diffuse + specular) / distance;
+        p.vx = iso_linear_to_srgb(p.vx * f);
+        p.vy = iso_linear_to_srgb(p.vy * f);
+        p.vz = iso_linear_to_srgb(p.vz * f);
+        p.vw = p.vw * f;
+    } else if (A.mode == HY_ISO_POSITION) {
+        p.vx = ipx2 / A.bbox_max[0];
+        p.vy = ipy2 / A.bbox_max[1];
+        p.vz = ipz2 / A.bbox_max[2];
+        p.vw = 1.f;
+    } else {
+        p.vx = nx;
+        p.vy = ny;
+        p.vz = nz;
+        p.vw = 1.f;
+    }
+    const float ddx = p.e0 - p.ox, ddy = p.e1 - p.oy, ddz = p.e2 - p.oz;
+    p.e3 = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
+    p.nsteps = 0;
     return samples;
 }
 
@@ -1353,7 +1408,7 @@ __device__ __forceinline__ long long run_main(Px &p, const ShadeArgs &A, const V
         return volume_main<PC, DT, PADDED, LEAN, GATHER, LOOP>(p, A, S);
     if (SHADER == HY_SHADER_BLOCKS) return blocks_main(p, A);
     if (SHADER == HY_SHADER_PAGING) return paging_main(p, A);
-    return iso_main<PC, DT, PADDED>(p, A, Vw, S);
+    return iso_main<LOOP == kLoopBatch2 ? 2 : LOOP == kLoopBatch4 ? 4 : 1, PC, DT, PADDED>(p, A, Vw, S);
 }
 
 // Ray generation (cuda_shading.cu:24-29 == cpu_shading.cc:14-21).
