@@ -112,8 +112,8 @@ __device__ __forceinline__ unsigned int shade_batch_unit(const BatchArgs &B, con
         gen_ray(bv.view, u.x, u.y, ox, oy, oz, dx, dy, dz);
         if (COMPOSITE) {
             float4 aux;
-            samples = unsigned(composite_ray<SHADER, PC, DT, PADDED, GATHER>(A, bv.view, S, ox, oy, oz, dx,
-                                                                    dy, dz, v, aux));
+            samples = unsigned(composite_ray<SHADER, PC, DT, PADDED, GATHER, LOOP>(
+                A, bv.view, S, ox, oy, oz, dx, dy, dz, v, aux));
         } else {
             Px p;
             samples = unsigned(emit<SHADER, PC, DT, PADDED, LEAN, GATHER, LOOP>(
@@ -195,12 +195,13 @@ __device__ __forceinline__ void batch_body(const BatchArgs &B) {
 #ifndef HY_BATCH_COMPOSITE_GATHER_MIN_BLOCKS
 #define HY_BATCH_COMPOSITE_GATHER_MIN_BLOCKS 5
 #endif
-template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE, int GATHER = 0>
+template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE, int GATHER = 0,
+          int LOOP = kLoopOne>
 __global__ void __launch_bounds__(kMaxBlockThreads,
                                   (COMPOSITE && GATHER) ? HY_BATCH_COMPOSITE_GATHER_MIN_BLOCKS
                                                         : HY_BATCH_MIN_BLOCKS)
     batch_kernel(const __grid_constant__ BatchArgs B) {
-    batch_body<SHADER, PC, DT, PADDED, COMPOSITE, false, GATHER>(B);
+    batch_body<SHADER, PC, DT, PADDED, COMPOSITE, false, GATHER, LOOP>(B);
 }
 
 // The lean march over u8 bricks with an apron holds its state in 56
@@ -238,12 +239,13 @@ __global__ void __maxnreg__((lean_regs<DT, PADDED, GATHER, LOOP>()))
 
 // The lean march's samples in flight (volume_batches), where steps_per_iter
 // leaves it open: four (128 registers) for a batch of fewer than 8 warps of
-// rays a scheduler, which is bound by latency; else two at 64 registers, for
-// bricks of 32 voxels and more: 16 views of the 1024^3 volume 25.6 ms against
-// 25.7 with one at 48 registers (26.5 for two at 72 or 80, 29.9 for four at
-// 96), 11 views of a 99x213x412 volume 887 against 946 us, 9 views of 128^3
-// bricks 157 against 175; with 16^3 bricks a batch ends at a brick face
-// after a few steps and one sample at a time is faster (526 against 558 us).
+// rays a scheduler, which is bound by latency; else two at 64 registers where
+// cells are free of effect and bricks have 32 voxels and more: 16 views of
+// the 1024^3 volume 25.6 ms against 25.7 with one at 48 registers (26.5 for
+// two at 72 or 80, 29.9 for four at 96), 11 views of a 99x213x412 volume 887
+// against 946 us; with 16^3 bricks a batch ends at a brick face after a few
+// steps and one at a time is faster (526 against 558 us), and with no free
+// cells as well (24 views of 512^3 tubes 1458 against 1643 us).
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
 const void *pick_lean(const ShadeArgs &a, int steps_per_iter, long long rays) {
     if (a.ert > 0.f)
@@ -254,10 +256,15 @@ const void *pick_lean(const ShadeArgs &a, int steps_per_iter, long long rays) {
             if (steps_per_iter == 0 && rays < 8 * 32ll * a.schedulers)
                 return reinterpret_cast<const void *>(
                     &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopBatch4>);
-            if (steps_per_iter == 2 || a.vol.P >= 34)
+                        if (steps_per_iter == 2 || (steps_per_iter == 0 && a.skip.d && a.vol.P >= 34))
                 return reinterpret_cast<const void *>(
                     &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopBatch2>);
         }
+    }
+    if constexpr (PADDED) {
+        if (a.skip.d)
+            return reinterpret_cast<const void *>(
+                &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopSkip>);
     }
     return reinterpret_cast<const void *>(&batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopOne>);
 }
@@ -268,7 +275,15 @@ const void *pick_c(const ShadeArgs &a, int steps_per_iter, long long rays) {
         // the Volume shader's per-brick segments sample by gathers too
         if constexpr (SHADER == HY_SHADER_VOLUME && DT == HY_DTYPE_U8 && PADDED) {
             if (a.vol.tex && HY_BATCH_COMPOSITE_GATHER)
-                return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, PADDED, 1, true>);
+                return a.skip.d ? reinterpret_cast<const void *>(
+                                      &batch_kernel<SHADER, PC, DT, PADDED, 1, true, kLoopSkip>)
+                                : reinterpret_cast<const void *>(
+                                      &batch_kernel<SHADER, PC, DT, PADDED, 1, true>);
+        }
+        if constexpr (SHADER == HY_SHADER_VOLUME && PADDED) {
+            if (a.skip.d)
+                return reinterpret_cast<const void *>(
+                    &batch_kernel<SHADER, PC, DT, PADDED, 1, false, kLoopSkip>);
         }
         return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, PADDED, 1>);
     }
@@ -454,14 +469,15 @@ int launch(hy_batch *b, uint8_t *out) {
         int rc = layout(b);
         if (rc) return rc;
     }
-    // the skip grid follows the knots; a launch that gains or loses it is a
-    // new graph
+    // the skip grid follows the knots; a batch that gains or loses it is
+    // another kernel and graph
     SkipGrid skip;
     int rc = hy_skip_view(ctx, b->vol, &b->params, &skip);
     if (rc) return rc;
     if (skip.d != b->base.skip.d) {
         b->base.skip = skip;
-        drop_graph(b);
+        rc = layout(b);
+        if (rc) return rc;
     }
     const int count = b->params.count_samples ? 1 : 0;
     if (!b->exec || b->graph_out != out || b->graph_count != count) {
@@ -532,6 +548,8 @@ extern "C" int hy_batch_create(hy_ctx *ctx, const hy_volume *vol, const hy_shade
             return hy_fail(ctx, HY_ERR_INVALID, "batch: bad view size or output offset");
     }
     HY_CUDA(ctx, cudaSetDevice(ctx->device));
+    rc = hy_skip_view(ctx, vol, params, &base.skip);
+    if (rc) return rc;
     hy_batch *b = new hy_batch();
     b->ctx = ctx;
     b->vol = vol;

@@ -190,6 +190,11 @@ struct hy_skip {
     unsigned char *grid[2] = {nullptr, nullptr};
     bool valid[2] = {false, false};
     hy_skip_ranges key[2];
+    // how many cells have their smallest voxel in value bin i or above and
+    // their largest in bin j or below (kSkipBins^2), and the cells that are
+    // sampled at all
+    std::vector<int> hist;
+    long long sampled = 0;
 };
 
 struct hy_volume {

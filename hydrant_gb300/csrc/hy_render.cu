@@ -67,7 +67,8 @@ __device__ __forceinline__ void render_body(const ShadeArgs &A) {
         float4 v, aux;
         if (COMPOSITE) {
             samples = unsigned(
-                composite_ray<SHADER, PC, DT, PADDED, GATHER>(A, A.view, S, ox, oy, oz, dx, dy, dz, v, aux));
+                composite_ray<SHADER, PC, DT, PADDED, GATHER, LOOP>(A, A.view, S, ox, oy, oz, dx, dy,
+                                                                  dz, v, aux));
         } else {
             Px p;
             samples = unsigned(emit<SHADER, PC, DT, PADDED, LEAN, GATHER, LOOP>(
@@ -95,9 +96,9 @@ __device__ __forceinline__ void render_body(const ShadeArgs &A) {
     count_samples(A, samples);
 }
 
-template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE>
+template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE, int LOOP = kLoopOne>
 __global__ void __launch_bounds__(kThreads) render_kernel(const __grid_constant__ ShadeArgs A) {
-    render_body<SHADER, PC, DT, PADDED, COMPOSITE, false>(A);
+    render_body<SHADER, PC, DT, PADDED, COMPOSITE, false, false, LOOP>(A);
 }
 
 // The Isosurface march with 2 or 4 samples in flight (80 and 128 registers).
@@ -125,8 +126,8 @@ __global__ void HY_RENDER_LEAN_BOUNDS render_lean_kernel(const __grid_constant__
     render_body<SHADER, PC, DT, PADDED, 0, true, false, LOOP>(A);
 }
 // The same march sampling by texture gathers (u8 bricks with an apron in
-// the volume's gather textures), one sample at a time, for early termination
-// and for paged caches: 64-view step, one launch per view, 169.6 ms at 48
+// the volume's gather textures), one sample at a time, for large views with
+// nothing to pass over, early termination and paged caches: 64-view step, one launch per view, 169.6 ms at 48
 // registers against 172.4 at 56, 173.1 at 64 and 198.8 for the loads
 // (HY_RENDER_GATHER=0 builds the per-view path without gathers).
 #ifndef HY_RENDER_GATHER
@@ -192,10 +193,10 @@ __global__ void __launch_bounds__(kThreads) render_group_kernel(const __grid_con
 // Volume 147 -> 163 and Isosurface 231 -> 237 Gsamples/s against 80
 // registers and 6 blocks unbounded (Blocks is 3 % faster unbounded and keeps
 // render_kernel).
-template <int SHADER, int PC, int DT, bool PADDED>
+template <int SHADER, int PC, int DT, bool PADDED, int LOOP = kLoopOne>
 __global__ void __launch_bounds__(kThreads, 8)
     render_composite_kernel(const __grid_constant__ ShadeArgs A) {
-    render_body<SHADER, PC, DT, PADDED, 1, false>(A);
+    render_body<SHADER, PC, DT, PADDED, 1, false, false, LOOP>(A);
 }
 // The Volume shader's per-brick compositing sampling by gathers (u8 bricks
 // with an apron), 64 registers (8 blocks): 64-view step of per-view launches
@@ -206,10 +207,10 @@ __global__ void __launch_bounds__(kThreads, 8)
 #ifndef HY_RENDER_COMPOSITE_GATHER_BLOCKS
 #define HY_RENDER_COMPOSITE_GATHER_BLOCKS 8
 #endif
-template <int SHADER, int PC, int DT, bool PADDED>
+template <int SHADER, int PC, int DT, bool PADDED, int LOOP>
 __global__ void __launch_bounds__(kThreads, HY_RENDER_COMPOSITE_GATHER_BLOCKS)
     render_composite_gather_kernel(const __grid_constant__ ShadeArgs A) {
-    render_body<SHADER, PC, DT, PADDED, 1, false, true>(A);
+    render_body<SHADER, PC, DT, PADDED, 1, false, true, LOOP>(A);
 }
 
 // ---- reference-layout film passes ------------------------------------------
@@ -369,12 +370,14 @@ void launch_group(const ShadeArgs &a, cudaStream_t s) {
 // The lean march of one view in the form its size wants, by the warps (of 32
 // rays) a scheduler would get.  u8 by gathers, 1-voxel steps, us at 0.8, 3.4,
 // 13.5 and 54 warps (256^3, 512^3, 512^3, 512^3 blobs at 128^2, 256^2, 512^2,
-// 1024^2): 8 lanes a ray 65, 244, 783, 2871; 4 samples in flight 97, 196, 363,
-// 1100; 2 in flight 112, 247, 323, 904; one sample at a time 163, 361, 364, 941
-// (the last column row with boxes on all sides).  f32 (200^3, quarter-voxel
-// steps): 97, 155, 449, 1643; 163, 169, 230, 587; 191, 198, 248, 526; 288, 286,
-// 311, 581.  Without an apron only the group and the plain march are built:
-// 83, 228, 738 against 233, 235, 400.
+// 1024^2), half the cells free of effect: 8 lanes a ray 65, 244, 783, 2871; 4
+// samples in flight 97, 196, 363, 1100; 2 in flight 112, 247, 323, 904; one at
+// a time 163, 361, 364, 941 (without the skip grid 163, 479, 491, 1336).  No
+// free cells: 63, 297, 1017, 3867; 83, 208, 483, 1571; 106, 281, 436, 1328; 163,
+// 425, 443, 1293.  f32 (200^3, quarter-voxel steps, free cells): 97, 155, 449,
+// 1643; 163, 169, 230, 587; 191, 198, 248, 526; 288, 286, 311, 581.  Without an
+// apron only the group and the plain march are built: 83, 228, 738 against
+// 230, 231, 392.
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
 void launch_lean(const ShadeArgs &a, cudaStream_t s) {
     const dim3 g = grid_of(a);
@@ -399,25 +402,40 @@ void launch_lean(const ShadeArgs &a, cudaStream_t s) {
     }
     if (rays < 8 * per_warp)
         render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
-    else
+    else if (a.skip.d || rays < 24 * per_warp)
         render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch2><<<g, kThreads, sm, s>>>(a);
+    else if constexpr (GATHER != 0)
+        render_lean_gather_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopOne><<<g, kThreads, sm, s>>>(a);
+    else
+        render_lean_kernel<SHADER, PC, DT, PADDED, kLoopOne><<<g, kThreads, sm, s>>>(a);
 }
 
 template <int SHADER, int PC, int DT, bool PADDED>
 void launch_fused(const ShadeArgs &a, cudaStream_t s) {
+    const dim3 g = grid_of(a);
+    const size_t sm = smem_bytes(a);
     if (a.composite) {
+        if constexpr (SHADER == HY_SHADER_VOLUME && PADDED) {
+            if constexpr (HY_RENDER_COMPOSITE_GATHER && DT == HY_DTYPE_U8) {
+                if (a.vol.tex) {
+                    if (a.skip.d)
+                        render_composite_gather_kernel<SHADER, PC, DT, PADDED, kLoopSkip>
+                            <<<g, kThreads, sm, s>>>(a);
+                    else
+                        render_composite_gather_kernel<SHADER, PC, DT, PADDED, kLoopOne>
+                            <<<g, kThreads, sm, s>>>(a);
+                    return;
+                }
+            }
+            if (a.skip.d) {
+                render_composite_kernel<SHADER, PC, DT, PADDED, kLoopSkip><<<g, kThreads, sm, s>>>(a);
+                return;
+            }
+        }
         if constexpr (SHADER == HY_SHADER_BLOCKS)
-            render_kernel<SHADER, PC, DT, PADDED, 1><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
-        else if constexpr (HY_RENDER_COMPOSITE_GATHER && SHADER == HY_SHADER_VOLUME &&
-                           DT == HY_DTYPE_U8 && PADDED) {
-            if (a.vol.tex)
-                render_composite_gather_kernel<SHADER, PC, DT, PADDED>
-                    <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
-            else
-                render_composite_kernel<SHADER, PC, DT, PADDED>
-                    <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
-        } else
-            render_composite_kernel<SHADER, PC, DT, PADDED><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+            render_kernel<SHADER, PC, DT, PADDED, 1><<<g, kThreads, sm, s>>>(a);
+        else
+            render_composite_kernel<SHADER, PC, DT, PADDED><<<g, kThreads, sm, s>>>(a);
         return;
     }
     if constexpr (SHADER == HY_SHADER_VOLUME) {
@@ -426,10 +444,10 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
                 if (a.vol.paged_gather) {  // a pager's cache in gather textures
                     if (a.ert > 0.f)
                         render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherPaged, kLoopErt>
-                            <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+                            <<<g, kThreads, sm, s>>>(a);
                     else
                         render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherPaged, kLoopOne>
-                            <<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+                            <<<g, kThreads, sm, s>>>(a);
                     return;
                 }
             }
@@ -451,13 +469,19 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
         const long long rays = (long long)a.view.W * a.view.H, per_warp = 32ll * a.schedulers;
         if (rays < 24 * per_warp && a.vol.P <= kMaxBatchesP) {
             if (rays < 8 * per_warp)
-                render_iso_kernel<PC, DT, kLoopBatch4><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+                render_iso_kernel<PC, DT, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
             else
-                render_iso_kernel<PC, DT, kLoopBatch2><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+                render_iso_kernel<PC, DT, kLoopBatch2><<<g, kThreads, sm, s>>>(a);
             return;
         }
     }
-    render_kernel<SHADER, PC, DT, PADDED, 0><<<grid_of(a), kThreads, smem_bytes(a), s>>>(a);
+    if constexpr (SHADER == HY_SHADER_VOLUME && PADDED) {
+        if (a.skip.d) {
+            render_kernel<SHADER, PC, DT, PADDED, 0, kLoopSkip><<<g, kThreads, sm, s>>>(a);
+            return;
+        }
+    }
+    render_kernel<SHADER, PC, DT, PADDED, 0><<<g, kThreads, sm, s>>>(a);
 }
 
 // Instantiations: Blocks reads no bricks; u8 volumes with a 1-voxel apron and

@@ -868,19 +868,17 @@ struct VolumeMarch {
 //            alone stopping would not free its warp).  A lane stops only when
 //            its own ray is that opaque, whichever lanes vote with it, so what
 //            it leaves out adds at most 1 - A.ert per channel;
+//  kLoopSkip the steps of kLoopOne, with the samples without effect passed
+//            over (skip_free).  Kept apart: with nothing to pass over the
+//            looks and their registers cost the march 3 to 5 %;
 //  kLoopBatch2, kLoopBatch4  volume_batches with 2 or 4 samples in flight.
-constexpr int kLoopOne = 0, kLoopErt = 1, kLoopBatch2 = 2, kLoopBatch4 = 4;
+constexpr int kLoopOne = 0, kLoopErt = 1, kLoopSkip = 3, kLoopBatch2 = 2, kLoopBatch4 = 4;
 template <int PC, int DT, bool PADDED, bool LEAN = false, int GATHER = 0, int LOOP = kLoopOne>
 __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, const Shared &S) {
     unsigned int samples = 0;
     VolumeMarch m;
     m.init(p, A.step);
-    if constexpr (LOOP == kLoopErt) {
-        while (p.nsteps > 0) {
-            if (!m.step<PC, DT, PADDED, LEAN, GATHER>(p, A, S, samples)) break;
-            if (__all_sync(__activemask(), p.vw >= A.ert)) break;
-        }
-    } else {
+    if constexpr (LOOP == kLoopSkip) {
         bool go = true;
         int hint = A.skip.d != nullptr;
         while (go && p.nsteps > 0) {
@@ -893,6 +891,11 @@ __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, cons
             do {
                 go = m.step<PC, DT, PADDED, LEAN, GATHER>(p, A, S, samples);
             } while (go && p.nsteps > 0 && --r > 0);
+        }
+    } else {
+        while (p.nsteps > 0) {
+            if (!m.step<PC, DT, PADDED, LEAN, GATHER>(p, A, S, samples)) break;
+            if (LOOP == kLoopErt && __all_sync(__activemask(), p.vw >= A.ert)) break;
         }
     }
     return samples;
@@ -1497,7 +1500,7 @@ __device__ __forceinline__ float vol_linear_to_srgb(float x) {  // volume.cc:175
 // per-partition bbox of dbuf_renderer.hpp:38-40) and the partials are
 // composited front to back with volume.cc:267-280 (Volume),
 // isosurface.cc:272-290 (depth-min, Isosurface) or the over operator (Blocks).
-template <int SHADER, int PC, int DT, bool PADDED, int GATHER = 0>
+template <int SHADER, int PC, int DT, bool PADDED, int GATHER = 0, int LOOP = kLoopOne>
 __device__ __forceinline__ long long composite_ray(const ShadeArgs &A, const ViewArgs &Vw,
                                                    const Shared &S, float ox,
                                                    float oy, float oz, float dx, float dy,
@@ -1547,9 +1550,8 @@ __device__ __forceinline__ long long composite_ray(const ShadeArgs &A, const Vie
         if (__ldg(&V.info[bid].x) == 0) {
             const float bx = float(cell[0]), by = float(cell[1]), bz = float(cell[2]);
             Px p;
-            samples += emit<SHADER, PC, DT, PADDED, false, GATHER>(p, A, Vw, S, ox, oy, oz, dx, dy, dz,
-                                                                   bx, by, bz, bx + 1.f, by + 1.f,
-                                                                   bz + 1.f);
+            samples += emit<SHADER, PC, DT, PADDED, false, GATHER, LOOP>(
+                p, A, Vw, S, ox, oy, oz, dx, dy, dz, bx, by, bz, bx + 1.f, by + 1.f, bz + 1.f);
             if (SHADER == HY_SHADER_VOLUME) {
                 if (first) {
                     acc = make_float4(p.vx, p.vy, p.vz, p.vw);

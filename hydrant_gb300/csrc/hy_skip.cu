@@ -103,6 +103,31 @@ __global__ void cell_minmax_kernel(const __grid_constant__ CellArgs a, MinMax<T>
     }
 }
 
+// Value bins of the cells' min/max histogram: 64 over [0, 1], the outer ones
+// open (a u8 voxel u is u / 255).
+constexpr int kBins = 64;
+__device__ __forceinline__ int value_bin(float v) {
+    return min(max(int(v * float(kBins)), 0), kBins - 1);
+}
+
+// hist[i][j]: cells with smallest voxel in bin i and largest in bin j.
+template <typename T>
+__global__ void cell_hist_kernel(const MinMax<T> *__restrict__ mm, long long n, float scale,
+                                 int *__restrict__ hist) {
+    __shared__ int h[kBins * kBins];
+    for (int i = threadIdx.x; i < kBins * kBins; i += blockDim.x) h[i] = 0;
+    __syncthreads();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const MinMax<T> m = mm[i];
+        if (!(m.lo > m.hi))
+            atomicAdd(&h[value_bin(float(m.lo) * scale) * kBins + value_bin(float(m.hi) * scale)], 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kBins * kBins; i += blockDim.x)
+        if (h[i]) atomicAdd(&hist[i], h[i]);
+}
+
 struct ClassArgs {
     hy_skip_ranges r;
     float scale;  // voxel -> sample value: 1/255 (u8) or 1
@@ -173,6 +198,58 @@ int classify(hy_volume *v, const hy_skip_ranges &r, unsigned char *grid) {
     return HY_OK;
 }
 
+// The cells' histogram on the host, summed so that hist[i * kBins + j] counts
+// the cells with lo in bin >= i and hi in bin <= j.
+template <typename T>
+int cell_hist(hy_volume *v) {
+    hy_ctx *ctx = v->ctx;
+    hy_skip &s = v->skip;
+    int *dev = reinterpret_cast<int *>(s.grid[0]);  // 16 KB of the grids, unused until a render
+    int *own = nullptr;
+    if (s.cells * 8 < (long long)(sizeof(int) * kBins * kBins)) {
+        HY_CUDA(ctx, cudaMalloc(&own, sizeof(int) * kBins * kBins));
+        dev = own;
+    }
+    s.hist.assign(kBins * kBins, 0);
+    cudaError_t e = cudaMemsetAsync(dev, 0, sizeof(int) * kBins * kBins, ctx->stream);
+    if (e == cudaSuccess) {
+        const unsigned blocks = unsigned(std::min<long long>((s.cells + 255) / 256, 4 * ctx->sms));
+        cell_hist_kernel<T><<<blocks, 256, 0, ctx->stream>>>(
+            static_cast<const MinMax<T> *>(s.minmax), s.cells, sizeof(T) == 1 ? 1.f / 255.f : 1.f, dev);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(s.hist.data(), dev, sizeof(int) * kBins * kBins, cudaMemcpyDeviceToHost,
+                            ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (own) cudaFree(own);
+    if (e != cudaSuccess) return hy_cuda_fail(ctx, e, "volume: skip grid");
+    for (int i = kBins - 1; i >= 0; --i)
+        for (int j = 0; j < kBins; ++j) {
+            int &h = s.hist[i * kBins + j];
+            h += (i + 1 < kBins ? s.hist[(i + 1) * kBins + j] : 0) +
+                 (j > 0 ? s.hist[i * kBins + j - 1] : 0) -
+                 (i + 1 < kBins && j > 0 ? s.hist[(i + 1) * kBins + j - 1] : 0);
+        }
+    s.sampled = s.hist[kBins - 1];
+    return HY_OK;
+}
+
+// Cells free of effect for these ranges, to a value bin's width and no more
+// than there are.
+long long free_cells(const hy_skip &s, const hy_skip_ranges &r) {
+    long long n = 0;
+    for (int k = 0; k < r.n; ++k) {
+        // the bins that lie in the range (the outer ones are open)
+        const float lo = std::ceil(std::max(r.lo[k], 0.f) * kBins);
+        const float hi = std::floor(std::min(r.hi[k], 1.f) * kBins) - 1.f;
+        const int i = int(std::min(std::max(lo, 0.f), float(kBins)));
+        const int j = int(std::min(std::max(hi, -1.f), float(kBins - 1)));
+        if (i < kBins && j >= i) n += s.hist[i * kBins + j];
+    }
+    return n;
+}
+
 bool same_ranges(const hy_skip_ranges &a, const hy_skip_ranges &b) {
     return a.n == b.n && std::memcmp(a.lo, b.lo, sizeof(float) * a.n) == 0 &&
            std::memcmp(a.hi, b.hi, sizeof(float) * a.n) == 0;
@@ -236,7 +313,7 @@ int hy_skip_build(hy_volume *v) {
         cell_minmax_kernel<float><<<v->nbricks, threads, 0, ctx->stream>>>(
             a, static_cast<MinMax<float> *>(s.minmax));
     HY_CUDA(ctx, cudaGetLastError());
-    return HY_OK;
+    return u8 ? cell_hist<unsigned char>(v) : cell_hist<float>(v);
 }
 
 // The value ranges in which a sample leaves a Volume march as it is: between
@@ -296,6 +373,10 @@ int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy
             return HY_OK;
         which = 0;
         r = ctx->tf_ranges;
+        // With less than a tenth of the cells free the looks cost more than
+        // the samples passed over: a march without a free cell takes 3 to 5 %
+        // longer with the grid than without.
+        if (free_cells(s, r) * 10 < s.sampled) return HY_OK;
     } else if (p->shader == HY_SHADER_ISOSURFACE) {
         // crossed: value and 0 on different sides of the isovalue
         which = 1;
