@@ -299,9 +299,21 @@ const void *pick_c(const ShadeArgs &a, int steps_per_iter, long long rays) {
     return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, PADDED, 0>);
 }
 
+// the Blocks shader's modes
+template <int COMPOSITE>
+const void *pick_blocks(const ShadeArgs &a) {
+    return a.mode == HY_BLOCKS_VOLUME
+               ? reinterpret_cast<const void *>(
+                     &batch_kernel<HY_SHADER_BLOCKS, 0, HY_DTYPE_U8, false, COMPOSITE, 0, kBlocksVolume>)
+               : reinterpret_cast<const void *>(
+                     &batch_kernel<HY_SHADER_BLOCKS, 0, HY_DTYPE_U8, false, COMPOSITE, 0, kBlocksSolid>);
+}
+
 template <int SHADER>
 const void *pick_shader(const ShadeArgs &a, int spi, long long rays) {
-    if constexpr (SHADER == HY_SHADER_BLOCKS || SHADER == HY_SHADER_PAGING) {
+    if constexpr (SHADER == HY_SHADER_BLOCKS) {
+        return a.composite ? pick_blocks<1>(a) : pick_blocks<0>(a);
+    } else if constexpr (SHADER == HY_SHADER_PAGING) {
         return pick_c<SHADER, 0, HY_DTYPE_U8, false>(a, spi, rays);
     } else {
         const bool padded = a.vol.pad > 0;

@@ -432,9 +432,12 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
                 return;
             }
         }
-        if constexpr (SHADER == HY_SHADER_BLOCKS)
-            render_kernel<SHADER, PC, DT, PADDED, 1><<<g, kThreads, sm, s>>>(a);
-        else
+        if constexpr (SHADER == HY_SHADER_BLOCKS) {
+            if (a.mode == HY_BLOCKS_VOLUME)
+                render_kernel<SHADER, PC, DT, PADDED, 1, kBlocksVolume><<<g, kThreads, sm, s>>>(a);
+            else
+                render_kernel<SHADER, PC, DT, PADDED, 1, kBlocksSolid><<<g, kThreads, sm, s>>>(a);
+        } else
             render_composite_kernel<SHADER, PC, DT, PADDED><<<g, kThreads, sm, s>>>(a);
         return;
     }
@@ -481,7 +484,14 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
             return;
         }
     }
-    render_kernel<SHADER, PC, DT, PADDED, 0><<<g, kThreads, sm, s>>>(a);
+    if constexpr (SHADER == HY_SHADER_BLOCKS) {
+        if (a.mode == HY_BLOCKS_VOLUME)
+            render_kernel<SHADER, PC, DT, PADDED, 0, kBlocksVolume><<<g, kThreads, sm, s>>>(a);
+        else
+            render_kernel<SHADER, PC, DT, PADDED, 0, kBlocksSolid><<<g, kThreads, sm, s>>>(a);
+    } else {
+        render_kernel<SHADER, PC, DT, PADDED, 0><<<g, kThreads, sm, s>>>(a);
+    }
 }
 
 // Instantiations: Blocks reads no bricks; u8 volumes with a 1-voxel apron and

@@ -873,6 +873,8 @@ struct VolumeMarch {
 //            looks and their registers cost the march 3 to 5 %;
 //  kLoopBatch2, kLoopBatch4  volume_batches with 2 or 4 samples in flight.
 constexpr int kLoopOne = 0, kLoopErt = 1, kLoopSkip = 3, kLoopBatch2 = 2, kLoopBatch4 = 4;
+// the Blocks shader's modes, each in its own kernel (fewer registers)
+constexpr int kBlocksVolume = 5, kBlocksSolid = 6;
 template <int PC, int DT, bool PADDED, bool LEAN = false, int GATHER = 0, int LOOP = kLoopOne>
 __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, const Shared &S) {
     unsigned int samples = 0;
@@ -1137,52 +1139,133 @@ __device__ __forceinline__ unsigned int volume_group(Px &p, bool on, const Shade
     return samples;
 }
 
-// VisBlocksShaderKernel::main (blocks_shader.cu:16-50).
-__device__ __forceinline__ long long blocks_main(Px &p, const ShadeArgs &A) {
+// VisBlocksShaderKernel::main (blocks_shader.cu:16-50), Solid mode: the first
+// brick that is not empty colours the ray.
+__device__ __forceinline__ long long blocks_solid(Px &p, const ShadeArgs &A) {
     const DevVolume &V = A.vol;
-    long long samples = 0;
     const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
     const float rx = 1.f / p.dx, ry = 1.f / p.dy, rz = 1.f / p.dz;
-    const float opacity_threshold = 0.95f;
     const float hx = A.bbox_max[0] - 1.f, hy = A.bbox_max[1] - 1.f, hz = A.bbox_max[2] - 1.f;
     const float ex = A.bbox_max[0] - 0.f, ey = A.bbox_max[1] - 0.f, ez = A.bbox_max[2] - 0.f;
     const float sx = p.dx * A.step, sy = p.dy * A.step, sz = p.dz * A.step;
     while (p.nsteps > 0) {
-        float ipx = floorf(p.ox), ipy = floorf(p.oy), ipz = floorf(p.oz);
-        int bid = thumb_index(V, ipx, ipy, ipz);
-        int cd = __ldg(&V.info[bid].x);
-        if (cd) {
-            p.nsteps -= skip_nblock_steps(p, rx, ry, rz, ipx, ipy, ipz, cd, cdu, A.step);
-        } else {
-            float rpx = fclamp(ipx, 0.f, hx) / ex, rpy = fclamp(ipy, 0.f, hy) / ey,
-                  rpz = fclamp(ipz, 0.f, hz) / ez;
-            ++samples;
-            if (A.mode == HY_BLOCKS_VOLUME) {
-                const float mean = __ldg(&V.mean[bid]);
-                const float cx = rpx * A.density * mean, cy = rpy * A.density * mean,
-                            cz = rpz * A.density * mean, cw = 1.f * A.density * mean;
-                const float t = 1.f - p.vw;
-                p.vx = p.vx + cx * t;
-                p.vy = p.vy + cy * t;
-                p.vz = p.vz + cz * t;
-                p.vw = p.vw + cw * t;
-                if (p.vw > opacity_threshold) {
-                    p.nsteps = 0;
-                    break;
-                }
-            } else {
-                p.vx = rpx;
-                p.vy = rpy;
-                p.vz = rpz;
-                p.vw = 1.f;
-                p.nsteps = 0;
-                break;
-            }
+        const float ipx = floorf(p.ox), ipy = floorf(p.oy), ipz = floorf(p.oz);
+        const int cd = __ldg(&V.info[thumb_index(V, ipx, ipy, ipz)].x);
+        if (!cd) {
+            p.vx = fclamp(ipx, 0.f, hx) / ex;
+            p.vy = fclamp(ipy, 0.f, hy) / ey;
+            p.vz = fclamp(ipz, 0.f, hz) / ez;
+            p.vw = 1.f;
+            p.nsteps = 0;
+            return 1;
         }
+        p.nsteps -= skip_nblock_steps(p, rx, ry, rz, ipx, ipy, ipz, cd, cdu, A.step);
         p.ox = p.ox + sx;
         p.oy = p.oy + sy;
         p.oz = p.oz + sz;
         p.nsteps -= 1;
+    }
+    return 0;
+}
+
+// The same in Volume mode.  A brick has one colour, so its lookups (page
+// table, mean) and the three divisions of its colour are made once per brick;
+// how many steps certainly stay in it follows from the nearest face
+// (approximate division, the brick shrunk by more than the steps' roundings,
+// as in skip_free), and those take only the compositing and the position's
+// additions, four at a time.  At most 32 steps before the warp's rays look at
+// their bricks again together: with runs to the face (up to 127) the rays that
+// reach theirs wait for the others.  512^3 tubes, 1024^2, composited / in one
+// march: 6.88 / 6.05 ms with the lookups on every step, 1.76 / 2.21 once per
+// brick, 1.57 / 1.91 four steps at a time, 1.30 / 1.54 in runs of 32 (1.39 /
+// 1.72 of 64, 1.34 / 1.50 of 16); at 128^2 1.62 / 1.05 ms and now 0.15 / 0.16.
+// Bound by issue: some 14 instructions a step.
+__device__ __forceinline__ long long blocks_volume(Px &p, const ShadeArgs &A) {
+    const DevVolume &V = A.vol;
+    unsigned int samples = 0;
+    const float opacity_threshold = 0.95f;
+    const float hx = A.bbox_max[0] - 1.f, hy = A.bbox_max[1] - 1.f, hz = A.bbox_max[2] - 1.f;
+    const float ex = A.bbox_max[0] - 0.f, ey = A.bbox_max[1] - 0.f, ez = A.bbox_max[2] - 0.f;
+    const float sx = p.dx * A.step, sy = p.dy * A.step, sz = p.dz * A.step;
+    // 128 roundings of an ulp of the largest coordinate, and the division's
+    SkipGrid box;
+    box.cell = 1.f;
+    box.shrink = (fmaxf(fmaxf(V.gmx, V.gmy), V.gmz) + 2.f) * 1.6e-5f + 4e-6f;
+    float ipx = __int_as_float(0x7f800000), ipy = ipx, ipz = ipx;
+    int cd = 0;
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+    while (p.nsteps > 0) {
+        const float fx = floorf(p.ox), fy = floorf(p.oy), fz = floorf(p.oz);
+        if (!(fx == ipx && fy == ipy && fz == ipz)) {  // another brick (or NaN)
+            ipx = fx;
+            ipy = fy;
+            ipz = fz;
+            const int bid = thumb_index(V, ipx, ipy, ipz);
+            cd = __ldg(&V.info[bid].x);
+            if (!cd) {
+                const float rpx = fclamp(ipx, 0.f, hx) / ex, rpy = fclamp(ipy, 0.f, hy) / ey,
+                            rpz = fclamp(ipz, 0.f, hz) / ez;
+                const float mean = __ldg(&V.mean[bid]);
+                c = make_float4(rpx * A.density * mean, rpy * A.density * mean,
+                                rpz * A.density * mean, 1.f * A.density * mean);
+            }
+        }
+        if (cd) {
+            const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
+            p.nsteps -= skip_nblock_steps(p, 1.f / p.dx, 1.f / p.dy, 1.f / p.dz, ipx, ipy, ipz, cd,
+                                          cdu, A.step);
+            p.ox = p.ox + sx;
+            p.oy = p.oy + sy;
+            p.oz = p.oz + sz;
+            p.nsteps -= 1;
+            continue;
+        }
+        const float m = fminf(fminf(steps_to_face(p.ox, sx, ipx, 1.f, 0.f, box),
+                                    steps_to_face(p.oy, sy, ipy, 1.f, 0.f, box)),
+                              steps_to_face(p.oz, sz, ipz, 1.f, 0.f, box));
+        const int n = min(1 + int(fminf(fmaxf(m, 0.f), 31.f)), p.nsteps);
+        int i = 0;
+        auto sample = [&]() {
+            const float t = 1.f - p.vw;
+            const float2 txy = mul2(f2(c.x, c.y), f2(t, t)), tzw = mul2(f2(c.z, c.w), f2(t, t));
+            p.vx = __fadd_rn(p.vx, txy.x);
+            p.vy = __fadd_rn(p.vy, txy.y);
+            p.vz = __fadd_rn(p.vz, tzw.x);
+            p.vw = __fadd_rn(p.vw, tzw.y);
+        };
+        auto advance = [&]() {
+            p.ox = p.ox + sx;
+            p.oy = p.oy + sy;
+            p.oz = p.oz + sz;
+        };
+        // Four steps between two looks at the opacity, which does not fall
+        // while 0 <= c.w <= 1: when it passed the threshold among them they
+        // are taken again one by one.
+        if (c.w >= 0.f && c.w <= 1.f) {
+            while (i + 4 <= n) {
+                const Px q = p;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    sample();
+                    advance();
+                }
+                if (p.vw > opacity_threshold) {
+                    p = q;
+                    break;
+                }
+                i += 4;
+            }
+        }
+        for (; i < n; ++i) {
+            sample();
+            if (p.vw > opacity_threshold) {
+                p.nsteps = 0;
+                return samples + unsigned(i + 1);
+            }
+            advance();
+        }
+        samples += unsigned(n);
+        p.nsteps -= n;
     }
     return samples;
 }
@@ -1409,7 +1492,11 @@ __device__ __forceinline__ long long run_main(Px &p, const ShadeArgs &A, const V
         return volume_batches<4, PC, DT, PADDED, GATHER>(p, A, S);
     else if (SHADER == HY_SHADER_VOLUME)
         return volume_main<PC, DT, PADDED, LEAN, GATHER, LOOP>(p, A, S);
-    if (SHADER == HY_SHADER_BLOCKS) return blocks_main(p, A);
+    if (SHADER == HY_SHADER_BLOCKS) {
+        if (LOOP == kBlocksSolid || (LOOP != kBlocksVolume && A.mode != HY_BLOCKS_VOLUME))
+            return blocks_solid(p, A);
+        return blocks_volume(p, A);
+    }
     if (SHADER == HY_SHADER_PAGING) return paging_main(p, A);
     return iso_main<LOOP == kLoopBatch2 ? 2 : LOOP == kLoopBatch4 ? 4 : 1, PC, DT, PADDED>(p, A, Vw, S);
 }

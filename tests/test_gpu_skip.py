@@ -202,3 +202,22 @@ def test_captured_render_follows_the_knots(ctx):
         del g
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("density", [0.0, 1e-3, 0.05, 0.7, 3.0, -0.4])
+@pytest.mark.parametrize("composite", [False, True])
+def test_blocks(ctx, density, composite):
+    """The Blocks march takes a brick's steps in runs: opacities that pass the
+    threshold early, late and never, fall, or leave [0, 1]; rays along the axes;
+    bricks of fewer and of more steps than a run."""
+    for bs, rate in ((8, 0.25), (32, 1.0), (24, 2.0)):
+        c = Case(ctx, voxels("u8", (64, 48, 50)), bs, 1)
+        try:
+            for cam in (camera(), camera("ptu", a=(0.0, 0.0, 2.2)),
+                        camera("ptu", a=(0.1, 0.2, 0.05), target=(1.0, 0.3, 0.2))):
+                check(c, cam, 61, 47, f"{density} bs{bs}", shader="Blocks", mode="Volume",
+                      density=density, sample_rate=rate, composite=composite)
+                check(c, cam, 33, 35, f"solid bs{bs}", shader="Blocks", mode="Solid",
+                      density=density, sample_rate=rate, composite=composite)
+        finally:
+            c.close()
