@@ -20,7 +20,7 @@ CSRC = PKG / "csrc"
 BUILD = PKG / "_build"
 LIB = PKG / "libhydrant_gb300.so"
 
-SOURCES = ["hy_api.cc", "hy_volume.cu", "hy_skip.cu", "hy_render.cu", "hy_batch.cu", "hy_page.cu", "hy_diff.cu",
+SOURCES = ["hy_api.cc", "hy_volume.cu", "hy_skip.cu", "hy_render.cu", "hy_pass.cu", "hy_batch.cu", "hy_page.cu", "hy_diff.cu",
            "hy_synth.cc", "hy_store_io.cc"]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -13,33 +13,12 @@
 #include <algorithm>
 #include <cstring>
 
-#include "hy_shade.cuh"
+#include "hy_tile.cuh"
 
 using namespace hy;
 using namespace hy::dev;
 
 namespace {
-
-constexpr int kTileW = 16, kTileH = 8, kThreads = 128;
-
-__device__ __forceinline__ void load_shared(const ShadeArgs &A, float4 *tf, float *lut) {
-    stage_tf(A.tf, A.ntf, tf);
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = float(i) / 255.f;
-    __syncthreads();
-}
-
-__device__ __forceinline__ void tile_xy(int &x, int &y) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    x = blockIdx.x * kTileW + (warp & 1) * 8 + (lane & 7);
-    y = blockIdx.y * kTileH + (warp >> 1) * 4 + (lane >> 3);
-}
-
-__device__ __forceinline__ void count_samples(const ShadeArgs &A, long long samples) {
-    if (!A.count) return;
-    unsigned long long s = (unsigned long long)samples;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0 && s) atomicAdd(A.counter, s);
-}
 
 // StdVec4Pixel::write_to (pixel_template.hpp:11-20), RGBA: alpha = saturate(v.a).
 __device__ __forceinline__ uchar4 quantise(const ShadeArgs &A, float4 v) {
@@ -213,153 +192,6 @@ __global__ void __launch_bounds__(kThreads, HY_RENDER_COMPOSITE_GATHER_BLOCKS)
     render_body<SHADER, PC, DT, PADDED, 1, false, true, LOOP>(A);
 }
 
-// ---- reference-layout film passes ------------------------------------------
-
-template <int SHADER>
-__device__ __forceinline__ size_t film_bytes() {
-    return (SHADER == HY_SHADER_BLOCKS || SHADER == HY_SHADER_PAGING) ? 48 : 64;
-}
-
-template <int SHADER>
-__device__ __forceinline__ void store_film(void *film, size_t idx, const Px &p) {
-    float4 *q = reinterpret_cast<float4 *>(static_cast<char *>(film) + idx * film_bytes<SHADER>());
-    q[0] = make_float4(p.ox, p.oy, p.oz, p.dx);
-    q[1] = make_float4(p.dy, p.dz, __int_as_float(p.nsteps), __int_as_float(p.step_size));
-    q[2] = make_float4(p.vx, p.vy, p.vz, p.vw);
-    if (SHADER != HY_SHADER_BLOCKS && SHADER != HY_SHADER_PAGING)
-        q[3] = make_float4(p.e0, p.e1, p.e2, p.e3);
-}
-
-template <int SHADER>
-__device__ __forceinline__ Px load_film(const void *film, size_t idx) {
-    const float4 *q =
-        reinterpret_cast<const float4 *>(static_cast<const char *>(film) + idx * film_bytes<SHADER>());
-    Px p;
-    float4 a = q[0], b = q[1], c = q[2];
-    p.ox = a.x;
-    p.oy = a.y;
-    p.oz = a.z;
-    p.dx = a.w;
-    p.dy = b.x;
-    p.dz = b.y;
-    p.nsteps = __float_as_int(b.z);
-    p.step_size = __float_as_int(b.w);
-    p.vx = c.x;
-    p.vy = c.y;
-    p.vz = c.z;
-    p.vw = c.w;
-    if (SHADER != HY_SHADER_BLOCKS && SHADER != HY_SHADER_PAGING) {
-        float4 d = q[3];
-        p.e0 = d.x;
-        p.e1 = d.y;
-        p.e2 = d.z;
-        p.e3 = d.w;
-    } else {
-        p.e0 = p.e1 = p.e2 = p.e3 = 0.f;
-    }
-    return p;
-}
-
-// ray_emit_kernel_impl (cuda_shading.cu:14-35)
-template <int SHADER, int DT>
-__global__ void __launch_bounds__(kThreads) emit_pass_kernel(const __grid_constant__ ShadeArgs A) {
-    extern __shared__ float4 smem[];
-    float4 *tf = smem;
-    float *lut = reinterpret_cast<float *>(smem + A.ntf + kTfPad);
-    load_shared(A, tf, lut);
-    const Shared S = make_shared(tf, A.ntf, lut);
-    int x, y;
-    tile_xy(x, y);
-    long long samples = 0;
-    if (x < A.view.W && y < A.view.H) {
-        float ox, oy, oz, dx, dy, dz;
-        gen_ray(A.view, x, y, ox, oy, oz, dx, dy, dz);
-        Px p;
-        samples = emit<SHADER, 0, DT, false>(p, A, A.view, S, ox, oy, oz, dx, dy, dz, 0.f, 0.f, 0.f,
-                                             A.bbox_max[0], A.bbox_max[1], A.bbox_max[2]);
-        store_film<SHADER>(A.film, size_t(y) * A.view.W + x, p);
-    }
-    count_samples(A, samples);
-}
-
-// ray_march_kernel_impl (cuda_shading.cu:41-54): resumes every pixel.
-template <int SHADER, int DT>
-__global__ void __launch_bounds__(kThreads) march_pass_kernel(const __grid_constant__ ShadeArgs A) {
-    extern __shared__ float4 smem[];
-    float4 *tf = smem;
-    float *lut = reinterpret_cast<float *>(smem + A.ntf + kTfPad);
-    load_shared(A, tf, lut);
-    const Shared S = make_shared(tf, A.ntf, lut);
-    int x, y;
-    tile_xy(x, y);
-    long long samples = 0;
-    if (x < A.view.W && y < A.view.H) {
-        const size_t idx = size_t(y) * A.view.W + x;
-        Px p = load_film<SHADER>(A.film, idx);
-        samples = run_main<SHADER, 0, DT, false>(p, A, A.view, S);
-        store_film<SHADER>(A.film, idx, p);
-    }
-    count_samples(A, samples);
-}
-
-// pixel_kernel_impl (cuda_shading.cu:60-74): film -> uchar3 via write_to.
-template <int SHADER>
-__global__ void __launch_bounds__(kThreads) pixel_pass_kernel(const __grid_constant__ ShadeArgs A) {
-    int x, y;
-    tile_xy(x, y);
-    if (x >= A.view.W || y >= A.view.H) return;
-    const size_t idx = size_t(y) * A.view.W + x;
-    Px p = load_film<SHADER>(A.film, idx);
-    unsigned char *d = static_cast<unsigned char *>(A.dst) + idx * 3;
-    if (p.vw != 0.f) {
-        d[0] = saturate_u8(p.vx);
-        d[1] = saturate_u8(p.vy);
-        d[2] = saturate_u8(p.vz);
-    } else {
-        d[0] = A.clear_u8[0];
-        d[1] = A.clear_u8[1];
-        d[2] = A.clear_u8[2];
-    }
-}
-
-// fetch_kernel_impl (cuda_shading.cu:80-94): VolumeShaderKernel::fetch
-// (volume_shader.cu:23-30), IsosurfaceShaderKernel::fetch
-// (isosurface_shader.cu:41-48) and PagingShaderKernel::fetch
-// (paging_shader.cu:16-22, uchar3 pixels).  The Blocks shader has no fetch.
-template <int SHADER>
-__global__ void __launch_bounds__(kThreads) fetch_pass_kernel(const __grid_constant__ ShadeArgs A) {
-    int x, y;
-    tile_xy(x, y);
-    if (x >= A.view.W || y >= A.view.H) return;
-    const size_t idx = size_t(y) * A.view.W + x;
-    Px p = load_film<SHADER>(A.film, idx);
-    if (SHADER == HY_SHADER_VOLUME) {
-        float4 *d = reinterpret_cast<float4 *>(static_cast<char *>(A.dst) + idx * 32);
-        d[0] = make_float4(p.e0, p.e1, p.e2, p.e3);
-        d[1] = make_float4(p.vx, p.vy, p.vz, p.vw);
-    } else if (SHADER == HY_SHADER_ISOSURFACE) {
-        unsigned char *d = static_cast<unsigned char *>(A.dst) + idx * 8;
-        d[0] = saturate_u8(p.vx);
-        d[1] = saturate_u8(p.vy);
-        d[2] = saturate_u8(p.vz);
-        d[3] = 0;
-        *reinterpret_cast<float *>(d + 4) = p.e3;
-    } else if (SHADER == HY_SHADER_PAGING) {
-        unsigned char *d = static_cast<unsigned char *>(A.dst) + idx * 3;
-        d[0] = saturate_u8(p.vx);
-        d[1] = saturate_u8(p.vy);
-        d[2] = saturate_u8(p.vz);
-    }
-}
-
-size_t smem_bytes(const ShadeArgs &a) {
-    return size_t(a.ntf + kTfPad) * sizeof(float4) + 256 * sizeof(float);
-}
-
-dim3 grid_of(const ShadeArgs &a) {
-    return dim3((a.view.W + kTileW - 1) / kTileW, (a.view.H + kTileH - 1) / kTileH);
-}
-
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
 void launch_group(const ShadeArgs &a, cudaStream_t s) {
     const dim3 g((a.view.W + 2 * kGroupW - 1) / (2 * kGroupW),
@@ -520,33 +352,6 @@ int dispatch_fused(const ShadeArgs &a, cudaStream_t s) {
     return HY_OK;
 }
 
-template <int SHADER>
-void dispatch_pass(const ShadeArgs &a, int pass, cudaStream_t s) {
-    const dim3 g = grid_of(a);
-    const size_t sm = smem_bytes(a);
-    const bool f32 = a.vol.dtype == HY_DTYPE_F32;
-    switch (pass) {
-        case HY_PASS_RAY_EMIT:
-            if (f32)
-                emit_pass_kernel<SHADER, HY_DTYPE_F32><<<g, kThreads, sm, s>>>(a);
-            else
-                emit_pass_kernel<SHADER, HY_DTYPE_U8><<<g, kThreads, sm, s>>>(a);
-            break;
-        case HY_PASS_RAY_MARCH:
-            if (f32)
-                march_pass_kernel<SHADER, HY_DTYPE_F32><<<g, kThreads, sm, s>>>(a);
-            else
-                march_pass_kernel<SHADER, HY_DTYPE_U8><<<g, kThreads, sm, s>>>(a);
-            break;
-        case HY_PASS_PIXEL:
-            pixel_pass_kernel<SHADER><<<g, kThreads, 0, s>>>(a);
-            break;
-        default:
-            fetch_pass_kernel<SHADER><<<g, kThreads, 0, s>>>(a);
-            break;
-    }
-}
-
 unsigned char sat_host(float f) {
     float x = f * 255.f;
     x = (x < 0.f) ? 0.f : x;
@@ -658,34 +463,6 @@ int hy_launch_render(hy_ctx *ctx, const ShadeArgs &a) {
     HY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->stats_pending = true;
     ctx->pend_count = a.count;
-    ctx->pend_pixels = (int64_t)a.view.W * a.view.H;
-    return HY_OK;
-}
-
-int hy_launch_pass(hy_ctx *ctx, const ShadeArgs &a, int pass, bool reset_counter) {
-    int rc = hy_check_paged_gather(ctx, a, false);
-    if (rc) return rc;
-    if (reset_counter && a.count && pass <= HY_PASS_RAY_MARCH)
-        HY_CUDA(ctx, cudaMemsetAsync(ctx->counter_dev, 0, sizeof(unsigned long long), ctx->stream));
-    HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    switch (a.shader) {
-        case HY_SHADER_VOLUME:
-            dispatch_pass<HY_SHADER_VOLUME>(a, pass, ctx->stream);
-            break;
-        case HY_SHADER_BLOCKS:
-            dispatch_pass<HY_SHADER_BLOCKS>(a, pass, ctx->stream);
-            break;
-        case HY_SHADER_PAGING:
-            dispatch_pass<HY_SHADER_PAGING>(a, pass, ctx->stream);
-            break;
-        default:
-            dispatch_pass<HY_SHADER_ISOSURFACE>(a, pass, ctx->stream);
-            break;
-    }
-    HY_CUDA(ctx, cudaGetLastError());
-    HY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
-    ctx->stats_pending = true;
-    ctx->pend_count = a.count && pass <= HY_PASS_RAY_MARCH;
     ctx->pend_pixels = (int64_t)a.view.W * a.view.H;
     return HY_OK;
 }
@@ -804,6 +581,11 @@ extern "C" int hy_shade_pass(hy_ctx *ctx, const hy_volume *vol, const hy_shader_
     ShadeArgs a;
     int rc = hy_fill_args(ctx, vol, p, view, W, H, &a);
     if (rc) return rc;
+    if (pass <= HY_PASS_RAY_MARCH) {
+        HY_CUDA(ctx, cudaSetDevice(ctx->device));
+        rc = hy_skip_view(ctx, vol, p, &a.skip);
+        if (rc) return rc;
+    }
     a.film = film_dev;
     a.dst = dst_dev;
     if (clear_rgb)

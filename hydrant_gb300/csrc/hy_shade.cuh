@@ -903,14 +903,14 @@ __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, cons
     return samples;
 }
 
-// The lean Volume march with U samples of the ray in flight: a step's taps
+// The Volume march (Default mode) with U samples of the ray in flight: a step's taps
 // do not depend on the sample before it (only its position does, by one
 // addition), so the next U positions are stepped first, their taps fetched
 // together, and their colours composited in order -- the floats of
 // volume_main.  A batch takes the samples in the brick of its first one; the
 // sample after which the step size changes ends it (the samples fetched
 // beyond are dropped).
-template <int U, int PC, int DT, bool PADDED, int GATHER>
+template <int U, int PC, int DT, bool PADDED, bool LEAN, int GATHER>
 __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, const Shared &S) {
     const DevVolume &V = A.vol;
     unsigned int samples = 0;
@@ -940,7 +940,7 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
             float qx[U], qy[U], qz[U], v[U];
             Footprint fp[U];
             bool ok = true;
-            int n = 0;
+            int n = 0, left = p.nsteps;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 qx[u] = u ? qx[u ? u - 1 : 0] + m.sx : p.ox;
@@ -951,8 +951,8 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
                     ux = qx[u] - m.c.ipx;
                     uy = qy[u] - m.c.ipy;
                     uz = qz[u] - m.c.ipz;
-                    ok = ok & unit_interval(ux) & unit_interval(uy) & unit_interval(uz) &
-                         (p.nsteps > u * ss);
+                    left -= ss;
+                    ok = ok & unit_interval(ux) & unit_interval(uy) & unit_interval(uz) & (left > 0);
                     ux = ok ? ux : lx;
                     uy = ok ? uy : ly;
                     uz = ok ? uz : lz;
@@ -990,6 +990,12 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
                 const float2 cxy = mul2(f2(c.x, c.y), f2(c.w, c.w));
                 c.z = c.z * c.w;
                 if (u < n) {
+                    if (!LEAN) {
+                        p.e0 = p.e0 + cxy.x * p.e3;
+                        p.e1 = p.e1 + cxy.y * p.e3;
+                        p.e2 = p.e2 + c.z * p.e3;
+                        p.e3 = p.e3 * (1.f - c.w);
+                    }
                     const float t = 1.f - p.vw;
                     const float2 txy = mul2(cxy, f2(t, t)), tzw = mul2(f2(c.z, c.w), f2(t, t));
                     p.vx = __fadd_rn(p.vx, txy.x);
@@ -1487,9 +1493,9 @@ template <int SHADER, int PC, int DT, bool PADDED, bool LEAN = false, int GATHER
 __device__ __forceinline__ long long run_main(Px &p, const ShadeArgs &A, const ViewArgs &Vw,
                                              const Shared &S) {
     if constexpr (SHADER == HY_SHADER_VOLUME && LOOP == kLoopBatch2)
-        return volume_batches<2, PC, DT, PADDED, GATHER>(p, A, S);
+        return volume_batches<2, PC, DT, PADDED, LEAN, GATHER>(p, A, S);
     else if constexpr (SHADER == HY_SHADER_VOLUME && LOOP == kLoopBatch4)
-        return volume_batches<4, PC, DT, PADDED, GATHER>(p, A, S);
+        return volume_batches<4, PC, DT, PADDED, LEAN, GATHER>(p, A, S);
     else if (SHADER == HY_SHADER_VOLUME)
         return volume_main<PC, DT, PADDED, LEAN, GATHER, LOOP>(p, A, S);
     if (SHADER == HY_SHADER_BLOCKS) {

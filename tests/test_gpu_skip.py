@@ -221,3 +221,35 @@ def test_blocks(ctx, density, composite):
                       density=density, sample_rate=rate, composite=composite)
         finally:
             c.close()
+
+
+@pytest.mark.parametrize("shader,mode", [("Volume", "Default"), ("Volume", "Partition"),
+                                         ("Isosurface", "Position"), ("Blocks", "Volume"),
+                                         ("Blocks", "Solid")])
+@pytest.mark.parametrize("dtype,pad", [("u8", 1), ("u8", 0), ("f32", 1)])
+def test_films(ctx, shader, mode, dtype, pad):
+    """The emit pass leaves the plain march's film, byte for byte, in each form
+    (sizes on both sides of 155,648 and 466,944 rays), and a march pass leaves
+    the film of rays that have marched to their end."""
+    torch = pytest.importorskip("torch")
+    c = Case(ctx, voxels(dtype, (70, 61, 52)), 32, pad, tf=knots("ends"))
+    try:
+        fb = 48 if shader == "Blocks" else 64
+        for W, H in ((41, 33), (395, 393), (397, 394), (690, 680)):
+            cam = camera(a=(-50.0, 20.0, 1.9))
+            p = hy.shader_params(shader=shader, mode=mode, sample_rate=0.5, density=0.3, rank=0.4)
+            if shader == "Isosurface":
+                hy.iso_lighting(c.vol, cam, p)
+            view = hy.camera_view(c.vol, cam)
+            film = torch.zeros(H * W * fb, dtype=torch.uint8, device="cuda")
+            hy.shade_pass(ctx, c.vol, p, hy._abi.PASS_RAY_EMIT, view, film.data_ptr(), W, H)
+            ctx.synchronize()
+            ref = orc.render(c.ov, c.tf, orc.params_from(p), view_array(view), W, H, want_film=True)
+            got = film.cpu().numpy().reshape(H, W, fb)
+            assert np.array_equal(got, ref["film"]), (shader, mode, W, H)
+        before = film.clone()
+        hy.shade_pass(ctx, c.vol, p, hy._abi.PASS_RAY_MARCH, None, film.data_ptr(), W, H)
+        ctx.synchronize()
+        assert torch.equal(before, film)
+    finally:
+        c.close()
