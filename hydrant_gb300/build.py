@@ -45,7 +45,7 @@ def nvcc() -> str:
 
 
 def extra_flags() -> list[str]:
-    """Macro settings for tuning builds (e.g. "-DHY_DIFF_MIN_BLOCKS=6"), from
+    """Macro settings for tuning builds (e.g. "-DHY_BATCH_GATHER_REGS=56"), from
     HYDRANT_GB300_NVCC_DEFINES; only -D options are taken."""
     return [f for f in os.environ.get("HYDRANT_GB300_NVCC_DEFINES", "").split() if f.startswith("-D")]
 

@@ -67,6 +67,7 @@ struct DiffArgs {
     // s + 1 of a footprint is always P rows below slice s
     unsigned long long gtex;
     int gper;
+    unsigned int gmagic;  // floor(2^32 / gper) + 1: s / gper = umulhi(s, gmagic) for s < 2^16
 };
 
 // Trilinear footprint of the padded brick at brick-local x in [0,1] (the
@@ -128,55 +129,93 @@ __device__ __forceinline__ float diff_sample(const DiffArgs &a, float lx, float 
     return diff_fetch(a, c);
 }
 
-// diff_sample through the gather texture: the same fractions and lerps, the
-// eight taps by two gathers (slices iz and iz + 1 of the padded volume,
-// whose texels repeat the clamped border exactly as diff_cell's indices do).
-// In the interior a footprint's lower index lies in [0, P - 2], so the
-// whole-number texel coordinates stay inside the slice's tile.
-__device__ __forceinline__ float diff_sample_gather(const DiffArgs &a, float lx, float ly,
-                                                    float lz) {
-    const int P = a.n + 2;
-    const float fd = float(P);
-    const float2 kl = mul2(f2(a.k, a.k), f2(lx, ly));
-    const float2 fxy = mul2(f2(fd, fd), f2(__fadd_rn(kl.x, a.b), __fadd_rn(kl.y, a.b)));
-    const float fz = fd * (a.k * lz + a.b);
-    const float ux = fxy.x - .5f, uy = fxy.y - .5f, uz = fz - .5f;
-    const float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
-    const float2 axy = sub2(f2(ux, uy), f2(flx, fly));
-    const float az = uz - flz;
-    const int iz = int(flz);
-    const int col = iz / a.gper, row = iz - col * a.gper;
-    const float X = float(col * P + 1) + flx, Y = float(row * P + 1) + fly;
-    const float4 g0 = gather_r(a.gtex, X, Y), g1 = gather_r(a.gtex, X, Y + fd);
-    // gather order: w = (x, y), z = (x + 1, y), x = (x, y + 1), y = (x + 1, y + 1)
-    const float2 c00 = f2(g0.w, g1.w), c01 = f2(g0.z, g1.z);
-    const float2 c10 = f2(g0.x, g1.x), c11 = f2(g0.y, g1.y);
-    const float2 bxy = sub2(f2(1.f, 1.f), axy);
-    const float bz = 1.f - az;
-    const float2 bx2 = f2(bxy.x, bxy.x), ax2 = f2(axy.x, axy.x);
-    const float2 X0 = lerp2(c00, bx2, c01, ax2);
-    const float2 X1 = lerp2(c10, bx2, c11, ax2);
-    const float2 Yv = lerp2(X0, f2(bxy.y, bxy.y), X1, f2(axy.y, axy.y));
-    const float2 Z = mul2(Yv, f2(bz, az));
-    return __fadd_rn(Z.x, Z.y);
+// U samples' values at positions q: through the gather texture (the fractions
+// and lerps of diff_sample, the eight taps by two gathers from slices iz and
+// iz + 1 of the padded volume, whose texels repeat the clamped border exactly as
+// diff_cell's indices do; in the interior a footprint's lower index lies in
+// [0, P - 2], so the whole-number texel coordinates stay inside the slice's
+// tile), or by loads.  All footprints first, then all taps, then the lerps, so
+// that the fetches are in flight together.
+template <int U, bool GATHER>
+__device__ __forceinline__ void diff_values(const DiffArgs &a, const float (&qx)[U],
+                                            const float (&qy)[U], const float (&qz)[U],
+                                            float (&v)[U]) {
+    if constexpr (!GATHER) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            v[u] = diff_sample(a, qx[u] - floorf(qx[u]), qy[u] - floorf(qy[u]),
+                               qz[u] - floorf(qz[u]));
+    } else {
+        const float fd = float(a.n + 2);
+        float X[U], Y[U], az[U];
+        float2 axy[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float lx = qx[u] - floorf(qx[u]), ly = qy[u] - floorf(qy[u]),
+                        lz = qz[u] - floorf(qz[u]);
+            const float2 kl = mul2(f2(a.k, a.k), f2(lx, ly));
+            const float2 fxy = mul2(f2(fd, fd), f2(__fadd_rn(kl.x, a.b), __fadd_rn(kl.y, a.b)));
+            const float fz = fd * (a.k * lz + a.b);
+            const float ux = fxy.x - .5f, uy = fxy.y - .5f, uz = fz - .5f;
+            const float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
+            axy[u] = sub2(f2(ux, uy), f2(flx, fly));
+            az[u] = uz - flz;
+            const int iz = int(flz);
+            const int col = int(__umulhi(unsigned(iz), a.gmagic)), row = iz - col * a.gper;
+            // whole numbers below 2^24: exact in any order
+            X[u] = __fmaf_rn(float(col), fd, flx + 1.f);
+            Y[u] = __fmaf_rn(float(row), fd, fly + 1.f);
+        }
+        float4 g0[U], g1[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            g0[u] = gather_r(a.gtex, X[u], Y[u]);
+            g1[u] = gather_r(a.gtex, X[u], Y[u] + fd);
+        }
+        // gather order: w = (x, y), z = (x + 1, y), x = (x, y + 1), y = (x + 1, y + 1)
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            v[u] = trilerp(f2(g0[u].w, g1[u].w), f2(g0[u].z, g1[u].z), f2(g0[u].x, g1[u].x),
+                           f2(g0[u].y, g1[u].y), axy[u], az[u]);
+    }
 }
 
-// The padded volume into the gather texture: one thread per texel of a
-// slice row (x), rows (y) and slices (z) on the grid's other axes.
-__global__ void diff_fill_kernel(const float *__restrict__ vol, int n, int gper,
-                                 unsigned long long surf) {
-    const int P = n + 2;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, s = blockIdx.z;
-    if (x >= P) return;
-    const int vx = min(max(x - 1, 0), n - 1), vy = min(max(y - 1, 0), n - 1),
-              vz = min(max(s - 1, 0), n - 1);
-    const float v = vol[(size_t(vz) * n + vy) * n + vx];
+// The padded volume into the gather texture.  A block takes kFillRows rows of a
+// slice, its threads texel pairs along them (8-byte surface writes; single
+// texels when P is odd).  256^3: 20-30 us (67 MB read, 69 MB written) against
+// 103 us with a thread per texel in 200 k blocks.
+constexpr int kFillRows = 32;
+template <bool PAIRS>
+__global__ void __launch_bounds__(256) diff_fill_kernel(const float *__restrict__ vol, int n,
+                                                        int gper, unsigned long long surf) {
+    const int P = n + 2, s = blockIdx.y;
+    const int vz = min(max(s - 1, 0), n - 1);
     const cudaSurfaceObject_t so = cudaSurfaceObject_t(surf);
     const int col = s / gper, row = s - col * gper;
-    surf2Dwrite(v, so, (col * P + x) * int(sizeof(float)), row * P + y, cudaBoundaryModeZero);
-    if (row == 0 && col > 0)
-        surf2Dwrite(v, so, ((col - 1) * P + x) * int(sizeof(float)), gper * P + y,
-                    cudaBoundaryModeZero);
+    const bool twice = row == 0 && col > 0;
+    constexpr int W = PAIRS ? 2 : 1;
+    const int lane = threadIdx.x & 63;
+    const int y1 = min((int(blockIdx.x) + 1) * kFillRows, P);
+    for (int y = blockIdx.x * kFillRows + (threadIdx.x >> 6); y < y1; y += 4) {
+        const float *src = vol + (size_t(vz) * n + min(max(y - 1, 0), n - 1)) * n;
+        for (int x = lane * W; x < P; x += 64 * W) {
+            const float v0 = src[min(max(x - 1, 0), n - 1)];
+            if constexpr (PAIRS) {
+                const float2 v = make_float2(v0, src[min(x, n - 1)]);
+                surf2Dwrite(v, so, (col * P + x) * int(sizeof(float)), row * P + y,
+                            cudaBoundaryModeZero);
+                if (twice)
+                    surf2Dwrite(v, so, ((col - 1) * P + x) * int(sizeof(float)), gper * P + y,
+                                cudaBoundaryModeZero);
+            } else {
+                surf2Dwrite(v0, so, (col * P + x) * int(sizeof(float)), row * P + y,
+                            cudaBoundaryModeZero);
+                if (twice)
+                    surf2Dwrite(v0, so, ((col - 1) * P + x) * int(sizeof(float)), gper * P + y,
+                                cudaBoundaryModeZero);
+            }
+        }
+    }
 }
 
 // emit against the unit box; returns nsteps, sets o and d
@@ -205,26 +244,26 @@ __device__ __forceinline__ int diff_emit(const DiffArgs &a, int view, int x, int
     return min(a.max_steps, int((tfar - tnear) / a.step));
 }
 
-// transfer function value and its derivative in s
-__device__ __forceinline__ float4 tf_eval(const float4 *tf, int n, float s, int &i, int &j,
-                                          float &al, bool &inb) {
-    const float fn = float(n);
-    const float fx = fn * s;
-    inb = (0.f <= fx && fx <= fn);
-    if (!inb) {
-        i = j = 0;
-        al = 0.f;
-        return make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+// Where a value falls among the knots staged by stage_tf (end knots repeated,
+// two zero knots after them): between entries k and k + 1 at fraction al; out
+// of [0, 1] (or NaN) between the zeros.
+struct TfAt {
+    int k;
+    float al;
+    bool in;
+};
+__device__ __forceinline__ TfAt tf_at(int n, float fn, float s) {
+    float fx = fn * s;
+    const bool in = 0.f <= fx && fx <= fn;
+    fx = in ? fx : 0.f;
     const float u = fx - .5f;
     const float flr = floorf(u);
-    al = u - flr;
-    const int fi = int(flr);
-    i = max(fi, 0);
-    j = min(fi + 1, n - 1);
-    const float4 p = tf[i], q = tf[j];
-    const float bb = 1.f - al;
-    const float2 b2 = f2(bb, bb), a2 = f2(al, al);
+    return TfAt{in ? int(flr) + 1 : n + 2, u - flr, in};
+}
+__device__ __forceinline__ float4 tf_value(const float4 *tf, const TfAt &t) {
+    const float4 p = tf[t.k], q = tf[t.k + 1];
+    const float bb = 1.f - t.al;
+    const float2 b2 = f2(bb, bb), a2 = f2(t.al, t.al);
     const float2 rg = lerp2(f2(p.x, p.y), b2, f2(q.x, q.y), a2);
     const float2 ba = lerp2(f2(p.z, p.w), b2, f2(q.z, q.w), a2);
     return make_float4(rg.x, rg.y, ba.x, ba.y);
@@ -237,10 +276,16 @@ __device__ __forceinline__ void pixel_of(const DiffArgs &a, int &x, int &y, int 
     view = blockIdx.z;
 }
 
-template <bool GATHER>
-__global__ void __launch_bounds__(128) diff_forward_kernel(const __grid_constant__ DiffArgs a) {
-    __shared__ float4 tf[kMaxKnots];
-    for (int i = threadIdx.x; i < a.ntf; i += blockDim.x) tf[i] = a.tf[i];
+// U steps of a ray at a time: their taps are fetched together (a step's
+// position does not depend on the sample before it).  256^3, four views of
+// 512^2, K = 32: 5.30 ms by loads one at a time, 1.9 ms by gathers with 4 in
+// flight (L1 86 % busy: the texture's f32 wavefronts); 3 views of 75x51 over
+// 48^3 104 and 50 us.
+template <int U, bool GATHER>
+__global__ void __launch_bounds__(128, U >= 4 ? 4 : 8)
+    diff_forward_kernel(const __grid_constant__ DiffArgs a) {
+    __shared__ float4 tf[kMaxKnots + kTfPad];
+    stage_tf(a.tf, a.ntf, tf);
     __syncthreads();
     int x, y, view;
     pixel_of(a, x, y, view);
@@ -251,34 +296,48 @@ __global__ void __launch_bounds__(128) diff_forward_kernel(const __grid_constant
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     const float sx = dx * a.step, sy = dy * a.step, sz = dz * a.step;  // step_size 1
     float4 *cp = a.ckpt ? a.ckpt + ray * a.max_ckpt : nullptr;
-    int until_ckpt = 0;  // a checkpoint before steps 0, K, 2K, ...
-    for (int s = 0; s < nsteps; ++s) {
-        if (until_ckpt == 0) {
-            if (cp) *cp++ = make_float4(ox, oy, oz, v.w);
-            until_ckpt = a.K;
+    const float fn = float(a.ntf);
+    int left = nsteps;
+    while (left > 0) {
+        // a checkpoint before steps 0, K, 2K, ...
+        if (cp) *cp++ = make_float4(ox, oy, oz, v.w);
+        int cnt = a.ckpt ? min(a.K, left) : left;
+        left -= cnt;
+        while (cnt > 0) {
+            float qx[U], qy[U], qz[U], val[U];
+            qx[0] = ox;
+            qy[0] = oy;
+            qz[0] = oz;
+#pragma unroll
+            for (int u = 1; u < U; ++u) {
+                const bool on = u < cnt;  // beyond the segment: the last position again
+                qx[u] = on ? qx[u - 1] + sx : qx[u - 1];
+                qy[u] = on ? qy[u - 1] + sy : qy[u - 1];
+                qz[u] = on ? qz[u - 1] + sz : qz[u - 1];
+            }
+            diff_values<U, GATHER>(a, qx, qy, qz, val);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                float4 ub = tf_value(tf, tf_at(a.ntf, fn, val[u]));
+                ub.w = ub.w * a.density;
+                const float w = ub.w;
+                const float2 uxy = mul2(f2(ub.x, ub.y), f2(w, w));
+                ub.z = ub.z * w;
+                if (u < cnt) {
+                    const float t = 1.f - v.w;
+                    // packed products, scalar sums (see mul2)
+                    const float2 txy = mul2(uxy, f2(t, t)), tzw = mul2(f2(ub.z, ub.w), f2(t, t));
+                    v.x = __fadd_rn(v.x, txy.x);
+                    v.y = __fadd_rn(v.y, txy.y);
+                    v.z = __fadd_rn(v.z, tzw.x);
+                    v.w = __fadd_rn(v.w, tzw.y);
+                }
+            }
+            ox = qx[U - 1] + sx;
+            oy = qy[U - 1] + sy;
+            oz = qz[U - 1] + sz;
+            cnt -= U;
         }
-        --until_ckpt;
-        const float ipx = floorf(ox), ipy = floorf(oy), ipz = floorf(oz);
-        const float val = GATHER ? diff_sample_gather(a, ox - ipx, oy - ipy, oz - ipz)
-                                 : diff_sample(a, ox - ipx, oy - ipy, oz - ipz);
-        int i, j;
-        float al;
-        bool inb;
-        float4 ub = tf_eval(tf, a.ntf, val, i, j, al, inb);
-        ub.w = ub.w * a.density;
-        const float w = ub.w;
-        const float2 uxy = mul2(f2(ub.x, ub.y), f2(w, w));
-        ub.z = ub.z * w;
-        const float t = 1.f - v.w;
-        // packed products, scalar sums (see mul2)
-        const float2 txy = mul2(uxy, f2(t, t)), tzw = mul2(f2(ub.z, ub.w), f2(t, t));
-        v.x = __fadd_rn(v.x, txy.x);
-        v.y = __fadd_rn(v.y, txy.y);
-        v.z = __fadd_rn(v.z, tzw.x);
-        v.w = __fadd_rn(v.w, tzw.y);
-        ox = ox + sx;
-        oy = oy + sy;
-        oz = oz + sz;
     }
     a.image[ray] = v;
     if (a.nsteps_out) a.nsteps_out[ray] = nsteps;
@@ -288,22 +347,22 @@ __global__ void __launch_bounds__(128) diff_forward_kernel(const __grid_constant
 // interval and a voxel cell, so gradients are summed in registers and flushed
 // (one atomic per knot channel / cell corner) only when those change.
 struct GradAcc {
-    int ki = -1, kj = -1;
+    int k = -1;  // knot entries k and k + 1 of stage_tf
     float4 acc_i = make_float4(0.f, 0.f, 0.f, 0.f), acc_j = make_float4(0.f, 0.f, 0.f, 0.f);
     Cell cell;
     bool has_cell = false;
     float cacc[8];
 
     __device__ __forceinline__ void flush_knots(float4 *gtf) {
-        if (ki < 0) return;
-        atomicAdd(&gtf[ki].x, acc_i.x);
-        atomicAdd(&gtf[ki].y, acc_i.y);
-        atomicAdd(&gtf[ki].z, acc_i.z);
-        atomicAdd(&gtf[ki].w, acc_i.w);
-        atomicAdd(&gtf[kj].x, acc_j.x);
-        atomicAdd(&gtf[kj].y, acc_j.y);
-        atomicAdd(&gtf[kj].z, acc_j.z);
-        atomicAdd(&gtf[kj].w, acc_j.w);
+        if (k < 0) return;
+        atomicAdd(&gtf[k].x, acc_i.x);
+        atomicAdd(&gtf[k].y, acc_i.y);
+        atomicAdd(&gtf[k].z, acc_i.z);
+        atomicAdd(&gtf[k].w, acc_i.w);
+        atomicAdd(&gtf[k + 1].x, acc_j.x);
+        atomicAdd(&gtf[k + 1].y, acc_j.y);
+        atomicAdd(&gtf[k + 1].z, acc_j.z);
+        atomicAdd(&gtf[k + 1].w, acc_j.w);
         acc_i = make_float4(0.f, 0.f, 0.f, 0.f);
         acc_j = acc_i;
     }
@@ -325,10 +384,9 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
                                                     float4 *gtf, GradAcc &G, const float4 &g,
                                                     float4 &R, float px, float py, float pz,
                                                     float val, float T) {
-    int i, j;
-    float al;
-    bool inb;
-    const float4 q = tf_eval(tf, a.ntf, val, i, j, al, inb);
+    const TfAt at = tf_at(a.ntf, float(a.ntf), val);
+    const float4 q = tf_value(tf, at);
+    const float al = at.al;
     const float aa = q.w * a.density;
     // The gradient arithmetic has no float-exact counterpart to follow, so it
     // uses fused multiply-adds (the file is compiled with contraction off).
@@ -344,15 +402,14 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
     const float2 Rxy = fma2(om2, f2(R.x, R.y), mul2(f2(q.x, q.y), f2(aa, aa)));
     const float2 Rzw = fma2(om2, f2(R.z, R.w), f2(q.z * aa, aa));
     R = make_float4(Rxy.x, Rxy.y, Rzw.x, Rzw.y);
-    if (!inb) return;
+    if (!at.in) return;
     // gradient of the TF output (r, g, b, A)
     const float2 gqxy = mul2(gcxy, f2(aa, aa)), gqzw = mul2(f2(gcz, da), f2(aa, a.density));
     const float4 gq = make_float4(gqxy.x, gqxy.y, gqzw.x, gqzw.y);
     const float bb = 1.f - al;
-    if (i != G.ki || j != G.kj) {
+    if (at.k != G.k) {
         G.flush_knots(gtf);
-        G.ki = i;
-        G.kj = j;
+        G.k = at.k;
     }
     {
         const float2 b2 = f2(bb, bb), a2 = f2(al, al);
@@ -364,7 +421,7 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
         G.acc_j = make_float4(jxy.x, jxy.y, jzw.x, jzw.y);
     }
     // d TF / d s = (knot_j - knot_i) * n
-    const float4 kj = tf[j], ki = tf[i];
+    const float4 kj = tf[at.k + 1], ki = tf[at.k];
     const float fn = float(a.ntf);
     const float ds = fn * __fmaf_rn(gq.w, kj.w - ki.w,
                                     __fmaf_rn(gq.z, kj.z - ki.z,
@@ -408,22 +465,20 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
 // s additions: the positions agree to a few ulps, and the trilinear weights'
 // derivative is continuous across cell faces, so a sample that lands in the
 // neighbouring cell gets the same gradient to first order).
-// HY_DIFF_MIN_BLOCKS: resident 128-thread blocks per SM the register budget
-// is fitted to.  6 (80 registers, 36 bytes spilled, 24 warps) against the
-// compiler's 96 registers and 20 warps, 256^3 f32, 16 views of 512^2, K = 32:
-// adjoint 2.35 vs 2.55 ms/view; 8 (64 registers, 100 bytes spilled): 2.45.
-#ifndef HY_DIFF_MIN_BLOCKS
-#define HY_DIFF_MIN_BLOCKS 6
-#endif
-template <bool GATHER>
-__global__ void __launch_bounds__(128, HY_DIFF_MIN_BLOCKS)
+// BLOCKS: resident 128-thread blocks per SM the registers are fitted to.  256^3,
+// four views of 512^2, K = 32, forward and adjoint: 8 blocks (64 registers)
+// 9.71 ms, 6 (80) 10.1, 5 10.2, 4 10.6; launches of fewer than 8 warps of
+// rays a scheduler are bound by latency and take 4 (128 registers) with
+// four samples of the recompute in flight: 3 views of 75x51 over 48^3 446
+// against 492 us.
+template <int U, int BLOCKS, bool GATHER>
+__global__ void __launch_bounds__(128, BLOCKS)
     diff_backward_kernel(const __grid_constant__ DiffArgs a) {
-    __shared__ float4 tf[kMaxKnots];
-    __shared__ float4 gtf[kMaxKnots];
-    for (int i = threadIdx.x; i < a.ntf; i += blockDim.x) {
-        tf[i] = a.tf[i];
+    __shared__ float4 tf[kMaxKnots + kTfPad];
+    __shared__ float4 gtf[kMaxKnots + 2];  // gradients of stage_tf's entries 0 .. ntf + 1
+    stage_tf(a.tf, a.ntf, tf);
+    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x)
         gtf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
     __syncthreads();
     int x, y, view;
     pixel_of(a, x, y, view);
@@ -438,27 +493,39 @@ __global__ void __launch_bounds__(128, HY_DIFF_MIN_BLOCKS)
         const int K = a.K;
         float2 seg_vw[kMaxK];  // (sample value, v.w before the sample)
         const int nseg = (nsteps + K - 1) / K;
+        const float fn = float(a.ntf);
         GradAcc G;
         const float4 *cps = a.ckpt + ray * a.max_ckpt;
         for (int seg = nseg - 1; seg >= 0; --seg) {
             const float4 c = cps[seg];
             float ox = c.x, oy = c.y, oz = c.z, vw = c.w;
             const int cnt = min(K, nsteps - seg * K);
-            // recompute the segment: values and v.w before each sample
-            for (int s = 0; s < cnt; ++s) {
-                const float ipx = floorf(ox), ipy = floorf(oy), ipz = floorf(oz);
-                const float val = GATHER ? diff_sample_gather(a, ox - ipx, oy - ipy, oz - ipz)
-                                         : diff_sample(a, ox - ipx, oy - ipy, oz - ipz);
-                seg_vw[s] = make_float2(val, vw);
-                int i, j;
-                float al;
-                bool inb;
-                const float4 ub = tf_eval(tf, a.ntf, val, i, j, al, inb);
-                const float aa = ub.w * a.density;
-                vw = vw + aa * (1.f - vw);
-                ox = ox + sx;
-                oy = oy + sy;
-                oz = oz + sz;
+            // recompute the segment: values and v.w before each sample, U
+            // samples' taps in flight
+            for (int s = 0; s < cnt; s += U) {
+                float qx[U], qy[U], qz[U], val[U];
+                qx[0] = ox;
+                qy[0] = oy;
+                qz[0] = oz;
+#pragma unroll
+                for (int u = 1; u < U; ++u) {
+                    const bool on = s + u < cnt;
+                    qx[u] = on ? qx[u - 1] + sx : qx[u - 1];
+                    qy[u] = on ? qy[u - 1] + sy : qy[u - 1];
+                    qz[u] = on ? qz[u - 1] + sz : qz[u - 1];
+                }
+                diff_values<U, GATHER>(a, qx, qy, qz, val);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const float aa = tf_value(tf, tf_at(a.ntf, fn, val[u])).w * a.density;
+                    if (s + u < cnt) {
+                        seg_vw[s + u] = make_float2(val[u], vw);
+                        vw = vw + aa * (1.f - vw);
+                    }
+                }
+                ox = qx[U - 1] + sx;
+                oy = qy[U - 1] + sy;
+                oz = qz[U - 1] + sz;
             }
             for (int s = cnt - 1; s >= 0; --s) {
                 const float fs = float(s);
@@ -472,12 +539,14 @@ __global__ void __launch_bounds__(128, HY_DIFF_MIN_BLOCKS)
         G.flush_cell(a.dvol);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < a.ntf; i += blockDim.x) {
+    // entry i is knot clamp(i - 1, 0, ntf - 1)
+    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x) {
         const float4 v = gtf[i];
-        if (v.x != 0.f) atomicAdd(a.dtf + 4 * i + 0, v.x);
-        if (v.y != 0.f) atomicAdd(a.dtf + 4 * i + 1, v.y);
-        if (v.z != 0.f) atomicAdd(a.dtf + 4 * i + 2, v.z);
-        if (v.w != 0.f) atomicAdd(a.dtf + 4 * i + 3, v.w);
+        float *d = a.dtf + 4 * min(max(i - 1, 0), a.ntf - 1);
+        if (v.x != 0.f) atomicAdd(d + 0, v.x);
+        if (v.y != 0.f) atomicAdd(d + 1, v.y);
+        if (v.z != 0.f) atomicAdd(d + 2, v.z);
+        if (v.w != 0.f) atomicAdd(d + 3, v.w);
     }
 }
 
@@ -525,18 +594,9 @@ int fill_diff(hy_ctx *ctx, const hy_diff_params *p, const float *vol, const floa
 
 dim3 diff_grid(const DiffArgs &a) { return dim3((a.W + 15) / 16, (a.H + 7) / 8, a.nviews); }
 
-// HY_DIFF_GATHER: the adjoint's segment recompute (1) -- and the forward
-// too (2) -- sample the volume through a gather texture refreshed from the
-// caller's volume at each call (the refresh inside the timed launch); 0:
-// loads only.  256^3 f32, 16 views of 512^2, 32 knots, K = 32, per view:
-//   0: forward 1.34 ms, forward + adjoint 3.70 ms (2.79x), fit iteration 59.9 ms
-//   1: forward 1.34 ms, forward + adjoint 3.45 ms (2.58x), fit iteration 55.1 ms
-//   2: forward 0.88 ms, forward + adjoint 2.97 ms (3.38x), fit iteration 47.5 ms
-// 1 is the default: 2 gives the fastest fit, but its forward + adjoint is
-// more than three times its (faster) forward.
-#ifndef HY_DIFF_GATHER
-#define HY_DIFF_GATHER 1
-#endif
+// Both passes sample the volume through a gather texture refreshed from the
+// caller's volume at each call (inside the timed launch); by loads where the
+// device cannot make it.
 struct DiffGather {
     cudaArray_t arr = nullptr;
     unsigned long long tex = 0, surf = 0;
@@ -599,11 +659,15 @@ int diff_gather_refresh(hy_ctx *ctx, const float *vol, int n, DiffArgs &a, bool 
         ctx->diff_gather = g;
     }
     const int P = n + 2;
-    diff_fill_kernel<<<dim3((P + 127) / 128, P, P), 128, 0, ctx->stream>>>(vol, n, g->gper,
-                                                                          g->surf);
+    const dim3 grid((P + kFillRows - 1) / kFillRows, P);
+    if (P % 2 == 0)
+        diff_fill_kernel<true><<<grid, 256, 0, ctx->stream>>>(vol, n, g->gper, g->surf);
+    else
+        diff_fill_kernel<false><<<grid, 256, 0, ctx->stream>>>(vol, n, g->gper, g->surf);
     HY_CUDA(ctx, cudaGetLastError());
     a.gtex = g->tex;
     a.gper = g->gper;
+    a.gmagic = unsigned((1ull << 32) / unsigned(g->gper) + 1);
     *ok = true;
     return HY_OK;
 }
@@ -644,14 +708,12 @@ extern "C" int hy_diff_forward(hy_ctx *ctx, const hy_diff_params *p, const float
     // the texture's refresh is part of the timed launch
     HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     bool gathers = false;
-    if (HY_DIFF_GATHER >= 2) {
-        rc = diff_gather_refresh(ctx, vol_dev, p->n, a, &gathers);
-        if (rc) return rc;
-    }
+    rc = diff_gather_refresh(ctx, vol_dev, p->n, a, &gathers);
+    if (rc) return rc;
     if (gathers)
-        diff_forward_kernel<true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
+        diff_forward_kernel<4, true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
     else
-        diff_forward_kernel<false><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
+        diff_forward_kernel<1, false><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
     HY_CUDA(ctx, cudaGetLastError());
     HY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->stats_pending = true;
@@ -685,14 +747,14 @@ extern "C" int hy_diff_backward(hy_ctx *ctx, const hy_diff_params *p, const floa
     // the texture's refresh is part of the timed launch
     HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     bool gathers = false;
-    if (HY_DIFF_GATHER >= 1) {
-        rc = diff_gather_refresh(ctx, vol_dev, p->n, a, &gathers);
-        if (rc) return rc;
-    }
-    if (gathers)
-        diff_backward_kernel<true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
+    rc = diff_gather_refresh(ctx, vol_dev, p->n, a, &gathers);
+    if (rc) return rc;
+    if (gathers && (long long)W * H * nviews < 8 * 32ll * 4 * ctx->sms)
+        diff_backward_kernel<4, 4, true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
+    else if (gathers)
+        diff_backward_kernel<2, 8, true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
     else
-        diff_backward_kernel<false><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
+        diff_backward_kernel<1, 6, false><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
     HY_CUDA(ctx, cudaGetLastError());
     HY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->stats_pending = true;
