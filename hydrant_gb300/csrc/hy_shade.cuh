@@ -691,6 +691,21 @@ __device__ __forceinline__ float steps_to_face(float o, float s, float q, float 
 __device__ __forceinline__ int skip_plane(const SkipGrid &G, float sx, float sy, float sz) {
     return (int(sx < 0.f) + 2 * int(sy < 0.f) + 4 * int(sz < 0.f)) * G.plane;
 }
+// o after n steps of s, each rounded, at once: false where that is not known.
+// While o stays in one binade (ulp u), o + s = o + S + r with S the
+// rounded step, a multiple of u, and |r| <= u / 2; every o + S is a multiple
+// of u, so each step rounds to exactly o + S unless r is a tie (then the
+// parity of o decides).  S = fl(fl(o + s) - o) and r = s - S are exact there,
+// and fma(n, S, o) is too.  The last value may not be the binade's first
+// (below it the ulp halves).  n >= 1.
+__device__ __forceinline__ bool jump(float o, float s, float n, float &on) {
+    const float S = (o + s) - o, r = s - S;
+    on = __fmaf_rn(n, S, o);
+    const unsigned int bo = __float_as_uint(o), bn = __float_as_uint(on);
+    const unsigned int e = bo & 0x7f800000u;
+    return ((bo ^ bn) & 0xff800000u) == 0u && (bn & 0x7fffffu) != 0u && e >= (25u << 23) &&
+           fabsf(r) != __uint_as_float(e - (24u << 23));
+}
 // The byte of the cell at (x, y, z); 0 outside the grid and for NaN.
 __device__ __forceinline__ int skip_cell(const SkipGrid &G, int plane, float x, float y, float z,
                                          float &qx, float &qy, float &qz) {
@@ -700,8 +715,12 @@ __device__ __forceinline__ int skip_cell(const SkipGrid &G, int plane, float x, 
     if (!(qx >= 0.f && qx < G.fcx && qy >= 0.f && qy < G.fcy && qz >= 0.f && qz < G.fcz)) return 0;
     return __ldg(G.d + (plane + (int(qz) * G.cy + int(qy)) * G.cx + int(qx)));
 }
-__device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, float sy, float sz, int step_size,
-                                          unsigned int &samples) {
+// JUMP: runs of 12 steps and more by jump().  512^3 tubes' isosurface 984 ->
+// 935 us, f32 blobs 256 -> 248; the u8 march, whose runs are short at 1-voxel
+// steps, loses 1 % (896 -> 903) and keeps the additions.
+template <bool JUMP>
+__device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, float sy, float sz,
+                                          int step_size, unsigned int &samples) {
     const int plane = skip_plane(G, sx, sy, sz);
     while (p.nsteps > 0) {
         float qx, qy, qz;
@@ -716,6 +735,18 @@ __device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, fl
         n = min(n, ss == 1u ? left : (left + ss - 1u) / ss);
         samples += n;
         p.nsteps -= int(n * ss);
+        if (JUMP && n >= 12) {
+            float jx, jy, jz;
+            const bool ok = jump(p.ox, sx, float(n), jx) & jump(p.oy, sy, float(n), jy) &
+                            jump(p.oz, sz, float(n), jz);
+            if (ok) {
+                p.ox = jx;
+                p.oy = jy;
+                p.oz = jz;
+                continue;
+            }
+        }
+#pragma unroll 4
         for (; n > 0; --n) {
             p.ox = p.ox + sx;
             p.oy = p.oy + sy;
@@ -885,7 +916,7 @@ __device__ __forceinline__ long long volume_main(Px &p, const ShadeArgs &A, cons
         int hint = A.skip.d != nullptr;
         while (go && p.nsteps > 0) {
             if (hint) {
-                skip_free(p, A.skip, m.sx, m.sy, m.sz, p.step_size, samples);
+                skip_free<DT == HY_DTYPE_F32>(p, A.skip, m.sx, m.sy, m.sz, p.step_size, samples);
                 if (p.nsteps <= 0) break;
             }
             hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, A.skip.fstride);
@@ -919,7 +950,7 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
     int hint = A.skip.d != nullptr;
     while (p.nsteps > 0) {
         if (hint) {
-            skip_free(p, A.skip, m.sx, m.sy, m.sz, p.step_size, samples);
+            skip_free<DT == HY_DTYPE_F32>(p, A.skip, m.sx, m.sy, m.sz, p.step_size, samples);
             if (p.nsteps <= 0) break;
         }
         hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, A.skip.fstride);
@@ -1051,7 +1082,7 @@ __device__ __forceinline__ unsigned int volume_group(Px &p, bool on, const Shade
     while (__any_sync(full, p.nsteps > 0)) {
         if (hint && p.nsteps > 0) {
             unsigned int n = 0;
-            skip_free(p, A.skip, m.sx, m.sy, m.sz, p.step_size, n);
+            skip_free<DT == HY_DTYPE_F32>(p, A.skip, m.sx, m.sy, m.sz, p.step_size, n);
             if (j == 0) samples += n;
         }
         hint = skip_hint(p, A.skip, m.sx, m.sy, m.sz, float(K));
@@ -1364,7 +1395,7 @@ __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const V
     int hint = A.skip.d != nullptr;
     while (p.nsteps > 0 && !hit) {
         if (hint) {
-            skip_free(p, A.skip, sx, sy, sz, 1, samples);
+            skip_free<true>(p, A.skip, sx, sy, sz, 1, samples);
             if (p.nsteps <= 0) break;
         }
         hint = skip_hint(p, A.skip, sx, sy, sz, A.skip.fstride);
