@@ -25,108 +25,86 @@
 
 namespace {
 
+// Rows of a padded brick: a warp takes a row (its z, y and x clamped to the
+// volume, as the apron replicates the border), its lanes consecutive voxels.
+// What bounds both kernels is issue; a thread per voxel with 64-bit divisions
+// took 5.1 + 6.9 ms for 1024^3 u8 (one block per brick for the statistics:
+// 0.8 ms for a single 64^3 brick, 6.5 ms for 128^3), these 1.0 + 1.2.
+struct BrickArgs {
+    int dim[3];
+    int bs, pad, P;
+    int gx, gy;
+};
+
+__device__ __forceinline__ long long row_base(const BrickArgs &a, int bid, int z, int y) {
+    const int by = (bid / a.gx) % a.gy, bz = bid / (a.gx * a.gy);
+    const int Y = min(max(by * a.bs + y - a.pad, 0), a.dim[1] - 1);
+    const int Z = min(max(bz * a.bs + z - a.pad, 0), a.dim[2] - 1);
+    return ((long long)Z * a.dim[1] + Y) * a.dim[0];
+}
+
+// Emptiness and the sum of the core voxels of brick blockIdx.x, rows of the
+// slices of part blockIdx.y of gridDim.y: part sums are added up on the host.
 template <typename T>
-__global__ void brick_stats_kernel(const T *__restrict__ raw, int dx, int dy, int dz, int bs,
-                                   int pad, int gx, int gy, unsigned int *__restrict__ nonempty,
-                                   double *__restrict__ core_sum) {
-    const int bid = blockIdx.x;
-    const int bx = bid % gx, by = (bid / gx) % gy, bz = bid / (gx * gy);
-    const int P = bs + 2 * pad;
-    const long long P3 = (long long)P * P * P;
-    unsigned int any = 0;
+__global__ void __launch_bounds__(256) brick_stats_kernel(const T *__restrict__ raw,
+                                                          const __grid_constant__ BrickArgs a,
+                                                          unsigned int *__restrict__ nonempty,
+                                                          double *__restrict__ core_sum) {
+    const int bid = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int bx = bid % a.gx, P = a.P;
+    const int z0 = int((long long)P * blockIdx.y / gridDim.y),
+              z1 = int((long long)P * (blockIdx.y + 1) / gridDim.y);
+    const int hi = a.pad + a.bs;
+    bool any = false;
     double sum = 0.0;
-    for (long long i = threadIdx.x; i < P3; i += blockDim.x) {
-        int x = int(i % P), y = int((i / P) % P), z = int(i / ((long long)P * P));
-        int X = min(max(bx * bs + x - pad, 0), dx - 1);
-        int Y = min(max(by * bs + y - pad, 0), dy - 1);
-        int Z = min(max(bz * bs + z - pad, 0), dz - 1);
-        T v = raw[((long long)Z * dy + Y) * dx + X];
-        if (v != T(0)) any = 1;
-        bool core = x >= pad && x < pad + bs && y >= pad && y < pad + bs && z >= pad && z < pad + bs;
-        if (core) sum += double(v);
-    }
-    // block reduction
-    __shared__ double ssum[32];
-    __shared__ unsigned int sany[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_down_sync(0xffffffffu, sum, o);
-        any |= __shfl_down_sync(0xffffffffu, any, o);
-    }
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        ssum[warp] = sum;
-        sany[warp] = any;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        int nw = blockDim.x >> 5;
-        sum = lane < nw ? ssum[lane] : 0.0;
-        any = lane < nw ? sany[lane] : 0u;
-        for (int o = 16; o > 0; o >>= 1) {
-            sum += __shfl_down_sync(0xffffffffu, sum, o);
-            any |= __shfl_down_sync(0xffffffffu, any, o);
+    unsigned long long whole = 0;  // u8: exact, and no FP64 (slow on this GPU)
+    for (int r = z0 * P + warp; r < z1 * P; r += 8) {
+        const int z = r / P, y = r - z * P;
+        const T *row = raw + row_base(a, bid, z, y);
+        const bool core = z >= a.pad && z < hi && y >= a.pad && y < hi;
+        unsigned int rs = 0;  // a row's sum fits: P * 255
+        for (int x = lane; x < P; x += 32) {
+            const T v = row[min(max(bx * a.bs + x - a.pad, 0), a.dim[0] - 1)];
+            any |= v != T(0);
+            if constexpr (sizeof(T) == 1)
+                if (x >= a.pad && x < hi) rs += v;
         }
-        if (lane == 0) {
-            nonempty[bid] = any;
-            core_sum[bid] = sum;
+        if constexpr (sizeof(T) == 1) {
+            if (core) whole += rs;
+        } else if (core) {  // the core again (L1): full warps of FP64 additions
+            for (int x = a.pad + lane; x < hi; x += 32)
+                sum += double(row[min(bx * a.bs + x - a.pad, a.dim[0] - 1)]);
         }
+    }
+    if constexpr (sizeof(T) == 1) sum = double(whole);
+    __shared__ double ssum[8];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if (lane == 0) ssum[warp] = sum;
+    const int some = __syncthreads_or(any);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) sum += ssum[w];
+        const size_t i = size_t(bid) * gridDim.y + blockIdx.y;
+        nonempty[i] = some != 0;
+        core_sum[i] = sum;
     }
 }
 
 template <typename T>
-__global__ void brick_fill_kernel(const T *__restrict__ raw, int dx, int dy, int dz, int bs,
-                                  int pad, int gx, int gy, const int *__restrict__ slot_brick,
-                                  unsigned char *__restrict__ pool, long long slot_stride,
-                                  int slot0) {
-    const int slot = slot0 + blockIdx.y;
-    const int bid = slot_brick[slot];
-    const int bx = bid % gx, by = (bid / gx) % gy, bz = bid / (gx * gy);
-    const int P = bs + 2 * pad;
-    const long long P3 = (long long)P * P * P;
+__global__ void __launch_bounds__(256) brick_fill_kernel(const T *__restrict__ raw,
+                                                         const __grid_constant__ BrickArgs a,
+                                                         const int *__restrict__ slot_brick,
+                                                         unsigned char *__restrict__ pool,
+                                                         long long slot_stride, int slot0) {
+    const int slot = slot0 + blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int bid = slot_brick[slot], bx = bid % a.gx, P = a.P;
     T *dst = reinterpret_cast<T *>(pool + (long long)slot * slot_stride);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < P3;
-         i += (long long)gridDim.x * blockDim.x) {
-        int x = int(i % P), y = int((i / P) % P), z = int(i / ((long long)P * P));
-        int X = min(max(bx * bs + x - pad, 0), dx - 1);
-        int Y = min(max(by * bs + y - pad, 0), dy - 1);
-        int Z = min(max(bz * bs + z - pad, 0), dz - 1);
-        dst[i] = raw[((long long)Z * dy + Y) * dx + X];
+    for (int r = blockIdx.x * 8 + warp; r < P * P; r += gridDim.x * 8) {
+        const int z = r / P, y = r - z * P;
+        const T *row = raw + row_base(a, bid, z, y);
+        T *out = dst + (long long)r * P;
+        for (int x = lane; x < P; x += 32)
+            out[x] = row[min(max(bx * a.bs + x - a.pad, 0), a.dim[0] - 1)];
     }
-}
-
-// Chebyshev distance transform over the brick grid by 26-neighbour dilation.
-void chebyshev_transform(const std::vector<unsigned int> &nonempty, const int g[3],
-                         std::vector<int> &out) {
-    const int n = g[0] * g[1] * g[2];
-    const int cap = std::max(g[0], std::max(g[1], g[2]));
-    out.assign(n, -1);
-    for (int i = 0; i < n; ++i)
-        if (nonempty[i]) out[i] = 0;
-    std::vector<int> next;
-    for (int r = 1; r <= cap; ++r) {
-        next = out;
-        bool changed = false;
-        for (int z = 0; z < g[2]; ++z)
-            for (int y = 0; y < g[1]; ++y)
-                for (int x = 0; x < g[0]; ++x) {
-                    int id = (z * g[1] + y) * g[0] + x;
-                    if (out[id] >= 0) continue;
-                    for (int k = 0; k < 27; ++k) {
-                        int X = x + k % 3 - 1, Y = y + (k / 3) % 3 - 1, Z = z + k / 9 - 1;
-                        if (X < 0 || Y < 0 || Z < 0 || X >= g[0] || Y >= g[1] || Z >= g[2])
-                            continue;
-                        if (out[(Z * g[1] + Y) * g[0] + X] == r - 1) {
-                            next[id] = r;
-                            changed = true;
-                            break;
-                        }
-                    }
-                }
-        out.swap(next);
-        if (!changed) break;
-    }
-    for (int i = 0; i < n; ++i)
-        if (out[i] < 0) out[i] = cap;
 }
 
 // ---- gather textures ---------------------------------------------------------
@@ -216,6 +194,26 @@ int gather_check(hy_ctx *ctx, bool *ok) {
     return HY_OK;
 }
 
+// Slots first .. first + gridDim.y - 1 of the pool into a gather texture: a
+// brick's P^2 rows of P voxels are P^2 texel rows (slot i of the texture in
+// column i % cols, row block i / cols).  Texel pairs where P is even.  One
+// kernel for all bricks: a 2-D copy call per brick took half of a 1024^3
+// volume's upload.
+template <typename U>
+__global__ void __launch_bounds__(256) gather_fill_kernel(const unsigned char *__restrict__ pool,
+                                                          long long slot_stride, int P, int first,
+                                                          int slot0, int cols,
+                                                          cudaSurfaceObject_t surf) {
+    const int i = slot0 + blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x0 = (i % cols) * P, y0 = (i / cols) * P * P;
+    const U *src = reinterpret_cast<const U *>(pool + (long long)(first + i) * slot_stride);
+    const int W = P / int(sizeof(U));
+    for (int r = blockIdx.x * 8 + warp; r < P * P; r += gridDim.x * 8)
+        for (int x = lane; x < W; x += 32)
+            surf2Dwrite(src[(long long)r * W + x], surf, x0 + x * int(sizeof(U)), y0 + r,
+                        cudaBoundaryModeZero);
+}
+
 void free_gather(hy_volume *v) {
     for (auto t : v->atlas_tex) cudaDestroyTextureObject(cudaTextureObject_t(t));
     for (auto a : v->atlas) cudaFreeArray(a);
@@ -243,33 +241,45 @@ int build_gather(hy_volume *vol) {
     const int n = vol->resident;
     if ((long long)per * hy::kResidentGatherTextures < n) return HY_OK;  // more than two textures hold
     std::vector<hy::TexEntry> table(n);
-    cudaChannelFormatDesc cd = cudaCreateChannelDesc(8, 0, 0, 0, cudaChannelFormatKindUnsigned);
+    std::vector<cudaSurfaceObject_t> surfs;  // for the fill alone
+    auto drop_surfs = [&] {
+        cudaStreamSynchronize(ctx->stream);
+        for (auto sf : surfs) cudaDestroySurfaceObject(sf);
+        surfs.clear();
+    };
     for (int first = 0; first < n; first += per) {
         const int cnt = std::min(per, n - first);
         const int ucols = std::min(cols, cnt), urows = (cnt + cols - 1) / cols;
         cudaArray_t arr = nullptr;
-        cudaError_t e = cudaMallocArray(&arr, &cd, size_t(ucols) * P, size_t(urows) * brick_rows,
-                                        cudaArrayTextureGather);
-        if (e != cudaSuccess) {
+        unsigned long long t = 0, sf = 0;
+        rc = hy_gather_texture_create(ctx, size_t(ucols) * P, size_t(urows) * brick_rows, &arr, &t,
+                                      &sf);
+        if (rc) {
+            drop_surfs();
             free_gather(vol);
-            return hy_cuda_fail(ctx, e, "volume: gather texture allocation");
+            return rc;
         }
         vol->atlas.push_back(arr);
-        cudaTextureObject_t t = make_gather_texture(arr, &e);
-        if (e != cudaSuccess) {
-            free_gather(vol);
-            return hy_cuda_fail(ctx, e, "volume: gather texture object");
+        vol->atlas_tex.push_back(t);
+        surfs.push_back(cudaSurfaceObject_t(sf));
+        const unsigned gx = unsigned(std::min<long long>((brick_rows + 7) / 8, 64));
+        for (int s0 = 0; s0 < cnt; s0 += 65535) {
+            const dim3 grid(gx, unsigned(std::min(65535, cnt - s0)));
+            if (P % 2 == 0)
+                gather_fill_kernel<unsigned short><<<grid, 256, 0, ctx->stream>>>(
+                    vol->pool, (long long)vol->slot_stride, P, first, s0, cols, surfs.back());
+            else
+                gather_fill_kernel<unsigned char><<<grid, 256, 0, ctx->stream>>>(
+                    vol->pool, (long long)vol->slot_stride, P, first, s0, cols, surfs.back());
         }
-        vol->atlas_tex.push_back((unsigned long long)t);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) {
+            drop_surfs();
+            free_gather(vol);
+            return hy_cuda_fail(ctx, e, "volume: gather texture fill");
+        }
         for (int i = 0; i < cnt; ++i) {
             const int slot = first + i, cx = i % cols, ry = i / cols;
-            e = cudaMemcpy2DToArrayAsync(arr, size_t(cx) * P, size_t(ry) * brick_rows,
-                                         vol->pool + size_t(slot) * vol->slot_stride, P, P,
-                                         brick_rows, cudaMemcpyDeviceToDevice, ctx->stream);
-            if (e != cudaSuccess) {
-                free_gather(vol);
-                return hy_cuda_fail(ctx, e, "volume: gather texture fill");
-            }
             table[slot] = hy::TexEntry{float(cx * P), float(ry * brick_rows),
                                        int(vol->atlas_tex.size()) - 1, 0};
         }
@@ -298,6 +308,7 @@ int build_gather(hy_volume *vol) {
         e = cudaMemcpyAsync(vol->info4_dev, info4.data(), size_t(vol->nbricks) * sizeof(int4),
                             cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    drop_surfs();
     if (e != cudaSuccess) {
         free_gather(vol);
         return hy_cuda_fail(ctx, e, "volume: gather table");
@@ -347,21 +358,32 @@ int upload_impl(hy_volume *vol, const void *host) {
     HY_UP(cudaMalloc(&raw, nvox * sizeof(T)));
     HY_UP(cudaMemcpyAsync(raw, host, nvox * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
     const int nb = vol->nbricks;
-    HY_UP(cudaMalloc(&ne_dev, nb * sizeof(unsigned int)));
-    HY_UP(cudaMalloc(&sum_dev, nb * sizeof(double)));
-    brick_stats_kernel<T><<<nb, 256, 0, ctx->stream>>>(raw, d.dim[0], d.dim[1], d.dim[2],
-                                                       d.block_size, d.padding, vol->grid[0],
-                                                       vol->grid[1], ne_dev, sum_dev);
+    // enough blocks for the GPU when there are few bricks
+    const int parts = std::max(1, std::min(vol->P, 8 * ctx->sms / nb));
+    const size_t np = size_t(nb) * parts;
+    const BrickArgs ba{{d.dim[0], d.dim[1], d.dim[2]}, d.block_size, d.padding, vol->P,
+                       vol->grid[0], vol->grid[1]};
+    HY_UP(cudaMalloc(&ne_dev, np * sizeof(unsigned int)));
+    HY_UP(cudaMalloc(&sum_dev, np * sizeof(double)));
+    brick_stats_kernel<T><<<dim3(unsigned(nb), unsigned(parts)), 256, 0, ctx->stream>>>(
+        raw, ba, ne_dev, sum_dev);
     HY_UP(cudaGetLastError());
-    std::vector<unsigned int> ne(nb);
-    std::vector<double> sums(nb);
-    HY_UP(cudaMemcpyAsync(ne.data(), ne_dev, nb * sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                          ctx->stream));
-    HY_UP(cudaMemcpyAsync(sums.data(), sum_dev, nb * sizeof(double), cudaMemcpyDeviceToHost,
+    std::vector<unsigned int> ne_part(np);
+    std::vector<double> sum_part(np);
+    HY_UP(cudaMemcpyAsync(ne_part.data(), ne_dev, np * sizeof(unsigned int),
+                          cudaMemcpyDeviceToHost, ctx->stream));
+    HY_UP(cudaMemcpyAsync(sum_part.data(), sum_dev, np * sizeof(double), cudaMemcpyDeviceToHost,
                           ctx->stream));
     HY_UP(cudaStreamSynchronize(ctx->stream));
+    std::vector<unsigned char> ne(nb, 0);
+    std::vector<double> sums(nb, 0.0);
+    for (int i = 0; i < nb; ++i)
+        for (int k = 0; k < parts; ++k) {
+            ne[i] |= ne_part[size_t(i) * parts + k] ? 1 : 0;
+            sums[i] += sum_part[size_t(i) * parts + k];
+        }
 
-    chebyshev_transform(ne, vol->grid, vol->cheb);
+    hy_chebyshev_transform(ne, vol->grid, vol->cheb);
     const double ncore = double(d.block_size) * d.block_size * d.block_size;
     vol->mean.resize(nb);
     for (int i = 0; i < nb; ++i)
@@ -383,13 +405,11 @@ int upload_impl(hy_volume *vol, const void *host) {
         HY_UP(cudaMalloc(&slot_brick_dev, slot_brick.size() * sizeof(int)));
         HY_UP(cudaMemcpyAsync(slot_brick_dev, slot_brick.data(), slot_brick.size() * sizeof(int),
                               cudaMemcpyHostToDevice, ctx->stream));
-        const long long P3 = (long long)vol->P * vol->P * vol->P;
+        const unsigned gx = unsigned(std::min<long long>(((long long)vol->P * vol->P + 7) / 8, 64));
         for (int s0 = 0; s0 < vol->resident; s0 += 65535) {
             const int n = std::min(65535, vol->resident - s0);
-            dim3 grid(unsigned((P3 + 255) / 256 < 512 ? (P3 + 255) / 256 : 512), unsigned(n));
-            brick_fill_kernel<T><<<grid, 256, 0, ctx->stream>>>(
-                raw, d.dim[0], d.dim[1], d.dim[2], d.block_size, d.padding, vol->grid[0],
-                vol->grid[1], slot_brick_dev, vol->pool, (long long)vol->slot_stride, s0);
+            brick_fill_kernel<T><<<dim3(gx, unsigned(n)), 256, 0, ctx->stream>>>(
+                raw, ba, slot_brick_dev, vol->pool, (long long)vol->slot_stride, s0);
             HY_UP(cudaGetLastError());
         }
     }
