@@ -110,6 +110,22 @@ struct SkipGrid {
     float fstride;
 };
 
+// One brick move of a pager: store bytes at `src` -> cache slot `dst`.
+struct GatherItem {
+    long long src;
+    int dst;
+    int pad_;
+};
+
+// Where a pager's cache keeps its slots (after ncoarse coarse bricks): a pool,
+// or gather textures of gper bricks in gcols columns through their surfaces.
+struct CacheLayout {
+    const unsigned char *pool;
+    long long stride;
+    int ncoarse, gper, gcols;
+    unsigned long long surf[kMaxGatherTextures];
+};
+
 // Everything one shading launch reads; passed as a __grid_constant__ kernel
 // parameter (the reference copies its shader struct into a 16 KiB
 // __constant__ buffer per launch, cuda_shading.cu:5-10).
@@ -185,9 +201,11 @@ struct hy_skip {
     int c[3] = {0, 0, 0};
     long long cells = 0;
     float shrink = 0.f;
-    void *minmax = nullptr;
-    unsigned char *tmp = nullptr, *tmp2 = nullptr;  // one allocation with the grids
+    void *minmax = nullptr;  // per cell of the volume; paged: per brick's coarse stand-in
+    void *slots = nullptr;   // paged: per cache slot
+    int reg_base = 0;        // paged: registry ids from here on are slots
     unsigned char *grid[2] = {nullptr, nullptr};
+    unsigned int *bits = nullptr;  // work planes (in grid[0]'s allocation)
     bool valid[2] = {false, false};
     hy_skip_ranges key[2];
     // how many cells have their smallest voxel in value bin i or above and
@@ -289,6 +307,13 @@ void hy_chebyshev_transform(const std::vector<unsigned char> &nonempty, const in
 int hy_skip_build(hy_volume *v);
 void hy_skip_free(hy_volume *v);
 int hy_skip_view(hy_ctx *ctx, const hy_volume *v, const hy_shader_params *p, hy::SkipGrid *out);
+// A realtime pager's volume: cells per cache slot (hy_skip_slots after each
+// fill, on the fill's stream) and per coarse stand-in; the grid is renewed
+// after hy_skip_page_table_changed by the next hy_skip_view.
+int hy_skip_build_paged(hy_volume *v, const hy_store *store, int nslots, int reg_base);
+int hy_skip_slots(hy_volume *v, const hy::GatherItem *items, int n, const hy::CacheLayout &l,
+                  cudaStream_t stream);
+void hy_skip_page_table_changed(hy_volume *v);
 void hy_skip_tf_ranges(const float *rgba, int n, hy_skip_ranges *r, float *alpha_max);
 
 // error helpers (hy_api.cc)

@@ -697,16 +697,21 @@ extern "C" int hy_cull(const hy_volume *vol, const hy_view *view, const float re
 // ---------------------------------------------------------------------------
 namespace {
 
-// One brick move of a realtime frame: store bytes at `src` -> cache slot `dst`.
-struct GatherItem {
-    long long src;
-    int dst;
-    int pad_;
-};
+// Blocks per brick of the fills below: a block's reads of host memory are a
+// chain of 16 bytes a thread at the link's latency (a 287 KB brick by one block
+// of 256 threads took 90 us, whatever the number of bricks up to one per SM),
+// so fewer bricks than SMs are shared out over them: four frames of the
+// 1024x1024x512 volume (8 to 30 bricks a frame) 4.90 -> 4.63 ms.  Larger moves
+// reach the link's rate (210 GB/s, as a copy of the copy engine does) with a
+// block per brick; more blocks only take the march's place on the SMs (lossless
+// frame 3.71 ms, with 8 to 16 times the blocks 4.1 to 5.0).
+int fill_parts(const hy_ctx *ctx, int n) {
+    return std::max(1, std::min(16, ctx->sms / std::max(n, 1)));
+}
 
-// One block per brick: the slot is filled straight from the mapped pinned
-// store (the GPU reads host memory over the C2C link), 16 bytes per thread
-// and iteration; slot_stride is a multiple of 256 bytes.
+// The slot is filled straight from the mapped pinned store (the GPU reads host
+// memory over the C2C link), 16 bytes per thread and iteration; slot_stride is
+// a multiple of 256 bytes.
 __global__ void gather_bricks_kernel(const unsigned char *__restrict__ store,
                                      const GatherItem *__restrict__ items,
                                      unsigned char *__restrict__ pool, long long slot0,
@@ -715,30 +720,28 @@ __global__ void gather_bricks_kernel(const unsigned char *__restrict__ store,
     const uint4 *src = reinterpret_cast<const uint4 *>(store + it.src);
     uint4 *dst = reinterpret_cast<uint4 *>(pool + (slot0 + it.dst) * stride);
     const int n = int(stride / 16);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x)
+        dst[i] = src[i];
 }
 
-// The same moves into a cache held in gather textures: one block per brick
-// reads the record from the mapped pinned store (16 bytes per thread and
-// iteration) and writes it through the texture's surface, two texels per
+// The same moves into a cache held in gather textures: a brick's blocks
+// read the record from the mapped pinned store (16 bytes per thread and
+// iteration) and write it through the texture's surface, two texels per
 // write (P is even and every brick's column origin a multiple of P, so a
 // pair never straddles a row): record byte r = row * P + col lands at
 // texel (x0 + col, y0 + row).  Writes outside the array are dropped.
-struct GatherSurfaces {
-    unsigned long long s[hy::kMaxGatherTextures];
-};
 __global__ void fill_textures_kernel(const unsigned char *__restrict__ store,
-                                     const GatherItem *__restrict__ items, GatherSurfaces surf,
-                                     int P, int gper, int gcols, int slot0) {
+                                     const GatherItem *__restrict__ items,
+                                     const __grid_constant__ CacheLayout l, int P) {
     const GatherItem it = items[blockIdx.x];
-    const int g = slot0 + it.dst;
-    const int t = g / gper, i = g % gper;
-    const int x0 = (i % gcols) * P, y0 = (i / gcols) * P * P;
-    const cudaSurfaceObject_t so = cudaSurfaceObject_t(surf.s[t & (hy::kMaxGatherTextures - 1)]);
+    const int g = l.ncoarse + it.dst;
+    const int t = g / l.gper, i = g % l.gper;
+    const int x0 = (i % l.gcols) * P, y0 = (i / l.gcols) * P * P;
+    const cudaSurfaceObject_t so = cudaSurfaceObject_t(l.surf[t & (hy::kMaxGatherTextures - 1)]);
     const uint4 *src = reinterpret_cast<const uint4 *>(store + it.src);
     const int nbytes = P * P * P;
     const int nchunks = (nbytes + 15) / 16;
-    for (int j = threadIdx.x; j < nchunks; j += blockDim.x) {
+    for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < nchunks; j += gridDim.y * blockDim.x) {
         const uint4 q = src[j];
         const unsigned int w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -874,17 +877,18 @@ int move_bricks(hy_pager *pg, const int *bricks, const int *slots, int n, cudaSt
     HY_CUDA(ctx, cudaMemcpyAsync(dev, items, n * sizeof(GatherItem), cudaMemcpyHostToDevice,
                                  stream));
     HY_CUDA(ctx, cudaEventRecord(pg->gathered[buf], stream));
+    CacheLayout l{v->pool, (long long)v->slot_stride, pg->ncoarse, pg->gper, pg->gcols, {}};
+    for (int t = 0; t < hy::kMaxGatherTextures; ++t)
+        l.surf[t] = pg->surf[t] ? pg->surf[t] : pg->surf[0];
     if (pg->gathers) {
-        GatherSurfaces gs;
-        for (int t = 0; t < hy::kMaxGatherTextures; ++t)
-            gs.s[t] = pg->surf[t] ? pg->surf[t] : pg->surf[0];
-        fill_textures_kernel<<<n, 256, 0, stream>>>(pg->store->host_dev, dev, gs, v->P, pg->gper,
-                                                     pg->gcols, pg->ncoarse);
+        fill_textures_kernel<<<dim3(n, fill_parts(ctx, n)), 256, 0, stream>>>(pg->store->host_dev, dev, l, v->P);
     } else {
-        gather_bricks_kernel<<<n, 256, 0, stream>>>(pg->store->host_dev, dev, v->pool, pg->ncoarse,
+        gather_bricks_kernel<<<dim3(n, fill_parts(ctx, n)), 256, 0, stream>>>(pg->store->host_dev, dev, v->pool, pg->ncoarse,
                                                     (long long)v->slot_stride);
     }
     HY_CUDA(ctx, cudaGetLastError());
+    int rc = hy_skip_slots(v, dev, n, l, stream);
+    if (rc) return rc;
     pg->stats.uploads += n;
     pg->stats.upload_bytes += (int64_t)n * (int64_t)pg->store->slot_stride;
     return HY_OK;
@@ -1063,6 +1067,10 @@ extern "C" int hy_pager_create(hy_ctx *ctx, hy_store *store, const hy_pager_desc
     pg->stamp.assign(pg->nslots, -1);
     rc = upload_page_table(pg);
     if (rc) return fail(rc);
+    if (desc->mode == HY_PAGER_REALTIME) {
+        rc = hy_skip_build_paged(v, store, pg->nslots, pg->reg_base);
+        if (rc) return fail(rc);
+    }
     v->uploaded = true;
     *out = pg;
     return HY_OK;
@@ -1105,6 +1113,7 @@ extern "C" int hy_pager_destroy(hy_pager *pg) {
     if (pg->vol) {
         hy_volume *v = pg->vol;
         hy_volume_free_gather(v);
+        hy_skip_free(v);
         if (v->pool) cudaFree(v->pool);
         if (v->info_dev) cudaFree(v->info_dev);
         if (v->reg_dev) cudaFree(v->reg_dev);
@@ -1406,6 +1415,7 @@ int render_realtime(hy_pager *pg, const hy_shader_params *p, const hy_view &view
     if (rc) return rc;
     rc = upload_page_table(pg, pg->frame_buf);
     if (rc) return rc;
+    hy_skip_page_table_changed(v);
     pg->frame_buf ^= 1;
     int resident = 0;
     for (int s = 0; s < pg->nslots; ++s) resident += pg->owner[s] >= 0;

@@ -106,7 +106,7 @@ __global__ void HY_RENDER_LEAN_BOUNDS render_lean_kernel(const __grid_constant__
 }
 // The same march sampling by texture gathers (u8 bricks with an apron in
 // the volume's gather textures), one sample at a time, for large views with
-// nothing to pass over, early termination and paged caches: 64-view step, one launch per view, 169.6 ms at 48
+// nothing to pass over and for early termination: 64-view step, one launch per view, 169.6 ms at 48
 // registers against 172.4 at 56, 173.1 at 64 and 198.8 for the loads
 // (HY_RENDER_GATHER=0 builds the per-view path without gathers).
 #ifndef HY_RENDER_GATHER
@@ -115,9 +115,9 @@ __global__ void HY_RENDER_LEAN_BOUNDS render_lean_kernel(const __grid_constant__
 #ifndef HY_RENDER_GATHER_REGS
 #define HY_RENDER_GATHER_REGS 48
 #endif
-// The paged cache's march (each brick's own mapping, up to 16 textures):
-// 56 registers -- 21.2 ms per out-of-core frame against 24.6 at 48 (64 bytes
-// spilled) and 22.5 at 64.
+// The paged cache's march with early termination (each brick's own mapping, up
+// to 16 textures): 56 registers -- 21.2 ms per out-of-core frame against 24.6
+// at 48 (64 bytes spilled) and 22.5 at 64, measured without termination.
 #ifndef HY_RENDER_PAGED_GATHER_REGS
 #define HY_RENDER_PAGED_GATHER_REGS 56
 #endif
@@ -276,12 +276,23 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
     if constexpr (SHADER == HY_SHADER_VOLUME) {
         if (a.mode == HY_VOLUME_DEFAULT && !a.aux) {
             if constexpr (DT == HY_DTYPE_U8 && PADDED) {
-                if (a.vol.paged_gather) {  // a pager's cache in gather textures
+                if (a.vol.paged_gather) {
+                    // A pager's cache in gather textures: its lean march with
+                    // 4 samples in flight below 8 warps of rays a scheduler,
+                    // 2 above.  Four frames of the 1024x1024x512 noise volume
+                    // at 1024^2, half the visible bricks cached: 8.28 ms one
+                    // sample at a time, 5.29 with the skip grid, 4.91 two in
+                    // flight (5.45 four); 256^2 3.82, 3.57, 2.89 (2.40); opaque
+                    // knots 7.99, 8.05, 7.47 (8.19).
+                    const long long rays = (long long)a.view.W * a.view.H;
                     if (a.ert > 0.f)
                         render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherPaged, kLoopErt>
                             <<<g, kThreads, sm, s>>>(a);
+                    else if (rays < 8 * 32ll * a.schedulers)
+                        render_batches_kernel<SHADER, PC, DT, kGatherPaged, kLoopBatch4>
+                            <<<g, kThreads, sm, s>>>(a);
                     else
-                        render_lean_gather_kernel<SHADER, PC, DT, PADDED, kGatherPaged, kLoopOne>
+                        render_batches_kernel<SHADER, PC, DT, kGatherPaged, kLoopBatch2>
                             <<<g, kThreads, sm, s>>>(a);
                     return;
                 }

@@ -467,14 +467,15 @@ struct Footprint {
     float2 axy;
     float az;
 };
-template <int PC, bool GATHER>
+template <int PC, int GATHER>
 __device__ __forceinline__ Footprint footprint(const DevVolume &V, const BrickRef &b, float lx,
                                                float ly, float lz) {
     const int P = PC ? PC : V.P;
     const float fd = float(P);
-    const float k = GATHER ? V.map_k : b.k;
-    const float mbx = GATHER ? V.map_b : b.bx, mby = GATHER ? V.map_b : b.by,
-                mbz = GATHER ? V.map_b : b.bz;
+    constexpr bool one = GATHER == kGatherResident;  // every brick's mapping
+    const float k = one ? V.map_k : b.k;
+    const float mbx = one ? V.map_b : b.bx, mby = one ? V.map_b : b.by,
+                mbz = one ? V.map_b : b.bz;
     const float2 kl = mul2(f2(k, k), f2(lx, ly));
     const float2 fxy = mul2(f2(fd, fd), f2(__fadd_rn(kl.x, mbx), __fadd_rn(kl.y, mby)));
     const float fz = fd * (k * lz + mbz);
@@ -490,6 +491,40 @@ __device__ __forceinline__ Footprint footprint(const DevVolume &V, const BrickRe
         f.off = (int(flz) * P + int(fly)) * P + int(flx);
     }
     return f;
+}
+
+// The gathers of U samples of one brick of a paged cache: as gather2_indexed,
+// the texture named as a constant when the warp reads one.
+template <int U, int K>
+__device__ __forceinline__ void gathers_const(const DevVolume &V, const Footprint (&fp)[U],
+                                              float fd, float4 (&g0)[U], float4 (&g1)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) gather2_const<K>(V, fp[u].X, fp[u].Y, fd, g0[u], g1[u]);
+}
+template <int U>
+__device__ __forceinline__ void gathers_paged(const DevVolume &V, int which, unsigned int m,
+                                              const Footprint (&fp)[U], float fd, float4 (&g0)[U],
+                                              float4 (&g1)[U]) {
+    const int w0 = __shfl_sync(m, which, __ffs(m) - 1);
+    if (__all_sync(m, which == w0)) {
+        switch (w0) {
+            case 0: gathers_const<U, 0>(V, fp, fd, g0, g1); return;
+            case 1: gathers_const<U, 1>(V, fp, fd, g0, g1); return;
+            case 2: gathers_const<U, 2>(V, fp, fd, g0, g1); return;
+            case 3: gathers_const<U, 3>(V, fp, fd, g0, g1); return;
+            case 4: gathers_const<U, 4>(V, fp, fd, g0, g1); return;
+            case 5: gathers_const<U, 5>(V, fp, fd, g0, g1); return;
+            case 6: gathers_const<U, 6>(V, fp, fd, g0, g1); return;
+            case 7: gathers_const<U, 7>(V, fp, fd, g0, g1); return;
+            default: break;
+        }
+    }
+    const unsigned long long h = V.gtex[which];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        g0[u] = gather_r(h, fp[u].X, fp[u].Y);
+        g1[u] = gather_r(h, fp[u].X, fp[u].Y + fd);
+    }
 }
 
 // U samples of one brick by loads: all taps first, then the lerps, so that
@@ -989,14 +1024,16 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
                     uz = ok ? uz : lz;
                 }
                 n += ok;
-                fp[u] = footprint<PC, GATHER != 0>(V, m.c.br, ux, uy, uz);
+                fp[u] = footprint<PC, GATHER>(V, m.c.br, ux, uy, uz);
             }
             if constexpr (GATHER) {
                 const int P = PC ? PC : V.P;
                 const float fd = float(P);
                 float4 g0[U], g1[U];
                 const unsigned int am = __activemask();
-                if (__all_sync(am, m.c.br.which == 0)) {
+                if constexpr (GATHER == kGatherPaged) {
+                    gathers_paged<U>(V, m.c.br.which, am, fp, fd, g0, g1);
+                } else if (__all_sync(am, m.c.br.which == 0)) {
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         g0[u] = gather_r(V.gtex[0], fp[u].X, fp[u].Y);
@@ -1004,7 +1041,8 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
                     }
                 } else {
 #pragma unroll
-                    for (int u = 0; u < U; ++u) gather2(V, m.c.br.which, fp[u].X, fp[u].Y, fd, g0[u], g1[u]);
+                    for (int u = 0; u < U; ++u)
+                        gather2(V, m.c.br.which, fp[u].X, fp[u].Y, fd, g0[u], g1[u]);
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
@@ -1419,7 +1457,7 @@ __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const V
                     v[0] = sample_brick<PC, DT, PADDED>(c.br, V.P, lx, ly, lz, S.lut);
                 } else {
                     Footprint fp[U];
-                    fp[0] = footprint<PC, false>(V, c.br, lx, ly, lz);
+                    fp[0] = footprint<PC, 0>(V, c.br, lx, ly, lz);
                     bool ok = true;
 #pragma unroll
                     for (int u = 1; u < U; ++u) {
@@ -1433,7 +1471,7 @@ __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const V
                         uy = ok ? uy : ly;
                         uz = ok ? uz : lz;
                         n += ok;
-                        fp[u] = footprint<PC, false>(V, c.br, ux, uy, uz);
+                        fp[u] = footprint<PC, 0>(V, c.br, ux, uy, uz);
                     }
                     fetch_loads<U, PC, DT>(V, c.br, fp, v);
                 }

@@ -6,7 +6,7 @@
 // exact zero (v + 0 * t is v), or cannot cross the isovalue.  The upload
 // divides every brick into cells of about 8 voxels and keeps the smallest and
 // largest voxel a sample of the cell can touch.  Per transfer function (or
-// isovalue) four small kernels turn that into one byte per cell and direction
+// isovalue) six small kernels turn that into one byte per cell and direction
 // octant: 0, samples must be taken, or d > 0, the d^3 cells from this one on
 // in the ray's direction are free of effect, so a ray marches to the end of
 // that box with three additions per step (the positions round step by step
@@ -21,9 +21,8 @@
 // 103 and 95 us, the f32 view 192 and 219 us; 4 also takes eight times the
 // memory.
 //
-// Bound: the min/max kernel reads each voxel of the pool from DRAM once and
-// from L1 about twice per axis; the distance passes move a byte per cell and
-// live in L2 (1024^3 volume: 2 M cells, 14 planes).
+// Bound: the min/max kernel by L1 (each voxel about twice per axis); the
+// distances by writing a byte per cell and octant.
 
 #include <algorithm>
 #include <cmath>
@@ -34,19 +33,19 @@
 namespace {
 
 constexpr int kStride = 16;     // steps between two looks (hy_shade.cuh, skip_hint)
-constexpr int kMaxDist = 16;    // largest stored distance (box of 15 cells each way)
 constexpr long long kMaxGridCells = 1ll << 27;
 
 // Voxel range [lo, hi] (padded indices) that samples of cell c along one axis
 // can touch: positions l in [c, c + 1] / nc of the brick map to
-// u = bs * l + pad - 1/2 and read floor(u) and floor(u) + 1; 1e-3 voxels cover
-// the mapping's rounding (P <= 2^12 bricks: below 1e-3).
-__host__ __device__ inline void cell_taps(int c, int nc, int bs, int pad, int P, int *lo, int *hi) {
-    const float w = float(bs) / float(nc);
-    const int a = int(floorf(float(c) * w + float(pad) - .5f - 1e-3f));
-    const int b = int(floorf(float(c + 1) * w + float(pad) - .5f + 1e-3f)) + 1;
-    *lo = a < 0 ? 0 : a;
-    *hi = b > P - 1 ? P - 1 : b;
+// u = P * (k * l + b) - 1/2 and read floor(u) and floor(u) + 1; 1e-3 voxels cover
+// the mapping's rounding (P <= 2^12: below 1e-3).  A fine brick's mapping, or
+// a coarse stand-in's sub-box of its coarse brick.
+__device__ inline void cell_taps(int c, int nc, float k, float b, int P, int *lo, int *hi) {
+    const float s = 1.f / float(nc);
+    const int i = int(floorf(float(P) * (k * (float(c) * s) + b) - .5f - 1e-3f));
+    const int j = int(floorf(float(P) * (k * (float(c + 1) * s) + b) - .5f + 1e-3f)) + 1;
+    *lo = min(max(i, 0), P - 1);
+    *hi = min(max(j, 0), P - 1);
 }
 
 // What a cell keeps: the smallest and largest voxel, or lo > hi for a cell
@@ -57,28 +56,16 @@ struct MinMax {
     T lo, hi;
 };
 
-struct CellArgs {
-    const unsigned char *pool;
-    const hy::RegEntry *reg;
-    const int2 *info;
-    int gx, gy, gz;   // bricks
-    int nc;           // cells per brick edge
-    int bs, pad, P;
-};
-
-// gridDim.y blocks per brick, eight lanes per cell, each every eighth row of its taps
-// (a thread per cell, a serial chain of 1000 loads, took 91 us for 512 f32
-// bricks of 32^3 and 0.99 ms for 1024^3 u8).
+// The min/max of a brick's nc^3 cells, eight lanes per cell, each every eighth
+// row of its taps (a thread per cell, a serial chain of 1000 loads, took 91 us
+// for 512 f32 bricks of 32^3).  Blocks blockIdx.y of gridDim.y share a brick.
+// map: k and the offsets of the three axes; ld(x, y, z): a voxel; put(x, y, z,
+// m): the result of a cell.
 constexpr int kCellLanes = 8;
-template <typename T>
-__global__ void cell_minmax_kernel(const __grid_constant__ CellArgs a, MinMax<T> *__restrict__ out) {
-    const int b = blockIdx.x;
-    const int bx = b % a.gx, by = (b / a.gx) % a.gy, bz = b / (a.gx * a.gy);
-    const int2 in = a.info[b];
-    const bool sampled = in.x == 0 && in.y >= 0;
-    const T *v = reinterpret_cast<const T *>(a.pool + (sampled ? a.reg[in.y].offset : 0));
-    const int nc = a.nc, cells = nc * nc * nc;
-    const int cx = a.gx * nc, cy = a.gy * nc;
+template <typename T, typename Load, typename Put>
+__device__ __forceinline__ void brick_cells(int nc, int P, float4 map, bool sampled, Load ld,
+                                            Put put) {
+    const int cells = nc * nc * nc;
     const int k = threadIdx.x & (kCellLanes - 1);
     // whole warps go round together (the shuffles below)
     const int step = blockDim.x / kCellLanes;
@@ -89,17 +76,16 @@ __global__ void cell_minmax_kernel(const __grid_constant__ CellArgs a, MinMax<T>
         MinMax<T> m{T(1), T(0)};
         if (sampled) {
             int x0, x1, y0, y1, z0, z1;
-            cell_taps(x, nc, a.bs, a.pad, a.P, &x0, &x1);
-            cell_taps(y, nc, a.bs, a.pad, a.P, &y0, &y1);
-            cell_taps(z, nc, a.bs, a.pad, a.P, &z0, &z1);
-            T lo = v[((long long)z0 * a.P + y0) * a.P + x0], hi = lo;
+            cell_taps(x, nc, map.x, map.y, P, &x0, &x1);
+            cell_taps(y, nc, map.x, map.z, P, &y0, &y1);
+            cell_taps(z, nc, map.x, map.w, P, &z0, &z1);
+            T lo = ld(x0, y0, z0), hi = lo;
             int finite = 1;
             const int ny = y1 - y0 + 1, rows = ny * (z1 - z0 + 1);
             for (int r = k; r < rows; r += kCellLanes) {
                 const int dz = r / ny;
-                const T *row = v + ((long long)(z0 + dz) * a.P + y0 + (r - dz * ny)) * a.P;
                 for (int i = x0; i <= x1; ++i) {
-                    const T t = row[i];
+                    const T t = ld(i, y0 + (r - dz * ny), z0 + dz);
                     lo = t < lo ? t : lo;
                     hi = t > hi ? t : hi;
                     if constexpr (sizeof(T) == 4) finite &= fabsf(t) < 3e38f;
@@ -114,9 +100,81 @@ __global__ void cell_minmax_kernel(const __grid_constant__ CellArgs a, MinMax<T>
             }
             if (finite) m = MinMax<T>{lo, hi};
         }
-        if (k == 0 && c < cells)
-            out[((long long)(bz * nc + z) * cy + by * nc + y) * cx + bx * nc + x] = m;
+        if (k == 0 && c < cells) put(x, y, z, m);
     }
+}
+
+struct CellArgs {
+    const unsigned char *pool;
+    const hy::RegEntry *reg;
+    const int2 *info;
+    int gx, gy;  // bricks
+    int nc, P;
+};
+
+// A resident volume: brick blockIdx.x into the volume's grid of cells.
+template <typename T>
+__global__ void cell_minmax_kernel(const __grid_constant__ CellArgs a, MinMax<T> *__restrict__ out) {
+    const int b = blockIdx.x, nc = a.nc, P = a.P;
+    const int bx = b % a.gx, by = (b / a.gx) % a.gy, bz = b / (a.gx * a.gy);
+    const int2 in = a.info[b];
+    const bool sampled = in.x == 0 && in.y >= 0;
+    const hy::RegEntry e = a.reg[sampled ? in.y : 0];
+    const T *v = reinterpret_cast<const T *>(a.pool + e.offset);
+    const int cx = a.gx * nc, cy = a.gy * nc;
+    brick_cells<T>(
+        nc, P, make_float4(e.k, e.bx, e.by, e.bz), sampled,
+        [&](int x, int y, int z) { return v[((long long)z * P + y) * P + x]; },
+        [&](int x, int y, int z, MinMax<T> m) {
+            out[((long long)(bz * nc + z) * cy + by * nc + y) * cx + bx * nc + x] = m;
+        });
+}
+
+// A paged cache: the slots just filled (move list entry blockIdx.x), read back
+// from the pool or through the cache textures' surfaces; cells in
+// [slot][z][y][x] order.
+template <typename T, bool SURF>
+__global__ void slot_minmax_kernel(const hy::GatherItem *__restrict__ items,
+                                   const __grid_constant__ hy::CacheLayout l, int nc, int P,
+                                   float4 map, MinMax<T> *__restrict__ out) {
+    const int slot = items[blockIdx.x].dst;
+    const int g = l.ncoarse + slot;
+    MinMax<T> *o = out + (long long)slot * nc * nc * nc;
+    auto put = [&](int x, int y, int z, MinMax<T> m) { o[(z * nc + y) * nc + x] = m; };
+    if constexpr (SURF) {
+        const int t = g / l.gper, i = g % l.gper;
+        const int x0 = (i % l.gcols) * P, y0 = (i / l.gcols) * P * P;
+        const cudaSurfaceObject_t so =
+            cudaSurfaceObject_t(l.surf[t & (hy::kMaxGatherTextures - 1)]);
+        brick_cells<T>(
+            nc, P, map, true,
+            [&](int x, int y, int z) {
+                return T(surf2Dread<unsigned char>(so, x0 + x, y0 + z * P + y, cudaBoundaryModeZero));
+            },
+            put);
+    } else {
+        const T *v = reinterpret_cast<const T *>(l.pool + (long long)g * l.stride);
+        brick_cells<T>(
+            nc, P, map, true,
+            [&](int x, int y, int z) { return v[((long long)z * P + y) * P + x]; }, put);
+    }
+}
+
+// The coarse stand-in of brick blockIdx.x: its sub-box of coarse brick cid.
+template <typename T>
+__global__ void coarse_minmax_kernel(const unsigned char *__restrict__ coarse, long long stride,
+                                     const hy::RegEntry *__restrict__ reg, int gx, int gy, int sc,
+                                     int cgx, int cgy, int nc, int P, MinMax<T> *__restrict__ out) {
+    const int b = blockIdx.x;
+    const int x = b % gx, y = (b / gx) % gy, z = b / (gx * gy);
+    const int cid = ((z / sc) * cgy + y / sc) * cgx + x / sc;
+    const T *v = reinterpret_cast<const T *>(coarse + (long long)cid * stride);
+    const hy::RegEntry e = reg[b];
+    MinMax<T> *o = out + (long long)b * nc * nc * nc;
+    brick_cells<T>(
+        nc, P, make_float4(e.k, e.bx, e.by, e.bz), true,
+        [&](int i, int j, int k) { return v[((long long)k * P + j) * P + i]; },
+        [&](int i, int j, int k, MinMax<T> m) { o[(k * nc + j) * nc + i] = m; });
 }
 
 // Value bins of the cells' min/max histogram: 64 over [0, 1], the outer ones
@@ -147,7 +205,6 @@ __global__ void cell_hist_kernel(const MinMax<T> *__restrict__ mm, long long n, 
 struct ClassArgs {
     hy_skip_ranges r;
     float scale;  // voxel -> sample value: 1/255 (u8) or 1
-    long long n;
 };
 
 // 1: every sample of the cell lies in one of the ranges without effect; 0: it
@@ -156,60 +213,168 @@ struct ClassArgs {
 // most 3 * 3 * 2^-24 of the largest magnitude, u / 255 and n * s add one
 // rounding each: 2e-6 covers them three times over.
 template <typename T>
+__device__ __forceinline__ unsigned char cell_free(const ClassArgs &a, MinMax<T> m) {
+    if (m.lo > m.hi) return 0;
+    const float lo = float(m.lo) * a.scale, hi = float(m.hi) * a.scale;
+    const float e = 2e-6f * fmaxf(fabsf(lo), fabsf(hi)) + 1e-36f;  // and underflows
+    for (int k = 0; k < a.r.n; ++k)
+        if (lo - e >= a.r.lo[k] && hi + e <= a.r.hi[k]) return 1;
+    return 0;
+}
+// The grid is worked out in bits, 32 cells of a row to a word (rows padded with
+// zeros): free flags first, then per direction octant the cells from which a
+// cube of 2, 4, 8 and 16 free cells extends -- a cube of 2m is free when the
+// eight cubes of m at its corners are -- and last the distances as bytes, with
+// cubes of 3, 6 and 12 from overlapping ones of 2, 4 and 8.  A byte per cell
+// and scans along the axes took 130 us for a million cells; this takes 44.
+struct BitGrid {
+    int cx, cy, cz, w;   // cells per axis, words per row
+    unsigned int words;  // of one plane: below 2^27 (kMaxGridCells), so that
+                         // 32 threads a word number below 2^32
+};
+
+template <typename T>
 __global__ void classify_kernel(const __grid_constant__ ClassArgs a,
-                                const MinMax<T> *__restrict__ mm, unsigned char *__restrict__ out) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const MinMax<T> m = mm[i];
-    unsigned char free_ = 0;
-    if (!(m.lo > m.hi)) {
-        const float lo = float(m.lo) * a.scale, hi = float(m.hi) * a.scale;
-        const float e = 2e-6f * fmaxf(fabsf(lo), fabsf(hi)) + 1e-36f;  // and underflows
-        for (int k = 0; k < a.r.n; ++k)
-            if (lo - e >= a.r.lo[k] && hi + e <= a.r.hi[k]) free_ = 1;
+                                const __grid_constant__ BitGrid g,
+                                const MinMax<T> *__restrict__ mm, unsigned int *__restrict__ out) {
+    const unsigned int i = blockIdx.x * blockDim.x + threadIdx.x, word = i >> 5;
+    if (word >= g.words) return;  // whole warps
+    const unsigned int row = word / unsigned(g.w);
+    const int x = int(word - row * g.w) * 32 + int(i & 31);
+    const bool f = x < g.cx && cell_free(a, mm[(long long)row * g.cx + x]);
+    const unsigned int bits = __ballot_sync(0xffffffffu, f);
+    if ((i & 31) == 0) out[word] = bits;
+}
+// The same through a page table: a brick's cells are those of its slot, of its
+// coarse stand-in, or (empty or absent) to be looked at by the march.
+template <typename T>
+__global__ void classify_paged_kernel(const __grid_constant__ ClassArgs a,
+                                      const __grid_constant__ BitGrid g,
+                                      const int2 *__restrict__ info, int gx, int gy, int lg,
+                                      int reg_base, const MinMax<T> *__restrict__ slots,
+                                      const MinMax<T> *__restrict__ coarse,
+                                      unsigned int *__restrict__ out) {
+    const unsigned int i = blockIdx.x * blockDim.x + threadIdx.x, word = i >> 5;
+    if (word >= g.words) return;
+    const unsigned int row = word / unsigned(g.w);
+    const int x = int(word - row * g.w) * 32 + int(i & 31);
+    const int z = int(row / unsigned(g.cy)), y = int(row) - z * g.cy;
+    bool f = false;
+    if (x < g.cx) {  // nc = 1 << lg cells per brick edge
+        const int2 in = info[((z >> lg) * gy + (y >> lg)) * gx + (x >> lg)];
+        if (in.x == 0 && in.y >= 0) {
+            const int m = (1 << lg) - 1;
+            const int cell = ((((z & m) << lg) + (y & m)) << lg) + (x & m);
+            f = cell_free(a, in.y < reg_base ? coarse[((long long)in.y << (3 * lg)) + cell]
+                                             : slots[((long long)(in.y - reg_base) << (3 * lg)) + cell]);
+        }
     }
-    out[i] = free_;
+    const unsigned int bits = __ballot_sync(0xffffffffu, f);
+    if ((i & 31) == 0) out[word] = bits;
 }
 
-// One axis of the distance, both ways along it: the cells at stride `st`, n
-// of them; plane blockIdx.y of `in` holds free flags (first axis) or the
-// distances of the axes before, and gives the planes blockIdx.y (rays moving
-// up this axis) and blockIdx.y + gridDim.y (down) of `out`.  d(i) = the least
-// over k >= 0 of max(k, in(i +- k)), cells outside the grid 0.
-template <bool FIRST>
-__global__ void distance_kernel(const unsigned char *__restrict__ in,
-                                unsigned char *__restrict__ out, long long total, int n, int st) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const unsigned char *p = in + blockIdx.y * total;
-    const int c = int((i / st) % n);
-    auto at = [&](int k) -> int {
-        const int v = p[i + (long long)k * st];
-        return FIRST ? (v ? kMaxDist : 0) : v;
+// Word w of row (y, z) of `p` and the same cells moved by m along octant o's
+// x, anded; 0 outside the grid.
+__device__ __forceinline__ unsigned int row_pair(const unsigned int *__restrict__ p,
+                                                 const BitGrid &g, int w, int y, int z, int m,
+                                                 int o) {
+    if (y < 0 || y >= g.cy || z < 0 || z >= g.cz) return 0u;
+    const unsigned int *r = p + ((long long)z * g.cy + y) * g.w;
+    const unsigned int v = r[w];
+    if (!v) return 0u;
+    if (o & 1) return v & ((v << m) | (w > 0 ? r[w - 1] >> (32 - m) : 0u));
+    return v & ((v >> m) | (w + 1 < g.w ? r[w + 1] << (32 - m) : 0u));
+}
+// The cells whose eight corner cubes at distance m are all in `p`.
+__device__ __forceinline__ unsigned int cube_and(const unsigned int *__restrict__ p,
+                                                 const BitGrid &g, int w, int y, int z, int m,
+                                                 int o) {
+    const int dy = o & 2 ? -m : m, dz = o & 4 ? -m : m;
+    unsigned int v = row_pair(p, g, w, y, z, m, o);
+    if (v) v &= row_pair(p, g, w, y + dy, z, m, o);
+    if (v) v &= row_pair(p, g, w, y, z + dz, m, o);
+    if (v) v &= row_pair(p, g, w, y + dy, z + dz, m, o);
+    return v;
+}
+// Cubes of m (one plane for all octants, or eight) -> cubes of 2 m.
+__global__ void double_kernel(const unsigned int *__restrict__ in, int in_planes,
+                              const __grid_constant__ BitGrid g, int m,
+                              unsigned int *__restrict__ out) {
+    const unsigned int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.words) return;
+    const int o = blockIdx.y;
+    const unsigned int row = i / unsigned(g.w);
+    const int w = int(i - row * g.w), z = int(row / unsigned(g.cy)), y = int(row) - z * g.cy;
+    const long long plane = (long long)o * g.words;
+    out[plane + i] = cube_and(in + (in_planes > 1 ? plane : 0), g, w, y, z, m, o);
+}
+// Four cells' distances from their bits of the planes: 1 for each of the cubes
+// of 1, 2, 3 and 4, 2 for 6 and 8, 4 for 12 and 16.
+__global__ void distance_kernel(const unsigned int *__restrict__ f1,
+                                const unsigned int *__restrict__ cubes,
+                                const __grid_constant__ BitGrid g,
+                                unsigned char *__restrict__ out) {
+    const unsigned int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.words) return;
+    const int o = blockIdx.y;
+    const unsigned int row = i / unsigned(g.w);
+    const int w = int(i - row * g.w), z = int(row / unsigned(g.cy)), y = int(row) - z * g.cy;
+    const unsigned int *p = cubes + (long long)o * g.words;
+    const long long level = 8ll * g.words;  // planes of one cube size
+    const unsigned int b1 = f1[i], b2 = b1 ? p[i] : 0u, b4 = b2 ? p[level + i] : 0u,
+                       b8 = b4 ? p[2 * level + i] : 0u, b16 = b8 ? p[3 * level + i] : 0u;
+    const unsigned int b3 = b2 ? cube_and(p, g, w, y, z, 1, o) : 0u,
+                       b6 = b4 ? cube_and(p + level, g, w, y, z, 2, o) : 0u,
+                       b12 = b8 ? cube_and(p + 2 * level, g, w, y, z, 4, o) : 0u;
+    unsigned char *q = out + o * ((long long)g.cx * g.cy * g.cz) + (long long)row * g.cx + w * 32;
+    const int n = min(32, g.cx - w * 32);
+    // bits 0..3 to the low bits of four bytes
+    auto spread = [](unsigned int b, int k) {
+        return ((((b >> k) & 15u) * 0x00204081u) & 0x01010101u);
     };
-    int up = at(0), dn = up;
-    for (int k = 1; k < up; ++k) up = min(up, max(k, c + k >= n ? 0 : at(k)));
-    for (int k = 1; k < dn; ++k) dn = min(dn, max(k, c - k < 0 ? 0 : at(-k)));
-    out[blockIdx.y * total + i] = (unsigned char)up;
-    out[(blockIdx.y + gridDim.y) * total + i] = (unsigned char)dn;
+    unsigned int d[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        d[k] = spread(b1, 4 * k) + spread(b2, 4 * k) + spread(b3, 4 * k) + spread(b4, 4 * k) +
+               2u * (spread(b6, 4 * k) + spread(b8, 4 * k)) +
+               4u * (spread(b12, 4 * k) + spread(b16, 4 * k));
+    if ((g.cx & 31) == 0) {  // whole, aligned words of cells
+        reinterpret_cast<uint4 *>(q)[0] = make_uint4(d[0], d[1], d[2], d[3]);
+        reinterpret_cast<uint4 *>(q)[1] = make_uint4(d[4], d[5], d[6], d[7]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+            if (k < n) q[k] = (unsigned char)(d[k >> 2] >> (8 * (k & 3)));
+    }
+}
+
+BitGrid bit_grid(const hy_skip &s) {
+    const int w = (s.c[0] + 31) / 32;
+    return BitGrid{s.c[0], s.c[1], s.c[2], w, unsigned(w) * unsigned(s.c[1]) * unsigned(s.c[2])};
 }
 
 template <typename T>
 int classify(hy_volume *v, const hy_skip_ranges &r, unsigned char *grid) {
     hy_ctx *ctx = v->ctx;
     hy_skip &s = v->skip;
-    const long long n = s.cells;
-    const unsigned blocks = unsigned((n + 255) / 256);
-    ClassArgs a{r, sizeof(T) == 1 ? 1.f / 255.f : 1.f, n};
-    const long long cx = (long long)s.c[0], cxy = cx * s.c[1];
-    // free flags in the first plane of the result, then x (2 planes), y (4), z (8)
-    classify_kernel<T><<<blocks, 256, 0, ctx->stream>>>(
-        a, static_cast<const MinMax<T> *>(s.minmax), grid);
-    distance_kernel<true><<<dim3(blocks, 1), 256, 0, ctx->stream>>>(grid, s.tmp, n, s.c[0], 1);
-    distance_kernel<false><<<dim3(blocks, 2), 256, 0, ctx->stream>>>(s.tmp, s.tmp2, n, s.c[1],
-                                                                     int(cx));
-    distance_kernel<false><<<dim3(blocks, 4), 256, 0, ctx->stream>>>(s.tmp2, grid, n, s.c[2],
-                                                                     int(cxy));
+    const ClassArgs a{r, sizeof(T) == 1 ? 1.f / 255.f : 1.f};
+    const BitGrid g = bit_grid(s);
+    const unsigned by_cell = (g.words + 7) / 8, by_word = (g.words + 127) / 128;
+    unsigned int *f1 = s.bits, *cubes = s.bits + g.words;
+    int lg = 0;
+    while ((1 << lg) < s.nc) ++lg;
+    if (s.slots)
+        classify_paged_kernel<T><<<by_cell, 256, 0, ctx->stream>>>(
+            a, g, v->info_dev, v->grid[0], v->grid[1], lg, s.reg_base,
+            static_cast<const MinMax<T> *>(s.slots), static_cast<const MinMax<T> *>(s.minmax), f1);
+    else
+        classify_kernel<T><<<by_cell, 256, 0, ctx->stream>>>(
+            a, g, static_cast<const MinMax<T> *>(s.minmax), f1);
+    for (int k = 0; k < 4; ++k)
+        double_kernel<<<dim3(by_word, 8), 128, 0, ctx->stream>>>(
+            k ? cubes + (k - 1) * 8ll * g.words : f1, k ? 8 : 1, g, 1 << k,
+            cubes + k * 8ll * g.words);
+    distance_kernel<<<dim3(by_word, 8), 128, 0, ctx->stream>>>(f1, cubes, g, grid);
     HY_CUDA(ctx, cudaGetLastError());
     return HY_OK;
 }
@@ -222,7 +387,7 @@ int cell_hist(hy_volume *v) {
     hy_skip &s = v->skip;
     int *dev = reinterpret_cast<int *>(s.grid[0]);  // 16 KB of the grids, unused until a render
     int *own = nullptr;
-    if (s.cells * 8 < (long long)(sizeof(int) * kBins * kBins)) {
+    if (s.cells * 8 < (long long)(sizeof(int) * kBins * kBins)) {  // (or of its own)
         HY_CUDA(ctx, cudaMalloc(&own, sizeof(int) * kBins * kBins));
         dev = own;
     }
@@ -276,17 +441,20 @@ bool same_ranges(const hy_skip_ranges &a, const hy_skip_ranges &b) {
 void hy_skip_free(hy_volume *v) {
     hy_skip &s = v->skip;
     if (s.minmax) cudaFree(s.minmax);
-    if (s.tmp) cudaFree(s.tmp);
+    if (s.slots) cudaFree(s.slots);
+    if (s.grid[0]) cudaFree(s.grid[0]);
     s = hy_skip();
 }
 
-int hy_skip_build(hy_volume *v) {
-    hy_ctx *ctx = v->ctx;
+namespace {
+
+// Cells of a volume's bricks and the box margin; s.nc stays 0 where the
+// volume has no grid.  The interior sampler's bricks only (an apron: no
+// wrapped coordinates).
+void skip_geometry(hy_volume *v) {
     hy_skip &s = v->skip;
-    hy_skip_free(v);
     const int bs = v->desc.block_size;
-    // the interior sampler's bricks only (an apron: no wrapped coordinates)
-    if (v->desc.padding < 1 || v->resident <= 0 || v->P > 4096) return HY_OK;
+    if (v->desc.padding < 1 || v->P > 4096) return;
     int nc = 1;  // a power of two (positions scale exactly), cells of >= 8 voxels
     while (nc * 2 * 8 <= bs) nc *= 2;
     long long n = 1;
@@ -296,36 +464,64 @@ int hy_skip_build(hy_volume *v) {
         n *= s.c[i];
         gmax = std::max(gmax, v->grid[i]);
     }
-    if (n > kMaxGridCells) return HY_OK;
+    if (n > kMaxGridCells) return;
     // A run of up to 127 steps adds up to 127 roundings of half an ulp of
     // the largest coordinate; 4e-6 brick covers the run length's own
     // arithmetic.  Boxes shrink by this much, so that a run that stays in one
     // by this arithmetic stays in it step by step.
     const float ulp = std::nextafterf(float(gmax), 1e30f) - float(gmax);
     s.shrink = 128.f * ulp + 4e-6f;
-    if (s.shrink * float(nc) > .125f) return HY_OK;  // a volume of thousands of bricks an edge
+    if (s.shrink * float(nc) > .125f) return;  // a volume of thousands of bricks an edge
     s.nc = nc;
     s.cells = n;
+}
+
+// Threads and blocks per brick for brick_cells: enough for the GPU when there
+// are few bricks.
+dim3 cells_grid(const hy_volume *v, int bricks, int *threads) {
+    const int lanes = v->skip.nc * v->skip.nc * v->skip.nc * kCellLanes;
+    *threads = std::min(512, std::max(32, lanes));
+    const int rounds = (lanes + *threads - 1) / *threads;
+    return dim3(unsigned(bricks),
+                unsigned(std::max(1, std::min(rounds, 8 * v->ctx->sms / std::max(bricks, 1)))));
+}
+
+// The distances per transfer function and (iso) per isovalue, and the bit
+// planes they are worked out in, in one allocation.
+cudaError_t alloc_planes(hy_skip &s, bool iso) {
+    const size_t n = size_t(s.cells), grids = (n * (iso ? 16 : 8) + 255) / 256 * 256;
+    const cudaError_t e =
+        cudaMalloc(&s.grid[0], grids + size_t(bit_grid(s).words) * 33 * sizeof(unsigned int));
+    if (e != cudaSuccess) return e;
+    s.grid[1] = iso ? s.grid[0] + 8 * n : nullptr;
+    s.bits = reinterpret_cast<unsigned int *>(s.grid[0] + grids);
+    return e;
+}
+
+size_t mm_bytes(const hy_volume *v) {
+    return v->desc.dtype == HY_DTYPE_U8 ? sizeof(MinMax<unsigned char>) : sizeof(MinMax<float>);
+}
+
+}  // namespace
+
+int hy_skip_build(hy_volume *v) {
+    hy_ctx *ctx = v->ctx;
+    hy_skip &s = v->skip;
+    hy_skip_free(v);
+    if (v->resident <= 0) return HY_OK;
+    skip_geometry(v);
+    if (!s.nc) return HY_OK;
     const bool u8 = v->desc.dtype == HY_DTYPE_U8;
-    cudaError_t e = cudaMalloc(&s.minmax, size_t(n) * (u8 ? sizeof(MinMax<unsigned char>)
-                                                          : sizeof(MinMax<float>)));
-    // the distances per transfer function and per isovalue, and two work grids
-    if (e == cudaSuccess) e = cudaMalloc(&s.tmp, size_t(n) * (2 + 4 + 8 + 8));
+    cudaError_t e = cudaMalloc(&s.minmax, size_t(s.cells) * mm_bytes(v));
+    if (e == cudaSuccess) e = alloc_planes(s, true);
     if (e != cudaSuccess) {  // no room: the march samples every cell
         hy_skip_free(v);
         cudaGetLastError();
         return HY_OK;
     }
-    s.tmp2 = s.tmp + 2 * n;
-    s.grid[0] = s.tmp2 + 4 * n;
-    s.grid[1] = s.grid[0] + 8 * n;
-    CellArgs a{v->pool, v->reg_dev, v->info_dev, v->grid[0], v->grid[1], v->grid[2], nc, bs,
-               v->desc.padding, v->P};
-    const int threads = std::min(512, std::max(32, nc * nc * nc * kCellLanes));
-    // enough blocks for the GPU when there are few bricks
-    const int rounds = (nc * nc * nc * kCellLanes + threads - 1) / threads;
-    const dim3 grid(unsigned(v->nbricks),
-                    unsigned(std::max(1, std::min(rounds, 8 * ctx->sms / v->nbricks))));
+    CellArgs a{v->pool, v->reg_dev, v->info_dev, v->grid[0], v->grid[1], s.nc, v->P};
+    int threads;
+    const dim3 grid = cells_grid(v, v->nbricks, &threads);
     if (u8)
         cell_minmax_kernel<unsigned char><<<grid, threads, 0, ctx->stream>>>(
             a, static_cast<MinMax<unsigned char> *>(s.minmax));
@@ -335,6 +531,72 @@ int hy_skip_build(hy_volume *v) {
     HY_CUDA(ctx, cudaGetLastError());
     return u8 ? cell_hist<unsigned char>(v) : cell_hist<float>(v);
 }
+
+int hy_skip_build_paged(hy_volume *v, const hy_store *store, int nslots, int reg_base) {
+    hy_ctx *ctx = v->ctx;
+    hy_skip &s = v->skip;
+    hy_skip_free(v);
+    skip_geometry(v);
+    if (!s.nc) return HY_OK;
+    const bool u8 = v->desc.dtype == HY_DTYPE_U8;
+    const size_t per = size_t(s.nc) * s.nc * s.nc * mm_bytes(v);
+    unsigned char *coarse = nullptr;  // the coarse level, for its cells alone
+    s.reg_base = reg_base;
+    cudaError_t e = cudaMalloc(&s.slots, size_t(nslots) * per);
+    if (e == cudaSuccess) e = alloc_planes(s, !v->paged_gather);
+    if (e == cudaSuccess && reg_base > 0) {
+        e = cudaMalloc(&s.minmax, size_t(v->nbricks) * per);
+        if (e == cudaSuccess) e = cudaMalloc(&coarse, store->coarse.size());
+    }
+    if (e != cudaSuccess) {
+        hy_skip_free(v);
+        cudaGetLastError();
+        return HY_OK;
+    }
+    if (reg_base > 0) {
+        e = cudaMemcpyAsync(coarse, store->coarse.data(), store->coarse.size(),
+                            cudaMemcpyHostToDevice, ctx->stream);
+        int threads;
+        const dim3 grid = cells_grid(v, v->nbricks, &threads);
+        const int sc = 1 << store->coarse_level;
+        const int *cg = store->coarse_grid;
+        if (e == cudaSuccess && u8)
+            coarse_minmax_kernel<unsigned char><<<grid, threads, 0, ctx->stream>>>(
+                coarse, (long long)v->slot_stride, v->reg_dev, v->grid[0], v->grid[1], sc, cg[0],
+                cg[1], s.nc, v->P, static_cast<MinMax<unsigned char> *>(s.minmax));
+        else if (e == cudaSuccess)
+            coarse_minmax_kernel<float><<<grid, threads, 0, ctx->stream>>>(
+                coarse, (long long)v->slot_stride, v->reg_dev, v->grid[0], v->grid[1], sc, cg[0],
+                cg[1], s.nc, v->P, static_cast<MinMax<float> *>(s.minmax));
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        cudaFree(coarse);
+        if (e != cudaSuccess) return hy_cuda_fail(ctx, e, "pager: skip grid");
+    }
+    return HY_OK;
+}
+
+int hy_skip_slots(hy_volume *v, const hy::GatherItem *items, int n, const hy::CacheLayout &l,
+                  cudaStream_t stream) {
+    hy_skip &s = v->skip;
+    if (!s.slots || n <= 0) return HY_OK;
+    int threads;
+    const dim3 grid = cells_grid(v, n, &threads);
+    const float4 map = make_float4(v->k, v->b, v->b, v->b);
+    if (v->paged_gather)
+        slot_minmax_kernel<unsigned char, true><<<grid, threads, 0, stream>>>(
+            items, l, s.nc, v->P, map, static_cast<MinMax<unsigned char> *>(s.slots));
+    else if (v->desc.dtype == HY_DTYPE_U8)
+        slot_minmax_kernel<unsigned char, false><<<grid, threads, 0, stream>>>(
+            items, l, s.nc, v->P, map, static_cast<MinMax<unsigned char> *>(s.slots));
+    else
+        slot_minmax_kernel<float, false><<<grid, threads, 0, stream>>>(
+            items, l, s.nc, v->P, map, static_cast<MinMax<float> *>(s.slots));
+    HY_CUDA(v->ctx, cudaGetLastError());
+    return HY_OK;
+}
+
+void hy_skip_page_table_changed(hy_volume *v) { v->skip.valid[0] = v->skip.valid[1] = false; }
 
 // The value ranges in which a sample leaves a Volume march as it is: between
 // the first and last of a run of knots whose opacity is zero (the lerp of two
@@ -396,7 +658,8 @@ int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy
         // With less than a tenth of the cells free the looks cost more than
         // the samples passed over: a march without a free cell takes 3 to 5 %
         // longer with the grid than without.
-        if (free_cells(s, r) * 10 < s.sampled) return HY_OK;
+        // (a paged cache's cells are not counted.)
+        if (!s.slots && free_cells(s, r) * 10 < s.sampled) return HY_OK;
     } else if (p->shader == HY_SHADER_ISOSURFACE) {
         // crossed: value and 0 on different sides of the isovalue
         which = 1;
@@ -413,7 +676,7 @@ int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy
     } else {
         return HY_OK;
     }
-    if (r.n == 0) return HY_OK;
+    if (r.n == 0 || !s.grid[which]) return HY_OK;
     // A capture would replay against whatever knots the grid holds by then:
     // captured launches sample every cell.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
