@@ -198,8 +198,10 @@ __device__ __forceinline__ void batch_body(const BatchArgs &B) {
 template <int SHADER, int PC, int DT, bool PADDED, int COMPOSITE, int GATHER = 0,
           int LOOP = kLoopOne>
 __global__ void __launch_bounds__(kMaxBlockThreads,
-                                  (COMPOSITE && GATHER) ? HY_BATCH_COMPOSITE_GATHER_MIN_BLOCKS
-                                                        : HY_BATCH_MIN_BLOCKS)
+                                  LOOP == kLoopBatch4 ? 2
+                                  : (COMPOSITE && GATHER && LOOP == kLoopOne)
+                                      ? HY_BATCH_COMPOSITE_GATHER_MIN_BLOCKS
+                                      : HY_BATCH_MIN_BLOCKS)
     batch_kernel(const __grid_constant__ BatchArgs B) {
     batch_body<SHADER, PC, DT, PADDED, COMPOSITE, false, GATHER, LOOP>(B);
 }
@@ -269,21 +271,31 @@ const void *pick_lean(const ShadeArgs &a, int steps_per_iter, long long rays) {
     return reinterpret_cast<const void *>(&batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopOne>);
 }
 
+// the Volume shader's per-brick segments sample by gathers too
+template <int SHADER, int PC, int DT, int LOOP>
+const void *pick_composite(const ShadeArgs &a) {
+    if constexpr (SHADER == HY_SHADER_VOLUME && DT == HY_DTYPE_U8) {
+        if (a.vol.tex && HY_BATCH_COMPOSITE_GATHER)
+            return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, true, 1, true, LOOP>);
+    }
+    return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, true, 1, false, LOOP>);
+}
+
 template <int SHADER, int PC, int DT, bool PADDED>
 const void *pick_c(const ShadeArgs &a, int steps_per_iter, long long rays) {
     if (a.composite) {
-        // the Volume shader's per-brick segments sample by gathers too
-        if constexpr (SHADER == HY_SHADER_VOLUME && DT == HY_DTYPE_U8 && PADDED) {
-            if (a.vol.tex && HY_BATCH_COMPOSITE_GATHER)
-                return a.skip.d ? reinterpret_cast<const void *>(
-                                      &batch_kernel<SHADER, PC, DT, PADDED, 1, true, kLoopSkip>)
-                                : reinterpret_cast<const void *>(
-                                      &batch_kernel<SHADER, PC, DT, PADDED, 1, true>);
-        }
-        if constexpr (SHADER == HY_SHADER_VOLUME && PADDED) {
-            if (a.skip.d)
-                return reinterpret_cast<const void *>(
-                    &batch_kernel<SHADER, PC, DT, PADDED, 1, false, kLoopSkip>);
+        if constexpr (PADDED && (SHADER == HY_SHADER_VOLUME || SHADER == HY_SHADER_ISOSURFACE)) {
+            // samples in flight as for one view (pick_composite, hy_render.cu):
+            // six views of 200^2 and 300^2 978 -> 839 us, of 256^2 to 1024^2
+            // 3604 -> 3345 (three blocks an SM 3499)
+            constexpr bool volume = SHADER == HY_SHADER_VOLUME;
+            if (a.vol.P <= kMaxBatchesP && (!volume || a.mode == HY_VOLUME_DEFAULT)) {
+                if (rays < 8 * 32ll * a.schedulers)
+                    return pick_composite<SHADER, PC, DT, kLoopBatch4>(a);
+                if constexpr (volume)
+                    if (a.skip.d) return pick_composite<SHADER, PC, DT, kLoopBatch2>(a);
+            }
+            return pick_composite<SHADER, PC, DT, kLoopOne>(a);
         }
         return reinterpret_cast<const void *>(&batch_kernel<SHADER, PC, DT, PADDED, 1>);
     }

@@ -171,9 +171,9 @@ __global__ void __launch_bounds__(kThreads) render_group_kernel(const __grid_con
 // held to 64 registers (8 resident blocks): on the 512^3 tubes at 1024^2,
 // Volume 147 -> 163 and Isosurface 231 -> 237 Gsamples/s against 80
 // registers and 6 blocks unbounded (Blocks is 3 % faster unbounded and keeps
-// render_kernel).
-template <int SHADER, int PC, int DT, bool PADDED, int LOOP = kLoopOne>
-__global__ void __launch_bounds__(kThreads, 8)
+// render_kernel); 128 registers with four samples in flight.
+template <int SHADER, int PC, int DT, bool PADDED, int LOOP>
+__global__ void __launch_bounds__(kThreads, LOOP == kLoopBatch4 ? 4 : 8)
     render_composite_kernel(const __grid_constant__ ShadeArgs A) {
     render_body<SHADER, PC, DT, PADDED, 1, false, false, LOOP>(A);
 }
@@ -183,13 +183,48 @@ __global__ void __launch_bounds__(kThreads, 8)
 #ifndef HY_RENDER_COMPOSITE_GATHER
 #define HY_RENDER_COMPOSITE_GATHER 1
 #endif
-#ifndef HY_RENDER_COMPOSITE_GATHER_BLOCKS
-#define HY_RENDER_COMPOSITE_GATHER_BLOCKS 8
-#endif
 template <int SHADER, int PC, int DT, bool PADDED, int LOOP>
-__global__ void __launch_bounds__(kThreads, HY_RENDER_COMPOSITE_GATHER_BLOCKS)
+__global__ void __launch_bounds__(kThreads, LOOP == kLoopBatch4 ? 4 : 8)
     render_composite_gather_kernel(const __grid_constant__ ShadeArgs A) {
     render_body<SHADER, PC, DT, PADDED, 1, false, true, LOOP>(A);
+}
+
+template <int SHADER, int PC, int DT, bool PADDED, int LOOP>
+void launch_composite(const ShadeArgs &a, cudaStream_t s) {
+    const dim3 g = grid_of(a);
+    const size_t sm = smem_bytes(a);
+    if constexpr (HY_RENDER_COMPOSITE_GATHER && SHADER == HY_SHADER_VOLUME && PADDED &&
+                  DT == HY_DTYPE_U8) {
+        if (a.vol.tex) {
+            render_composite_gather_kernel<SHADER, PC, DT, PADDED, LOOP><<<g, kThreads, sm, s>>>(a);
+            return;
+        }
+    }
+    render_composite_kernel<SHADER, PC, DT, PADDED, LOOP><<<g, kThreads, sm, s>>>(a);
+}
+// Samples in flight by the warps of rays a scheduler gets.  512^3 blobs by
+// gathers, half the cells free, 128^2, 256^2, 512^2, 1024^2 (0.8, 3.4, 13.5, 54
+// warps): one sample at a time 549, 487, 523, 1321 us, two 393, 367, 466, 1249,
+// four 293, 276, 497, 1457; no free cells at 1024^2 1916, 1920, 2477.
+template <int SHADER, int PC, int DT, bool PADDED>
+void pick_composite(const ShadeArgs &a, cudaStream_t s) {
+    if constexpr (PADDED) {
+        constexpr bool volume = SHADER == HY_SHADER_VOLUME;
+        const long long rays = (long long)a.view.W * a.view.H, per_warp = 32ll * a.schedulers;
+        if (a.vol.P <= kMaxBatchesP && (!volume || a.mode == HY_VOLUME_DEFAULT)) {
+            if (rays < 8 * per_warp) {
+                launch_composite<SHADER, PC, DT, PADDED, kLoopBatch4>(a, s);
+                return;
+            }
+            if constexpr (volume) {
+                if (a.skip.d) {
+                    launch_composite<SHADER, PC, DT, PADDED, kLoopBatch2>(a, s);
+                    return;
+                }
+            }
+        }
+    }
+    launch_composite<SHADER, PC, DT, PADDED, kLoopOne>(a, s);
 }
 
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
@@ -247,30 +282,13 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
     const dim3 g = grid_of(a);
     const size_t sm = smem_bytes(a);
     if (a.composite) {
-        if constexpr (SHADER == HY_SHADER_VOLUME && PADDED) {
-            if constexpr (HY_RENDER_COMPOSITE_GATHER && DT == HY_DTYPE_U8) {
-                if (a.vol.tex) {
-                    if (a.skip.d)
-                        render_composite_gather_kernel<SHADER, PC, DT, PADDED, kLoopSkip>
-                            <<<g, kThreads, sm, s>>>(a);
-                    else
-                        render_composite_gather_kernel<SHADER, PC, DT, PADDED, kLoopOne>
-                            <<<g, kThreads, sm, s>>>(a);
-                    return;
-                }
-            }
-            if (a.skip.d) {
-                render_composite_kernel<SHADER, PC, DT, PADDED, kLoopSkip><<<g, kThreads, sm, s>>>(a);
-                return;
-            }
-        }
         if constexpr (SHADER == HY_SHADER_BLOCKS) {
             if (a.mode == HY_BLOCKS_VOLUME)
                 render_kernel<SHADER, PC, DT, PADDED, 1, kBlocksVolume><<<g, kThreads, sm, s>>>(a);
             else
                 render_kernel<SHADER, PC, DT, PADDED, 1, kBlocksSolid><<<g, kThreads, sm, s>>>(a);
         } else
-            render_composite_kernel<SHADER, PC, DT, PADDED><<<g, kThreads, sm, s>>>(a);
+            pick_composite<SHADER, PC, DT, PADDED>(a, s);
         return;
     }
     if constexpr (SHADER == HY_SHADER_VOLUME) {
