@@ -172,11 +172,8 @@ __device__ __forceinline__ void diff_values(const DiffArgs &a, const float (&qx)
             g0[u] = gather_r(a.gtex, X[u], Y[u]);
             g1[u] = gather_r(a.gtex, X[u], Y[u] + fd);
         }
-        // gather order: w = (x, y), z = (x + 1, y), x = (x, y + 1), y = (x + 1, y + 1)
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            v[u] = trilerp(f2(g0[u].w, g1[u].w), f2(g0[u].z, g1[u].z), f2(g0[u].x, g1[u].x),
-                           f2(g0[u].y, g1[u].y), axy[u], az[u]);
+        for (int u = 0; u < U; ++u) v[u] = gather_lerp(g0[u], g1[u], axy[u], az[u]);
     }
 }
 

@@ -397,6 +397,31 @@ __device__ __forceinline__ void gather2_indexed(const DevVolume &V, int which, f
     g1 = gather_r(h, X, Y + fd);
 }
 
+// The lerps of a footprint from its two gathers (slices z and z + 1).
+// gather order: w = (x, y), z = (x + 1, y), x = (x, y + 1), y = (x + 1, y + 1)
+__device__ __forceinline__ float gather_lerp(const float4 &g0, const float4 &g1, float2 axy,
+                                             float az) {
+#if HY_F32X2 && HY_GATHER_ROWS
+    // The x lerps row by row, each row's two taps as the gather returns them
+    // (adjacent registers): (x, y+1), (x+1, y+1) times (1-ax, ax) and
+    // (x+1, y), (x, y) times (ax, 1-ax), then one scalar add per row (IEEE
+    // addition commutes, so each row is fl(fl(c_x (1-ax)) + fl(c_x1 ax)) as
+    // in trilerp); then y per slice and z as there.
+    const float bx = 1.f - axy.x;
+    const float2 w10 = f2(bx, axy.x), w01 = f2(axy.x, bx);
+    const float2 r1z0 = mul2(f2(g0.x, g0.y), w10), r0z0 = mul2(f2(g0.z, g0.w), w01);
+    const float2 r1z1 = mul2(f2(g1.x, g1.y), w10), r0z1 = mul2(f2(g1.z, g1.w), w01);
+    const float2 X0 = f2(__fadd_rn(r0z0.x, r0z0.y), __fadd_rn(r0z1.x, r0z1.y));  // row y
+    const float2 X1 = f2(__fadd_rn(r1z0.x, r1z0.y), __fadd_rn(r1z1.x, r1z1.y));  // row y + 1
+    const float by = 1.f - axy.y, bz = 1.f - az;
+    const float2 Yv = lerp2(X0, f2(by, by), X1, f2(axy.y, axy.y));
+    const float2 Z = mul2(Yv, f2(bz, az));
+    return __fadd_rn(Z.x, Z.y);
+#else
+    return trilerp(f2(g0.w, g1.w), f2(g0.z, g1.z), f2(g0.x, g1.x), f2(g0.y, g1.y), axy, az);
+#endif
+}
+
 template <int PC, int GATHER = kGatherResident>
 __device__ __forceinline__ float sample_brick_gather(const DevVolume &V, const BrickRef &b,
                                                      int Prt, float lx, float ly, float lz) {
@@ -435,26 +460,7 @@ __device__ __forceinline__ float sample_brick_gather(const DevVolume &V, const B
         gather2_indexed(V, b.which, X, Y, fd, g0, g1);
     else
         gather2(V, b.which, X, Y, fd, g0, g1);
-    // gather order: w = (x, y), z = (x + 1, y), x = (x, y + 1), y = (x + 1, y + 1)
-#if HY_F32X2 && HY_GATHER_ROWS
-    // The x lerps row by row, each row's two taps as the gather returns them
-    // (adjacent registers): (x, y+1), (x+1, y+1) times (1-ax, ax) and
-    // (x+1, y), (x, y) times (ax, 1-ax), then one scalar add per row (IEEE
-    // addition commutes, so each row is fl(fl(c_x (1-ax)) + fl(c_x1 ax)) as
-    // in trilerp); then y per slice and z as there.
-    const float bx = 1.f - axy.x;
-    const float2 w10 = f2(bx, axy.x), w01 = f2(axy.x, bx);
-    const float2 r1z0 = mul2(f2(g0.x, g0.y), w10), r0z0 = mul2(f2(g0.z, g0.w), w01);
-    const float2 r1z1 = mul2(f2(g1.x, g1.y), w10), r0z1 = mul2(f2(g1.z, g1.w), w01);
-    const float2 X0 = f2(__fadd_rn(r0z0.x, r0z0.y), __fadd_rn(r0z1.x, r0z1.y));  // row y
-    const float2 X1 = f2(__fadd_rn(r1z0.x, r1z0.y), __fadd_rn(r1z1.x, r1z1.y));  // row y + 1
-    const float by = 1.f - axy.y, bz = 1.f - az;
-    const float2 Yv = lerp2(X0, f2(by, by), X1, f2(axy.y, axy.y));
-    const float2 Z = mul2(Yv, f2(bz, az));
-    return __fadd_rn(Z.x, Z.y);
-#else
-    return trilerp(f2(g0.w, g1.w), f2(g0.z, g1.z), f2(g0.x, g1.x), f2(g0.y, g1.y), axy, az);
-#endif
+    return gather_lerp(g0, g1, axy, az);
 }
 
 // A trilinear sample in three parts, for marches that keep several in flight:
@@ -1046,8 +1052,7 @@ __device__ __forceinline__ long long volume_batches(Px &p, const ShadeArgs &A, c
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
-                    v[u] = trilerp(f2(g0[u].w, g1[u].w), f2(g0[u].z, g1[u].z), f2(g0[u].x, g1[u].x),
-                                   f2(g0[u].y, g1[u].y), fp[u].axy, fp[u].az);
+                    v[u] = gather_lerp(g0[u], g1[u], fp[u].axy, fp[u].az);
             } else {
                 fetch_loads<U, PC, DT>(V, m.c.br, fp, v);
             }
