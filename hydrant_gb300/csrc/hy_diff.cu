@@ -374,17 +374,15 @@ struct GradAcc {
     }
 };
 
-// Back-propagates one sample: its position's cell, its value `val`, the
-// transmittance T before it and R (the colour composited behind it, updated
-// to include this sample).
+// Gradients of one sample: its value's place among the knots (`at`, q its knot
+// lerp, aa = q.w * density), the transmittance T before it, R the colour
+// composited behind it, its position.
 __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const float4 *tf,
                                                     float4 *gtf, GradAcc &G, const float4 &g,
-                                                    float4 &R, float px, float py, float pz,
-                                                    float val, float T) {
-    const TfAt at = tf_at(a.ntf, float(a.ntf), val);
-    const float4 q = tf_value(tf, at);
+                                                    const float4 &R, float px, float py, float pz,
+                                                    const TfAt &at, const float4 &q, float aa,
+                                                    float T) {
     const float al = at.al;
-    const float aa = q.w * a.density;
     // The gradient arithmetic has no float-exact counterpart to follow, so it
     // uses fused multiply-adds (the file is compiled with contraction off).
     // dL/dc = T g ; transmittance term through later samples
@@ -393,12 +391,6 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
     const float gdot = __fmaf_rn(g.w, R.w, __fmaf_rn(g.z, R.z, __fmaf_rn(g.y, R.y, g.x * R.x)));
     const float da =
         __fmaf_rn(-T, gdot, __fmaf_rn(gcz, q.z, __fmaf_rn(gcy, q.y, __fmaf_rn(gcx, q.x, gcw))));
-    // R_n = c_n + (1 - a_n) R_{n+1}
-    const float om = 1.f - aa;
-    const float2 om2 = f2(om, om);
-    const float2 Rxy = fma2(om2, f2(R.x, R.y), mul2(f2(q.x, q.y), f2(aa, aa)));
-    const float2 Rzw = fma2(om2, f2(R.z, R.w), f2(q.z * aa, aa));
-    R = make_float4(Rxy.x, Rxy.y, Rzw.x, Rzw.y);
     if (!at.in) return;
     // gradient of the TF output (r, g, b, A)
     const float2 gqxy = mul2(gcxy, f2(aa, aa)), gqzw = mul2(f2(gcz, da), f2(aa, a.density));
@@ -453,6 +445,15 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
     G.cacc[5] = c45.y;
     G.cacc[6] = c67.x;
     G.cacc[7] = c67.y;
+}
+
+// R_n = c_n + (1 - a_n) R_{n+1}
+__device__ __forceinline__ float4 diff_behind(const float4 &q, float aa, const float4 &R) {
+    const float om = 1.f - aa;
+    const float2 om2 = f2(om, om);
+    const float2 Rxy = fma2(om2, f2(R.x, R.y), mul2(f2(q.x, q.y), f2(aa, aa)));
+    const float2 Rzw = fma2(om2, f2(R.z, R.w), f2(q.z * aa, aa));
+    return make_float4(Rxy.x, Rxy.y, Rzw.x, Rzw.y);
 }
 
 // The adjoint walks a ray's segments back to front; a segment's recomputed
@@ -527,9 +528,191 @@ __global__ void __launch_bounds__(128, BLOCKS)
             for (int s = cnt - 1; s >= 0; --s) {
                 const float fs = float(s);
                 const float2 e = seg_vw[s];
+                const TfAt at = tf_at(a.ntf, fn, e.x);
+                const float4 q = tf_value(tf, at);
+                const float aa = q.w * a.density;
                 diff_adjoint_sample(a, tf, gtf, G, g, R, __fmaf_rn(fs, sx, c.x),
-                                    __fmaf_rn(fs, sy, c.y), __fmaf_rn(fs, sz, c.z), e.x,
+                                    __fmaf_rn(fs, sy, c.y), __fmaf_rn(fs, sz, c.z), at, q, aa,
                                     1.f - e.y);
+                R = diff_behind(q, aa, R);
+            }
+        }
+        G.flush_knots(gtf);
+        G.flush_cell(a.dvol);
+    }
+    __syncthreads();
+    // entry i is knot clamp(i - 1, 0, ntf - 1)
+    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x) {
+        const float4 v = gtf[i];
+        float *d = a.dtf + 4 * min(max(i - 1, 0), a.ntf - 1);
+        if (v.x != 0.f) atomicAdd(d + 0, v.x);
+        if (v.y != 0.f) atomicAdd(d + 1, v.y);
+        if (v.z != 0.f) atomicAdd(d + 2, v.z);
+        if (v.w != 0.f) atomicAdd(d + 3, v.w);
+    }
+}
+
+// Small launches: a ray's samples on kLanes neighbouring lanes.  A march of few
+// rays is a chain of samples waiting for their taps; here kLanes of them wait
+// together, and what has to go in order (compositing, the transmittance, the
+// colour behind) every lane of the group works out for itself from the others'
+// values, in the order and arithmetic of the kernels above.  A warp holds
+// 2x2 rays, a block 4 warps; the lanes of a group stay together (the shuffles
+// name the group), groups may part.  Below 2 warps of rays a scheduler: forward
+// and adjoint 8 lanes a ray against one, 3 views of 48^2 over 48^3 341 and 398
+// us, 2 of 64^2 over 128^3 476 and 682, 2 of 128x96 over 64^3 (1.3 warps) 385 and
+// 478, 2 of 200x150 over 64^3 (3 warps) 655 and 615, 2 of 200^2 over 128^3 (4
+// warps) 1513 and 907.
+constexpr int kLanes = 8;
+__device__ __forceinline__ bool group_pixel(const DiffArgs &a, int &x, int &y, int &view, int &j,
+                                            unsigned int &mask) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane / kLanes;
+    j = lane & (kLanes - 1);
+    mask = ((1u << kLanes) - 1u) << (lane - j);
+    x = blockIdx.x * 4 + (warp & 1) * 2 + (r & 1);
+    y = blockIdx.y * 4 + (warp >> 1) * 2 + (r >> 1);
+    view = blockIdx.z;
+    return x < a.W && y < a.H;
+}
+dim3 group_grid(const DiffArgs &a) { return dim3((a.W + 3) / 4, (a.H + 3) / 4, a.nviews); }
+
+// Lane j's position: j steps on (no further than step n - 1 of the group).
+__device__ __forceinline__ void group_position(int j, int n, float sx, float sy, float sz,
+                                               float &x, float &y, float &z) {
+#pragma unroll
+    for (int i = 1; i < kLanes; ++i)
+        if (i <= j && i < n) {
+            x = x + sx;
+            y = y + sy;
+            z = z + sz;
+        }
+}
+
+template <bool GATHER>
+__global__ void __launch_bounds__(128) diff_forward_group_kernel(const __grid_constant__ DiffArgs a) {
+    __shared__ float4 tf[kMaxKnots + kTfPad];
+    stage_tf(a.tf, a.ntf, tf);
+    __syncthreads();
+    int x, y, view, j;
+    unsigned int mask;
+    if (!group_pixel(a, x, y, view, j, mask)) return;  // whole groups
+    const size_t ray = (size_t(view) * a.H + y) * a.W + x;
+    float ox, oy, oz, dx, dy, dz;
+    const int nsteps = diff_emit(a, view, x, y, ox, oy, oz, dx, dy, dz);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float sx = dx * a.step, sy = dy * a.step, sz = dz * a.step;
+    float4 *cp = a.ckpt ? a.ckpt + ray * a.max_ckpt : nullptr;
+    const float fn = float(a.ntf);
+    int left = nsteps;
+    while (left > 0) {
+        if (cp) {
+            if (j == 0) *cp = make_float4(ox, oy, oz, v.w);
+            ++cp;
+        }
+        int cnt = a.ckpt ? min(a.K, left) : left;
+        left -= cnt;
+        for (; cnt > 0; cnt -= kLanes) {
+            const int n = min(cnt, kLanes);
+            float qx[1] = {ox}, qy[1] = {oy}, qz[1] = {oz}, val[1];
+            group_position(j, n, sx, sy, sz, qx[0], qy[0], qz[0]);
+            diff_values<1, GATHER>(a, qx, qy, qz, val);
+            float4 c = tf_value(tf, tf_at(a.ntf, fn, val[0]));
+            c.w = c.w * a.density;
+            c.x = c.x * c.w;
+            c.y = c.y * c.w;
+            c.z = c.z * c.w;
+#pragma unroll
+            for (int i = 0; i < kLanes; ++i) {
+                const float4 q = make_float4(
+                    __shfl_sync(mask, c.x, i, kLanes), __shfl_sync(mask, c.y, i, kLanes),
+                    __shfl_sync(mask, c.z, i, kLanes), __shfl_sync(mask, c.w, i, kLanes));
+                if (i < n) {
+                    const float t = 1.f - v.w;
+                    const float2 txy = mul2(f2(q.x, q.y), f2(t, t)), tzw = mul2(f2(q.z, q.w), f2(t, t));
+                    v.x = __fadd_rn(v.x, txy.x);
+                    v.y = __fadd_rn(v.y, txy.y);
+                    v.z = __fadd_rn(v.z, tzw.x);
+                    v.w = __fadd_rn(v.w, tzw.y);
+                }
+            }
+            ox = __shfl_sync(mask, qx[0], kLanes - 1, kLanes) + sx;
+            oy = __shfl_sync(mask, qy[0], kLanes - 1, kLanes) + sy;
+            oz = __shfl_sync(mask, qz[0], kLanes - 1, kLanes) + sz;
+        }
+    }
+    if (j) return;
+    a.image[ray] = v;
+    if (a.nsteps_out) a.nsteps_out[ray] = nsteps;
+}
+
+template <bool GATHER>
+__global__ void __launch_bounds__(128) diff_backward_group_kernel(const __grid_constant__ DiffArgs a) {
+    __shared__ float4 tf[kMaxKnots + kTfPad];
+    __shared__ float4 gtf[kMaxKnots + 2];  // gradients of stage_tf's entries 0 .. ntf + 1
+    stage_tf(a.tf, a.ntf, tf);
+    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x)
+        gtf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    int x, y, view, j;
+    unsigned int mask;
+    if (group_pixel(a, x, y, view, j, mask)) {
+        const size_t ray = (size_t(view) * a.H + y) * a.W + x;
+        const int nsteps = a.nsteps_out[ray];
+        const float4 g = a.dimage[ray];
+        float ox0, oy0, oz0, dx, dy, dz;
+        diff_emit(a, view, x, y, ox0, oy0, oz0, dx, dy, dz);
+        const float sx = dx * a.step, sy = dy * a.step, sz = dz * a.step;
+        float4 R = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int K = a.K, nseg = (nsteps + K - 1) / K;
+        const float fn = float(a.ntf);
+        GradAcc G;
+        const float4 *cps = a.ckpt + ray * a.max_ckpt;
+        for (int seg = nseg - 1; seg >= 0; --seg) {
+            const float4 c = cps[seg];
+            float ox = c.x, oy = c.y, oz = c.z, vw = c.w;
+            const int cnt = min(K, nsteps - seg * K);
+            float2 mine[kMaxK / kLanes];  // this lane's (sample value, v.w before it)
+            for (int s = 0; s < cnt; s += kLanes) {
+                const int n = min(cnt - s, kLanes);
+                float qx[1] = {ox}, qy[1] = {oy}, qz[1] = {oz}, val[1];
+                group_position(j, n, sx, sy, sz, qx[0], qy[0], qz[0]);
+                diff_values<1, GATHER>(a, qx, qy, qz, val);
+                const float aa = tf_value(tf, tf_at(a.ntf, fn, val[0])).w * a.density;
+                float before = vw;
+#pragma unroll
+                for (int i = 0; i < kLanes; ++i) {
+                    const float ai = __shfl_sync(mask, aa, i, kLanes);
+                    if (i == j) before = vw;
+                    if (i < n) vw = vw + ai * (1.f - vw);
+                }
+                mine[s / kLanes] = make_float2(val[0], before);
+                ox = __shfl_sync(mask, qx[0], kLanes - 1, kLanes) + sx;
+                oy = __shfl_sync(mask, qy[0], kLanes - 1, kLanes) + sy;
+                oz = __shfl_sync(mask, qz[0], kLanes - 1, kLanes) + sz;
+            }
+            for (int s = (cnt - 1) / kLanes * kLanes; s >= 0; s -= kLanes) {
+                const int n = min(cnt - s, kLanes);
+                const float2 e = mine[s / kLanes];
+                const TfAt at = tf_at(a.ntf, fn, e.x);
+                const float4 q = tf_value(tf, at);
+                const float aa = q.w * a.density;
+                float4 behind = R;
+#pragma unroll
+                for (int i = kLanes - 1; i >= 0; --i) {
+                    const float4 qi = make_float4(
+                        __shfl_sync(mask, q.x, i, kLanes), __shfl_sync(mask, q.y, i, kLanes),
+                        __shfl_sync(mask, q.z, i, kLanes), 0.f);
+                    const float ai = __shfl_sync(mask, aa, i, kLanes);
+                    if (i == j) behind = R;
+                    if (i < n) R = diff_behind(qi, ai, R);
+                }
+                if (j < n) {
+                    const float fs = float(s + j);
+                    diff_adjoint_sample(a, tf, gtf, G, g, behind, __fmaf_rn(fs, sx, c.x),
+                                        __fmaf_rn(fs, sy, c.y), __fmaf_rn(fs, sz, c.z), at, q, aa,
+                                        1.f - e.y);
+                }
+                __syncwarp(mask);
             }
         }
         G.flush_knots(gtf);
@@ -707,7 +890,10 @@ extern "C" int hy_diff_forward(hy_ctx *ctx, const hy_diff_params *p, const float
     bool gathers = false;
     rc = diff_gather_refresh(ctx, vol_dev, p->n, a, &gathers);
     if (rc) return rc;
-    if (gathers)
+    const long long rays = (long long)W * H * nviews, per_warp = 32ll * 4 * ctx->sms;
+    if (gathers && rays < 2 * per_warp)
+        diff_forward_group_kernel<true><<<group_grid(a), 128, 0, ctx->stream>>>(a);
+    else if (gathers)
         diff_forward_kernel<4, true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
     else
         diff_forward_kernel<1, false><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
@@ -746,7 +932,10 @@ extern "C" int hy_diff_backward(hy_ctx *ctx, const hy_diff_params *p, const floa
     bool gathers = false;
     rc = diff_gather_refresh(ctx, vol_dev, p->n, a, &gathers);
     if (rc) return rc;
-    if (gathers && (long long)W * H * nviews < 8 * 32ll * 4 * ctx->sms)
+    const long long rays = (long long)W * H * nviews, per_warp = 32ll * 4 * ctx->sms;
+    if (gathers && rays < 2 * per_warp)
+        diff_backward_group_kernel<true><<<group_grid(a), 128, 0, ctx->stream>>>(a);
+    else if (gathers && rays < 8 * per_warp)
         diff_backward_kernel<4, 4, true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
     else if (gathers)
         diff_backward_kernel<2, 8, true><<<diff_grid(a), 128, 0, ctx->stream>>>(a);
