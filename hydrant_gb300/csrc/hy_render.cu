@@ -167,6 +167,36 @@ __global__ void __launch_bounds__(kThreads) render_group_kernel(const __grid_con
     count_samples(A, samples);
 }
 
+// The Isosurface march of small launches: 8 lanes a ray (iso_group).
+template <int PC, int DT, bool PADDED>
+__global__ void __launch_bounds__(kThreads)
+    render_iso_group_kernel(const __grid_constant__ ShadeArgs A) {
+    extern __shared__ float4 smem[];
+    float4 *tf = smem;
+    float *lut = reinterpret_cast<float *>(smem + A.ntf + kTfPad);
+    load_shared(A, tf, lut);
+    const Shared S = make_shared(tf, A.ntf, lut);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane / kGroup;
+    const int x = (blockIdx.x * 2 + (warp & 1)) * kGroupW + r % kGroupW;
+    const int y = (blockIdx.y * 2 + (warp >> 1)) * kGroupH + r / kGroupW;
+    const bool on = x < A.view.W && y < A.view.H;
+    float ox, oy, oz, dx, dy, dz;
+    gen_ray(A.view, x, y, ox, oy, oz, dx, dy, dz);
+    Px p;
+    const bool hit = emit_setup<HY_SHADER_ISOSURFACE>(p, A, ox, oy, oz, dx, dy, dz, 0.f, 0.f, 0.f,
+                                                      A.bbox_max[0], A.bbox_max[1], A.bbox_max[2]);
+    int owner;
+    const unsigned int samples = iso_group<kGroup, PC, DT, PADDED>(p, on && hit, A, A.view, S, owner);
+    if (on && (lane & (kGroup - 1)) == owner) {
+        const float4 v = make_float4(p.vx, p.vy, p.vz, p.vw);
+        const size_t idx = size_t(y) * A.view.W + x;
+        A.rgba[idx] = quantise(A, v);
+        if (A.vout) A.vout[idx] = v;
+        if (A.aux) A.aux[idx] = make_float4(p.e3, 0.f, 0.f, 0.f);
+    }
+    count_samples(A, samples);
+}
+
 // The per-brick compositing variants of the Volume and Isosurface shaders,
 // held to 64 registers (8 resident blocks): on the 512^3 tubes at 1024^2,
 // Volume 147 -> 163 and Isosurface 231 -> 237 Gsamples/s against 80
@@ -322,6 +352,17 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
                 }
             }
             launch_lean<SHADER, PC, DT, PADDED, 0>(a, s);
+            return;
+        }
+    }
+    if constexpr (SHADER == HY_SHADER_ISOSURFACE) {
+        // Eight lanes a ray below 2 warps of rays a scheduler: 256^3 tubes at
+        // 128^2 (0.8 warps) 115 us against 271 with four samples in flight;
+        // 128^3 and 512^3 at 256^2 (3.4 warps) 281 and 258 against 167 and 449.
+        if ((long long)a.view.W * a.view.H < 2 * 32ll * a.schedulers) {
+            const dim3 gg((a.view.W + 2 * kGroupW - 1) / (2 * kGroupW),
+                          (a.view.H + 2 * kGroupH - 1) / (2 * kGroupH));
+            render_iso_group_kernel<PC, DT, PADDED><<<gg, kThreads, sm, s>>>(a);
             return;
         }
     }

@@ -1412,6 +1412,68 @@ __device__ __forceinline__ void normalize3(float &x, float &y, float &z) {
     z = z * r;
 }
 
+// A hit at p's position, whose sample in cursor c's brick is `value`: normal
+// (six samples), lighting, mode, depth (isosurface_shader.cu:72-118).
+template <int PC, int DT>
+__device__ __forceinline__ void iso_hit(Px &p, const BrickCursor &c, float value, const ShadeArgs &A,
+                                        const ViewArgs &Vw, const Shared &S) {
+    const DevVolume &V = A.vol;
+    const float prev_value = 0.0f;
+    const float iso = A.isovalue;
+    const BrickRef &br = c.br;
+    const float dt = A.step;
+    p.vx = A.surface[0];
+    p.vy = A.surface[1];
+    p.vz = A.surface[2];
+    p.vw = 1.f;
+    const float a = (iso - prev_value) / (value - prev_value);
+    const float qx = p.ox - dt * p.dx, qy = p.oy - dt * p.dy, qz = p.oz - dt * p.dz;
+    const float ia = 1.f - a;
+    const float ipx2 = ia * qx + a * p.ox, ipy2 = ia * qy + a * p.oy, ipz2 = ia * qz + a * p.oz;
+    // central difference in brick-local coordinates, dt = du * 2
+    const float lx = ipx2 - c.ipx, ly = ipy2 - c.ipy, lz = ipz2 - c.ipz;
+    const float g = A.du * 2.f;
+    float nnx = sample_brick<0, DT>(br, V.P, lx - g, ly - 0.f, lz - 0.f, S.lut) -
+                sample_brick<0, DT>(br, V.P, lx + g, ly + 0.f, lz + 0.f, S.lut);
+    float nny = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - g, lz - 0.f, S.lut) -
+                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + g, lz + 0.f, S.lut);
+    float nnz = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - 0.f, lz - g, S.lut) -
+                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + 0.f, lz + g, S.lut);
+    float wx, wy, wz, nx, ny, nz;
+    mat_vec4(A.to_world, ipx2, ipy2, ipz2, 1.f, wx, wy, wz);
+    mat_vec4(A.to_world, nnx, nny, nnz, 0.f, nx, ny, nz);
+    normalize3(nx, ny, nz);
+    float lx2 = Vw.light[0] - wx, ly2 = Vw.light[1] - wy, lz2 = Vw.light[2] - wz;
+    normalize3(lx2, ly2, lz2);
+    float hx = lx2 - wx, hy = ly2 - wy, hz = lz2 - wz;
+    normalize3(hx, hy, hz);
+    const float ambient = 0.2f;
+    const float diffuse = .6f * fclamp(lx2 * nx + ly2 * ny + lz2 * nz, 0.f, 1.f);
+    const float specular = .2f * powf(fclamp(hx * nx + hy * ny + hz * nz, 0.f, 1.f), 100.f);
+    const float ex = wx - Vw.eye[0], ey = wy - Vw.eye[1], ez = wz - Vw.eye[2];
+    const float distance = sqrtf(ex * ex + ey * ey + ez * ez) / 2.f;
+    if (A.mode == HY_ISO_COLOR) {
+        const float f = ambient + (diffuse + specular) / distance;
+        p.vx = iso_linear_to_srgb(p.vx * f);
+        p.vy = iso_linear_to_srgb(p.vy * f);
+        p.vz = iso_linear_to_srgb(p.vz * f);
+        p.vw = p.vw * f;
+    } else if (A.mode == HY_ISO_POSITION) {
+        p.vx = ipx2 / A.bbox_max[0];
+        p.vy = ipy2 / A.bbox_max[1];
+        p.vz = ipz2 / A.bbox_max[2];
+        p.vw = 1.f;
+    } else {
+        p.vx = nx;
+        p.vy = ny;
+        p.vz = nz;
+        p.vw = 1.f;
+    }
+    const float ddx = p.e0 - p.ox, ddy = p.e1 - p.oy, ddz = p.e2 - p.oz;
+    p.e3 = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
+    p.nsteps = 0;
+}
+
 // IsosurfaceShaderKernel::main (isosurface_shader.cu:50-125).  prev_value
 // stays 0, as in the reference (it is never updated there).  U samples of the
 // ray in flight (U > 1: bricks with an apron, as in volume_batches; the
@@ -1506,59 +1568,91 @@ __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const V
         } while (p.nsteps > 0 && r > 0);
     }
     if (!hit) return samples;
-    const BrickRef &br = c.br;
-    const float dt = A.step;
-    p.vx = A.surface[0];
-    p.vy = A.surface[1];
-    p.vz = A.surface[2];
-    p.vw = 1.f;
-    const float a = (iso - prev_value) / (value - prev_value);
-    const float qx = p.ox - dt * p.dx, qy = p.oy - dt * p.dy, qz = p.oz - dt * p.dz;
-    const float ia = 1.f - a;
-    const float ipx2 = ia * qx + a * p.ox, ipy2 = ia * qy + a * p.oy, ipz2 = ia * qz + a * p.oz;
-    // central difference in brick-local coordinates, dt = du * 2
-    const float lx = ipx2 - c.ipx, ly = ipy2 - c.ipy, lz = ipz2 - c.ipz;
-    const float g = A.du * 2.f;
-    float nnx = sample_brick<0, DT>(br, V.P, lx - g, ly - 0.f, lz - 0.f, S.lut) -
-                sample_brick<0, DT>(br, V.P, lx + g, ly + 0.f, lz + 0.f, S.lut);
-    float nny = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - g, lz - 0.f, S.lut) -
-                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + g, lz + 0.f, S.lut);
-    float nnz = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - 0.f, lz - g, S.lut) -
-                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + 0.f, lz + g, S.lut);
-    samples += 6;
-    float wx, wy, wz, nx, ny, nz;
-    mat_vec4(A.to_world, ipx2, ipy2, ipz2, 1.f, wx, wy, wz);
-    mat_vec4(A.to_world, nnx, nny, nnz, 0.f, nx, ny, nz);
-    normalize3(nx, ny, nz);
-    float lx2 = Vw.light[0] - wx, ly2 = Vw.light[1] - wy, lz2 = Vw.light[2] - wz;
-    normalize3(lx2, ly2, lz2);
-    float hx = lx2 - wx, hy = ly2 - wy, hz = lz2 - wz;
-    normalize3(hx, hy, hz);
-    const float ambient = 0.2f;
-    const float diffuse = .6f * fclamp(lx2 * nx + ly2 * ny + lz2 * nz, 0.f, 1.f);
-    const float specular = .2f * powf(fclamp(hx * nx + hy * ny + hz * nz, 0.f, 1.f), 100.f);
-    const float ex = wx - Vw.eye[0], ey = wy - Vw.eye[1], ez = wz - Vw.eye[2];
-    const float distance = sqrtf(ex * ex + ey * ey + ez * ez) / 2.f;
-    if (A.mode == HY_ISO_COLOR) {
-        const float f = ambient + (diffuse + specular) / distance;
-        p.vx = iso_linear_to_srgb(p.vx * f);
-        p.vy = iso_linear_to_srgb(p.vy * f);
-        p.vz = iso_linear_to_srgb(p.vz * f);
-        p.vw = p.vw * f;
-    } else if (A.mode == HY_ISO_POSITION) {
-        p.vx = ipx2 / A.bbox_max[0];
-        p.vy = ipy2 / A.bbox_max[1];
-        p.vz = ipz2 / A.bbox_max[2];
-        p.vw = 1.f;
-    } else {
-        p.vx = nx;
-        p.vy = ny;
-        p.vz = nz;
-        p.vw = 1.f;
+    iso_hit<PC, DT>(p, c, value, A, Vw, S);
+    return samples + 6;
+}
+
+// The march of a small launch: a ray's consecutive samples on K neighbouring
+// lanes, as in volume_group.  The lanes of a group stay together (the shuffles
+// name the group); `owner` is the lane that holds the ray's result: the one
+// whose sample crossed, or the first.  Every lane counts its share of samples.
+template <int K, int PC, int DT, bool PADDED>
+__device__ __forceinline__ unsigned int iso_group(Px &p, bool on, const ShadeArgs &A,
+                                                  const ViewArgs &Vw, const Shared &S, int &owner) {
+    const DevVolume &V = A.vol;
+    const int lane = threadIdx.x & 31, j = lane & (K - 1), base = lane - j;
+    const unsigned int mask = ((1u << K) - 1u) << base;
+    const float iso = A.isovalue;
+    const float prev_sign = fsign(0.0f - iso);  // as in iso_main
+    const float sx = p.dx * A.step, sy = p.dy * A.step, sz = p.dz * A.step;
+    unsigned int samples = 0;
+    BrickCursor c;
+    c.reset();
+    owner = 0;
+    if (!on) p.nsteps = 0;
+    int hint = A.skip.d != nullptr;
+    while (p.nsteps > 0) {
+        if (hint) {
+            unsigned int n = 0;
+            skip_free<true>(p, A.skip, sx, sy, sz, 1, n);
+            if (j == 0) samples += n;
+            if (p.nsteps <= 0) break;
+        }
+        hint = skip_hint(p, A.skip, sx, sy, sz, float(K));
+        float qx = p.ox, qy = p.oy, qz = p.oz;
+#pragma unroll
+        for (int i = 0; i < K - 1; ++i)
+            if (i < j) {
+                qx = qx + sx;
+                qy = qy + sy;
+                qz = qz + sz;
+            }
+        const bool valid = p.nsteps > j;
+        bool special = false, crossed = false;
+        float value = 0.f;
+        if (valid) {
+            float lx, ly, lz;
+            c.update(V, qx, qy, qz, lx, ly, lz);
+            special = c.cd != 0 || c.pg == -1;
+            if (!special) {
+                value = sample_brick<PC, DT, PADDED>(c.br, V.P, lx, ly, lz, S.lut);
+                crossed = prev_sign < 0.f   ? !(value < iso)
+                          : prev_sign > 0.f ? !(value > iso)
+                                            : (value < iso || value > iso);
+            }
+        }
+        const unsigned int sb = __ballot_sync(mask, special), cb = __ballot_sync(mask, crossed);
+        const int is = sb ? __ffs(sb) - 1 - base : K, ic = cb ? __ffs(cb) - 1 - base : K;
+        if (ic < is) {  // the first crossing, nothing special before it
+            owner = ic;
+            if (j == ic) {
+                samples += unsigned(ic + 1 + 6);
+                p.ox = qx;
+                p.oy = qy;
+                p.oz = qz;
+                iso_hit<PC, DT>(p, c, value, A, Vw, S);
+            }
+            break;
+        }
+        const int nv = min(K, p.nsteps), take = min(is, nv);
+        if (j == 0) samples += unsigned(take);
+        const int at = is < K ? is : K - 1;
+        p.ox = __shfl_sync(mask, qx, at, K);
+        p.oy = __shfl_sync(mask, qy, at, K);
+        p.oz = __shfl_sync(mask, qz, at, K);
+        p.nsteps -= take;
+        if (is < K) {
+            const float ipx = floorf(p.ox), ipy = floorf(p.oy), ipz = floorf(p.oz);
+            const int cd = __ldg(&V.info[thumb_index(V, ipx, ipy, ipz)].x);
+            if (cd == 0) break;  // page fault: the ray stops here
+            const float cdu = 1.f / gmax(gmax(fabsf(p.dx), fabsf(p.dy)), fabsf(p.dz));
+            p.nsteps -= skip_nblock_steps(p, 1.f / p.dx, 1.f / p.dy, 1.f / p.dz, ipx, ipy, ipz, cd,
+                                          cdu, A.step) + 1;
+        }
+        p.ox = p.ox + sx;
+        p.oy = p.oy + sy;
+        p.oz = p.oz + sz;
     }
-    const float ddx = p.e0 - p.ox, ddy = p.e1 - p.oy, ddz = p.e2 - p.oz;
-    p.e3 = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
-    p.nsteps = 0;
     return samples;
 }
 

@@ -133,6 +133,21 @@ def test_isosurface(ctx, iso, dtype):
         c.close()
 
 
+@pytest.mark.parametrize("dtype,pad", [("u8", 1), ("u8", 0), ("f32", 1)])
+def test_small_isosurfaces(ctx, dtype, pad):
+    """Isosurfaces with a ray's samples on eight lanes, up to the size where
+    they no longer are (2 warps of rays a scheduler: 38,912 rays), with and
+    without a surface in reach, and bricks the rays leap over."""
+    c = Case(ctx, voxels(dtype, (64, 48, 40)), 16, pad)
+    try:
+        for wh in ((1, 1), (9, 2), (37, 29), (197, 197), (198, 197)):
+            for iso, rate in ((0.4, 1.0), (0.05, 0.25), (0.97, 0.5), (-0.1, 0.5)):
+                check(c, camera(a=(-50.0, 20.0, 1.9)), *wh, f"{dtype} {pad} {wh} {iso}",
+                      shader="Isosurface", mode="Position", sample_rate=rate, isovalue=iso)
+    finally:
+        c.close()
+
+
 def test_brick_edges_and_axis_aligned_rays(ctx):
     """Brick edges that are no power of two and cameras along the axes (step
     components that are zero)."""
