@@ -80,20 +80,29 @@ struct Cell {
     float ax, ay, az;
 };
 
-__device__ __forceinline__ void diff_cell(const DiffArgs &a, float lx, float ly, float lz,
-                                          Cell &c) {
-    const int P = a.n + 2;
-    const float fd = float(P);
+// The footprint's lower padded indices (whole numbers) and the lerp fractions.
+__device__ __forceinline__ void diff_place(const DiffArgs &a, float lx, float ly, float lz,
+                                           float &flx, float &fly, float &flz, float &ax,
+                                           float &ay, float &az) {
+    const float fd = float(a.n + 2);
     // x and y in packed pairs (products summed by scalar adds), z alone
     const float2 kl = mul2(f2(a.k, a.k), f2(lx, ly));
     const float2 fxy = mul2(f2(fd, fd), f2(__fadd_rn(kl.x, a.b), __fadd_rn(kl.y, a.b)));
     const float fz = fd * (a.k * lz + a.b);
     const float ux = fxy.x - .5f, uy = fxy.y - .5f, uz = fz - .5f;
-    const float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
+    flx = floorf(ux);
+    fly = floorf(uy);
+    flz = floorf(uz);
     const float2 axy = sub2(f2(ux, uy), f2(flx, fly));
-    c.ax = axy.x;
-    c.ay = axy.y;
-    c.az = uz - flz;
+    ax = axy.x;
+    ay = axy.y;
+    az = uz - flz;
+}
+
+__device__ __forceinline__ void diff_cell(const DiffArgs &a, float lx, float ly, float lz,
+                                          Cell &c) {
+    float flx, fly, flz;
+    diff_place(a, lx, ly, lz, flx, fly, flz, c.ax, c.ay, c.az);
     const int ix = int(flx), iy = int(fly), iz = int(flz);
     // padded index i -> raw clamp(i - 1, 0, n - 1)
     const int n = a.n;
@@ -346,7 +355,7 @@ __global__ void __launch_bounds__(128, U >= 4 ? 4 : 8)
 struct GradAcc {
     int k = -1;  // knot entries k and k + 1 of stage_tf
     float4 acc_i = make_float4(0.f, 0.f, 0.f, 0.f), acc_j = make_float4(0.f, 0.f, 0.f, 0.f);
-    Cell cell;
+    float fx, fy, fz;  // the cell's padded lower indices (whole numbers)
     bool has_cell = false;
     float cacc[8];
 
@@ -363,14 +372,34 @@ struct GradAcc {
         acc_i = make_float4(0.f, 0.f, 0.f, 0.f);
         acc_j = acc_i;
     }
-    __device__ __forceinline__ void flush_cell(float *dvol) {
+    // The indices are worked out here and not per sample, and away from the
+    // border from one base: nearly every step some lane of the warp flushes
+    // (256^3, four views of 512^2: 9.50 -> 9.19 ms forward and adjoint).
+    __device__ __forceinline__ void flush_cell(const DiffArgs &a) {
         if (!has_cell) return;
-        const int idx[8] = {cell.r00 + cell.x0, cell.r00 + cell.x1, cell.r10 + cell.x0,
-                            cell.r10 + cell.x1, cell.r01 + cell.x0, cell.r01 + cell.x1,
-                            cell.r11 + cell.x0, cell.r11 + cell.x1};
+        // padded index i -> raw clamp(i - 1, 0, n - 1)
+        const int n = a.n, ix = int(fx), iy = int(fy), iz = int(fz);
+        const unsigned int m = unsigned(n - 1);
+        if (unsigned(ix - 1) < m && unsigned(iy - 1) < m && unsigned(iz - 1) < m) {
+            float *p = a.dvol + (((iz - 1) * n + iy - 1) * n + ix - 1);
+            float *q = p + n * n;
+            add2(p, cacc[0], cacc[1]);
+            add2(p + n, cacc[2], cacc[3]);
+            add2(q, cacc[4], cacc[5]);
+            add2(q + n, cacc[6], cacc[7]);
+            return;
+        }
+        const int x[2] = {iclamp(ix - 1, 0, n - 1), iclamp(ix, 0, n - 1)};
+        const int y[2] = {iclamp(iy - 1, 0, n - 1), iclamp(iy, 0, n - 1)};
+        const int z[2] = {iclamp(iz - 1, 0, n - 1), iclamp(iz, 0, n - 1)};
 #pragma unroll
         for (int t = 0; t < 8; ++t)
-            if (cacc[t] != 0.f) atomicAdd(dvol + idx[t], cacc[t]);
+            if (cacc[t] != 0.f)
+                atomicAdd(a.dvol + ((z[t >> 2] * n + y[(t >> 1) & 1]) * n + x[t & 1]), cacc[t]);
+    }
+    static __device__ __forceinline__ void add2(float *p, float u, float v) {
+        if (u != 0.f) atomicAdd(p, u);
+        if (v != 0.f) atomicAdd(p + 1, v);
     }
 };
 
@@ -416,18 +445,18 @@ __device__ __forceinline__ void diff_adjoint_sample(const DiffArgs &a, const flo
                                     __fmaf_rn(gq.z, kj.z - ki.z,
                                               __fmaf_rn(gq.y, kj.y - ki.y, gq.x * (kj.x - ki.x))));
     if (ds == 0.f) return;
-    Cell c;
-    diff_cell(a, px - floorf(px), py - floorf(py), pz - floorf(pz), c);
-    if (!G.has_cell || c.r00 + c.x0 != G.cell.r00 + G.cell.x0 ||
-        c.r11 + c.x1 != G.cell.r11 + G.cell.x1) {
-        G.flush_cell(a.dvol);
-        G.cell = c;
+    float cx, cy, cz, ax, ay, az;
+    diff_place(a, px - floorf(px), py - floorf(py), pz - floorf(pz), cx, cy, cz, ax, ay, az);
+    if (!G.has_cell || cx != G.fx || cy != G.fy || cz != G.fz) {
+        G.flush_cell(a);
+        G.fx = cx;
+        G.fy = cy;
+        G.fz = cz;
         G.has_cell = true;
 #pragma unroll
         for (int t = 0; t < 8; ++t) G.cacc[t] = 0.f;
     }
     // trilinear weights w = (x-weight) * (y-weight) * (z-weight), times ds
-    const float ax = c.ax, ay = c.ay, az = c.az;
     const float bx = 1.f - ax, by = 1.f - ay, bz = 1.f - az;
     const float2 ds2 = f2(ds, ds), yw = f2(by, ay);
     const float2 dz0 = mul2(ds2, mul2(yw, f2(bz, bz)));  // (d00, d10)
@@ -538,7 +567,7 @@ __global__ void __launch_bounds__(128, BLOCKS)
             }
         }
         G.flush_knots(gtf);
-        G.flush_cell(a.dvol);
+        G.flush_cell(a);
     }
     __syncthreads();
     // entry i is knot clamp(i - 1, 0, ntf - 1)
@@ -716,7 +745,7 @@ __global__ void __launch_bounds__(128) diff_backward_group_kernel(const __grid_c
             }
         }
         G.flush_knots(gtf);
-        G.flush_cell(a.dvol);
+        G.flush_cell(a);
     }
     __syncthreads();
     // entry i is knot clamp(i - 1, 0, ntf - 1)
