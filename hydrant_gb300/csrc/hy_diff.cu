@@ -419,6 +419,35 @@ struct GradAcc {
     }
 };
 
+// A block's sums of the gradients of stage_tf's entries 0 .. ntf + 1, in as
+// many copies as fit (a power of two, at most one a lane): neighbouring lanes,
+// whose values mostly lie in the same interval, add to different ones.  64^3,
+// two views of 200x150, 32 knots (4 copies) 440 -> 344 us forward and adjoint,
+// 256^3, four of 512^2 8.91 -> 8.81 ms; room for twice or four times the copies
+// (8 or 16 KB a block, out of the L1) 360 and 347 us, 8.77 and 8.92 ms.
+constexpr int kSums = kMaxKnots + 2;
+__device__ __forceinline__ int knot_copies(int ntf) {
+    int c = 1;
+    while (c < 32 && 2 * c * (ntf + 2) <= kSums) c *= 2;
+    return c;
+}
+
+// The block's sums into dtf: entry i is knot clamp(i - 1, 0, ntf - 1).
+__device__ __forceinline__ void add_knots(const DiffArgs &a, const float4 *sums, int copies) {
+    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x) {
+        float4 v = sums[i];
+        for (int c = 1; c < copies; ++c) {
+            const float4 w = sums[c * (a.ntf + 2) + i];
+            v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+        }
+        float *d = a.dtf + 4 * min(max(i - 1, 0), a.ntf - 1);
+        if (v.x != 0.f) atomicAdd(d + 0, v.x);
+        if (v.y != 0.f) atomicAdd(d + 1, v.y);
+        if (v.z != 0.f) atomicAdd(d + 2, v.z);
+        if (v.w != 0.f) atomicAdd(d + 3, v.w);
+    }
+}
+
 // Gradients of one sample: its value's place among the knots (`at`, q its knot
 // lerp, aa = q.w * density), the transmittance T before it, R the colour
 // composited behind it, its position.
@@ -515,11 +544,13 @@ template <int U, int BLOCKS, bool GATHER>
 __global__ void __launch_bounds__(128, BLOCKS)
     diff_backward_kernel(const __grid_constant__ DiffArgs a) {
     __shared__ float4 tf[kMaxKnots + kTfPad];
-    __shared__ float4 gtf[kMaxKnots + 2];  // gradients of stage_tf's entries 0 .. ntf + 1
+    __shared__ float4 sums[kSums];
     stage_tf(a.tf, a.ntf, tf);
-    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x)
-        gtf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int copies = knot_copies(a.ntf);
+    for (int i = threadIdx.x; i < copies * (a.ntf + 2); i += blockDim.x)
+        sums[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
+    float4 *gtf = sums + (threadIdx.x & (copies - 1)) * (a.ntf + 2);
     int x, y, view;
     pixel_of(a, x, y, view);
     if (x < a.W && y < a.H) {
@@ -583,15 +614,7 @@ __global__ void __launch_bounds__(128, BLOCKS)
         G.flush_cell(a);
     }
     __syncthreads();
-    // entry i is knot clamp(i - 1, 0, ntf - 1)
-    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x) {
-        const float4 v = gtf[i];
-        float *d = a.dtf + 4 * min(max(i - 1, 0), a.ntf - 1);
-        if (v.x != 0.f) atomicAdd(d + 0, v.x);
-        if (v.y != 0.f) atomicAdd(d + 1, v.y);
-        if (v.z != 0.f) atomicAdd(d + 2, v.z);
-        if (v.w != 0.f) atomicAdd(d + 3, v.w);
-    }
+    add_knots(a, sums, copies);
 }
 
 // Small launches: a ray's samples on kLanes neighbouring lanes.  A march of few
@@ -690,11 +713,13 @@ __global__ void __launch_bounds__(128) diff_forward_group_kernel(const __grid_co
 template <bool GATHER>
 __global__ void __launch_bounds__(128) diff_backward_group_kernel(const __grid_constant__ DiffArgs a) {
     __shared__ float4 tf[kMaxKnots + kTfPad];
-    __shared__ float4 gtf[kMaxKnots + 2];  // gradients of stage_tf's entries 0 .. ntf + 1
+    __shared__ float4 sums[kSums];
     stage_tf(a.tf, a.ntf, tf);
-    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x)
-        gtf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int copies = knot_copies(a.ntf);
+    for (int i = threadIdx.x; i < copies * (a.ntf + 2); i += blockDim.x)
+        sums[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
+    float4 *gtf = sums + (threadIdx.x & (copies - 1)) * (a.ntf + 2);
     int x, y, view, j;
     unsigned int mask;
     if (group_pixel(a, x, y, view, j, mask)) {
@@ -761,15 +786,7 @@ __global__ void __launch_bounds__(128) diff_backward_group_kernel(const __grid_c
         G.flush_cell(a);
     }
     __syncthreads();
-    // entry i is knot clamp(i - 1, 0, ntf - 1)
-    for (int i = threadIdx.x; i < a.ntf + 2; i += blockDim.x) {
-        const float4 v = gtf[i];
-        float *d = a.dtf + 4 * min(max(i - 1, 0), a.ntf - 1);
-        if (v.x != 0.f) atomicAdd(d + 0, v.x);
-        if (v.y != 0.f) atomicAdd(d + 1, v.y);
-        if (v.z != 0.f) atomicAdd(d + 2, v.z);
-        if (v.w != 0.f) atomicAdd(d + 3, v.w);
-    }
+    add_knots(a, sums, copies);
 }
 
 int fill_diff(hy_ctx *ctx, const hy_diff_params *p, const float *vol, const float *tf,
