@@ -938,7 +938,9 @@ def main_ours(args):
                 "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                 "frac": achieved / hbm, "peak_kind": peak_kind,
                 "traffic": (tps * samples) if tps else None,
-                "note": "8 B/sample algorithmic footprint; the march is bound by L1 latency and instruction issue, not HBM",
+                "note": "8 B/sample algorithmic footprint of the reference's march (samples that "
+                        "change nothing are counted and passed over unread); bound by "
+                        "instruction issue and gather latency, not HBM",
             },
             "issue_roofline": issue_roofline(ipsm, samples, mean_launch_s, ck, local),
             "cpu_baseline": cpu,
