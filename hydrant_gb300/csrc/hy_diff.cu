@@ -536,10 +536,9 @@ __device__ __forceinline__ float4 diff_behind(const float4 &q, float aa, const f
 // neighbouring cell gets the same gradient to first order).
 // BLOCKS: resident 128-thread blocks per SM the registers are fitted to.  256^3,
 // four views of 512^2, K = 32, forward and adjoint: 8 blocks (64 registers)
-// 9.71 ms, 6 (80) 10.1, 5 10.2, 4 10.6; launches of fewer than 8 warps of
-// rays a scheduler are bound by latency and take 4 (128 registers) with
-// four samples of the recompute in flight: 3 views of 75x51 over 48^3 446
-// against 492 us.
+// 8.78 ms, 6 (80) 9.03, 5 9.40; launches of fewer than 8 warps of rays a
+// scheduler are bound by latency and take 4 (128 registers) with four samples
+// of the recompute in flight: 2 of 200^2 over 128^3 (4 warps) 635 against 732 us.
 template <int U, int BLOCKS, bool GATHER>
 __global__ void __launch_bounds__(128, BLOCKS)
     diff_backward_kernel(const __grid_constant__ DiffArgs a) {
@@ -624,10 +623,10 @@ __global__ void __launch_bounds__(128, BLOCKS)
 // values, in the order and arithmetic of the kernels above.  A warp holds
 // 2x2 rays, a block 4 warps; the lanes of a group stay together (the shuffles
 // name the group), groups may part.  Below 2 warps of rays a scheduler: forward
-// and adjoint 8 lanes a ray against one, 3 views of 48^2 over 48^3 341 and 398
-// us, 2 of 64^2 over 128^3 476 and 682, 2 of 128x96 over 64^3 (1.3 warps) 385 and
-// 478, 2 of 200x150 over 64^3 (3 warps) 655 and 615, 2 of 200^2 over 128^3 (4
-// warps) 1513 and 907.
+// and adjoint 8 lanes a ray against one, 2 views of 64^2 over 128^3 311 and 541
+// us, 3 of 75x51 over 48^3 306 and 372, 2 of 128x96 over 64^3 (1.3 warps) 320 and
+// 337, 2 of 200x150 over 64^3 (3 warps) 380 and 353, 2 of 200^2 over 128^3 (4
+// warps) 941 and 635.
 constexpr int kLanes = 8;
 __device__ __forceinline__ bool group_pixel(const DiffArgs &a, int &x, int &y, int &view, int &j,
                                             unsigned int &mask) {
