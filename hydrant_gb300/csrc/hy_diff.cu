@@ -284,7 +284,7 @@ __device__ __forceinline__ void pixel_of(const DiffArgs &a, int &x, int &y, int 
 
 // U steps of a ray at a time: their taps are fetched together (a step's
 // position does not depend on the sample before it).  256^3, four views of
-// 512^2, K = 32: 5.30 ms by loads one at a time, 1.9 ms by gathers with 4 in
+// 512^2, K = 32: 5.30 ms by loads one at a time, 2.9 ms by gathers with 4 in
 // flight (L1 86 % busy: the texture's f32 wavefronts); 3 views of 75x51 over
 // 48^3 104 and 50 us.
 template <int U, bool GATHER>
