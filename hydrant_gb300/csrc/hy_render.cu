@@ -367,10 +367,11 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
         }
     }
     if constexpr (SHADER == HY_SHADER_ISOSURFACE && PADDED) {
-        // Samples in flight by the warps of rays a scheduler gets: 512^3 tubes
-        // at 256^2, 512^2 and 1024^2 (3.4, 13.5, 54 warps) 470, 596, 1160 us
-        // with four, 492, 590, 984 with two, 554, 602, 978 with one; 200^3 f32
-        // blobs at 600^2 (18.5 warps) 222, 216, 236.
+        // Samples in flight by the warps of rays a scheduler gets: 512^3 tubes at
+        // 256^2 and 512^2 (3.4, 13.5 warps) 414 and 468 us with one, 350 and 415
+        // with two, 337 with four at the first; 256^3 of 32^3 bricks at 256^2,
+        // 512^2, 670^2 339, 366, 444 with one, 230, 297, 385 with two, 194 with
+        // four at the first.
         const long long rays = (long long)a.view.W * a.view.H, per_warp = 32ll * a.schedulers;
         if (rays < 24 * per_warp && a.vol.P <= kMaxBatchesP) {
             if (rays < 8 * per_warp)
