@@ -167,34 +167,64 @@ __global__ void __launch_bounds__(kThreads) render_group_kernel(const __grid_con
     count_samples(A, samples);
 }
 
-// The Isosurface march of small launches: 8 lanes a ray (iso_group).
+// The Isosurface march of small launches: 8 lanes a ray (iso_group).  A block
+// takes 8x4 rays; their hits are shaded by one warp, a ray a lane: shading costs
+// a few hundred FP64 instructions a warp whether one lane or all take part
+// (linear_to_srgb), which at four rays a warp, where rays hit at once, was most
+// of the time (190^2 over 256^3 noise: 158 us, 40 this way, 32 with one ray a lane
+// throughout).
+constexpr int kIsoGroupThreads = 256, kIsoW = 8, kIsoH = 4;
 template <int PC, int DT, bool PADDED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kIsoGroupThreads)
     render_iso_group_kernel(const __grid_constant__ ShadeArgs A) {
     extern __shared__ float4 smem[];
+    __shared__ IsoHit hits[kIsoW * kIsoH];
+    __shared__ unsigned char found[kIsoW * kIsoH];
     float4 *tf = smem;
     float *lut = reinterpret_cast<float *>(smem + A.ntf + kTfPad);
     load_shared(A, tf, lut);
     const Shared S = make_shared(tf, A.ntf, lut);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane / kGroup;
-    const int x = (blockIdx.x * 2 + (warp & 1)) * kGroupW + r % kGroupW;
-    const int y = (blockIdx.y * 2 + (warp >> 1)) * kGroupH + r / kGroupW;
-    const bool on = x < A.view.W && y < A.view.H;
-    float ox, oy, oz, dx, dy, dz;
-    gen_ray(A.view, x, y, ox, oy, oz, dx, dy, dz);
-    Px p;
-    const bool hit = emit_setup<HY_SHADER_ISOSURFACE>(p, A, ox, oy, oz, dx, dy, dz, 0.f, 0.f, 0.f,
-                                                      A.bbox_max[0], A.bbox_max[1], A.bbox_max[2]);
-    int owner;
-    const unsigned int samples = iso_group<kGroup, PC, DT, PADDED>(p, on && hit, A, A.view, S, owner);
-    if (on && (lane & (kGroup - 1)) == owner) {
-        const float4 v = make_float4(p.vx, p.vy, p.vz, p.vw);
-        const size_t idx = size_t(y) * A.view.W + x;
-        A.rgba[idx] = quantise(A, v);
-        if (A.vout) A.vout[idx] = v;
-        if (A.aux) A.aux[idx] = make_float4(p.e3, 0.f, 0.f, 0.f);
+    const int ray = threadIdx.x / kGroup;
+    const int x = blockIdx.x * kIsoW + ray % kIsoW, y = blockIdx.y * kIsoH + ray / kIsoW;
+    {
+        const bool on = x < A.view.W && y < A.view.H;
+        float ox, oy, oz, dx, dy, dz;
+        gen_ray(A.view, x, y, ox, oy, oz, dx, dy, dz);
+        Px p;
+        const bool hit = emit_setup<HY_SHADER_ISOSURFACE>(p, A, ox, oy, oz, dx, dy, dz, 0.f, 0.f, 0.f,
+                                                          A.bbox_max[0], A.bbox_max[1],
+                                                          A.bbox_max[2]);
+        IsoHit h;
+        unsigned int samples;
+        const bool f = iso_group<kGroup, PC, DT, PADDED>(p, on && hit, A, S, h, samples);
+        if ((threadIdx.x & (kGroup - 1)) == 0) {
+            found[ray] = f;
+            if (f) hits[ray] = h;
+        }
+        count_samples(A, samples);
     }
-    count_samples(A, samples);
+    __syncthreads();
+    const int t = threadIdx.x;
+    const int px = blockIdx.x * kIsoW + t % kIsoW, py = blockIdx.y * kIsoH + t / kIsoW;
+    if (t >= kIsoW * kIsoH || px >= A.view.W || py >= A.view.H) return;
+    Px p;
+    p.vx = p.vy = p.vz = p.vw = 0.f;
+    p.e0 = A.view.ray_o[0];
+    p.e1 = A.view.ray_o[1];
+    p.e2 = A.view.ray_o[2];
+    p.e3 = __int_as_float(0x7f800000);  // INFINITY
+    if (found[t]) {
+        const IsoHit h = hits[t];
+        p.ox = h.o.x;
+        p.oy = h.o.y;
+        p.oz = h.o.z;
+        iso_shade(p, h.at, h.n.x, h.n.y, h.n.z, A, A.view);
+    }
+    const float4 v = make_float4(p.vx, p.vy, p.vz, p.vw);
+    const size_t idx = size_t(py) * A.view.W + px;
+    A.rgba[idx] = quantise(A, v);
+    if (A.vout) A.vout[idx] = v;
+    if (A.aux) A.aux[idx] = make_float4(p.e3, 0.f, 0.f, 0.f);
 }
 
 // The per-brick compositing variants of the Volume and Isosurface shaders,
@@ -357,12 +387,13 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
     }
     if constexpr (SHADER == HY_SHADER_ISOSURFACE) {
         // Eight lanes a ray below 2 warps of rays a scheduler: 256^3 tubes at
-        // 128^2 (0.8 warps) 115 us against 271 with four samples in flight;
-        // 128^3 and 512^3 at 256^2 (3.4 warps) 281 and 258 against 167 and 449.
+        // 128^2 (0.8 warps) 109 us against 191 with four samples in flight.
+        // Above, where rays march far (200^2 and 256^2, 2.1 and 3.4 warps) 131
+        // and 166 against 198 and 194, where they hit at once (noise) 49 and 68
+        // against 43 and 53.
         if ((long long)a.view.W * a.view.H < 2 * 32ll * a.schedulers) {
-            const dim3 gg((a.view.W + 2 * kGroupW - 1) / (2 * kGroupW),
-                          (a.view.H + 2 * kGroupH - 1) / (2 * kGroupH));
-            render_iso_group_kernel<PC, DT, PADDED><<<gg, kThreads, sm, s>>>(a);
+            const dim3 gg((a.view.W + kIsoW - 1) / kIsoW, (a.view.H + kIsoH - 1) / kIsoH);
+            render_iso_group_kernel<PC, DT, PADDED><<<gg, kIsoGroupThreads, sm, s>>>(a);
             return;
         }
     }

@@ -756,8 +756,8 @@ __device__ __forceinline__ int skip_cell(const SkipGrid &G, int plane, float x, 
     if (!(qx >= 0.f && qx < G.fcx && qy >= 0.f && qy < G.fcy && qz >= 0.f && qz < G.fcz)) return 0;
     return __ldg(G.d + (plane + (int(qz) * G.cy + int(qy)) * G.cx + int(qx)));
 }
-// JUMP: runs of 12 steps and more by jump().  512^3 tubes' isosurface 984 ->
-// 935 us, f32 blobs 256 -> 248; the u8 march, whose runs are short at 1-voxel
+// JUMP: runs of 12 steps and more by jump().  512^3 tubes' isosurface at 1024^2
+// 845 -> 736 us, f32 blobs 256 -> 248; the u8 march, whose runs are short at 1-voxel
 // steps, loses 1 % (896 -> 903) and keeps the additions.
 template <bool JUMP>
 __device__ __forceinline__ void skip_free(Px &p, const SkipGrid &G, float sx, float sy, float sz,
@@ -1412,33 +1412,25 @@ __device__ __forceinline__ void normalize3(float &x, float &y, float &z) {
     z = z * r;
 }
 
-// A hit at p's position, whose sample in cursor c's brick is `value`: normal
-// (six samples), lighting, mode, depth (isosurface_shader.cu:72-118).
-template <int PC, int DT>
-__device__ __forceinline__ void iso_hit(Px &p, const BrickCursor &c, float value, const ShadeArgs &A,
-                                        const ViewArgs &Vw, const Shared &S) {
-    const DevVolume &V = A.vol;
+// A hit at p's position, whose sample is `value` (isosurface_shader.cu:72-118):
+// the surface's position between the sample and the step before it,
+__device__ __forceinline__ float3 iso_position(const Px &p, float value, const ShadeArgs &A) {
     const float prev_value = 0.0f;
-    const float iso = A.isovalue;
-    const BrickRef &br = c.br;
     const float dt = A.step;
+    const float a = (A.isovalue - prev_value) / (value - prev_value);
+    const float qx = p.ox - dt * p.dx, qy = p.oy - dt * p.dy, qz = p.oz - dt * p.dz;
+    const float ia = 1.f - a;
+    return make_float3(ia * qx + a * p.ox, ia * qy + a * p.oy, ia * qz + a * p.oz);
+}
+// then, with the central difference (nnx, nny, nnz) there, normal, lighting,
+// mode and depth.
+__device__ __forceinline__ void iso_shade(Px &p, float3 at, float nnx, float nny, float nnz,
+                                          const ShadeArgs &A, const ViewArgs &Vw) {
+    const float ipx2 = at.x, ipy2 = at.y, ipz2 = at.z;
     p.vx = A.surface[0];
     p.vy = A.surface[1];
     p.vz = A.surface[2];
     p.vw = 1.f;
-    const float a = (iso - prev_value) / (value - prev_value);
-    const float qx = p.ox - dt * p.dx, qy = p.oy - dt * p.dy, qz = p.oz - dt * p.dz;
-    const float ia = 1.f - a;
-    const float ipx2 = ia * qx + a * p.ox, ipy2 = ia * qy + a * p.oy, ipz2 = ia * qz + a * p.oz;
-    // central difference in brick-local coordinates, dt = du * 2
-    const float lx = ipx2 - c.ipx, ly = ipy2 - c.ipy, lz = ipz2 - c.ipz;
-    const float g = A.du * 2.f;
-    float nnx = sample_brick<0, DT>(br, V.P, lx - g, ly - 0.f, lz - 0.f, S.lut) -
-                sample_brick<0, DT>(br, V.P, lx + g, ly + 0.f, lz + 0.f, S.lut);
-    float nny = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - g, lz - 0.f, S.lut) -
-                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + g, lz + 0.f, S.lut);
-    float nnz = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - 0.f, lz - g, S.lut) -
-                sample_brick<0, DT>(br, V.P, lx + 0.f, ly + 0.f, lz + g, S.lut);
     float wx, wy, wz, nx, ny, nz;
     mat_vec4(A.to_world, ipx2, ipy2, ipz2, 1.f, wx, wy, wz);
     mat_vec4(A.to_world, nnx, nny, nnz, 0.f, nx, ny, nz);
@@ -1472,6 +1464,25 @@ __device__ __forceinline__ void iso_hit(Px &p, const BrickCursor &c, float value
     const float ddx = p.e0 - p.ox, ddy = p.e1 - p.oy, ddz = p.e2 - p.oz;
     p.e3 = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
     p.nsteps = 0;
+}
+
+// Both, by one lane: the six samples lie in cursor c's brick, in its local
+// coordinates, dt = du * 2.
+template <int DT>
+__device__ __forceinline__ void iso_hit(Px &p, const BrickCursor &c, float value, const ShadeArgs &A,
+                                        const ViewArgs &Vw, const Shared &S) {
+    const DevVolume &V = A.vol;
+    const BrickRef &br = c.br;
+    const float3 at = iso_position(p, value, A);
+    const float lx = at.x - c.ipx, ly = at.y - c.ipy, lz = at.z - c.ipz;
+    const float g = A.du * 2.f;
+    const float nnx = sample_brick<0, DT>(br, V.P, lx - g, ly - 0.f, lz - 0.f, S.lut) -
+                      sample_brick<0, DT>(br, V.P, lx + g, ly + 0.f, lz + 0.f, S.lut);
+    const float nny = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - g, lz - 0.f, S.lut) -
+                      sample_brick<0, DT>(br, V.P, lx + 0.f, ly + g, lz + 0.f, S.lut);
+    const float nnz = sample_brick<0, DT>(br, V.P, lx - 0.f, ly - 0.f, lz - g, S.lut) -
+                      sample_brick<0, DT>(br, V.P, lx + 0.f, ly + 0.f, lz + g, S.lut);
+    iso_shade(p, at, nnx, nny, nnz, A, Vw);
 }
 
 // IsosurfaceShaderKernel::main (isosurface_shader.cu:50-125).  prev_value
@@ -1572,27 +1583,34 @@ __device__ __forceinline__ long long iso_main(Px &p, const ShadeArgs &A, const V
         p.nsteps -= 1;
     }
     if (!hit) return samples;
-    iso_hit<PC, DT>(p, c, value, A, Vw, S);
+    iso_hit<DT>(p, c, value, A, Vw, S);
     return samples + 6;
 }
 
+// A hit as iso_shade takes it.
+struct IsoHit {
+    float3 o, at, n;  // the crossing sample's position, the surface's, the central difference
+};
+
 // The march of a small launch: a ray's consecutive samples on K neighbouring
 // lanes, as in volume_group.  The lanes of a group stay together (the shuffles
-// name the group); `owner` is the lane that holds the ray's result: the one
-// whose sample crossed, or the first.  Every lane counts its share of samples.
+// name the group), all lanes of the warp call this (`on` false: no ray).  Every
+// lane of a group returns whether its ray hit, and where; the first lane counts
+// the group's samples.
 template <int K, int PC, int DT, bool PADDED>
-__device__ __forceinline__ unsigned int iso_group(Px &p, bool on, const ShadeArgs &A,
-                                                  const ViewArgs &Vw, const Shared &S, int &owner) {
+__device__ __forceinline__ bool iso_group(Px &p, bool on, const ShadeArgs &A, const Shared &S,
+                                          IsoHit &hit, unsigned int &samples) {
     const DevVolume &V = A.vol;
     const int lane = threadIdx.x & 31, j = lane & (K - 1), base = lane - j;
     const unsigned int mask = ((1u << K) - 1u) << base;
     const float iso = A.isovalue;
     const float prev_sign = fsign(0.0f - iso);  // as in iso_main
     const float sx = p.dx * A.step, sy = p.dy * A.step, sz = p.dz * A.step;
-    unsigned int samples = 0;
+    samples = 0;
     BrickCursor c;
     c.reset();
-    owner = 0;
+    int owner = -1;  // the lane whose sample crossed, and that sample
+    float hx = 0.f, hy = 0.f, hz = 0.f, hv = 0.f;
     if (!on) p.nsteps = 0;
     int hint = A.skip.d != nullptr;
     while (p.nsteps > 0) {
@@ -1628,14 +1646,12 @@ __device__ __forceinline__ unsigned int iso_group(Px &p, bool on, const ShadeArg
         const unsigned int sb = __ballot_sync(mask, special), cb = __ballot_sync(mask, crossed);
         const int is = sb ? __ffs(sb) - 1 - base : K, ic = cb ? __ffs(cb) - 1 - base : K;
         if (ic < is) {  // the first crossing, nothing special before it
+            if (j == 0) samples += unsigned(ic + 1 + 6);
             owner = ic;
-            if (j == ic) {
-                samples += unsigned(ic + 1 + 6);
-                p.ox = qx;
-                p.oy = qy;
-                p.oz = qz;
-                iso_hit<PC, DT>(p, c, value, A, Vw, S);
-            }
+            hx = qx;
+            hy = qy;
+            hz = qz;
+            hv = value;
             break;
         }
         const int nv = min(K, p.nsteps), take = min(is, nv);
@@ -1657,7 +1673,39 @@ __device__ __forceinline__ unsigned int iso_group(Px &p, bool on, const ShadeArg
         p.oy = p.oy + sy;
         p.oz = p.oz + sz;
     }
-    return samples;
+    // the warp's hits together, the six samples of a normal on six lanes
+    __syncwarp();
+    if (owner < 0) return false;
+    p.ox = __shfl_sync(mask, hx, owner, K);
+    p.oy = __shfl_sync(mask, hy, owner, K);
+    p.oz = __shfl_sync(mask, hz, owner, K);
+    const float value = __shfl_sync(mask, hv, owner, K);
+    BrickRef br{};
+    br.base = reinterpret_cast<const unsigned char *>(
+        __shfl_sync(mask, reinterpret_cast<unsigned long long>(c.br.base), owner, K));
+    br.k = __shfl_sync(mask, c.br.k, owner, K);
+    br.bx = __shfl_sync(mask, c.br.bx, owner, K);
+    br.by = __shfl_sync(mask, c.br.by, owner, K);
+    br.bz = __shfl_sync(mask, c.br.bz, owner, K);
+    const float3 at = iso_position(p, value, A);
+    const float lx = at.x - __shfl_sync(mask, c.ipx, owner, K),
+                ly = at.y - __shfl_sync(mask, c.ipy, owner, K),
+                lz = at.z - __shfl_sync(mask, c.ipz, owner, K);
+    const float g = A.du * 2.f;
+    // lane 2 a: below along axis a, lane 2 a + 1: above
+    const int axis = j >> 1;
+    const bool up = j & 1;
+    const float gx = axis == 0 ? g : 0.f, gy = axis == 1 ? g : 0.f, gz = axis == 2 ? g : 0.f;
+    float s = 0.f;
+    if (j < 6)
+        s = sample_brick<0, DT>(br, V.P, up ? lx + gx : lx - gx, up ? ly + gy : ly - gy,
+                                up ? lz + gz : lz - gz, S.lut);
+    const float n = s - __shfl_sync(mask, s, j | 1, K);
+    hit.o = make_float3(p.ox, p.oy, p.oz);
+    hit.at = at;
+    hit.n = make_float3(__shfl_sync(mask, n, 0, K), __shfl_sync(mask, n, 2, K),
+                        __shfl_sync(mask, n, 4, K));
+    return true;
 }
 
 template <int SHADER, int PC, int DT, bool PADDED, bool LEAN = false, int GATHER = 0,
