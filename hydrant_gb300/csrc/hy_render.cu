@@ -305,6 +305,13 @@ void launch_group(const ShadeArgs &a, cudaStream_t s) {
 // 1643; 163, 169, 230, 587; 191, 198, 248, 526; 288, 286, 311, 581.  Without an
 // apron only the group and the plain march are built: 83, 228, 738 against
 // 230, 231, 392.
+// Without free cells samples in flight end earlier.  256^3 blobs at 256^2, 320^2,
+// 380^2 and 400^2 (3.4, 5.3, 7.4, 8.2 warps): u8 by gathers 90, 125, 156 us with
+// four, 118, 144 and 160 with two at the last three, 147, 153, 162, 168 with
+// one; u8 by loads 118, 154, 188; 145, 172, 206; 150, 158, 169, 183; f32 135, 178,
+// 216; 161, 184, 220; 176, 197, 208, 212.  Rays that are soon opaque (density 0.3)
+// lose more where the line is too high: u8 by loads at 380^2 81 with four, 70
+// with two, 66 with one.
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
 void launch_lean(const ShadeArgs &a, cudaStream_t s) {
     const dim3 g = grid_of(a);
@@ -327,9 +334,10 @@ void launch_lean(const ShadeArgs &a, cudaStream_t s) {
             return;
         }
     }
-    if (rays < 8 * per_warp)
+    const int four = a.skip.d ? 8 : 5, two = GATHER ? 24 : DT == HY_DTYPE_F32 ? 8 : 0;
+    if (rays < four * per_warp)
         render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
-    else if (a.skip.d || rays < 24 * per_warp)
+    else if (a.skip.d || rays < two * per_warp)
         render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch2><<<g, kThreads, sm, s>>>(a);
     else if constexpr (GATHER != 0)
         render_lean_gather_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopOne><<<g, kThreads, sm, s>>>(a);
