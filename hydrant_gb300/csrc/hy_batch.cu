@@ -480,8 +480,23 @@ int layout(hy_batch *b) {
     return HY_OK;
 }
 
+// The launch is a graph of the batch's own, and the layout and the skip grid may
+// change before it: none of that can be part of a caller's capture.  Refused
+// before anything is touched, the capture and the batch stay as they are.
+int refuse_capture(hy_ctx *ctx) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HY_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return hy_fail(ctx, HY_ERR_STATE,
+                       "batch: the stream is capturing (a batch replays a graph of its own; "
+                       "capture hy_render_device per view)");
+    return HY_OK;
+}
+
 int launch(hy_batch *b, uint8_t *out) {
     hy_ctx *ctx = b->ctx;
+    int rc = refuse_capture(ctx);
+    if (rc) return rc;
     // the batch renders with the context's current transfer function: a new
     // table (hy_tf_set may have reallocated it) or knot count means new
     // kernel arguments, shared-memory size and graph
@@ -490,13 +505,13 @@ int launch(hy_batch *b, uint8_t *out) {
             return hy_fail(ctx, HY_ERR_STATE, "batch: Volume shader needs a transfer function");
         b->base.tf = ctx->tf_dev;
         b->base.ntf = ctx->ntf;
-        int rc = layout(b);
+        rc = layout(b);
         if (rc) return rc;
     }
     // the skip grid follows the knots; a batch that gains or loses it is
     // another kernel and graph
     SkipGrid skip;
-    int rc = hy_skip_view(ctx, b->vol, &b->params, &skip);
+    rc = hy_skip_view(ctx, b->vol, &b->params, &skip);
     if (rc) return rc;
     if (skip.d != b->base.skip.d) {
         b->base.skip = skip;
@@ -695,13 +710,15 @@ extern "C" int hy_batch_render(hy_batch *b, uint8_t *rgba_host) {
     if (!rgba_host) return hy_fail(b->ctx, HY_ERR_INVALID, "batch: null output");
     hy_ctx *ctx = b->ctx;
     HY_CUDA(ctx, cudaSetDevice(ctx->device));
+    int rc = refuse_capture(ctx);  // before the staging buffer is allocated
+    if (rc) return rc;
     if (uint8_t *direct = hy_mapped_device_ptr(rgba_host, 4)) {
-        int rc = launch(b, direct);
+        rc = launch(b, direct);
         if (rc) return rc;
         return hy_finish_stats(ctx);
     }
     void *stage = nullptr;
-    int rc = hy_stage(ctx, size_t(b->out_bytes), &stage);
+    rc = hy_stage(ctx, size_t(b->out_bytes), &stage);
     if (rc) return rc;
     rc = launch(b, static_cast<uint8_t *>(stage));
     if (rc) return rc;
@@ -716,6 +733,8 @@ extern "C" int hy_batch_autotune(hy_batch *b, uint8_t *rgba_dev, int32_t reps,
     if (!b || !rgba_dev) return HY_ERR_INVALID;
     hy_ctx *ctx = b->ctx;
     if (!hy_aligned(rgba_dev, 4)) return hy_fail(ctx, HY_ERR_INVALID, "batch: misaligned output (4-byte)");
+    int rc = refuse_capture(ctx);
+    if (rc) return rc;
     if (reps <= 0) reps = 3;
     const int tws[] = {8, 4, 16};
     const int grabs[] = {1, 2, 4};
@@ -727,7 +746,6 @@ extern "C" int hy_batch_autotune(hy_batch *b, uint8_t *rgba_dev, int32_t reps,
     cudaEvent_t e0, e1;
     HY_CUDA(ctx, cudaEventCreate(&e0));
     HY_CUDA(ctx, cudaEventCreate(&e1));
-    int rc = HY_OK;
     for (int bq = 0; bq < 2; ++bq)
     for (int tw : tws)
         for (int g : grabs)

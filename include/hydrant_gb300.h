@@ -491,7 +491,10 @@ int hy_batch_set_counting(hy_batch *batch, int32_t count_samples);
  * render.  Returns without waiting for the copy; `views` may be reused at once. */
 int hy_batch_update_views(hy_batch *batch, const hy_batch_view *views, int32_t nviews);
 int hy_batch_view_bytes(const hy_batch *batch, int64_t *bytes);
-/* Device output, asynchronous on the context's stream. */
+/* Device output, asynchronous on the context's stream.  The batch replays a
+ * graph of its own, so on a stream that is capturing this and the other calls
+ * that render a batch return HY_ERR_STATE and leave capture and batch as they
+ * are (capture hy_render_device per view instead). */
 int hy_batch_render_device(hy_batch *batch, uint8_t *rgba_dev);
 /* Host output; returns when the images are on the host.  rgba_host must
  * hold hy_batch_output_bytes bytes (as a cudaMemcpy destination must: a
@@ -515,9 +518,9 @@ int hy_batch_autotune(hy_batch *batch, uint8_t *rgba_dev, int32_t reps, hy_batch
  * synchronisation cost of cudaMalloc/cudaFree mid-frame.  Scratch lives in a
  * fixed ~33 KiB static device array that every GPU loading the library keeps
  * until exit.  The view descriptors are copied from host stack memory, so a
- * call on a stream that is capturing returns HY_ERR_STATE (capture the batch
- * path, hy_batch_*, instead).  Calls share that array: calls that overlap
- * on the GPU race.  More than 256 views is rejected with HY_ERR_INVALID.
+ * call on a stream that is capturing returns HY_ERR_STATE (capture
+ * hy_render_device per view instead).  Calls share that array: calls that
+ * overlap on the GPU race.  More than 256 views is rejected with HY_ERR_INVALID.
  * rgba_dev must hold at least max over views of rgba_offset + width*height*4
  * bytes (there is no size argument to check it against).
  * Asynchronous on the context's stream; count_samples is ignored. */
