@@ -385,12 +385,7 @@ template <typename T>
 int cell_hist(hy_volume *v) {
     hy_ctx *ctx = v->ctx;
     hy_skip &s = v->skip;
-    int *dev = reinterpret_cast<int *>(s.grid[0]);  // 16 KB of the grids, unused until a render
-    int *own = nullptr;
-    if (s.cells * 8 < (long long)(sizeof(int) * kBins * kBins)) {  // (or of its own)
-        HY_CUDA(ctx, cudaMalloc(&own, sizeof(int) * kBins * kBins));
-        dev = own;
-    }
+    int *dev = reinterpret_cast<int *>(s.grid[0]);  // the grids are unused until a render
     s.hist.assign(kBins * kBins, 0);
     cudaError_t e = cudaMemsetAsync(dev, 0, sizeof(int) * kBins * kBins, ctx->stream);
     if (e == cudaSuccess) {
@@ -403,7 +398,6 @@ int cell_hist(hy_volume *v) {
         e = cudaMemcpyAsync(s.hist.data(), dev, sizeof(int) * kBins * kBins, cudaMemcpyDeviceToHost,
                             ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (own) cudaFree(own);
     if (e != cudaSuccess) return hy_cuda_fail(ctx, e, "volume: skip grid");
     for (int i = kBins - 1; i >= 0; --i)
         for (int j = 0; j < kBins; ++j) {
@@ -486,10 +480,12 @@ dim3 cells_grid(const hy_volume *v, int bricks, int *threads) {
                 unsigned(std::max(1, std::min(rounds, 8 * v->ctx->sms / std::max(bricks, 1)))));
 }
 
-// The distances per transfer function and (iso) per isovalue, and the bit
-// planes they are worked out in, in one allocation.
+// The distances per transfer function and (iso) per isovalue (at least the
+// histogram's size: it is counted there), and the bit planes they are worked out
+// in, in one allocation.
 cudaError_t alloc_planes(hy_skip &s, bool iso) {
-    const size_t n = size_t(s.cells), grids = (n * (iso ? 16 : 8) + 255) / 256 * 256;
+    const size_t n = size_t(s.cells), hist = sizeof(int) * kBins * kBins,
+                 grids = (std::max(n * (iso ? 16 : 8), hist) + 255) / 256 * 256;
     const cudaError_t e =
         cudaMalloc(&s.grid[0], grids + size_t(bit_grid(s).words) * 33 * sizeof(unsigned int));
     if (e != cudaSuccess) return e;

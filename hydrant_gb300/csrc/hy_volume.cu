@@ -433,9 +433,10 @@ int upload_impl(hy_volume *vol, const void *host) {
 #undef HY_UP
     cleanup();
     vol->uploaded = true;
-    const int rc = hy_skip_build(vol);
+    // what the upload needs first: the skip grid gives way where memory is short
+    const int rc = build_gather(vol);
     if (rc) return rc;
-    return build_gather(vol);
+    return hy_skip_build(vol);
 }
 
 }  // namespace
