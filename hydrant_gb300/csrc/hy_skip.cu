@@ -34,6 +34,10 @@ namespace {
 
 constexpr int kStride = 16;     // steps between two looks (hy_shade.cuh, skip_hint)
 constexpr long long kMaxGridCells = 1ll << 27;
+// A ray crosses few cells of a smaller volume (below 64^3 voxels), and the grid's
+// part of its upload shows: 16^3 u8 209 and 258 us, 32^3 f32 90 and 148 (215 and
+// 176 by the upload before the grid).
+constexpr long long kMinGridCells = 512;
 
 // Voxel range [lo, hi] (padded indices) that samples of cell c along one axis
 // can touch: positions l in [c, c + 1] / nc of the brick map to
@@ -104,18 +108,25 @@ __device__ __forceinline__ void brick_cells(int nc, int P, float4 map, bool samp
     }
 }
 
+// Value bins of the cells' min/max histogram: 64 over [0, 1], the outer ones
+// open (a u8 voxel u is u / 255).
+constexpr int kBins = 64;
+
 struct CellArgs {
     const unsigned char *pool;
     const hy::RegEntry *reg;
     const int2 *info;
     int gx, gy;  // bricks
     int nc, P;
+    int *hist;   // cleared for the histogram's kernel
 };
 
 // A resident volume: brick blockIdx.x into the volume's grid of cells.
 template <typename T>
 __global__ void cell_minmax_kernel(const __grid_constant__ CellArgs a, MinMax<T> *__restrict__ out) {
     const int b = blockIdx.x, nc = a.nc, P = a.P;
+    if (b == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < kBins * kBins; i += blockDim.x) a.hist[i] = 0;
     const int bx = b % a.gx, by = (b / a.gx) % a.gy, bz = b / (a.gx * a.gy);
     const int2 in = a.info[b];
     const bool sampled = in.x == 0 && in.y >= 0;
@@ -177,9 +188,6 @@ __global__ void coarse_minmax_kernel(const unsigned char *__restrict__ coarse, l
         [&](int i, int j, int k, MinMax<T> m) { o[(k * nc + j) * nc + i] = m; });
 }
 
-// Value bins of the cells' min/max histogram: 64 over [0, 1], the outer ones
-// open (a u8 voxel u is u / 255).
-constexpr int kBins = 64;
 __device__ __forceinline__ int value_bin(float v) {
     return min(max(int(v * float(kBins)), 0), kBins - 1);
 }
@@ -382,30 +390,26 @@ int classify(hy_volume *v, const hy_skip_ranges &r, unsigned char *grid) {
 // The cells' histogram on the host, summed so that hist[i * kBins + j] counts
 // the cells with lo in bin >= i and hi in bin <= j.
 template <typename T>
-int cell_hist(hy_volume *v) {
+int cell_hist(hy_volume *v, int *dev) {
     hy_ctx *ctx = v->ctx;
     hy_skip &s = v->skip;
-    int *dev = reinterpret_cast<int *>(s.grid[0]);  // the grids are unused until a render
-    s.hist.assign(kBins * kBins, 0);
-    cudaError_t e = cudaMemsetAsync(dev, 0, sizeof(int) * kBins * kBins, ctx->stream);
-    if (e == cudaSuccess) {
-        const unsigned blocks = unsigned(std::min<long long>((s.cells + 255) / 256, 4 * ctx->sms));
-        cell_hist_kernel<T><<<blocks, 256, 0, ctx->stream>>>(
-            static_cast<const MinMax<T> *>(s.minmax), s.cells, sizeof(T) == 1 ? 1.f / 255.f : 1.f, dev);
-        e = cudaGetLastError();
-    }
+    s.hist.resize(kBins * kBins);
+    const unsigned blocks = unsigned(std::min<long long>((s.cells + 255) / 256, 4 * ctx->sms));
+    cell_hist_kernel<T><<<blocks, 256, 0, ctx->stream>>>(
+        static_cast<const MinMax<T> *>(s.minmax), s.cells, sizeof(T) == 1 ? 1.f / 255.f : 1.f, dev);
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s.hist.data(), dev, sizeof(int) * kBins * kBins, cudaMemcpyDeviceToHost,
                             ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return hy_cuda_fail(ctx, e, "volume: skip grid");
-    for (int i = kBins - 1; i >= 0; --i)
+    for (int i = kBins - 1; i >= 0; --i) {
+        int row = 0;
         for (int j = 0; j < kBins; ++j) {
-            int &h = s.hist[i * kBins + j];
-            h += (i + 1 < kBins ? s.hist[(i + 1) * kBins + j] : 0) +
-                 (j > 0 ? s.hist[i * kBins + j - 1] : 0) -
-                 (i + 1 < kBins && j > 0 ? s.hist[(i + 1) * kBins + j - 1] : 0);
+            row += s.hist[i * kBins + j];
+            s.hist[i * kBins + j] = row + (i + 1 < kBins ? s.hist[(i + 1) * kBins + j] : 0);
         }
+    }
     s.sampled = s.hist[kBins - 1];
     return HY_OK;
 }
@@ -434,8 +438,10 @@ bool same_ranges(const hy_skip_ranges &a, const hy_skip_ranges &b) {
 
 void hy_skip_free(hy_volume *v) {
     hy_skip &s = v->skip;
-    if (s.minmax) cudaFree(s.minmax);
-    if (s.slots) cudaFree(s.slots);
+    if (s.slots) {  // paged; else minmax lies in grid[0]'s allocation
+        cudaFree(s.slots);
+        if (s.minmax) cudaFree(s.minmax);
+    }
     if (s.grid[0]) cudaFree(s.grid[0]);
     s = hy_skip();
 }
@@ -458,7 +464,7 @@ void skip_geometry(hy_volume *v) {
         n *= s.c[i];
         gmax = std::max(gmax, v->grid[i]);
     }
-    if (n > kMaxGridCells) return;
+    if (n < kMinGridCells || n > kMaxGridCells) return;
     // A run of up to 127 steps adds up to 127 roundings of half an ulp of
     // the largest coordinate; 4e-6 brick covers the run length's own
     // arithmetic.  Boxes shrink by this much, so that a run that stays in one
@@ -481,16 +487,17 @@ dim3 cells_grid(const hy_volume *v, int bricks, int *threads) {
 }
 
 // The distances per transfer function and (iso) per isovalue (at least the
-// histogram's size: it is counted there), and the bit planes they are worked out
-// in, in one allocation.
-cudaError_t alloc_planes(hy_skip &s, bool iso) {
+// histogram's size: it is counted there), the bit planes they are worked out in
+// and `minmax` bytes of the cells' own (0: none), in one allocation.
+cudaError_t alloc_planes(hy_skip &s, bool iso, size_t minmax) {
     const size_t n = size_t(s.cells), hist = sizeof(int) * kBins * kBins,
-                 grids = (std::max(n * (iso ? 16 : 8), hist) + 255) / 256 * 256;
-    const cudaError_t e =
-        cudaMalloc(&s.grid[0], grids + size_t(bit_grid(s).words) * 33 * sizeof(unsigned int));
+                 grids = (std::max(n * (iso ? 16 : 8), hist) + 255) / 256 * 256,
+                 planes = (size_t(bit_grid(s).words) * 33 * sizeof(unsigned int) + 255) / 256 * 256;
+    const cudaError_t e = cudaMalloc(&s.grid[0], grids + planes + minmax);
     if (e != cudaSuccess) return e;
     s.grid[1] = iso ? s.grid[0] + 8 * n : nullptr;
     s.bits = reinterpret_cast<unsigned int *>(s.grid[0] + grids);
+    if (minmax) s.minmax = s.grid[0] + grids + planes;
     return e;
 }
 
@@ -508,14 +515,15 @@ int hy_skip_build(hy_volume *v) {
     skip_geometry(v);
     if (!s.nc) return HY_OK;
     const bool u8 = v->desc.dtype == HY_DTYPE_U8;
-    cudaError_t e = cudaMalloc(&s.minmax, size_t(s.cells) * mm_bytes(v));
-    if (e == cudaSuccess) e = alloc_planes(s, true);
+    const cudaError_t e = alloc_planes(s, true, size_t(s.cells) * mm_bytes(v));
     if (e != cudaSuccess) {  // no room: the march samples every cell
         hy_skip_free(v);
         cudaGetLastError();
         return HY_OK;
     }
-    CellArgs a{v->pool, v->reg_dev, v->info_dev, v->grid[0], v->grid[1], s.nc, v->P};
+    int *hist = reinterpret_cast<int *>(s.grid[0]);  // the grids are unused until a render
+    const CellArgs a{v->pool,    v->reg_dev, v->info_dev, v->grid[0],
+                     v->grid[1], s.nc,       v->P,        hist};
     int threads;
     const dim3 grid = cells_grid(v, v->nbricks, &threads);
     if (u8)
@@ -525,7 +533,7 @@ int hy_skip_build(hy_volume *v) {
         cell_minmax_kernel<float><<<grid, threads, 0, ctx->stream>>>(
             a, static_cast<MinMax<float> *>(s.minmax));
     HY_CUDA(ctx, cudaGetLastError());
-    return u8 ? cell_hist<unsigned char>(v) : cell_hist<float>(v);
+    return u8 ? cell_hist<unsigned char>(v, hist) : cell_hist<float>(v, hist);
 }
 
 int hy_skip_build_paged(hy_volume *v, const hy_store *store, int nslots, int reg_base) {
@@ -539,7 +547,7 @@ int hy_skip_build_paged(hy_volume *v, const hy_store *store, int nslots, int reg
     unsigned char *coarse = nullptr;  // the coarse level, for its cells alone
     s.reg_base = reg_base;
     cudaError_t e = cudaMalloc(&s.slots, size_t(nslots) * per);
-    if (e == cudaSuccess) e = alloc_planes(s, !v->paged_gather);
+    if (e == cudaSuccess) e = alloc_planes(s, !v->paged_gather, 0);
     if (e == cudaSuccess && reg_base > 0) {
         e = cudaMalloc(&s.minmax, size_t(v->nbricks) * per);
         if (e == cudaSuccess) e = cudaMalloc(&coarse, store->coarse.size());
