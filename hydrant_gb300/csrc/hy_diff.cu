@@ -834,7 +834,8 @@ dim3 diff_grid(const DiffArgs &a) { return dim3((a.W + 15) / 16, (a.H + 7) / 8, 
 
 // Both passes sample the volume through a gather texture refreshed from the
 // caller's volume at each call (inside the timed launch); by loads where the
-// device cannot make it.
+// device cannot make it, and while the stream is captured: a graph would keep the
+// texture after the context has replaced it.
 struct DiffGather {
     cudaArray_t arr = nullptr;
     unsigned long long tex = 0, surf = 0;
@@ -855,6 +856,9 @@ void free_diff_gather(DiffGather *g) {
 // samples by loads.
 int diff_gather_refresh(hy_ctx *ctx, const float *vol, int n, DiffArgs &a, bool *ok) {
     *ok = false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HY_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return HY_OK;
     DiffGather *g = static_cast<DiffGather *>(ctx->diff_gather);
     if (!g || g->n != n) {
         free_diff_gather(g);

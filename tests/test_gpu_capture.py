@@ -67,3 +67,74 @@ def test_batch_refuses_a_capturing_stream(ctx, warm):
     finally:
         b.close()
         vol.close()
+
+
+def diff_case(ctx, n=24, seed=4):
+    torch = pytest.importorskip("torch")
+    from hydrant_gb300 import fit
+    from tests.test_gpu_diff_forms import inputs
+
+    vol, tf, views, _ = inputs(ctx, n, 2, 9)
+    r = fit.DiffRenderer(ctx, n, views, 33, 21, 9, density=0.7, ckpt_k=5)
+    tv, tt = torch.from_numpy(vol).cuda(), torch.from_numpy(tf).cuda()
+    img = torch.zeros(2, 21, 33, 4, device="cuda")
+    dimg = torch.rand(2, 21, 33, 4, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+    dvol, dtf = torch.zeros_like(tv), torch.zeros_like(tt)
+    lib = hy.lib()
+
+    def forward():
+        ctx.check(lib.hy_diff_forward(
+            ctx.handle, C.byref(r.p), C.c_void_p(tv.data_ptr()), C.c_void_p(tt.data_ptr()), r.views,
+            r.nviews, r.W, r.H, C.c_void_p(img.data_ptr()), C.c_void_p(r.ckpt.data_ptr()),
+            C.c_void_p(r.nsteps.data_ptr())))
+
+    def backward():
+        ctx.check(lib.hy_diff_backward(
+            ctx.handle, C.byref(r.p), C.c_void_p(tv.data_ptr()), C.c_void_p(tt.data_ptr()), r.views,
+            r.nviews, r.W, r.H, C.c_void_p(dimg.data_ptr()), C.c_void_p(r.ckpt.data_ptr()),
+            C.c_void_p(r.nsteps.data_ptr()), C.c_void_p(dvol.data_ptr()), C.c_void_p(dtf.data_ptr())))
+
+    return forward, backward, img, dvol, dtf, tv, (r, tt, dimg)
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_captured_differentiable_passes(warm):
+    """Forward and adjoint are captured on a fresh context and on one that has
+    its texture, and replay what the calls give, also after the context has
+    rendered a volume of another edge and after the voxels changed."""
+    torch = pytest.importorskip("torch")
+    ctx = hy.Context(0)
+    forward, backward, img, dvol, dtf, tv, keep = diff_case(ctx)
+    torch.cuda.synchronize()
+    if warm:
+        forward()
+        backward()
+    ctx.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(ctx.stream)):
+        forward()
+        backward()
+    other = diff_case(ctx, 40)
+    torch.cuda.synchronize()
+    other[0]()
+    other[1]()
+    ctx.synchronize()
+    for scale in (1.0, 0.5):
+        tv *= scale
+        torch.cuda.synchronize()
+        img.zero_(), dvol.zero_(), dtf.zero_()
+        torch.cuda.synchronize()
+        forward()
+        backward()
+        ctx.synchronize()
+        want = [t.clone() for t in (img, dvol, dtf)]
+        img.zero_(), dvol.zero_(), dtf.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(img, want[0])
+        # float atomics in another order: 24^3 x 2 views of some 100 samples a ray
+        for a, b in zip((dvol, dtf), want[1:]):
+            assert torch.linalg.norm((a - b).double()) <= 1e-5 * torch.linalg.norm(b.double())
+    del g
+    ctx.close()
