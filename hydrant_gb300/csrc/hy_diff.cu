@@ -839,7 +839,7 @@ dim3 diff_grid(const DiffArgs &a) { return dim3((a.W + 15) / 16, (a.H + 7) / 8, 
 struct DiffGather {
     cudaArray_t arr = nullptr;
     unsigned long long tex = 0, surf = 0;
-    int n = 0, gper = 0;
+    int w = 0, h = 0;  // texels
 };
 
 void free_diff_gather(DiffGather *g) {
@@ -850,66 +850,76 @@ void free_diff_gather(DiffGather *g) {
     delete g;
 }
 
-// The context's texture of an n^3 volume, (re)made for n, filled from vol on
-// the stream.  *ok = false (no error) when this device cannot make it (an
-// edge too large for a gather texture, or no memory left): the caller then
-// samples by loads.
+// Slices per column in h rows (plus the repeated one; less than 2: too few rows)
+// and the columns of the footprints' lower slices.
+int slices_per_column(int P, int h) { return std::max(0, std::min(h / P, P) - 1); }
+int slice_columns(int P, int gper) { return (P - 2) / gper + 1; }
+
+DiffGather *make_diff_gather(int w, int h) {
+    DiffGather *g = new DiffGather();
+    g->w = w;
+    g->h = h;
+    cudaChannelFormatDesc cd = cudaCreateChannelDesc(32, 0, 0, 0, cudaChannelFormatKindFloat);
+    cudaError_t e = cudaMallocArray(&g->arr, &cd, size_t(w), size_t(h),
+                                    cudaArrayTextureGather | cudaArraySurfaceLoadStore);
+    cudaResourceDesc rd;
+    std::memset(&rd, 0, sizeof(rd));
+    rd.resType = cudaResourceTypeArray;
+    rd.res.array.array = g->arr;
+    cudaTextureDesc td;
+    std::memset(&td, 0, sizeof(td));
+    td.addressMode[0] = td.addressMode[1] = cudaAddressModeClamp;
+    td.filterMode = cudaFilterModePoint;
+    td.readMode = cudaReadModeElementType;
+    td.normalizedCoords = 0;
+    cudaTextureObject_t t = 0;
+    cudaSurfaceObject_t so = 0;
+    if (e == cudaSuccess) e = cudaCreateTextureObject(&t, &rd, &td, nullptr);
+    if (e == cudaSuccess) g->tex = (unsigned long long)t;
+    if (e == cudaSuccess) e = cudaCreateSurfaceObject(&so, &rd);
+    if (e == cudaSuccess) g->surf = (unsigned long long)so;
+    if (e == cudaSuccess) return g;
+    free_diff_gather(g);  // e.g. no room: the loads serve this call
+    cudaGetLastError();
+    return nullptr;
+}
+
+// The context's texture, filled from the n^3 volume on the stream.  A texture
+// that holds a smaller volume's slices too is kept for it (edges that alternate
+// neither allocate nor wait), one too small is replaced once the launches that
+// read it are through.  *ok = false (no error): by loads.
 int diff_gather_refresh(hy_ctx *ctx, const float *vol, int n, DiffArgs &a, bool *ok) {
     *ok = false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     HY_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone) return HY_OK;
     DiffGather *g = static_cast<DiffGather *>(ctx->diff_gather);
-    if (!g || g->n != n) {
-        free_diff_gather(g);
-        ctx->diff_gather = nullptr;
+    const int P = n + 2;
+    int gper = g ? slices_per_column(P, g->h) : 0;
+    if (gper < 2 || (long long)slice_columns(P, gper) * P > g->w) {
         int gw = 0, gh = 0;
         HY_CUDA(ctx, cudaDeviceGetAttribute(&gw, cudaDevAttrMaxTexture2DGatherWidth, ctx->device));
         HY_CUDA(ctx, cudaDeviceGetAttribute(&gh, cudaDevAttrMaxTexture2DGatherHeight, ctx->device));
-        const int P = n + 2;
-        const int gper = gh / P - 1;  // slices per column, plus the repeated one
-        if (gper < 1) return HY_OK;
-        const int cols = (P - 2) / gper + 1;  // columns of the footprints' lower slices
-        if ((long long)cols * P > gw) return HY_OK;
-        g = new DiffGather();
-        g->n = n;
-        g->gper = gper;
-        cudaChannelFormatDesc cd = cudaCreateChannelDesc(32, 0, 0, 0, cudaChannelFormatKindFloat);
-        cudaError_t e = cudaMallocArray(&g->arr, &cd, size_t(cols) * P, size_t(gper + 1) * P,
-                                        cudaArrayTextureGather | cudaArraySurfaceLoadStore);
-        cudaResourceDesc rd;
-        std::memset(&rd, 0, sizeof(rd));
-        rd.resType = cudaResourceTypeArray;
-        rd.res.array.array = g->arr;
-        cudaTextureDesc td;
-        std::memset(&td, 0, sizeof(td));
-        td.addressMode[0] = td.addressMode[1] = cudaAddressModeClamp;
-        td.filterMode = cudaFilterModePoint;
-        td.readMode = cudaReadModeElementType;
-        td.normalizedCoords = 0;
-        cudaTextureObject_t t = 0;
-        cudaSurfaceObject_t so = 0;
-        if (e == cudaSuccess) e = cudaCreateTextureObject(&t, &rd, &td, nullptr);
-        if (e == cudaSuccess) g->tex = (unsigned long long)t;
-        if (e == cudaSuccess) e = cudaCreateSurfaceObject(&so, &rd);
-        if (e == cudaSuccess) g->surf = (unsigned long long)so;
-        if (e != cudaSuccess) {  // e.g. no room: the loads serve this call
+        gper = slices_per_column(P, gh);
+        if (gper < 2 || (long long)slice_columns(P, gper) * P > gw) return HY_OK;
+        if (g) {
+            HY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             free_diff_gather(g);
-            cudaGetLastError();
-            return HY_OK;
+            ctx->diff_gather = nullptr;
         }
+        g = make_diff_gather(slice_columns(P, gper) * P, (gper + 1) * P);
+        if (!g) return HY_OK;
         ctx->diff_gather = g;
     }
-    const int P = n + 2;
     const dim3 grid((P + kFillRows - 1) / kFillRows, P);
     if (P % 2 == 0)
-        diff_fill_kernel<true><<<grid, 256, 0, ctx->stream>>>(vol, n, g->gper, g->surf);
+        diff_fill_kernel<true><<<grid, 256, 0, ctx->stream>>>(vol, n, gper, g->surf);
     else
-        diff_fill_kernel<false><<<grid, 256, 0, ctx->stream>>>(vol, n, g->gper, g->surf);
+        diff_fill_kernel<false><<<grid, 256, 0, ctx->stream>>>(vol, n, gper, g->surf);
     HY_CUDA(ctx, cudaGetLastError());
     a.gtex = g->tex;
-    a.gper = g->gper;
-    a.gmagic = unsigned((1ull << 32) / unsigned(g->gper) + 1);
+    a.gper = gper;
+    a.gmagic = unsigned((1ull << 32) / unsigned(gper) + 1);
     *ok = true;
     return HY_OK;
 }

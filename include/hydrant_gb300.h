@@ -421,8 +421,9 @@ int hy_pager_render_host(hy_pager *pager, const hy_shader_params *params, const 
  * the transfer function and the trilinear weights, accumulating into
  * caller-zeroed gradient buffers.  All pointers are device pointers; views is
  * a host array; both calls are asynchronous on the context's stream.  They
- * sample through a texture of the volume's size that the context keeps; without
- * room for it, and on a stream that is capturing, by loads. */
+ * sample through a texture that the context keeps until it is destroyed, as large
+ * as the largest volume it has rendered (some 4 n^3 bytes); without room for it,
+ * and on a stream that is capturing, by loads. */
 typedef struct hy_diff_params {
     int32_t n;            /* volume edge (voxels); bbox = [0,1]^3 */
     float sample_rate;    /* step = (1/n) / 4 / sample_rate */

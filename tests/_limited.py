@@ -22,7 +22,7 @@ WRAP = r"""
 static std::mutex mu;
 static std::map<const void *, size_t> sizes;
 static size_t live = 0, limit = ~size_t(0), most = 0;
-static int arrays = 1;
+static int arrays = 1, array_calls = 0;
 static bool take(size_t n) {
     std::lock_guard<std::mutex> l(mu);
     if (live + n > limit) return false;
@@ -60,6 +60,7 @@ cudaError_t __wrap_cudaFree(void *p) {
 cudaError_t __wrap_cudaMallocArray(cudaArray_t *a, const cudaChannelFormatDesc *d, size_t w,
                                    size_t h, unsigned int flags) {
     const size_t n = (size_t)(d->x + d->y + d->z + d->w) / 8 * w * (h ? h : 1);
+    ++array_calls;
     if (!arrays || !take(n)) return cudaErrorMemoryAllocation;
     cudaError_t e = __real_cudaMallocArray(a, d, w, h, flags);
     if (e == cudaSuccess) keep(*a, n);
@@ -73,6 +74,7 @@ void test_memory_limit(size_t n) { limit = n; most = live; }
 size_t test_memory_live(void) { return live; }
 size_t test_memory_most(void) { return most; }
 void test_memory_arrays(int allowed) { arrays = allowed; }
+int test_memory_array_calls(void) { return array_calls; }
 }
 """
 

@@ -53,3 +53,60 @@ def test_upload_without_room_for_its_grid(limited):
     """A volume that fits without the skip grid is uploaded, with its gather
     textures, and renders the same images."""
     assert "ok" in _limited.run(limited, UPLOAD)
+
+
+DIFF = """
+import numpy as np, torch
+import hydrant_gb300 as hy
+from hydrant_gb300 import fit
+from oracle import oracle as orc
+from tests.test_gpu_diff_forms import inputs
+ctx = hy.Context(0)
+cases = []
+for n, W, H in ((40, 33, 21), (24, 17, 13), (39, 20, 9), (23, 395, 394), (9, 31, 7)):
+    vol, tf, views, va = inputs(ctx, n, 2, 7)
+    r = fit.DiffRenderer(ctx, n, views, W, H, 7, density=0.7, ckpt_k=5)
+    ref = orc.diff_forward(vol, tf, va, W, H, density=0.7)
+    cases.append((r, torch.from_numpy(vol).cuda(), torch.from_numpy(tf).cuda(), ref))
+torch.cuda.synchronize()
+mem.test_memory_arrays({arrays})
+calls = mem.test_memory_array_calls()
+# the edges in turn, nothing waited for in between
+images = [[r.forward(v, t) for r, v, t, _ in cases] for _ in range(3)]
+grads = [r.backward(v, t, 2 * im) for (r, v, t, _), im in zip(cases, images[0])]
+torch.cuda.synchronize()
+for turn in images:
+    for im, (_, _, _, ref) in zip(turn, cases):
+        assert np.array_equal(im.cpu().numpy(), ref)
+for dv, dt in grads:
+    assert torch.isfinite(dv).all() and dv.abs().sum() > 0 and dt.abs().sum() > 0
+made = mem.test_memory_array_calls() - calls
+print("made", made)
+"""
+
+
+@pytest.mark.parametrize("arrays", [1, 0])
+def test_differentiable_edges_in_turn(limited, arrays):
+    """Volumes of several edges on one context: one texture, the largest's,
+    serves all; without one every call samples by loads (and asks again).  The
+    images are the oracle's."""
+    out = _limited.run(limited, DIFF.format(arrays=arrays))
+    assert int(out.split("made")[1]) == (1 if arrays else 20)
+
+
+FALLBACK = """
+import hydrant_gb300 as hy
+import tests.test_gpu_diff_forms as forms
+mem.test_memory_arrays(0)
+ctx = hy.Context(0)
+for case in ((23, 2, 17, 13, 5, 1, 1.0), (24, 2, 33, 7, 16, 3, 1.0), (9, 3, 20, 20, 1, 64, 2.0),
+             (24, 1, 395, 394, 16, 7, 0.5), (24, 1, 395, 395, 256, 32, 0.5)):
+    forms.test_forward_and_gradients(ctx, *case)
+forms.test_values_out_of_range(ctx)
+print("ok")
+"""
+
+
+def test_differentiable_passes_by_loads(limited):
+    """Forward and gradients where the texture cannot be made."""
+    assert "ok" in _limited.run(limited, FALLBACK)
