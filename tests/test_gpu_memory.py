@@ -110,3 +110,30 @@ print("ok")
 def test_differentiable_passes_by_loads(limited):
     """Forward and gradients where the texture cannot be made."""
     assert "ok" in _limited.run(limited, FALLBACK)
+
+
+FEW_RAYS = """
+import numpy as np, torch
+import hydrant_gb300 as hy
+from hydrant_gb300 import fit
+from oracle import oracle as orc
+from tests.test_gpu_diff_forms import inputs
+ctx = hy.Context(0)
+vol, tf, views, va = inputs(ctx, 384, 1, 9)
+tv, tt = torch.from_numpy(vol).cuda(), torch.from_numpy(tf).cuda()
+for W, H, rate, texture in ((9, 7, 0.25, 0), (40, 33, 0.25, 1), (9, 7, 1.0, 1)):
+    r = fit.DiffRenderer(ctx, 384, views, W, H, 9, sample_rate=rate, ckpt_k=7)
+    ref = orc.diff_forward(vol, tf, va, W, H, sample_rate=rate)
+    calls = mem.test_memory_array_calls()
+    mem.test_memory_arrays(texture)
+    for keep in (True, False):
+        assert np.array_equal(r.forward(tv, tt, keep=keep).cpu().numpy(), ref), (W, rate)
+    assert (mem.test_memory_array_calls() > calls) == (texture == 1 and rate < 1), (W, rate)
+print("ok")
+"""
+
+
+def test_few_rays_over_a_large_volume(limited):
+    """A forward that takes fewer samples than the texture's refresh is worth
+    goes by loads and makes none."""
+    assert "ok" in _limited.run(limited, FEW_RAYS)
