@@ -511,7 +511,7 @@ int launch(hy_batch *b, uint8_t *out) {
     // the skip grid follows the knots; a batch that gains or loses it is
     // another kernel and graph
     SkipGrid skip;
-    rc = hy_skip_view(ctx, b->vol, &b->params, &skip);
+    rc = hy_skip_view(ctx, b->vol, &b->params, &skip, false);
     if (rc) return rc;
     if (skip.d != b->base.skip.d) {
         b->base.skip = skip;
@@ -554,7 +554,9 @@ int launch(hy_batch *b, uint8_t *out) {
         b->graph_out = out;
         b->graph_count = count;
     }
-    HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+    rc = hy_time_begin(ctx, false);  // the graph clears the counter
+    if (!rc) rc = hy_skip_view(ctx, b->vol, &b->params, &skip);
+    if (rc) return rc;
     HY_CUDA(ctx, cudaGraphLaunch(b->exec, ctx->stream));
     HY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->stats_pending = true;
@@ -872,7 +874,7 @@ extern "C" int hy_render_views_noalloc(hy_ctx *ctx, const hy_volume *vol,
     if (rc) return rc;
     base.count = 0;  // sample counting is not available on this entry point
     HY_CUDA(ctx, cudaSetDevice(ctx->device));
-    rc = hy_skip_view(ctx, vol, params, &base.skip);
+    rc = hy_skip_view(ctx, vol, params, &base.skip, false);
     if (rc) return rc;
     // The descriptors are copied from this call's stack: a captured copy
     // would replay from a dead address, so capture is refused.
@@ -950,7 +952,9 @@ extern "C" int hy_render_views_noalloc(hy_ctx *ctx, const hy_volume *vol,
     HY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     HY_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     void *kargs[] = {&args};
-    HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+    rc = hy_time_begin(ctx, false);
+    if (!rc) rc = hy_skip_view(ctx, vol, params, &base.skip);
+    if (rc) return rc;
     HY_CUDA(ctx, cudaLaunchKernel(kernel, dim3(sms * std::max(per_sm, 1)), dim3(threads), kargs,
                                   smem, ctx->stream));
     HY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));

@@ -303,10 +303,12 @@ void hy_chebyshev_transform(const std::vector<unsigned char> &nonempty, const in
 // Skip grid (hy_skip.cu): built from the brick pool by the upload, freed with
 // it; hy_skip_view brings it in line with the context's knots (or the
 // isovalue) on the context's stream and fills a launch's view of it, with a
-// null grid where the launch has to sample every cell.
+// null grid where the launch has to sample every cell (refresh false: the view
+// alone, to choose a kernel by).
 int hy_skip_build(hy_volume *v);
 void hy_skip_free(hy_volume *v);
-int hy_skip_view(hy_ctx *ctx, const hy_volume *v, const hy_shader_params *p, hy::SkipGrid *out);
+int hy_skip_view(hy_ctx *ctx, const hy_volume *v, const hy_shader_params *p, hy::SkipGrid *out,
+                 bool refresh = true);
 // A realtime pager's volume: cells per cache slot (hy_skip_slots after each
 // fill, on the fill's stream) and per coarse stand-in; the grid is renewed
 // after hy_skip_page_table_changed by the next hy_skip_view.
@@ -339,11 +341,13 @@ uint8_t *hy_mapped_device_ptr(void *host, uintptr_t align);
 // staging buffer (hy_api.cc)
 int hy_stage(hy_ctx *ctx, size_t bytes, void **out);
 
-// launchers (hy_render.cu)
+// launchers (hy_render.cu, hy_pass.cu).  hy_time_begin opens the time that
+// hy_render_stats.ms gives, before the skip grid is brought up to date; the
+// launcher closes it.  reset_counter = false: the sample counter keeps counting
+// from the previous passes (a pager frame made of several passes).
+int hy_time_begin(hy_ctx *ctx, bool reset_counter);
 int hy_launch_render(hy_ctx *ctx, const hy::ShadeArgs &args);
-// reset_counter = false: the sample counter keeps counting from the previous
-// passes (a pager frame made of several passes)
-int hy_launch_pass(hy_ctx *ctx, const hy::ShadeArgs &args, int pass, bool reset_counter = true);
+int hy_launch_pass(hy_ctx *ctx, const hy::ShadeArgs &args, int pass);
 int hy_finish_stats(hy_ctx *ctx);
 int hy_fill_args(hy_ctx *ctx, const hy_volume *vol, const hy_shader_params *p, const hy_view *view,
                  int W, int H, hy::ShadeArgs *a);

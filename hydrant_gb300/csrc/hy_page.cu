@@ -1263,7 +1263,8 @@ int render_lossless(hy_pager *pg, const hy_shader_params *p, const hy_camera *ca
         for (size_t i = 0; i < cur.size(); ++i) pg->page[cur[i]] = cur_slots[i];
         rc = upload_page_table(pg, k & 1);
         if (rc) return rc;
-        rc = hy_launch_pass(ctx, a, k == 0 ? HY_PASS_RAY_EMIT : HY_PASS_RAY_MARCH, false);
+        rc = hy_time_begin(ctx, false);
+        if (!rc) rc = hy_launch_pass(ctx, a, k == 0 ? HY_PASS_RAY_EMIT : HY_PASS_RAY_MARCH);
         if (rc) return rc;
         HY_CUDA(ctx, cudaEventRecord(pg->marched[k & 1], ctx->stream));
         ++pg->stats.passes;

@@ -236,12 +236,7 @@ void dispatch_pass(const ShadeArgs &a, int pass, cudaStream_t s) {
 
 }  // namespace
 
-int hy_launch_pass(hy_ctx *ctx, const ShadeArgs &a, int pass, bool reset_counter) {
-    int rc = hy_check_paged_gather(ctx, a, false);
-    if (rc) return rc;
-    if (reset_counter && a.count && pass <= HY_PASS_RAY_MARCH)
-        HY_CUDA(ctx, cudaMemsetAsync(ctx->counter_dev, 0, sizeof(unsigned long long), ctx->stream));
-    HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+int hy_launch_pass(hy_ctx *ctx, const ShadeArgs &a, int pass) {
     switch (a.shader) {
         case HY_SHADER_VOLUME:
             dispatch_pass<HY_SHADER_VOLUME>(a, pass, ctx->stream);

@@ -550,11 +550,14 @@ int hy_check_paged_gather(hy_ctx *ctx, const ShadeArgs &a, bool fused) {
                    "Paging shaders; create the pager with HY_PAGER_LOADS for this use");
 }
 
-int hy_launch_render(hy_ctx *ctx, const ShadeArgs &a) {
-    int rc = hy_check_paged_gather(ctx, a, true);
-    if (rc) return rc;
-    if (a.count) HY_CUDA(ctx, cudaMemsetAsync(ctx->counter_dev, 0, sizeof(unsigned long long), ctx->stream));
+int hy_time_begin(hy_ctx *ctx, bool reset_counter) {
+    if (reset_counter)
+        HY_CUDA(ctx, cudaMemsetAsync(ctx->counter_dev, 0, sizeof(unsigned long long), ctx->stream));
     HY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+    return HY_OK;
+}
+
+int hy_launch_render(hy_ctx *ctx, const ShadeArgs &a) {
     switch (a.shader) {
         case HY_SHADER_VOLUME:
             dispatch_fused<HY_SHADER_VOLUME>(a, ctx->stream);
@@ -605,12 +608,13 @@ extern "C" int hy_render_device(hy_ctx *ctx, const hy_volume *vol, const hy_shad
     ShadeArgs a;
     int rc = hy_fill_args(ctx, vol, p, view, W, H, &a);
     if (rc) return rc;
-    rc = hy_skip_view(ctx, vol, p, &a.skip);
-    if (rc) return rc;
     a.rgba = reinterpret_cast<uchar4 *>(rgba_dev);
     a.vout = reinterpret_cast<float4 *>(v_dev);
     a.aux = reinterpret_cast<float4 *>(aux_dev);
-    return hy_launch_render(ctx, a);
+    rc = hy_check_paged_gather(ctx, a, true);
+    if (!rc) rc = hy_time_begin(ctx, a.count);
+    if (!rc) rc = hy_skip_view(ctx, vol, p, &a.skip);
+    return rc ? rc : hy_launch_render(ctx, a);
 }
 
 uint8_t *hy_mapped_device_ptr(void *host, uintptr_t align) {
@@ -633,8 +637,6 @@ extern "C" int hy_render(hy_ctx *ctx, const hy_volume *vol, const hy_shader_para
     int rc = hy_fill_args(ctx, vol, p, view, W, H, &a);
     if (rc) return rc;
     HY_CUDA(ctx, cudaSetDevice(ctx->device));
-    rc = hy_skip_view(ctx, vol, p, &a.skip);
-    if (rc) return rc;
     // outputs in pinned, mapped host memory are written by the kernel itself
     // (as in hy_batch_render); the others are staged in device memory and
     // copied once
@@ -662,7 +664,10 @@ extern "C" int hy_render(hy_ctx *ctx, const hy_volume *vol, const hy_shader_para
     a.rgba = reinterpret_cast<uchar4 *>(place(rgba_d, rgba_b));
     if (v_out) a.vout = reinterpret_cast<float4 *>(place(v_d, f4_b));
     if (aux_out) a.aux = reinterpret_cast<float4 *>(place(aux_d, f4_b));
-    rc = hy_launch_render(ctx, a);
+    rc = hy_check_paged_gather(ctx, a, true);
+    if (!rc) rc = hy_time_begin(ctx, a.count);
+    if (!rc) rc = hy_skip_view(ctx, vol, p, &a.skip);
+    if (!rc) rc = hy_launch_render(ctx, a);
     if (rc) return rc;
     if (!rgba_d)
         HY_CUDA(ctx, cudaMemcpyAsync(rgba_out, a.rgba, npx * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -691,14 +696,15 @@ extern "C" int hy_shade_pass(hy_ctx *ctx, const hy_volume *vol, const hy_shader_
     ShadeArgs a;
     int rc = hy_fill_args(ctx, vol, p, view, W, H, &a);
     if (rc) return rc;
-    if (pass <= HY_PASS_RAY_MARCH) {
-        HY_CUDA(ctx, cudaSetDevice(ctx->device));
-        rc = hy_skip_view(ctx, vol, p, &a.skip);
-        if (rc) return rc;
-    }
     a.film = film_dev;
     a.dst = dst_dev;
     if (clear_rgb)
         for (int i = 0; i < 3; ++i) a.clear_u8[i] = clear_rgb[i];
-    return hy_launch_pass(ctx, a, pass);
+    rc = hy_check_paged_gather(ctx, a, false);
+    if (rc) return rc;
+    const bool marches = pass <= HY_PASS_RAY_MARCH;
+    HY_CUDA(ctx, cudaSetDevice(ctx->device));
+    rc = hy_time_begin(ctx, a.count && marches);
+    if (!rc && marches) rc = hy_skip_view(ctx, vol, p, &a.skip);
+    return rc ? rc : hy_launch_pass(ctx, a, pass);
 }

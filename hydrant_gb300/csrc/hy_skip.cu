@@ -644,7 +644,8 @@ void hy_skip_tf_ranges(const float *rgba, int n, hy_skip_ranges *r, float *alpha
     }
 }
 
-int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy::SkipGrid *out) {
+int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy::SkipGrid *out,
+                 bool refresh) {
     std::memset(out, 0, sizeof(*out));
     out->stride = 1 << 30;
     hy_volume *v = const_cast<hy_volume *>(cv);  // the grids are a cache of its bricks
@@ -686,7 +687,7 @@ int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     HY_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone) return HY_OK;
-    if (!s.valid[which] || !same_ranges(r, s.key[which])) {
+    if (refresh && (!s.valid[which] || !same_ranges(r, s.key[which]))) {
         s.valid[which] = false;
         const int rc = v->desc.dtype == HY_DTYPE_U8 ? classify<unsigned char>(v, r, s.grid[which])
                                                     : classify<float>(v, r, s.grid[which]);

@@ -180,7 +180,8 @@ typedef struct hy_volume_info {
 typedef struct hy_render_stats {
     int64_t samples;        /* trilinear brick samples of the last render (count_samples=1) */
     int64_t pixels;
-    float ms;               /* device time of the last render's kernels */
+    float ms;               /* device time of the last render's kernels, the ones that
+                               prepare it (the skip grid, after new knots) among them */
 } hy_render_stats;
 
 /* ---- context ----------------------------------------------------------------
