@@ -343,7 +343,9 @@ class Batch:
         return c
 
     def set_config(self, tile_w=8, grab=1, block_warps=4, blocks_per_sm=0, block_queue=1,
-                   steps_per_iter=1) -> None:
+                   steps_per_iter=0) -> None:
+        """hy_batch_config; the defaults are the library's (steps_per_iter 0: a
+        ray's samples in flight by the library's rule)."""
         c = HyBatchConfig(tile_w, grab, block_warps, blocks_per_sm, block_queue, steps_per_iter)
         self.ctx.check(lib().hy_batch_set_config(self.handle, C.byref(c)))
 
