@@ -86,6 +86,17 @@ __global__ void __launch_bounds__(kThreads, pass_blocks(LOOP, GATHER))
     count_samples(A, samples);
 }
 
+// Whether a film's pixel is one that a march leaves: the step size its opacity
+// asks for, nothing that 0 * t would turn into NaN.  Others (a film that the caller
+// wrote) take every sample, as the step size may change at one without effect.
+template <int SHADER>
+__device__ __forceinline__ bool march_state(const Px &p) {
+    if (SHADER != HY_SHADER_VOLUME) return true;
+    const float big = 3e38f;
+    return fabsf(p.vw) < big && fabsf(p.e3) < big &&
+           (!(p.vw >= HY_T85) || p.step_size == (p.vw >= HY_T93 ? 16 : 4));
+}
+
 // ray_march_kernel_impl (cuda_shading.cu:41-54): resumes every pixel that has
 // steps left (the others keep their bytes).
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER, int LOOP>
@@ -103,7 +114,10 @@ __global__ void __launch_bounds__(kThreads, pass_blocks(LOOP, GATHER))
         const size_t idx = size_t(y) * A.view.W + x;
         Px p = load_film<SHADER>(A.film, idx);
         if (p.nsteps > 0) {
-            samples = run_main<SHADER, PC, DT, PADDED, false, GATHER, LOOP>(p, A, A.view, S);
+            if (SHADER != HY_SHADER_VOLUME || LOOP == kLoopOne || march_state<SHADER>(p))
+                samples = run_main<SHADER, PC, DT, PADDED, false, GATHER, LOOP>(p, A, A.view, S);
+            else
+                samples = run_main<SHADER, PC, DT, PADDED, false, GATHER, kLoopOne>(p, A, A.view, S);
             store_film<SHADER>(A.film, idx, p);
         }
     }
