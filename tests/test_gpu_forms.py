@@ -4,8 +4,10 @@ images, floats and sample counts equal, bit for bit."""
 import numpy as np
 import pytest
 
-from tests._harness import Case, camera
-from tests.test_gpu_skip import check, voxels
+import hydrant_gb300 as hy
+from oracle import oracle as orc
+from tests._harness import Case, camera, view_array
+from tests.test_gpu_skip import check, knots, voxels
 
 pytestmark = pytest.mark.gpu
 
@@ -27,4 +29,87 @@ def test_no_free_cells(ctx, wh, dtype):
             check(c, camera(), *wh, f"{wh} {dtype} {density}", shader="Volume", sample_rate=0.5,
                   density=density)
     finally:
+        c.close()
+
+
+@pytest.mark.parametrize("bs", [64, 128])
+@pytest.mark.parametrize("wh", [(31, 27), (197, 200), (396, 395), (690, 684)])
+def test_compile_time_edges(ctx, bs, wh):
+    """Bricks of 64^3 and 128^3 voxels with an apron (compile-time edges of 66 and
+    130): every form of the Volume and Isosurface march, in one march, composited
+    and over films."""
+    torch = pytest.importorskip("torch")
+    dims = (150, 140, 133)
+    c = Case(ctx, voxels("u8", dims), bs, 1, tf=knots("ends"))
+    W, H = wh
+    try:
+        for composite in (False, True):
+            check(c, camera(a=(-50.0, 20.0, 1.9)), W, H, f"{bs} {wh} {composite}", shader="Volume",
+                  sample_rate=0.25, density=0.2, composite=composite)
+            check(c, camera(a=(-50.0, 20.0, 1.9)), W, H, f"{bs} {wh} {composite} iso",
+                  shader="Isosurface", mode="Position", sample_rate=0.25, isovalue=0.4,
+                  composite=composite)
+        for shader, mode in (("Volume", "Default"), ("Isosurface", "Position")):
+            for gather in (True, False):
+                c.vol.set_gather_sampling(gather)
+                cam = camera(a=(-50.0, 20.0, 1.9))
+                p = hy.shader_params(shader=shader, mode=mode, sample_rate=0.25, density=0.2,
+                                     isovalue=0.4)
+                if shader == "Isosurface":
+                    hy.iso_lighting(c.vol, cam, p)
+                view = hy.camera_view(c.vol, cam)
+                # the emit pass in one go, and cut short with march passes after it
+                ref = orc.render(c.ov, c.tf, orc.params_from(p), view_array(view), W, H,
+                                 want_film=True)["film"]
+                film = torch.zeros(H * W * 64, dtype=torch.uint8, device="cuda")
+                torch.cuda.synchronize()
+                hy.shade_pass(ctx, c.vol, p, hy._abi.PASS_RAY_EMIT, view, film.data_ptr(), W, H)
+                ctx.synchronize()
+                assert np.array_equal(film.cpu().numpy().reshape(H, W, 64), ref), (shader, gather)
+                p.max_steps = 60
+                part = orc.render(c.ov, c.tf, orc.params_from(p), view_array(view), W, H,
+                                  want_film=True)["film"].copy()
+                part.view(np.int32)[..., 6][part.view(np.int32)[..., 6] == 0] = 40
+                dev = torch.from_numpy(part.copy()).cuda()
+                torch.cuda.synchronize()
+                hy.shade_pass(ctx, c.vol, p, hy._abi.PASS_RAY_MARCH, None, dev.data_ptr(), W, H)
+                ctx.synchronize()
+                orc.march_film(c.ov, c.tf, orc.params_from(p), part, W, H, nthreads=8)
+                assert np.array_equal(dev.cpu().numpy(), part), (shader, gather)
+    finally:
+        c.vol.set_gather_sampling(True)
+        c.close()
+
+
+@pytest.mark.parametrize("bs", [16, 64, 128])
+@pytest.mark.parametrize("gather", [True, False])
+def test_batch_by_the_rule(ctx, bs, gather):
+    """Batches whose samples in flight the library chooses (steps_per_iter 0), below
+    and above 8 warps of rays a scheduler, with and without free cells, composited
+    too, view by view against the oracle."""
+    c = Case(ctx, voxels("u8", (150, 140, 133)), bs, 1)
+    c.vol.set_gather_sampling(gather)
+    try:
+        for name, tf in (("ends", knots("ends")), ("dense", dense_knots())):
+            ctx.set_transfer_fn(tf)
+            for sizes in (((60, 50), (33, 71)), ((410, 400), (64, 64))):
+                for composite in (False, True):
+                    p = hy.shader_params(shader="Volume", sample_rate=0.25, density=0.2,
+                                         composite=composite)
+                    views = [(hy.camera_view(c.vol, camera(a=(20.0 * i, 30.0, 2.0))), W, H)
+                             for i, (W, H) in enumerate(sizes)]
+                    b = hy.Batch(ctx, c.vol, p, views)
+                    try:
+                        assert b.config.steps_per_iter == 0
+                        b.set_counting(True)
+                        got, n, want = b.render(), ctx.stats().samples, 0
+                        for img, (view, W, H) in zip(got, views):
+                            r = orc.render(c.ov, tf, orc.params_from(p), view_array(view), W, H)
+                            want += r["samples"]
+                            assert np.array_equal(img, r["rgba"]), (name, W, H, composite)
+                        assert n == want, (name, sizes, composite)
+                    finally:
+                        b.close()
+    finally:
+        c.vol.set_gather_sampling(True)
         c.close()
