@@ -171,11 +171,13 @@ __global__ void slot_minmax_kernel(const hy::GatherItem *__restrict__ items,
     }
 }
 
-// The coarse stand-in of brick blockIdx.x: its sub-box of coarse brick cid.
+// The coarse stand-in of brick blockIdx.x (of one that is not empty): its sub-box
+// of coarse brick cid.
 template <typename T>
 __global__ void coarse_minmax_kernel(const unsigned char *__restrict__ coarse, long long stride,
-                                     const hy::RegEntry *__restrict__ reg, int gx, int gy, int sc,
-                                     int cgx, int cgy, int nc, int P, MinMax<T> *__restrict__ out) {
+                                     const hy::RegEntry *__restrict__ reg,
+                                     const int2 *__restrict__ info, int gx, int gy, int sc, int cgx,
+                                     int cgy, int nc, int P, MinMax<T> *__restrict__ out) {
     const int b = blockIdx.x;
     const int x = b % gx, y = (b / gx) % gy, z = b / (gx * gy);
     const int cid = ((z / sc) * cgy + y / sc) * cgx + x / sc;
@@ -183,7 +185,7 @@ __global__ void coarse_minmax_kernel(const unsigned char *__restrict__ coarse, l
     const hy::RegEntry e = reg[b];
     MinMax<T> *o = out + (long long)b * nc * nc * nc;
     brick_cells<T>(
-        nc, P, make_float4(e.k, e.bx, e.by, e.bz), true,
+        nc, P, make_float4(e.k, e.bx, e.by, e.bz), info[b].x == 0,
         [&](int i, int j, int k) { return v[((long long)k * P + j) * P + i]; },
         [&](int i, int j, int k, MinMax<T> m) { o[(k * nc + j) * nc + i] = m; });
 }
@@ -566,16 +568,20 @@ int hy_skip_build_paged(hy_volume *v, const hy_store *store, int nslots, int reg
         const int *cg = store->coarse_grid;
         if (e == cudaSuccess && u8)
             coarse_minmax_kernel<unsigned char><<<grid, threads, 0, ctx->stream>>>(
-                coarse, (long long)v->slot_stride, v->reg_dev, v->grid[0], v->grid[1], sc, cg[0],
-                cg[1], s.nc, v->P, static_cast<MinMax<unsigned char> *>(s.minmax));
+                coarse, (long long)v->slot_stride, v->reg_dev, v->info_dev, v->grid[0], v->grid[1], sc,
+                cg[0], cg[1], s.nc, v->P, static_cast<MinMax<unsigned char> *>(s.minmax));
         else if (e == cudaSuccess)
             coarse_minmax_kernel<float><<<grid, threads, 0, ctx->stream>>>(
-                coarse, (long long)v->slot_stride, v->reg_dev, v->grid[0], v->grid[1], sc, cg[0],
-                cg[1], s.nc, v->P, static_cast<MinMax<float> *>(s.minmax));
+                coarse, (long long)v->slot_stride, v->reg_dev, v->info_dev, v->grid[0], v->grid[1], sc,
+                cg[0], cg[1], s.nc, v->P, static_cast<MinMax<float> *>(s.minmax));
         if (e == cudaSuccess) e = cudaGetLastError();
+        int *hist = reinterpret_cast<int *>(s.grid[0]);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(hist, 0, sizeof(int) * kBins * kBins, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         cudaFree(coarse);
         if (e != cudaSuccess) return hy_cuda_fail(ctx, e, "pager: skip grid");
+        return u8 ? cell_hist<unsigned char>(v, hist) : cell_hist<float>(v, hist);
     }
     return HY_OK;
 }
@@ -662,9 +668,9 @@ int hy_skip_view(hy_ctx *ctx, const hy_volume *cv, const hy_shader_params *p, hy
         r = ctx->tf_ranges;
         // With less than a tenth of the cells free the looks cost more than
         // the samples passed over: a march without a free cell takes 3 to 5 %
-        // longer with the grid than without.
-        // (a paged cache's cells are not counted.)
-        if (!s.slots && free_cells(s, r) * 10 < s.sampled) return HY_OK;
+        // longer with the grid than without.  A paged cache's cells are
+        // counted on the coarse stand-ins (without a coarse level: not).
+        if (!s.hist.empty() && free_cells(s, r) * 10 < s.sampled) return HY_OK;
     } else if (p->shader == HY_SHADER_ISOSURFACE) {
         // crossed: value and 0 on different sides of the isovalue
         which = 1;

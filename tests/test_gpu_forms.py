@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import hydrant_gb300 as hy
+from hydrant_gb300 import _abi
 from oracle import oracle as orc
 from tests._harness import Case, camera, view_array
 from tests.test_gpu_skip import check, knots, voxels
@@ -113,3 +114,42 @@ def test_batch_by_the_rule(ctx, bs, gather):
     finally:
         c.vol.set_gather_sampling(True)
         c.close()
+
+
+@pytest.mark.parametrize("sampler", [_abi.PAGER_LOADS, _abi.PAGER_GATHERS])
+@pytest.mark.parametrize("level", [0, 2])
+def test_paged_with_few_free_cells(ctx, sampler, level):
+    """Realtime frames whose knots are transparent where hardly a cell lies (no grid
+    by the coarse stand-ins' count; without a coarse level always one), then where
+    most lie, then nowhere."""
+    torch = pytest.importorskip("torch")
+    vox = np.maximum(voxels("u8", (96, 64, 80)), 1)
+    vol, ov = hy.Volume(ctx, vox, 16, 1), orc.OracleVolume(vox, 16, 1)
+    store = hy.Store.from_volume(vol)
+    if level:
+        store.build_coarse(level)
+        ov.build_coarse(level)
+    pg = hy.Pager(ctx, store, max(4, vol.info.nonempty // 3), _abi.PAGER_REALTIME, sampler=sampler)
+    few = dense_knots()
+    few[7:, 3] = 0
+    try:
+        for f, tf in enumerate((few, knots("first"), dense_knots())):
+            cam = hy.camera_orbit((25.0 + 40.0 * f, 30.0, 1.4))
+            for W, H in ((57, 43), (317, 315), (397, 394)):
+                ctx.set_transfer_fn(tf)
+                p = hy.shader_params(shader="Volume", sample_rate=0.5, density=0.3,
+                                     count_samples=True)
+                out = torch.zeros(W * H * 4, dtype=torch.uint8, device="cuda")
+                torch.cuda.synchronize()
+                pg.render(p, cam, W, H, out.data_ptr())
+                samples = ctx.stats().samples
+                ov.set_present(pg.present())
+                op = orc.params_from(p)
+                op.lowest_blkcnt = ov.lowest_blkcnt if level else 0
+                ref = orc.render(ov, tf, op, view_array(hy.camera_view(pg.volume, cam)), W, H)
+                assert np.array_equal(out.cpu().numpy().reshape(H, W, 4), ref["rgba"]), (f, W)
+                assert samples == ref["samples"], (f, W)
+    finally:
+        pg.close()
+        store.close()
+        vol.close()
