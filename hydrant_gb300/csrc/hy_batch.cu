@@ -241,7 +241,9 @@ __global__ void __maxnreg__((lean_regs<DT, PADDED, GATHER, LOOP>()))
 
 // The lean march's samples in flight (volume_batches), where steps_per_iter
 // leaves it open: four (128 registers) for a batch of fewer than 8 warps of
-// rays a scheduler, which is bound by latency; else two at 64 registers where
+// rays a scheduler, which is bound by latency (5 by loads without free cells: three
+// views of 250x200 f32, 7.7 warps, dense knots, bricks of 16^3 151 us with four, 124
+// with one); else two at 64 registers where
 // cells are free of effect and bricks have 32 voxels and more: 16 views of
 // the 1024^3 volume 25.6 ms against 25.7 with one at 48 registers (26.5 for
 // two at 72 or 80, 29.9 for four at 96), 11 views of a 99x213x412 volume 887
@@ -255,10 +257,11 @@ const void *pick_lean(const ShadeArgs &a, int steps_per_iter, long long rays) {
             &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopErt>);
     if constexpr (PADDED) {
         if (steps_per_iter != 1 && a.vol.P <= kMaxBatchesP) {
-            if (steps_per_iter == 0 && rays < 8 * 32ll * a.schedulers)
+            if (steps_per_iter == 0 &&
+                rays < (GATHER || a.skip.d ? 8 : 5) * 32ll * a.schedulers)
                 return reinterpret_cast<const void *>(
                     &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopBatch4>);
-                        if (steps_per_iter == 2 || (steps_per_iter == 0 && a.skip.d && a.vol.P >= 34))
+            if (steps_per_iter == 2 || (steps_per_iter == 0 && a.skip.d && a.vol.P >= 34))
                 return reinterpret_cast<const void *>(
                     &batch_lean_kernel<SHADER, PC, DT, PADDED, GATHER, kLoopBatch2>);
         }

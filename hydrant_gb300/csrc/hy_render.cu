@@ -311,7 +311,9 @@ void launch_group(const ShadeArgs &a, cudaStream_t s) {
 // one; u8 by loads 118, 154, 188; 145, 172, 206; 150, 158, 169, 183; f32 135, 178,
 // 216; 161, 184, 220; 176, 197, 208, 212.  Rays that are soon opaque (density 0.3)
 // lose more where the line is too high: u8 by loads at 380^2 81 with four, 70
-// with two, 66 with one.
+// with two, 66 with one.  In bricks of fewer than 32 voxels a batch ends at a face
+// after a few steps: f32 by loads at 360x400, bricks of 16^3, 132 with two, 124
+// with one.
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
 void launch_lean(const ShadeArgs &a, cudaStream_t s) {
     const dim3 g = grid_of(a);
@@ -334,7 +336,8 @@ void launch_lean(const ShadeArgs &a, cudaStream_t s) {
             return;
         }
     }
-    const int four = a.skip.d ? 8 : 5, two = GATHER ? 24 : DT == HY_DTYPE_F32 ? 8 : 0;
+    const int four = a.skip.d ? 8 : 5,
+              two = a.vol.P < 34 ? 0 : GATHER ? 24 : DT == HY_DTYPE_F32 ? 8 : 0;
     if (rays < four * per_warp)
         render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
     else if (a.skip.d || rays < two * per_warp)
@@ -410,10 +413,12 @@ void launch_fused(const ShadeArgs &a, cudaStream_t s) {
         // 256^2 and 512^2 (3.4, 13.5 warps) 414 and 468 us with one, 350 and 415
         // with two, 337 with four at the first; 256^3 of 32^3 bricks at 256^2,
         // 512^2, 670^2 339, 366, 444 with one, 230, 297, 385 with two, 194 with
-        // four at the first.
+        // four at the first.  Two from 6 warps on: over 56 volumes and isovalues
+        // at 380^2 (7.4 warps) both take as long, but where rays hit soon (noise,
+        // 360x400) 138 with four, 123 with two or one.
         const long long rays = (long long)a.view.W * a.view.H, per_warp = 32ll * a.schedulers;
         if (rays < 24 * per_warp && a.vol.P <= kMaxBatchesP) {
-            if (rays < 8 * per_warp)
+            if (rays < 6 * per_warp)
                 render_iso_kernel<PC, DT, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
             else
                 render_iso_kernel<PC, DT, kLoopBatch2><<<g, kThreads, sm, s>>>(a);

@@ -33,6 +33,31 @@ def test_no_free_cells(ctx, wh, dtype):
         c.close()
 
 
+@pytest.mark.parametrize("wh", [(341, 342), (342, 342), (395, 396)])
+@pytest.mark.parametrize("dtype,bs", [("u8", 16), ("u8", 32), ("f32", 16), ("f32", 32)])
+def test_lines_between_the_forms(ctx, wh, dtype, bs):
+    """Isosurfaces on both sides of 6 warps of rays a scheduler (116,736 rays), and
+    dense knots in bricks below and from 32 voxels on, per view and batched."""
+    c = Case(ctx, voxels(dtype, (70, 61, 52)), bs, 1, tf=dense_knots())
+    W, H = wh
+    try:
+        check(c, camera(), W, H, f"{wh} {dtype} {bs} iso", shader="Isosurface", mode="Position",
+              sample_rate=0.5, isovalue=0.4)
+        check(c, camera(), W, H, f"{wh} {dtype} {bs}", shader="Volume", sample_rate=0.5, density=0.2)
+        p = hy.shader_params(shader="Volume", sample_rate=0.5, density=0.2)
+        view = hy.camera_view(c.vol, camera())
+        for sizes in ([(W, H)], [(W, H // 2), (W, H // 4)]):
+            b = hy.Batch(ctx, c.vol, p, [(view, w, h) for w, h in sizes])
+            try:
+                for img, (w, h) in zip(b.render(), sizes):
+                    r = orc.render(c.ov, c.tf, orc.params_from(p), view_array(view), w, h)
+                    assert np.array_equal(img, r["rgba"]), (w, h)
+            finally:
+                b.close()
+    finally:
+        c.close()
+
+
 @pytest.mark.parametrize("bs", [64, 128])
 @pytest.mark.parametrize("wh", [(31, 27), (197, 200), (396, 395), (690, 684)])
 def test_compile_time_edges(ctx, bs, wh):
