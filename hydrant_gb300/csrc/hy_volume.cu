@@ -25,55 +25,124 @@
 
 namespace {
 
-// Rows of a padded brick: a warp takes a row (its z, y and x clamped to the
-// volume, as the apron replicates the border), its lanes consecutive voxels.
-// What bounds both kernels is issue; a thread per voxel with 64-bit divisions
-// took 5.1 + 6.9 ms for 1024^3 u8 (one block per brick for the statistics:
-// 0.8 ms for a single 64^3 brick, 6.5 ms for 128^3), these 1.0 + 1.2.
+// Rows of a padded brick (z, y and x clamped to the volume, as the apron replicates
+// the border).  Long rows go to a warp each, its lanes consecutive voxels; of short
+// ones (short_rows) a block takes as many at a time as its threads hold, kRows of
+// these loaded before the first is used.  What bounds both kernels is issue, and
+// FP64 for f32 sums; a thread per voxel with 64-bit divisions took 5.1 + 4.8 ms for
+// 1024^3 u8 in bricks of 64^3 (one block per brick for the statistics: 0.8 ms for a
+// single 64^3 brick, 6.5 ms for 128^3), a warp a row 2.8 + 1.6, short rows 2.2 + 2.2.
+// 200x150x171 f32 in bricks of 16^3, us: 49 + 57 a thread per voxel, 91 + 67 a warp a
+// row, 37 + 24 short rows; of 32^3 121 + 58, 57 + 31, 40 + 29.
 struct BrickArgs {
     int dim[3];
     int bs, pad, P;
     int gx, gy;
 };
+constexpr int kThreads = 256, kRows = 4;
+template <typename T>
+__host__ __device__ constexpr bool short_rows(int P) {
+    return P <= (sizeof(T) == 1 ? 40 : 72);
+}
 
-__device__ __forceinline__ long long row_base(const BrickArgs &a, int bid, int z, int y) {
-    const int by = (bid / a.gx) % a.gy, bz = bid / (a.gx * a.gy);
-    const int Y = min(max(by * a.bs + y - a.pad, 0), a.dim[1] - 1);
-    const int Z = min(max(bz * a.bs + z - a.pad, 0), a.dim[2] - 1);
-    return ((long long)Z * a.dim[1] + Y) * a.dim[0];
+// Where a brick's padded rows lie in the volume.
+struct BrickOrigin {
+    int x, y, z;
+    __device__ __forceinline__ BrickOrigin(const BrickArgs &a, int bid) {
+        const int q = bid / a.gx, bz = q / a.gy;
+        x = (bid - q * a.gx) * a.bs - a.pad;
+        y = (q - bz * a.gy) * a.bs - a.pad;
+        z = bz * a.bs - a.pad;
+    }
+    __device__ __forceinline__ long long row(const BrickArgs &a, int pz, int py) const {
+        const int Y = min(max(y + py, 0), a.dim[1] - 1), Z = min(max(z + pz, 0), a.dim[2] - 1);
+        return ((long long)Z * a.dim[1] + Y) * a.dim[0];
+    }
+    __device__ __forceinline__ int column(const BrickArgs &a, int px) const {
+        return min(max(x + px, 0), a.dim[0] - 1);
+    }
+};
+
+// This thread's rows of the box [x0, x1) x [y0, y1) x [z0, z1) of a padded brick,
+// of which `group` of `groups` blocks takes its share: get(ok, x, y, z) for kRows of
+// them, then put(k, ok, x, y, z) for the same ones.
+template <typename Get, typename Put>
+__device__ __forceinline__ void brick_rows(int x0, int x1, int y0, int y1, int z0, int z1, int group,
+                                           int groups, Get get, Put put) {
+    const int nx = x1 - x0, ny = y1 - y0, cols = min(nx, kThreads), rows = kThreads / cols;
+    const int row = threadIdx.x / cols, col = threadIdx.x - row * cols;
+    if (row >= rows) return;
+    const int first = group * rows + row, stride = groups * rows;
+    for (int x = x0 + col; x < x1; x += cols) {
+        int z = first / ny, y = y0 + first - z * ny;
+        z += z0;
+        while (z < z1) {
+            int ky[kRows], kz[kRows];
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                ky[k] = y;
+                kz[k] = z;
+                y += stride;
+                while (y >= y1) {
+                    y -= ny;
+                    ++z;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) get(k, kz[k] < z1, x, ky[k], kz[k]);
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) put(k, kz[k] < z1, x, ky[k], kz[k]);
+        }
+    }
 }
 
 // Emptiness and the sum of the core voxels of brick blockIdx.x, rows of the
 // slices of part blockIdx.y of gridDim.y: part sums are added up on the host.
-template <typename T>
-__global__ void __launch_bounds__(256) brick_stats_kernel(const T *__restrict__ raw,
-                                                          const __grid_constant__ BrickArgs a,
-                                                          unsigned int *__restrict__ nonempty,
-                                                          double *__restrict__ core_sum) {
+template <typename T, bool SHORT>
+__global__ void __launch_bounds__(kThreads) brick_stats_kernel(const T *__restrict__ raw,
+                                                               const __grid_constant__ BrickArgs a,
+                                                               unsigned int *__restrict__ nonempty,
+                                                               double *__restrict__ core_sum) {
     const int bid = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bx = bid % a.gx, P = a.P;
+    const int P = a.P, hi = a.pad + a.bs;
     const int z0 = int((long long)P * blockIdx.y / gridDim.y),
               z1 = int((long long)P * (blockIdx.y + 1) / gridDim.y);
-    const int hi = a.pad + a.bs;
+    const BrickOrigin o(a, bid);
     bool any = false;
     double sum = 0.0;
     unsigned long long whole = 0;  // u8: exact, and no FP64 (slow on this GPU)
-    for (int r = z0 * P + warp; r < z1 * P; r += 8) {
-        const int z = r / P, y = r - z * P;
-        const T *row = raw + row_base(a, bid, z, y);
-        const bool core = z >= a.pad && z < hi && y >= a.pad && y < hi;
-        unsigned int rs = 0;  // a row's sum fits: P * 255
-        for (int x = lane; x < P; x += 32) {
-            const T v = row[min(max(bx * a.bs + x - a.pad, 0), a.dim[0] - 1)];
-            any |= v != T(0);
+    if constexpr (SHORT) {
+        T v[kRows];
+        auto load = [&](int k, bool ok, int x, int y, int z) {
+            v[k] = ok ? raw[o.row(a, z, y) + o.column(a, x)] : T(0);
+        };
+        brick_rows(0, P, 0, P, z0, z1, 0, 1, load, [&](int k, bool, int x, int y, int z) {
+            any |= v[k] != T(0);
             if constexpr (sizeof(T) == 1)
-                if (x >= a.pad && x < hi) rs += v;
-        }
-        if constexpr (sizeof(T) == 1) {
-            if (core) whole += rs;
-        } else if (core) {  // the core again (L1): full warps of FP64 additions
-            for (int x = a.pad + lane; x < hi; x += 32)
-                sum += double(row[min(bx * a.bs + x - a.pad, a.dim[0] - 1)]);
+                if (x >= a.pad && x < hi && y >= a.pad && y < hi && z >= a.pad && z < hi)
+                    whole += v[k];
+        });
+        // f32: the core again (L1), full warps of FP64 additions
+        if constexpr (sizeof(T) != 1)
+            brick_rows(a.pad, hi, a.pad, hi, max(z0, a.pad), min(z1, hi), 0, 1, load,
+                       [&](int k, bool, int, int, int) { sum += double(v[k]); });
+    } else {
+        for (int r = z0 * P + warp; r < z1 * P; r += 8) {
+            const int z = r / P, y = r - z * P;
+            const T *row = raw + o.row(a, z, y);
+            const bool core = z >= a.pad && z < hi && y >= a.pad && y < hi;
+            unsigned int rs = 0;  // a row's sum fits: P * 255
+            for (int x = lane; x < P; x += 32) {
+                const T t = row[o.column(a, x)];
+                any |= t != T(0);
+                if constexpr (sizeof(T) == 1)
+                    if (x >= a.pad && x < hi) rs += t;
+            }
+            if constexpr (sizeof(T) == 1) {
+                if (core) whole += rs;
+            } else if (core) {
+                for (int x = a.pad + lane; x < hi; x += 32) sum += double(row[o.column(a, x)]);
+            }
         }
     }
     if constexpr (sizeof(T) == 1) sum = double(whole);
@@ -89,21 +158,33 @@ __global__ void __launch_bounds__(256) brick_stats_kernel(const T *__restrict__ 
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) brick_fill_kernel(const T *__restrict__ raw,
-                                                         const __grid_constant__ BrickArgs a,
-                                                         const int *__restrict__ slot_brick,
-                                                         unsigned char *__restrict__ pool,
-                                                         long long slot_stride, int slot0) {
-    const int slot = slot0 + blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bid = slot_brick[slot], bx = bid % a.gx, P = a.P;
+template <typename T, bool SHORT>
+__global__ void __launch_bounds__(kThreads) brick_fill_kernel(const T *__restrict__ raw,
+                                                              const __grid_constant__ BrickArgs a,
+                                                              const int *__restrict__ slot_brick,
+                                                              unsigned char *__restrict__ pool,
+                                                              long long slot_stride, int slot0) {
+    const int slot = slot0 + blockIdx.y, P = a.P;
+    const BrickOrigin o(a, slot_brick[slot]);
     T *dst = reinterpret_cast<T *>(pool + (long long)slot * slot_stride);
-    for (int r = blockIdx.x * 8 + warp; r < P * P; r += gridDim.x * 8) {
-        const int z = r / P, y = r - z * P;
-        const T *row = raw + row_base(a, bid, z, y);
-        T *out = dst + (long long)r * P;
-        for (int x = lane; x < P; x += 32)
-            out[x] = row[min(max(bx * a.bs + x - a.pad, 0), a.dim[0] - 1)];
+    if constexpr (!SHORT) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int r = blockIdx.x * 8 + warp; r < P * P; r += gridDim.x * 8) {
+            const int z = r / P, y = r - z * P;
+            const T *row = raw + o.row(a, z, y);
+            T *out = dst + (long long)r * P;
+            for (int x = lane; x < P; x += 32) out[x] = row[o.column(a, x)];
+        }
+    } else {
+        T v[kRows];
+        brick_rows(
+            0, P, 0, P, 0, P, blockIdx.x, gridDim.x,
+            [&](int k, bool ok, int x, int y, int z) {
+                if (ok) v[k] = raw[o.row(a, z, y) + o.column(a, x)];
+            },
+            [&](int k, bool ok, int x, int y, int z) {
+                if (ok) dst[((long long)z * P + y) * P + x] = v[k];
+            });
     }
 }
 
@@ -365,8 +446,10 @@ int upload_impl(hy_volume *vol, const void *host) {
                        vol->grid[0], vol->grid[1]};
     HY_UP(cudaMalloc(&ne_dev, np * sizeof(unsigned int)));
     HY_UP(cudaMalloc(&sum_dev, np * sizeof(double)));
-    brick_stats_kernel<T><<<dim3(unsigned(nb), unsigned(parts)), 256, 0, ctx->stream>>>(
-        raw, ba, ne_dev, sum_dev);
+    const bool rows_short = short_rows<T>(vol->P);
+    const auto stats = rows_short ? &brick_stats_kernel<T, true> : &brick_stats_kernel<T, false>;
+    stats<<<dim3(unsigned(nb), unsigned(parts)), kThreads, 0, ctx->stream>>>(raw, ba, ne_dev,
+                                                                             sum_dev);
     HY_UP(cudaGetLastError());
     std::vector<unsigned int> ne_part(np);
     std::vector<double> sum_part(np);
@@ -405,10 +488,14 @@ int upload_impl(hy_volume *vol, const void *host) {
         HY_UP(cudaMalloc(&slot_brick_dev, slot_brick.size() * sizeof(int)));
         HY_UP(cudaMemcpyAsync(slot_brick_dev, slot_brick.data(), slot_brick.size() * sizeof(int),
                               cudaMemcpyHostToDevice, ctx->stream));
-        const unsigned gx = unsigned(std::min<long long>(((long long)vol->P * vol->P + 7) / 8, 64));
+        // rows a block takes at a time
+        const int rows = rows_short ? kRows * (kThreads / vol->P) : kThreads / 32;
+        const unsigned gx =
+            unsigned(std::min<long long>(((long long)vol->P * vol->P + rows - 1) / rows, 64));
+        const auto fill = rows_short ? &brick_fill_kernel<T, true> : &brick_fill_kernel<T, false>;
         for (int s0 = 0; s0 < vol->resident; s0 += 65535) {
             const int n = std::min(65535, vol->resident - s0);
-            brick_fill_kernel<T><<<dim3(gx, unsigned(n)), 256, 0, ctx->stream>>>(
+            fill<<<dim3(gx, unsigned(n)), kThreads, 0, ctx->stream>>>(
                 raw, ba, slot_brick_dev, vol->pool, (long long)vol->slot_stride, s0);
             HY_UP(cudaGetLastError());
         }
