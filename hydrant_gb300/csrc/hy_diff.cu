@@ -924,20 +924,21 @@ int diff_gather_refresh(hy_ctx *ctx, const float *vol, int n, DiffArgs &a, bool 
     return HY_OK;
 }
 
-// Whether the forward is worth the texture's refresh, which takes some 1.5 ps a
-// voxel while the volume stays in L2 and 3.3 ps beyond.  By loads, up to 64 k rays
-// wait about as long as one: 0.5 us a step for a few rays or a volume in L2, else
-// 1 us.  One view of 768^3 at 8^2, 32^2 and 256^2: 1430, 3200, 2920 us by loads and
+// Whether the forward is worth the texture's refresh, which takes a launch and some
+// 1.5 ps a voxel while the volume stays in L2 and 3.3 ps beyond.  By loads, up to 64 k
+// rays wait about as long as one: 0.3 us a step while the volume stays in L1, 0.5 us
+// for a few rays or a volume in L2, else 1 us.  One view of 768^3 at 8^2, 32^2 and 256^2: 1430, 3200, 2920 us by loads and
 // 1860, 1880, 2740 through the texture; a quarter of the steps, 394, 925 and (128^2)
 // 934 against 1520, 1520 and 1570; 512^3 at 8^2 968 and 664, a quarter of the
-// steps 265 and 442.  The adjoint, whose samples cost several times as much, is
-// always worth it.
+// steps 265 and 442; 33^3, 33 steps, 27 and 33; 64^3, 64 steps, 50 and 33.  The
+// adjoint, whose samples cost several times as much, is always worth it.
 bool forward_through_texture(const DiffArgs &a, long long rays) {
     const double voxels = double(a.n) * a.n * a.n;
     const bool in_l2 = voxels * 4 < 100e6;
-    const double refresh = voxels * (in_l2 ? 1.5e-6 : 3.3e-6);
+    const double refresh = 15. + voxels * (in_l2 ? 1.5e-6 : 3.3e-6);
     const double steps = std::min<double>(a.max_steps, 1.0 / a.step);
-    const double loads = steps * (in_l2 || rays < 512 ? .5 : 1.) * std::max(1., double(rays) / 65536);
+    const double step = voxels * 4 < 128e3 ? .3 : in_l2 || rays < 512 ? .5 : 1.;
+    const double loads = steps * step * std::max(1., double(rays) / 65536);
     return refresh < .75 * loads;
 }
 

@@ -88,10 +88,11 @@ print("made", made)
 @pytest.mark.parametrize("arrays", [1, 0])
 def test_differentiable_edges_in_turn(limited, arrays):
     """Volumes of several edges on one context: one texture, the largest's,
-    serves all; without one every call samples by loads (and asks again).  The
-    images are the oracle's."""
+    serves all; without one every call samples by loads (and asks again, but for
+    the 9^3 forward, which is over before a texture pays).  The images are the
+    oracle's."""
     out = _limited.run(limited, DIFF.format(arrays=arrays))
-    assert int(out.split("made")[1]) == (1 if arrays else 20)
+    assert int(out.split("made")[1]) == (1 if arrays else 17)
 
 
 FALLBACK = """
