@@ -313,6 +313,7 @@ void launch_group(const ShadeArgs &a, cudaStream_t s) {
 // lose more where the line is too high: u8 by loads at 380^2 81 with four, 70
 // with two, 66 with one.  In bricks of fewer than 32 voxels a batch ends at a face
 // after a few steps: f32 by loads at 360x400, bricks of 16^3, 132 with two, 124
+// with one; a paged pool of 32^3 bricks at 300^2 (4.6 warps) 221 with four, 200
 // with one.
 template <int SHADER, int PC, int DT, bool PADDED, int GATHER>
 void launch_lean(const ShadeArgs &a, cudaStream_t s) {
@@ -336,7 +337,7 @@ void launch_lean(const ShadeArgs &a, cudaStream_t s) {
             return;
         }
     }
-    const int four = a.skip.d ? 8 : 5,
+    const int four = a.skip.d ? 8 : GATHER ? 5 : 4,
               two = a.vol.P < 34 ? 0 : GATHER ? 24 : DT == HY_DTYPE_F32 ? 8 : 0;
     if (rays < four * per_warp)
         render_batches_kernel<SHADER, PC, DT, GATHER, kLoopBatch4><<<g, kThreads, sm, s>>>(a);
