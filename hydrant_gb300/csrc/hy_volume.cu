@@ -73,6 +73,7 @@ __device__ __forceinline__ void brick_rows(int x0, int x1, int y0, int y1, int z
     const int row = threadIdx.x / cols, col = threadIdx.x - row * cols;
     if (row >= rows) return;
     const int first = group * rows + row, stride = groups * rows;
+    const int sz = stride / ny, sy = stride - sz * ny;
     for (int x = x0 + col; x < x1; x += cols) {
         int z = first / ny, y = y0 + first - z * ny;
         z += z0;
@@ -82,8 +83,9 @@ __device__ __forceinline__ void brick_rows(int x0, int x1, int y0, int y1, int z
             for (int k = 0; k < kRows; ++k) {
                 ky[k] = y;
                 kz[k] = z;
-                y += stride;
-                while (y >= y1) {
+                y += sy;
+                z += sz;
+                if (y >= y1) {
                     y -= ny;
                     ++z;
                 }
