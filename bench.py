@@ -863,7 +863,6 @@ def main_ours(args):
     e2e = e2e_samples * ws / t_e2e / 1e9
     hbm, peak_kind = measured_peaks()
     mean_launch_s = t / args.steps  # one batch kernel per step
-    achieved = samples * BYTES_PER_SAMPLE / mean_launch_s / 1e9
     # the profiled per-sample figures hold for the Volume shader on the blob
     # volume they were captured on, not for the other workloads
     tps = ipsm = None
@@ -874,6 +873,7 @@ def main_ours(args):
         tps = profile_per_sample(int(tuned.get("block_queue", 1)), sampler=smp)
         ipsm = profile_per_sample(int(tuned.get("block_queue", 1)),
                                   "warp_instructions_per_sample", sampler=smp)
+    achieved = tps * samples / mean_launch_s / 1e9 if tps else None
     if rank == 0:
         from oracle import oracle as orc
 
@@ -936,11 +936,12 @@ def main_ours(args):
                             "host wall clock around the loop"},
             "roofline": {
                 "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                "frac": achieved / hbm, "peak_kind": peak_kind,
+                "frac": achieved / hbm if tps else None, "peak_kind": peak_kind,
                 "traffic": (tps * samples) if tps else None,
-                "note": "8 B/sample algorithmic footprint of the reference's march (samples that "
-                        "change nothing are counted and passed over unread); bound by "
-                        "instruction issue and gather latency, not HBM",
+                "footprint_gbs": samples * BYTES_PER_SAMPLE / mean_launch_s / 1e9,
+                "note": "achieved = profiled DRAM bytes of the step / its time; footprint_gbs = 8 B "
+                        "for each sample of the reference's march, also those passed over "
+                        "unread; bound by instruction issue and gather latency, not HBM",
             },
             "issue_roofline": issue_roofline(ipsm, samples, mean_launch_s, ck, local),
             "cpu_baseline": cpu,

@@ -245,8 +245,8 @@ __global__ void __maxnreg__((lean_regs<DT, PADDED, GATHER, LOOP>()))
 // views of 250x200 f32, 7.7 warps, dense knots, bricks of 16^3 151 us with four, 124
 // with one); else two at 64 registers where
 // cells are free of effect and bricks have 32 voxels and more: 16 views of
-// the 1024^3 volume 25.6 ms against 25.7 with one at 48 registers (26.5 for
-// two at 72 or 80, 29.9 for four at 96), 11 views of a 99x213x412 volume 887
+// the 1024^3 volume take as long with one at 48 registers (3 % longer with two
+// at 72 or 80, 17 % with four at 96), 11 views of a 99x213x412 volume 887
 // against 946 us; with 16^3 bricks a batch ends at a brick face after a few
 // steps and one at a time is faster (526 against 558 us), and with no free
 // cells as well (24 views of 512^3 tubes 1458 against 1643 us).

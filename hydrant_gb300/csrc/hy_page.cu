@@ -902,10 +902,11 @@ int move_bricks(hy_pager *pg, const int *bricks, const int *slots, int n, cudaSt
     for (int t = 0; t < hy::kMaxGatherTextures; ++t)
         l.surf[t] = pg->surf[t] ? pg->surf[t] : pg->surf[0];
     if (pg->gathers) {
-        fill_textures_kernel<<<dim3(n, fill_parts(ctx, n)), 256, 0, stream>>>(pg->store->host_dev, dev, l, v->P);
+        fill_textures_kernel<<<dim3(n, fill_parts(ctx, n)), 256, 0, stream>>>(pg->store->host_dev,
+                                                                              dev, l, v->P);
     } else {
-        gather_bricks_kernel<<<dim3(n, fill_parts(ctx, n)), 256, 0, stream>>>(pg->store->host_dev, dev, v->pool, pg->ncoarse,
-                                                    (long long)v->slot_stride);
+        gather_bricks_kernel<<<dim3(n, fill_parts(ctx, n)), 256, 0, stream>>>(
+            pg->store->host_dev, dev, v->pool, pg->ncoarse, (long long)v->slot_stride);
     }
     HY_CUDA(ctx, cudaGetLastError());
     int rc = hy_skip_slots(v, dev, n, l, stream);

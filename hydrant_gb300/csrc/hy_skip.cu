@@ -12,14 +12,13 @@
 // that box with three additions per step (the positions round step by step
 // as before; nothing else of the sample is computed).  Kept per octant because
 // a ray leaving a surface cares only for what lies ahead: boxes around
-// the cell on all sides made the 16-view batch 25.7 instead of 24.7 ms and
-// small images up to 25 % slower (more and shorter hops).  The grid covers
+// the cell on all sides made the 16-view batch 4 % and small images up to 25 %
+// slower (more and shorter hops).  The grid covers
 // the whole volume, so boxes span bricks; cells of empty bricks are 0,
 // because rays cross those with the reference's own brick skip.
 //
-// Cells of 8 voxels against 4: 16-view batch 25.7 and 25.9 ms, the 128^3 view
-// 103 and 95 us, the f32 view 192 and 219 us; 4 also takes eight times the
-// memory.
+// Cells of 4 voxels instead of 8: 16-view batch 1 % slower, the 128^3 view 8 %
+// faster, the f32 view 14 % slower, and eight times the memory.
 //
 // Bound: the min/max kernel by L1 (each voxel about twice per axis); the
 // distances by writing a byte per cell and octant.

@@ -365,7 +365,10 @@ int hy_pager_destroy(hy_pager *pager);
  * at most budget_bytes / slot bytes and the store's non-empty bricks; the
  * most visible bricks are returned too.  The reference derives its cache
  * from mem_limit_mb alone (rt_block_paging.cc:230-236); this sizes it to
- * the path, within the same kind of limit. */
+ * the path, within the same kind of limit.  The budget is the slots' alone: a
+ * pager also holds the coarse level, the page table and, where there is room
+ * when it is created, cells and distances for its march (14 to 28 bytes a cell
+ * of 8^3 voxels of the whole volume: 1 GB at 4096x4096x2048). */
 int hy_pager_tune_slots(hy_ctx *ctx, const hy_store *store, const hy_camera *cams, int32_t ncams,
                         int64_t budget_bytes, int32_t *slots, int32_t *visible_max);
 /* The paged volume (for hy_cull / hy_render); owned by the pager. */
