@@ -33,6 +33,16 @@ int hy_stage(hy_ctx *ctx, size_t bytes, void **out) {
     return HY_OK;
 }
 
+bool hy_room_for(size_t bytes) {
+    if (bytes < (size_t(16) << 20)) return true;
+    size_t free_b = 0, total = 0;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return free_b >= bytes && free_b - bytes >= total / 50;
+}
+
 extern "C" int hy_ctx_create(int device, hy_ctx **out) {
     if (!out) return HY_ERR_INVALID;
     *out = nullptr;

@@ -907,7 +907,8 @@ int diff_gather_refresh(hy_ctx *ctx, const float *vol, int n, DiffArgs &a, bool 
             free_diff_gather(g);
             ctx->diff_gather = nullptr;
         }
-        g = make_diff_gather(slice_columns(P, gper) * P, (gper + 1) * P);
+        const int w = slice_columns(P, gper) * P, h = (gper + 1) * P;
+        g = hy_room_for(size_t(w) * h * sizeof(float)) ? make_diff_gather(w, h) : nullptr;
         if (!g) return HY_OK;
         ctx->diff_gather = g;
     }

@@ -338,6 +338,11 @@ uint8_t *hy_mapped_device_ptr(void *host, uintptr_t align);
         if (e_ != cudaSuccess) return hy_cuda_fail(ctx, e_, #call); \
     } while (0)
 
+// Whether `bytes` of device memory that a call can do without (skip grids, the
+// differentiable passes' texture) leave a fiftieth of the device for what it
+// cannot: staging, films, the caller's own.  Small amounts are not asked for.
+bool hy_room_for(size_t bytes);
+
 // staging buffer (hy_api.cc)
 int hy_stage(hy_ctx *ctx, size_t bytes, void **out);
 

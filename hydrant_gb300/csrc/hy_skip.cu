@@ -494,6 +494,7 @@ cudaError_t alloc_planes(hy_skip &s, bool iso, size_t minmax) {
     const size_t n = size_t(s.cells), hist = sizeof(int) * kBins * kBins,
                  grids = (std::max(n * (iso ? 16 : 8), hist) + 255) / 256 * 256,
                  planes = (size_t(bit_grid(s).words) * 33 * sizeof(unsigned int) + 255) / 256 * 256;
+    if (!hy_room_for(grids + planes + minmax)) return cudaErrorMemoryAllocation;
     const cudaError_t e = cudaMalloc(&s.grid[0], grids + planes + minmax);
     if (e != cudaSuccess) return e;
     s.grid[1] = iso ? s.grid[0] + 8 * n : nullptr;
@@ -547,7 +548,9 @@ int hy_skip_build_paged(hy_volume *v, const hy_store *store, int nslots, int reg
     const size_t per = size_t(s.nc) * s.nc * s.nc * mm_bytes(v);
     unsigned char *coarse = nullptr;  // the coarse level, for its cells alone
     s.reg_base = reg_base;
-    cudaError_t e = cudaMalloc(&s.slots, size_t(nslots) * per);
+    const size_t cells = size_t(nslots) * per + (reg_base > 0 ? size_t(v->nbricks) * per : 0);
+    cudaError_t e = hy_room_for(cells) ? cudaMalloc(&s.slots, size_t(nslots) * per)
+                                       : cudaErrorMemoryAllocation;
     if (e == cudaSuccess) e = alloc_planes(s, !v->paged_gather, 0);
     if (e == cudaSuccess && reg_base > 0) {
         e = cudaMalloc(&s.minmax, size_t(v->nbricks) * per);

@@ -426,8 +426,8 @@ int hy_pager_render_host(hy_pager *pager, const hy_shader_params *params, const 
  * caller-zeroed gradient buffers.  All pointers are device pointers; views is
  * a host array; both calls are asynchronous on the context's stream.  They
  * sample through a texture that the context keeps until it is destroyed, as large
- * as the largest volume it has rendered (some 4 n^3 bytes); without room for it,
- * and on a stream that is capturing, by loads. */
+ * as the largest volume it has rendered (some 4 n^3 bytes); where that would leave
+ * less than a fiftieth of the device, and on a stream that is capturing, by loads. */
 typedef struct hy_diff_params {
     int32_t n;            /* volume edge (voxels); bbox = [0,1]^3 */
     float sample_rate;    /* step = (1/n) / 4 / sample_rate */

@@ -70,6 +70,16 @@ cudaError_t __wrap_cudaFreeArray(cudaArray_t a) {
     give(a);
     return __real_cudaFreeArray(a);
 }
+cudaError_t __real_cudaMemGetInfo(size_t *, size_t *);
+cudaError_t __wrap_cudaMemGetInfo(size_t *f, size_t *t) {
+    cudaError_t e = __real_cudaMemGetInfo(f, t);
+    std::lock_guard<std::mutex> l(mu);
+    if (e == cudaSuccess && limit < *t) {
+        *t = limit;
+        *f = limit > live ? limit - live : 0;
+    }
+    return e;
+}
 void test_memory_limit(size_t n) { limit = n; most = live; }
 size_t test_memory_live(void) { return live; }
 size_t test_memory_most(void) { return most; }
@@ -96,7 +106,7 @@ def build(folder: Path) -> Path:
         pytest.skip("the library's object files are not here")
     src, lib = folder / "wrap.cc", folder / "liblimited.so"
     src.write_text(WRAP)
-    names = ("cudaMalloc", "cudaFree", "cudaMallocArray", "cudaFreeArray")
+    names = ("cudaMalloc", "cudaFree", "cudaMallocArray", "cudaFreeArray", "cudaMemGetInfo")
     cmd = [hb.nvcc(), *hb.ARCH, "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-o", str(lib),
            str(src), *map(str, objs), *(f"-Xlinker=--wrap={n}" for n in names), "-lpthread"]
     r = subprocess.run(cmd, capture_output=True, text=True)

@@ -138,3 +138,38 @@ def test_few_rays_over_a_large_volume(limited):
     """A forward that takes fewer samples than the texture's refresh is worth
     goes by loads and makes none."""
     assert "ok" in _limited.run(limited, FEW_RAYS)
+
+
+ROOM = """
+import numpy as np
+import hydrant_gb300 as hy
+ctx = hy.Context(0)
+k = np.random.default_rng(1).random((9, 4)).astype(np.float32); k[:3, 3] = 0
+ctx.set_transfer_fn(k)
+vox = np.ones((768, 768, 768), np.uint8)
+vox[300:420, 300:420, 300:420] = hy.synth_blobs_u8(3, (120, 120, 120), 9)
+p = hy.shader_params(shader="Volume", sample_rate=0.5, density=0.3)
+def volume(limit):
+    start = mem.test_memory_live()
+    mem.test_memory_limit(start + limit)
+    v = hy.Volume(ctx, vox, 64, 1)
+    used = mem.test_memory_live() - start
+    img = hy.render(ctx, v, p, hy.camera_view(v, hy.camera_orbit((25.0, 65.0, 2.2))), 300, 200).rgba
+    v.close()
+    mem.test_memory_limit((1 << 64) - 1)
+    return used, img
+full, want = volume(1 << 40)
+distances = 96 ** 3 * 16
+# 1 GB of bricks and textures, 20 MB of grid: with 8 MB more, less than a fiftieth is left
+less, img = volume(full + (8 << 20))
+assert less < full - distances and np.array_equal(img, want), (less, full)
+some, img = volume(full + (64 << 20))
+assert some == full and np.array_equal(img, want), (some, full)
+print("ok")
+"""
+
+
+def test_the_grid_leaves_room(limited):
+    """A grid of 20 MB is not taken where it would leave less than a fiftieth of the
+    device: the staging buffer of the render after it still fits."""
+    assert "ok" in _limited.run(limited, ROOM)
